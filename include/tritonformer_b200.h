@@ -137,6 +137,17 @@ int tfb_cross_entropy_bwd(const void* logits, const int64_t* labels, const float
                           int64_t rows, int64_t vocab, int64_t logits_ld, int64_t dlogits_ld,
                           int dtype, void* stream);
 
+/* The loss of a causal language model over (batch, seq) positions (transformer.py:330-344 of the reference, which
+ * copies logits[:, :-1] and labels[:, 1:] first): position t of a sequence is scored against labels[b, t + 1], the last
+ * one against nothing, and *loss is the fp32 mean over the batch * (seq - 1) scored positions.  row_loss and lse hold
+ * batch * seq floats (row_loss is scratch).  A label outside [0, vocab) contributes zero loss and zero gradient.
+ * bwd: dlogits = (softmax - onehot) * *grad / (batch * (seq - 1)), grad one fp32 value on the device.          */
+int tfb_lm_loss_fwd(const void* logits, const int64_t* labels, float* loss, float* row_loss, float* lse,
+                    int64_t batch, int64_t seq, int64_t vocab, int64_t logits_ld, int dtype, void* stream);
+int tfb_lm_loss_bwd(const void* logits, const int64_t* labels, const float* lse, const float* grad, void* dlogits,
+                    int64_t batch, int64_t seq, int64_t vocab, int64_t logits_ld, int64_t dlogits_ld, int dtype,
+                    void* stream);
+
 /* ---------------------------------------------------------- ReLU grad / bias grad
  * Replaces mask_grad (tritonformer/kernels/activation.py:7-44) without mutating the
  * incoming gradient: dz = act > 0 ? dy : 0 for n contiguous elements.          */

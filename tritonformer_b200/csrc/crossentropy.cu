@@ -21,10 +21,17 @@ __device__ __forceinline__ void online_merge(float& m, float& s, float m2, float
   s = a + b;
 }
 
+// Label of a row: labels[row], or with shift_seq > 0 (rows = sequences of that length) the label of the next position
+// of the same sequence; the last position of a sequence has none.
+__device__ __forceinline__ int64_t label_of(const int64_t* __restrict__ labels, int64_t row, int64_t shift_seq) {
+  if (shift_seq == 0) return labels[row];
+  return (row + 1) % shift_seq == 0 ? -1 : labels[row + 1];
+}
+
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(CE_THREADS) ce_fwd_kernel(
     const T* __restrict__ logits, const int64_t* __restrict__ labels, T* __restrict__ loss,
-    float* __restrict__ loss_f32, float* __restrict__ lse, int vocab, int64_t ld) {
+    float* __restrict__ loss_f32, float* __restrict__ lse, int vocab, int64_t ld, int64_t shift_seq) {
   grid_dependency_wait();
   allow_dependents();
   __shared__ float sm_m[CE_THREADS / 32], sm_s[CE_THREADS / 32];
@@ -74,10 +81,10 @@ __global__ void __launch_bounds__(CE_THREADS) ce_fwd_kernel(
     for (int w = 1; w < CE_THREADS / 32; ++w) online_merge(m, s, sm_m[w], sm_s[w]);
     const float l = (m + log2f(s)) * kLn2;
     lse[row] = l;
-    const int64_t lab = labels[row];
+    const int64_t lab = label_of(labels, row, shift_seq);
     float v = 0.f;
     if (lab >= 0 && lab < vocab) v = l - Num<T>::to_f(xr[lab]);
-    loss[row] = Num<T>::from_f(v);
+    if (loss) loss[row] = Num<T>::from_f(v);
     if (loss_f32) loss_f32[row] = v;
   }
 }
@@ -85,17 +92,18 @@ __global__ void __launch_bounds__(CE_THREADS) ce_fwd_kernel(
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(CE_THREADS) ce_bwd_kernel(
     const T* __restrict__ logits, const int64_t* __restrict__ labels, const float* __restrict__ lse,
-    const T* __restrict__ grad, int64_t grad_stride, T* __restrict__ dlogits, int vocab, int64_t ld,
-    int64_t dld) {
+    const T* __restrict__ grad, int64_t grad_stride, const float* __restrict__ grad_all, float grad_scale,
+    T* __restrict__ dlogits, int vocab, int64_t ld, int64_t dld, int64_t shift_seq) {
   grid_dependency_wait();
   allow_dependents();
   const int64_t row = blockIdx.x;
   const T* xr = logits + row * ld;
   T* dr = dlogits + row * dld;
-  const int64_t lab64 = labels[row];
+  const int64_t lab64 = label_of(labels, row, shift_seq);
   const bool valid = lab64 >= 0 && lab64 < vocab;
   const int lab = valid ? (int)lab64 : -1;
-  const float g = valid ? Num<T>::to_f(grad[row * grad_stride]) : 0.f;
+  // one fp32 gradient for every row (of their mean), or the rows' own
+  const float g = !valid ? 0.f : grad_all ? *grad_all * grad_scale : Num<T>::to_f(grad[row * grad_stride]);
   const float l2 = lse[row] * kLog2e;
   if (VEC) {
     const int nvec = vocab >> 3;
@@ -123,6 +131,44 @@ __global__ void __launch_bounds__(CE_THREADS) ce_bwd_kernel(
   }
 }
 
+// out[0] = sum of n row losses / count, in a fixed order.
+constexpr int CE_SUM_THREADS = 1024;
+__global__ void __launch_bounds__(CE_SUM_THREADS) ce_mean_kernel(const float* __restrict__ loss, float* __restrict__ out,
+                                                                 int64_t n, float count) {
+  grid_dependency_wait();
+  allow_dependents();
+  __shared__ float part[CE_SUM_THREADS / 32];
+  float s = 0.f;
+  for (int64_t i = threadIdx.x; i < n; i += CE_SUM_THREADS) s += loss[i];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = warp_sum(part[threadIdx.x]);
+    if (threadIdx.x == 0) *out = s / count;
+  }
+}
+
+template <typename T>
+static int launch_ce_fwd(const void* logits, const int64_t* labels, void* loss, float* loss_f32, float* lse, int64_t rows,
+                         int64_t vocab, int64_t ld, int64_t shift_seq, cudaStream_t st) {
+  const bool vec = vocab % 8 == 0 && ld % 8 == 0 && aligned16(logits);
+  launch_overlapped(vec ? ce_fwd_kernel<T, true> : ce_fwd_kernel<T, false>, dim3((unsigned)rows), dim3(CE_THREADS), 0, st,
+                    (const T*)logits, labels, (T*)loss, loss_f32, lse, (int)vocab, ld, shift_seq);
+  return launched("cross_entropy_fwd");
+}
+
+template <typename T>
+static int launch_ce_bwd(const void* logits, const int64_t* labels, const float* lse, const void* grad, int64_t grad_stride,
+                         const float* grad_all, float grad_scale, void* dlogits, int64_t rows, int64_t vocab, int64_t ld,
+                         int64_t dld, int64_t shift_seq, cudaStream_t st) {
+  const bool vec = vocab % 8 == 0 && ld % 8 == 0 && dld % 8 == 0 && aligned16(logits) && aligned16(dlogits);
+  launch_overlapped(vec ? ce_bwd_kernel<T, true> : ce_bwd_kernel<T, false>, dim3((unsigned)rows), dim3(CE_THREADS), 0, st,
+                    (const T*)logits, labels, lse, (const T*)grad, grad_stride, grad_all, grad_scale, (T*)dlogits, (int)vocab,
+                    ld, dld, shift_seq);
+  return launched("cross_entropy_bwd");
+}
+
 }  // namespace tfb
 
 using namespace tfb;
@@ -134,14 +180,7 @@ extern "C" int tfb_cross_entropy_fwd(const void* logits, const int64_t* labels, 
   TFB_REQUIRE(logits_ld >= vocab, "cross_entropy_fwd: row stride smaller than vocab");
   if (rows == 0) return TFB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const bool vec = vocab % 8 == 0 && logits_ld % 8 == 0 && aligned16(logits);
-  TFB_DISPATCH_16(dtype, T, {
-    if (vec)
-      launch_overlapped(ce_fwd_kernel<T, true>, dim3((unsigned)rows), dim3(CE_THREADS), 0, st, (const T*)logits, labels, (T*)loss, loss_f32, lse, (int)vocab, logits_ld);
-    else
-      launch_overlapped(ce_fwd_kernel<T, false>, dim3((unsigned)rows), dim3(CE_THREADS), 0, st, (const T*)logits, labels, (T*)loss, loss_f32, lse, (int)vocab, logits_ld);
-  })
-  return launched("cross_entropy_fwd");
+  TFB_DISPATCH_16(dtype, T, { return launch_ce_fwd<T>(logits, labels, loss, loss_f32, lse, rows, vocab, logits_ld, 0, st); })
 }
 
 extern "C" int tfb_cross_entropy_bwd(const void* logits, const int64_t* labels, const float* lse,
@@ -152,15 +191,36 @@ extern "C" int tfb_cross_entropy_bwd(const void* logits, const int64_t* labels, 
   TFB_REQUIRE(logits_ld >= vocab && dlogits_ld >= vocab, "cross_entropy_bwd: row stride smaller than vocab");
   if (rows == 0) return TFB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const bool vec = vocab % 8 == 0 && logits_ld % 8 == 0 && dlogits_ld % 8 == 0 && aligned16(logits) &&
-                   aligned16(dlogits);
   TFB_DISPATCH_16(dtype, T, {
-    if (vec)
-      launch_overlapped(ce_bwd_kernel<T, true>, dim3((unsigned)rows), dim3(CE_THREADS), 0, st, (const T*)logits, labels, lse, (const T*)grad, grad_stride, (T*)dlogits, (int)vocab,
-          logits_ld, dlogits_ld);
-    else
-      launch_overlapped(ce_bwd_kernel<T, false>, dim3((unsigned)rows), dim3(CE_THREADS), 0, st, (const T*)logits, labels, lse, (const T*)grad, grad_stride, (T*)dlogits, (int)vocab,
-          logits_ld, dlogits_ld);
+    return launch_ce_bwd<T>(logits, labels, lse, grad, grad_stride, nullptr, 1.f, dlogits, rows, vocab, logits_ld, dlogits_ld, 0,
+                            st);
   })
-  return launched("cross_entropy_bwd");
+}
+
+extern "C" int tfb_lm_loss_fwd(const void* logits, const int64_t* labels, float* loss, float* row_loss, float* lse,
+                               int64_t batch, int64_t seq, int64_t vocab, int64_t logits_ld, int dtype, void* stream) {
+  TFB_REQUIRE(batch >= 0 && seq > 0 && vocab > 0 && vocab < (1LL << 31) - 8, "lm_loss_fwd: bad shape");
+  TFB_REQUIRE(logits_ld >= vocab, "lm_loss_fwd: row stride smaller than vocab");
+  cudaStream_t st = (cudaStream_t)stream;
+  const int64_t rows = batch * seq;
+  if (rows > 0) {
+    int rc = TFB_OK;
+    TFB_DISPATCH_16(dtype, T, { rc = launch_ce_fwd<T>(logits, labels, nullptr, row_loss, lse, rows, vocab, logits_ld, seq, st); })
+    if (rc) return rc;
+  }
+  launch_overlapped(ce_mean_kernel, dim3(1), dim3(CE_SUM_THREADS), 0, st, (const float*)row_loss, loss, rows,
+                    (float)(batch * (seq - 1)));
+  return launched("lm_loss_fwd");
+}
+
+extern "C" int tfb_lm_loss_bwd(const void* logits, const int64_t* labels, const float* lse, const float* grad, void* dlogits,
+                               int64_t batch, int64_t seq, int64_t vocab, int64_t logits_ld, int64_t dlogits_ld, int dtype,
+                               void* stream) {
+  TFB_REQUIRE(batch >= 0 && seq > 0 && vocab > 0 && vocab < (1LL << 31) - 8, "lm_loss_bwd: bad shape");
+  TFB_REQUIRE(logits_ld >= vocab && dlogits_ld >= vocab, "lm_loss_bwd: row stride smaller than vocab");
+  if (batch == 0) return TFB_OK;
+  TFB_DISPATCH_16(dtype, T, {
+    return launch_ce_bwd<T>(logits, labels, lse, nullptr, 0, grad, 1.f / (float)(batch * (seq - 1)), dlogits, batch * seq, vocab,
+                            logits_ld, dlogits_ld, seq, (cudaStream_t)stream);
+  })
 }

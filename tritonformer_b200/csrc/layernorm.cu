@@ -415,19 +415,17 @@ __global__ void __launch_bounds__(256, 2) ln_bwd_split_kernel(
     slot = (slot + 1) % LN_DEPTH;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (has) {
+  // the row groups add their sums one after the other: a fixed order, so the result does not depend on timing
+  for (int g = 0; g < RG; ++g) {
+    if (has && rg == g) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (RG > 1) {
-        atomicAdd(&fold[c * 8 + j], acc_a[j]);
-        atomicAdd(&fold[d + c * 8 + j], acc_b[j]);
-      } else {
-        fold[c * 8 + j] = acc_a[j];
-        fold[d + c * 8 + j] = acc_b[j];
+      for (int j = 0; j < 8; ++j) {
+        fold[c * 8 + j] += acc_a[j];
+        fold[d + c * 8 + j] += acc_b[j];
       }
     }
+    __syncthreads();
   }
-  __syncthreads();
   float* pa = partials + (int64_t)blockIdx.x * 2 * d;
   for (int i = threadIdx.x; i < 2 * d; i += blockDim.x) pa[i] = fold[i];
 }

@@ -7,9 +7,7 @@ position-table gradients in one pass over the incoming gradient, without a sort.
 import torch
 from torch.autograd import Function
 
-from . import _lib
-from . import linear as _linear
-from ._amp import amp_backward, amp_forward
+from . import _host, _lib
 
 
 def embedding_forward(input_ids, tok, pos=None):
@@ -54,35 +52,9 @@ def embedding_backward(input_ids, dout, dtok, dpos=None, vocab=None):
         dpos.shape[0] if dpos is not None else 0, _lib.dtype_code(ref.dtype), _lib.stream_ptr(ref.device)))
 
 
-def _grad_target(p):
-    """(buffer to add into, whether it is p.grad itself)."""
-    if _linear.accumulating() and p.grad is not None and p.grad.is_contiguous() \
-            and p.grad.dtype == p.dtype and p.grad.shape == p.shape:
-        return p.grad, True
-    return torch.zeros_like(p, memory_format=torch.contiguous_format), False
-
-
 class Embedding(Function):
-    """out[b, t] = tok[input_ids[b, t]] (+ pos[t]).  `pos` may be None.
+    """out[b, t] = tok[input_ids[b, t]] (+ pos[t]): apply(input_ids, tok, pos).  `pos` may be None.
 
     Under autocast the tables are cast to the region's 16-bit type like the inputs of the other Functions, so
     a model kept in fp32 works; the table gradients come back in the tables' own dtype."""
-
-    @staticmethod
-    @amp_forward
-    def forward(ctx, input_ids, tok, pos):
-        ctx.save_for_backward(input_ids, tok, pos)
-        return embedding_forward(input_ids, tok, pos)
-
-    @staticmethod
-    @amp_backward
-    def backward(ctx, grad_output):
-        input_ids, tok, pos = ctx.saved_tensors
-        dtok, tok_in_place = (None, True)  # a frozen table gets no gradient buffer at all
-        if ctx.needs_input_grad[1]:
-            dtok, tok_in_place = _grad_target(tok)
-        dpos, pos_in_place = (None, True)
-        if pos is not None and ctx.needs_input_grad[2]:
-            dpos, pos_in_place = _grad_target(pos)
-        embedding_backward(input_ids, grad_output, dtok, dpos, vocab=tok.shape[0])
-        return None, None if tok_in_place else dtok, None if pos_in_place else dpos
+    apply = staticmethod(_host.embedding)

@@ -2,8 +2,7 @@
 import torch
 from torch.autograd import Function
 
-from . import _lib
-from ._amp import amp_backward, amp_forward
+from . import _host, _lib
 
 
 def _rows(t: torch.Tensor) -> torch.Tensor:
@@ -61,18 +60,5 @@ def layernorm_backward(dy, x, alpha, stats, dres=None, into=None, overwrite=Fals
 
 
 class LayerNorm(Function):
-    """y = alpha * (x - mean) / sqrt(var + eps) + beta over the last dimension."""
-
-    @staticmethod
-    @amp_forward
-    def forward(ctx, input, alpha, beta, eps):
-        y, stats = layernorm_forward(input, alpha, beta, eps)
-        ctx.save_for_backward(input, alpha, stats)
-        return y
-
-    @staticmethod
-    @amp_backward
-    def backward(ctx, grad_output):
-        x, alpha, stats = ctx.saved_tensors
-        dx, dalpha, dbeta = layernorm_backward(grad_output.to(x.dtype), x, alpha, stats)
-        return dx, dalpha.view(alpha.shape), dbeta.view(alpha.shape), None
+    """y = alpha * (x - mean) / sqrt(var + eps) + beta over the last dimension: apply(input, alpha, beta, eps)."""
+    apply = staticmethod(_host.layernorm)

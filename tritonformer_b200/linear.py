@@ -1,12 +1,15 @@
 """Linear autograd Functions (drop-in for tritonformer/linear.py:10-102).
 
+`.apply` runs the native host path (csrc/host): checks, allocation, launches and the autograd node in one call.  The
+Python bodies below are the same operators spelled out; they run while the benchmark records or times GEMM calls
+(PROFILE, TIMING).
+
 Weights are stored (in_features, out_features) and applied as x @ W.  Every product -- forward,
 input gradient and weight gradient -- is one call of the same GEMM entry point with different
 operand strides; the weight gradient contracts over all B*T rows at once in fp32 instead of
 producing per-batch partials and summing them.  Bias and ReLU are applied in the GEMM epilogue.
 The incoming gradient is never modified (the reference masks it in place).
 """
-import collections
 import os
 import contextlib
 import ctypes
@@ -14,7 +17,7 @@ import ctypes
 import torch
 from torch.autograd import Function
 
-from . import _lib
+from . import _host, _lib
 from ._amp import amp_backward, amp_forward
 
 
@@ -98,45 +101,44 @@ def accumulate_into_grad(enabled: bool = True, overwrite: bool = False, written=
         yield
         return
     previous = (_overwrite, _written, DEFER_WEIGHT_GRAD_JOIN)
+    _collect_written()
     _accumulate_depth += 1
     _overwrite, _written = bool(overwrite), (written if overwrite else None)
     DEFER_WEIGHT_GRAD_JOIN = bool(defer_weight_grads)
+    _tell_host()
     try:
         yield
     finally:
+        _collect_written()
         _accumulate_depth -= 1
         _overwrite, _written, DEFER_WEIGHT_GRAD_JOIN = previous
+        _tell_host()
         join_weight_grads()
 
 
-# GEMM scratch, newest last; at most _MAX_WORKSPACES are kept per process.  An entry that falls out is
-# returned to the caching allocator, which hands it out again only in the order of the stream it was
-# allocated on, so kernels still in flight on that stream keep their scratch.
-_workspaces = collections.OrderedDict()
-_MAX_WORKSPACES = 8
+def _tell_host():
+    """The native host path delivers gradients the way the block in force says."""
+    _host.set_grad_mode(_accumulate_depth > 0, _overwrite, DEFER_WEIGHT_GRAD_JOIN, FORK_WEIGHT_GRAD)
+
+
+def _collect_written():
+    """Moves the buffers the native host path overwrote into the set of the block in force."""
+    pointers = _host.take_written()
+    if _written is not None:
+        _written.update(pointers)
 
 
 def _gemm_workspace(device, stream):
     """Scratch the GEMM uses to share the contraction of a tile between SMs: arrival counters (kept zero by
-    the kernels, so cleared only here) and one fp32 partial tile per SM.  One per device and stream, since calls
+    the kernels, so cleared only once) and one fp32 partial tile per SM.  One per device and stream, since calls
     that share it must be stream-ordered."""
-    key = (device, stream)
-    ws = _workspaces.get(key)
-    if ws is None:
-        ws = torch.zeros(int(_lib.lib.tfb_gemm_workspace_bytes()), device=device, dtype=torch.uint8)
-        _workspaces[key] = ws
-        while len(_workspaces) > _MAX_WORKSPACES:
-            _workspaces.popitem(last=False)
-    else:
-        _workspaces.move_to_end(key)
-    return ws
+    return _host.gemm_workspace(device.index if device.index is not None else torch.cuda.current_device(), stream)
 
 
 def reset_workspaces():
     """Zeroes every cached GEMM workspace.  For use after the device status word was cleared: a split product
     that gave up can leave arrival counters non-zero."""
-    for ws in _workspaces.values():
-        ws.zero_()
+    _host.reset_workspaces()
 
 
 def gemm(a, a_sm, a_sk, b, b_sk, b_sn, m, n, k, bias=None, relu=False, out=None, accumulate=False,
@@ -244,12 +246,14 @@ def weight_grad(x, dy, w):
 # blocks of `transformer.py` are such a graph (the residual sums happen inside kernels, into fresh tensors).
 FORK_WEIGHT_GRAD = os.environ.get("TFB_FORK_DW", "1") != "0"
 DEFER_WEIGHT_GRAD_JOIN = False  # set by the accumulate_into_grad block in force
+_tell_host()
 _side_streams = {}
 _unjoined = {}  # (device index, compute stream handle) -> (compute stream, side stream) with work not yet joined
 
 
 def join_weight_grads():
     """Makes every compute stream wait for the weight-gradient products that still run on its side stream."""
+    _host.join_weight_grads()
     for main, side in list(_unjoined.values()):
         main.wait_stream(side)
     _unjoined.clear()
@@ -348,8 +352,17 @@ def _backward(ctx, grad_output, has_bias, has_relu):
     return dx, dw, db
 
 
+def instrumented():
+    """Whether GEMM calls are being recorded or timed (then the Python bodies run)."""
+    return PROFILE is not None or TIMING is not None
+
+
 class LinearNoBias(Function):
     """y = x @ W"""
+
+    @classmethod
+    def apply(cls, input, weight):
+        return super().apply(input, weight) if instrumented() else _host.linear(input, weight, None, False)
 
     @staticmethod
     @amp_forward
@@ -366,6 +379,10 @@ class LinearNoBias(Function):
 class LinearBias(Function):
     """y = x @ W + b"""
 
+    @classmethod
+    def apply(cls, input, weight, bias):
+        return super().apply(input, weight, bias) if instrumented() else _host.linear(input, weight, bias, False)
+
     @staticmethod
     @amp_forward
     def forward(ctx, input, weight, bias):
@@ -380,6 +397,10 @@ class LinearBias(Function):
 
 class LinearNoBiasReLU(Function):
     """y = relu(x @ W)"""
+
+    @classmethod
+    def apply(cls, input, weight):
+        return super().apply(input, weight) if instrumented() else _host.linear(input, weight, None, True)
 
     @staticmethod
     @amp_forward
@@ -396,6 +417,10 @@ class LinearNoBiasReLU(Function):
 
 class LinearBiasReLU(Function):
     """y = relu(x @ W + b)"""
+
+    @classmethod
+    def apply(cls, input, weight, bias):
+        return super().apply(input, weight, bias) if instrumented() else _host.linear(input, weight, bias, True)
 
     @staticmethod
     @amp_forward

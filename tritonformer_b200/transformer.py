@@ -7,9 +7,9 @@ dense_4h_to_h}}`, `final_layernorm`, `logits_out`, buffer `attn_bias`), same ini
 rule, pre-LN blocks, ReLU MLP, learned positions unless ALiBi is on, untied LM head.
 
 Two deliberate differences, both invisible in the results:
-  * the shifted loss is computed on the (B*T, V) logits in place -- the last position of each
-    sequence carries an out-of-range label, which the cross-entropy kernel skips -- instead of
-    copying logits[:, :-1] first (reference transformer.py:333-334);
+  * the shifted loss is computed on the (B*T, V) logits in place -- the cross-entropy kernel reads the
+    label of the next position and skips the last position of each sequence -- instead of copying
+    logits[:, :-1] first (reference transformer.py:333-334);
   * the mean over the B*(T-1) per-token losses is taken in fp32.
 """
 import math
@@ -19,15 +19,19 @@ from typing import List, Optional, Tuple
 import torch
 import torch.nn as nn
 
-from . import fast_causal_attention, fast_causal_attention_with_bias
+from . import _host, fast_causal_attention, fast_causal_attention_with_bias
+from . import attention as _attention
+from . import fused as _fused
+from . import linear as _linear
 from . import nn as tnn
-from .crossentropy import CrossEntropyLossFP32
+from .crossentropy import lm_loss
 from .embedding import Embedding
 from .fused import LayerNormFork, LinearResidual, MLPResidual, QKVProjection
 
-# The layer runs on fused Functions (residual adds, ReLU mask and the q/k/v input gradients folded into
-# kernel epilogues).  Set to False to run the layer module by module through the plain Functions,
-# exactly as the reference composes it; results agree to rounding.
+# The layer runs as one native autograd node (csrc/host/layer.cpp: residual adds, ReLU mask and the q/k/v input gradients
+# folded into kernel epilogues), or on the same fused Functions in Python while GEMM or attention calls are being
+# recorded or timed.  Set to False to run the layer module by module through the plain Functions, exactly as the
+# reference composes it; results agree to rounding.
 USE_FUSED_BLOCKS = True
 
 
@@ -150,6 +154,9 @@ class TransformerLayer(nn.Module):
         if not USE_FUSED_BLOCKS or not hidden_states.is_cuda:
             hidden_states = hidden_states + self.attention(self.input_layernorm(hidden_states), attn_bias)
             return hidden_states + self.mlp(self.post_attention_layernorm(hidden_states))
+        if not (_linear.instrumented() or _attention.TIMING is not None
+                or _fused.CAPTURE_ACTIVATION_PATTERN is not None):
+            return self._native(hidden_states, attn_bias)
         att, mlp = self.attention, self.mlp
         ln1, ln2 = self.input_layernorm, self.post_attention_layernorm
         normed, residual = LayerNormFork.apply(hidden_states, ln1.weight, ln1.bias, ln1.eps)
@@ -165,6 +172,26 @@ class TransformerLayer(nn.Module):
         normed, residual = LayerNormFork.apply(hidden_states, ln2.weight, ln2.bias, ln2.eps)
         return MLPResidual.apply(normed, mlp.dense_h_to_4h.weight, mlp.dense_h_to_4h.bias,
                                  mlp.dense_4h_to_h.weight, mlp.dense_4h_to_h.bias, residual)
+
+
+    def _native(self, hidden_states, attn_bias):
+        # the module dictionaries are read directly: attribute access through nn.Module costs as much as a kernel launch
+        modules = self._modules
+        att, mlp = modules["attention"]._modules, modules["mlp"]._modules
+        ln1, ln2 = modules["input_layernorm"], modules["post_attention_layernorm"]
+        fc1, fc2 = mlp["dense_h_to_4h"], mlp["dense_4h_to_h"]
+        heads = modules["attention"].num_attention_heads
+        if attn_bias is None:
+            bias = _NO_BIAS
+        else:
+            bias = _attention._resolve_bias(attn_bias, heads, hidden_states.shape[1], hidden_states.dtype)
+        return _host.layer(
+            hidden_states, ln1.weight, ln1.bias, att["q_proj"].weight, att["k_proj"].weight, att["v_proj"].weight,
+            att["out_proj"].weight, ln2.weight, ln2.bias, fc1.weight, fc1.bias, fc2.weight, fc2.bias,
+            bias.slopes, bias.rounded, bias.table, heads, ln1.eps, ln2.eps)
+
+
+_NO_BIAS = _attention._Bias()
 
 
 class Transformer(nn.Module):
@@ -225,9 +252,5 @@ class Transformer(nn.Module):
         logits = self.logits_out(hidden_states)
         if labels is None:
             return logits
-        # position t predicts token t+1; the last position of each sequence has no target
-        shifted = torch.full_like(labels, -1)
-        shifted[:, :-1] = labels[:, 1:]
-        per_token = CrossEntropyLossFP32.apply(logits.view(-1, logits.size(-1)), shifted.view(-1))
-        loss = per_token.sum() / (batch * (seq - 1))
+        loss = lm_loss(logits, labels)  # position t predicts token t+1; the last position of each sequence has no target
         return logits, loss
