@@ -239,9 +239,11 @@ struct AttentionFn : torch::autograd::Function<AttentionFn> {
       dk = at::empty_like(k);
       dv = at::empty_like(v);
     }
+    const int64_t nbytes = tfb_attention_bwd_scratch_bytes(shape.b, shape.h, shape.t, shape.hd);
+    Tensor scratch = at::empty({nbytes}, q.options().dtype(at::kByte));
     attention_backward(heads_of(q), heads_of(k), heads_of(v), heads_of(out), heads_of(d_out),
-                       static_cast<const float*>(lse.data_ptr()), heads_of(dq), heads_of(dk), heads_of(dv), shape, bias, q,
-                       dtype_code(q.scalar_type()), current_stream(q));
+                       static_cast<const float*>(lse.data_ptr()), heads_of(dq), heads_of(dk), heads_of(dv), shape, bias,
+                       scratch.data_ptr(), nbytes, dtype_code(q.scalar_type()), current_stream(q));
     return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };

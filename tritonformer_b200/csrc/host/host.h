@@ -114,7 +114,6 @@ std::tuple<Tensor, Tensor> layernorm_forward(const Tensor& x, const Tensor& alph
 // dalpha / dbeta: buffers to write, or with `add` to add to.  Returns dx.
 Tensor layernorm_backward(const Tensor& dy, const Tensor& x, const Tensor& alpha, const Tensor& stats, const Tensor& dres,
                           void* dalpha, void* dbeta, bool add);
-void column_sum_into(const Mat& x, void* out, int dtype, const Tensor& like, cudaStream_t stream);
 Tensor column_sum(const Tensor& x);
 Tensor relu_backward(const Tensor& dy, const Tensor& act);
 
@@ -135,6 +134,6 @@ void attention_forward(const Heads& q, const Heads& k, const Heads& v, const Hea
                        const Bias& bias, int dtype, cudaStream_t stream);
 void attention_backward(const Heads& q, const Heads& k, const Heads& v, const Heads& o, const Heads& d_o, const float* lse,
                         const Heads& dq, const Heads& dk, const Heads& dv, const AttnShape& s, const Bias& bias,
-                        const Tensor& like, int dtype, cudaStream_t stream);
+                        void* scratch, int64_t scratch_bytes, int dtype, cudaStream_t stream);
 
 }  // namespace tfb_host

@@ -280,13 +280,6 @@ Tensor layernorm_backward(const Tensor& dy, const Tensor& x, const Tensor& alpha
 }
 
 // ------------------------------------------------------------------------------------------ bias and ReLU gradients
-void column_sum_into(const Mat& x, void* out, int dtype, const Tensor& like, cudaStream_t stream) {
-  const int64_t n = tfb_colsum_partials(x.rows, x.cols);
-  Tensor partials = at::empty({n, x.cols}, like.options().dtype(at::kFloat));
-  check(tfb_colsum(x.p, out, static_cast<float*>(partials.data_ptr()), n, x.rows, x.cols, x.rows > 1 ? x.s0 : x.cols, dtype,
-                   stream));
-}
-
 Tensor column_sum(const Tensor& x) {
   Mat m = as_rows(x);
   if (m.s1 != 1) {
@@ -295,7 +288,10 @@ Tensor column_sum(const Tensor& x) {
     m.keep = c;
   }
   Tensor out = at::empty({m.cols}, x.options());
-  column_sum_into(m, out.data_ptr(), dtype_code(x.scalar_type()), x, current_stream(x));
+  const int64_t n = tfb_colsum_partials(m.rows, m.cols);
+  Tensor partials = at::empty({n, m.cols}, x.options().dtype(at::kFloat));
+  check(tfb_colsum(m.p, out.data_ptr(), static_cast<float*>(partials.data_ptr()), n, m.rows, m.cols,
+                   m.rows > 1 ? m.s0 : m.cols, dtype_code(x.scalar_type()), current_stream(x)));
   return out;
 }
 
@@ -324,14 +320,12 @@ void attention_forward(const Heads& q, const Heads& k, const Heads& v, const Hea
 
 void attention_backward(const Heads& q, const Heads& k, const Heads& v, const Heads& o, const Heads& d_o, const float* lse,
                         const Heads& dq, const Heads& dk, const Heads& dv, const AttnShape& s, const Bias& bias,
-                        const Tensor& like, int dtype, cudaStream_t stream) {
+                        void* scratch, int64_t scratch_bytes, int dtype, cudaStream_t stream) {
   const bool tab = bias.table.defined();
-  const int64_t nbytes = tfb_attention_bwd_scratch_bytes(s.b, s.h, s.t, s.hd);
-  Tensor scratch = at::empty({nbytes}, like.options().dtype(at::kByte));
   check(tfb_attention_bwd(q.p, k.p, v.p, o.p, d_o.p, lse, dq.p, dk.p, dv.p, s.b, s.h, s.t, s.hd, q.s, k.s, v.s, o.s, d_o.s, dq.s,
                           dk.s, dv.s, bias.slopes.defined() ? static_cast<const float*>(bias.slopes.data_ptr()) : nullptr,
                           bias.rounded, tab ? bias.table.data_ptr() : nullptr, tab ? bias.table.stride(0) : 0,
-                          tab ? bias.table.stride(1) : 0, scratch.data_ptr(), nbytes, dtype, stream, nullptr));
+                          tab ? bias.table.stride(1) : 0, scratch, scratch_bytes, dtype, stream, nullptr));
 }
 
 }  // namespace tfb_host
