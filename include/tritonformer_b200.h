@@ -160,6 +160,14 @@ int64_t tfb_colsum_partials(int64_t rows, int64_t cols);
 int tfb_colsum(const void* x, void* out, float* partials, int64_t n_partials,
                int64_t rows, int64_t cols, int64_t x_ld, int dtype, void* stream);
 
+/* What the backward of a linear layer needs before its products, in one pass: dz = act > 0 ? dy : 0 (act may be NULL: a
+ * copy) and, unless `sums` is NULL, sums[j] = sum_i dz[i,j] (scratch: tfb_colsum_partials() rows of `cols` floats).  dy and
+ * act may have any row pitch and any base; dz has 16-byte aligned rows (dz_ld a multiple of 8, at least cols rounded up
+ * to one; the padding is written with zeros), as the tcgen05 GEMM wants its operands.                          */
+int tfb_grad_rows(const void* dy, const void* act, void* dz, void* sums, float* partials, int64_t n_partials,
+                  int64_t rows, int64_t cols, int64_t dy_ld, int64_t act_ld, int64_t dz_ld, int dtype,
+                  void* stream);
+
 /* ------------------------------------------------------------------- embeddings
  * Replaces the two torch.nn.Embedding lookups and their sum at the head of
  * Transformer.forward (transformer.py:259-272, 311-321) and their gradients.
@@ -193,8 +201,9 @@ int tfb_embedding_bwd(const int64_t* ids, const void* dout, void* dtok, void* dp
  * fp16/bf16 operands, fp32 accumulation over the whole contraction, one rounding.
  * The weight gradient is this same call with the contraction over all B*T rows.
  * bias may be NULL; relu != 0 applies max(.,0) after the bias.
- * Shapes whose operand rows are 16-byte aligned run on the tcgen05/TMA kernel; the
- * rest run on a generic-stride tensor-core kernel.  `path` (may be NULL) receives
+ * Operands whose rows are 16-byte aligned run on the tcgen05/TMA kernels (C, bias, addend and mask may
+ * have any pitch and base; 16-byte aligned ones are faster); other operands run on a generic-stride
+ * tensor-core kernel (tfb_grad_rows packs such an operand).  `path` (may be NULL) receives
  * 1 for the tcgen05 kernel, 0 for the generic one.                              */
 int tfb_gemm(const void* a, const void* b, void* c, const void* bias,
              int64_t M, int64_t N, int64_t K,

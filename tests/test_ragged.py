@@ -1,0 +1,89 @@
+"""GPU: sizes whose rows are no multiple of 16 bytes, at the edges of the tiles and vectors of the kernels that take them:
+products with element-wise epilogues (one- and two-CTA kernels, split contraction, addend and mask), the operand packing
+with its mask and column sums, and the cross-entropy rows.  Bounds: one 16-bit rounding of the result (2^-11 / 2^-8 of
+its size) plus fp32 accumulation."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+EPS = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+
+
+def _close(got, want, dtype, terms=1):
+    err = (got.double() - want).abs()
+    # one rounding of the result, and fp32 sums of `terms` products of values of about one
+    bound = EPS[dtype] * want.abs() + 2.0 ** -22 * terms + 2.0 ** -24
+    assert (err <= 1.01 * bound).all(), (err - bound).max().item()
+
+
+# (M, N, K): one tile and its edges, several tiles, the pair kernel, split contractions; N odd or even without being 8k
+PRODUCTS = [(1, 1, 8), (31, 33, 64), (128, 127, 72), (129, 257, 128), (300, 250, 640), (640, 1001, 4096), (2600, 1290, 256),
+            (5000, 2050, 128)]
+
+
+@pytest.mark.parametrize("m,n,k", PRODUCTS)
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("form", ["plain", "bias_relu", "addend_mask"])
+def test_products_with_unaligned_output_rows(m, n, k, dtype, form):
+    from tritonformer_b200 import linear as L
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda").to(dtype)
+    w = (torch.randn(n, k, device="cuda") * k ** -0.5).to(dtype)  # applied transposed: its rows are aligned
+    want = a.double() @ w.double().t()
+    extra = {}
+    if form == "bias_relu":
+        bias = torch.randn(n, device="cuda").to(dtype)
+        want, extra = (want + bias.double()).clamp_min(0.0), {"bias": bias, "relu": True}
+    elif form == "addend_mask":
+        add, mask = (torch.randn(m, n, device="cuda").to(dtype) for _ in range(2))
+        want, extra = torch.where(mask > 0, want + add.double(), 0.0), {"addend": add, "mask": mask}
+    calls = []
+    L.PROFILE = calls
+    try:
+        got = L.gemm(a, k, 1, w, 1, k, m, n, k, **extra)
+    finally:
+        L.PROFILE = None
+    assert calls[0]["path"] == 1  # the tcgen05 kernels
+    _close(got, want, dtype, terms=k ** 0.5)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (7, 3), (33, 255), (64, 257), (1000, 1477), (4099, 9)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("offset", [0, 1, 5])
+def test_grad_rows(rows, cols, dtype, offset):
+    """The mask, the packing and the column sums, from every kind of base address."""
+    from tritonformer_b200 import _lib as L
+    dy = torch.randn(rows * cols + offset, device="cuda").to(dtype)[offset:].view(rows, cols)
+    act = torch.randn(rows * cols + offset, device="cuda").to(dtype)[offset:].view(rows, cols)
+    ld = -(-cols // 8) * 8
+    dz = torch.full((rows, ld), 7.0, device="cuda", dtype=dtype)
+    sums = torch.empty(cols, device="cuda", dtype=dtype)
+    n = L.lib.tfb_colsum_partials(rows, cols)
+    partials = torch.empty(n, cols, device="cuda")
+    L.check(L.lib.tfb_grad_rows(dy.data_ptr(), act.data_ptr(), dz.data_ptr(), sums.data_ptr(), partials.data_ptr(), n, rows,
+                                cols, cols, cols, ld, L.dtype_code(dtype), L.stream_ptr(dy.device)))
+    want = torch.where(act > 0, dy, torch.zeros_like(dy))
+    assert torch.equal(dz[:, :cols], want) and not dz[:, cols:].any()
+    _close(sums, want.double().sum(0), dtype, terms=rows)
+    L.check(L.lib.tfb_grad_rows(dy.data_ptr(), None, dz.data_ptr(), None, None, 0, rows, cols, cols, 0, ld,
+                                L.dtype_code(dtype), L.stream_ptr(dy.device)))
+    assert torch.equal(dz[:, :cols], dy)
+
+
+@pytest.mark.parametrize("cols", [1, 7, 9, 2047, 2049, 50257])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_lm_loss_of_an_odd_vocabulary(cols, dtype):
+    from tritonformer_b200.crossentropy import lm_loss
+    torch.manual_seed(cols)
+    b, t = 2, 9
+    logits = torch.randn(b, t, cols, device="cuda").to(dtype).requires_grad_(True)
+    labels = torch.randint(0, cols, (b, t), device="cuda")
+    ref = logits.detach().double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(ref[:, :-1].reshape(-1, cols), labels[:, 1:].reshape(-1))
+    loss = lm_loss(logits, labels)
+    assert abs(loss.item() - want.item()) <= 1e-5 * max(1.0, abs(want.item()))
+    (loss * 16.0).backward()
+    (want * 16.0).backward()
+    # exp2f of an fp32 difference: a few 1e-6 of the probability, then one rounding (or half a subnormal step)
+    err = (logits.grad.double() - ref.grad).abs()
+    assert (err <= (EPS[dtype] + 1e-5) * ref.grad.abs() + 1e-6 + 2.0 ** -25).all()

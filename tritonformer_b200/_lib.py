@@ -43,6 +43,7 @@ _SIGNATURES = {
     "tfb_relu_bwd": (_i32, [_vp, _vp, _vp, _i64, _i32, _vp]),
     "tfb_colsum_partials": (_i64, [_i64, _i64]),
     "tfb_colsum": (_i32, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _i32, _vp]),
+    "tfb_grad_rows": (_i32, [_vp] * 5 + [_i64] * 6 + [_i32, _vp]),
     "tfb_embedding_fwd": (_i32, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _vp]),
     "tfb_embedding_bwd_scratch_bytes": (_i64, [_i64] * 4),
     "tfb_embedding_bwd": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _i32, _vp]),

@@ -178,6 +178,61 @@ __device__ __forceinline__ void st_stream16(void* p, const uint4& v) {
                : "memory");
 }
 
+// Eight 16-bit values from an address of any (2-byte) alignment, `n` of them wanted (the rest of the result is
+// undefined): one or two aligned 16-byte loads and a shift.  Every load covers at least one wanted byte, and an aligned
+// 16-byte unit never crosses the end of an allocation, so nothing outside the allocation is touched.
+__device__ __forceinline__ uint4 load8_any(const void* p, int n) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  const uint32_t off = (uint32_t)(a & 15);
+  const uint4* q = reinterpret_cast<const uint4*>(a & ~uintptr_t(15));
+  const uint4 lo = ld_stream16(q);
+  if (off == 0) return lo;
+  uint4 hi = make_uint4(0, 0, 0, 0);
+  if (off + 2 * (uint32_t)n > 16) hi = ld_stream16(q + 1);
+  const uint32_t bits = (off & 2) * 8;
+  uint32_t w0, w1, w2, w3, w4;
+  switch (off >> 2) {
+    case 0: w0 = lo.x; w1 = lo.y; w2 = lo.z; w3 = lo.w; w4 = hi.x; break;
+    case 1: w0 = lo.y; w1 = lo.z; w2 = lo.w; w3 = hi.x; w4 = hi.y; break;
+    case 2: w0 = lo.z; w1 = lo.w; w2 = hi.x; w3 = hi.y; w4 = hi.z; break;
+    default: w0 = lo.w; w1 = hi.x; w2 = hi.y; w3 = hi.z; w4 = hi.w; break;
+  }
+  return make_uint4(__funnelshift_r(w0, w1, bits), __funnelshift_r(w1, w2, bits), __funnelshift_r(w2, w3, bits),
+                    __funnelshift_r(w3, w4, bits));
+}
+
+// Columns [first, last) of chunk `c` of a row whose chunks are cut at the 16-byte boundaries of `row`: all chunks but the
+// first and the last are whole vectors.  chunk_count() of them cover `cols` columns.
+struct Chunk {
+  int first, last;
+};
+template <typename T>
+__device__ __forceinline__ int chunk_shift(const T* row) {  // elements of the first boundary's vector that precede the row
+  return (int)((reinterpret_cast<uintptr_t>(row) & 15) / sizeof(T));
+}
+template <typename T>
+__device__ __forceinline__ int chunk_count(int shift, int cols) {
+  constexpr int W = 16 / sizeof(T);
+  return (cols + shift + W - 1) / W;
+}
+template <typename T>
+__device__ __forceinline__ Chunk chunk_at(int c, int shift, int cols) {
+  constexpr int W = 16 / sizeof(T);
+  const int s = c * W - shift;
+  return {s < 0 ? 0 : s, s + W < cols ? s + W : cols};
+}
+// Stores the values of a chunk (`f[0]` is column `first`).
+template <typename T>
+__device__ __forceinline__ void store_chunk(T* row, const Chunk& k, const float (&f)[8]) {
+  if (k.last - k.first == 8) {
+    st_stream16(row + k.first, pack8<T>(f));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j < k.last - k.first) row[k.first + j] = Num<T>::from_f(f[j]);
+  }
+}
+
 // Dispatch a 16-bit dtype code to a template instantiation.
 #define TFB_DISPATCH_16(dtype, T, ...)                                   \
   if ((dtype) == TFB_F16) { using T = __half; __VA_ARGS__ }              \

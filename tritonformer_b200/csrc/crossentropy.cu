@@ -54,14 +54,28 @@ __global__ void __launch_bounds__(CE_THREADS) ce_fwd_kernel(
 #pragma unroll
       for (int j = 0; j < 8; ++j) s += exp2f(fmaf(f[j], kLog2e, -m));
     }
-  } else {
-    for (int c = threadIdx.x; c < vocab; c += CE_THREADS) {
-      const float t = Num<T>::to_f(xr[c]) * kLog2e;
-      if (t > m) {
-        s *= exp2f(m - t);
-        m = t;
+  } else {  // rows of any alignment (a vocabulary that is no multiple of 8): vectors at the row's own boundaries
+    const int shift = chunk_shift(xr), chunks = chunk_count<T>(shift, vocab);
+    for (int c = threadIdx.x; c < chunks; c += CE_THREADS) {
+      const Chunk k = chunk_at<T>(c, shift, vocab);
+      const int n = k.last - k.first;
+      float f[8];
+      unpack8<T>(load8_any(xr + k.first, n), f);
+      float vm = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (j >= n) f[j] = -INFINITY;
+        vm = fmaxf(vm, f[j]);
       }
-      s += exp2f(t - m);
+      vm *= kLog2e;
+      if (vm > m) {
+        s *= exp2f(m - vm);
+        m = vm;
+      }
+      if (m != -INFINITY) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s += exp2f(fmaf(f[j], kLog2e, -m));
+      }
     }
   }
 #pragma unroll
@@ -123,10 +137,14 @@ __global__ void __launch_bounds__(CE_THREADS) ce_bwd_kernel(
       st_stream16(dr + (int64_t)c * 8, pack8<T>(f));
     }
   } else {
-    for (int c = threadIdx.x; c < vocab; c += CE_THREADS) {
-      float p = exp2f(fmaf(Num<T>::to_f(xr[c]), kLog2e, -l2));
-      if (c == lab) p -= 1.f;
-      dr[c] = Num<T>::from_f(p * g);
+    const int shift = chunk_shift(dr), chunks = chunk_count<T>(shift, vocab);
+    for (int c = threadIdx.x; c < chunks; c += CE_THREADS) {
+      const Chunk k = chunk_at<T>(c, shift, vocab);
+      float f[8];
+      unpack8<T>(load8_any(xr + k.first, k.last - k.first), f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = (exp2f(fmaf(f[j], kLog2e, -l2)) - (k.first + j == lab ? 1.f : 0.f)) * g;
+      store_chunk(dr, k, f);
     }
   }
 }

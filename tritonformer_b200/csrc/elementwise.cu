@@ -74,9 +74,93 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, fl
   }
 }
 
+// dz = act > 0 ? dy : 0 (act may be null: a copy) with the column sums of dz on the way: what the backward of a linear
+// layer needs before its two products, in one pass over dy and act.  dy and act may have any alignment and pitch; dz has
+// 16-byte aligned rows, so that the products can read it through TMA whatever the layer's width (a copy with act and
+// sums null packs an operand the same way).  HBM-bound; the work of a CTA is the one of colsum_kernel, four rows of a
+// thread in flight.  fp16 5015 x 2930 with mask and sums: see the table of the linear cases.
+constexpr int GR_ROWS = 4;
+template <typename T>
+__global__ void __launch_bounds__(256) grad_rows_kernel(const T* __restrict__ dy, const T* __restrict__ act,
+                                                        T* __restrict__ dz, float* __restrict__ partials, int64_t rows,
+                                                        int cols, int64_t dy_ld, int64_t act_ld, int64_t dz_ld) {
+  grid_dependency_wait();
+  allow_dependents();
+  __shared__ float sm[8][32][9];
+  const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5;
+  const int c0 = (blockIdx.x * 32 + cl) * 8;
+  const int n = min(8, cols - c0);
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+  if (n > 0) {
+    const int64_t step = (int64_t)gridDim.y * 8;
+    for (int64_t r0 = (int64_t)blockIdx.y * 8 + rl; r0 < rows; r0 += step * GR_ROWS) {
+      uint4 g[GR_ROWS], a[GR_ROWS];
+#pragma unroll
+      for (int i = 0; i < GR_ROWS; ++i) {
+        const int64_t r = r0 + i * step;
+        if (r >= rows) continue;
+        g[i] = load8_any(dy + r * dy_ld + c0, n);
+        if (act) a[i] = load8_any(act + r * act_ld + c0, n);
+      }
+#pragma unroll
+      for (int i = 0; i < GR_ROWS; ++i) {
+        const int64_t r = r0 + i * step;
+        if (r >= rows) continue;
+        float f[8];
+        unpack8<T>(g[i], f);
+        if (act) {
+          float m[8];
+          unpack8<T>(a[i], m);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] = m[j] > 0.f ? f[j] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (j >= n) f[j] = 0.f;  // the padding of a row
+          acc[j] += f[j];
+        }
+        *reinterpret_cast<uint4*>(dz + r * dz_ld + c0) = pack8<T>(f);
+      }
+    }
+  }
+  if (!partials) return;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sm[rl][cl][j] = acc[j];
+  __syncthreads();
+  const int cc = threadIdx.x, col = blockIdx.x * 256 + cc;
+  if (col < cols) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += sm[i][cc >> 3][cc & 7];
+    partials[(int64_t)blockIdx.y * cols + col] = s;
+  }
+}
+
 }  // namespace tfb
 
 using namespace tfb;
+
+extern "C" int tfb_grad_rows(const void* dy, const void* act, void* dz, void* sums, float* partials, int64_t n_partials,
+                             int64_t rows, int64_t cols, int64_t dy_ld, int64_t act_ld, int64_t dz_ld, int dtype,
+                             void* stream) {
+  TFB_REQUIRE(rows >= 0 && cols > 0 && cols < (1LL << 31) - 256, "grad_rows: bad shape");
+  TFB_REQUIRE(dy_ld >= cols && (!act || act_ld >= cols), "grad_rows: row stride smaller than cols");
+  TFB_REQUIRE(aligned16(dz) && dz_ld % 8 == 0 && dz_ld >= ceil_div(cols, 8) * 8, "grad_rows: dz rows must be 16-byte aligned");
+  TFB_REQUIRE(!sums || (partials && n_partials == tfb_colsum_partials(rows, cols)),
+              "grad_rows: scratch must hold tfb_colsum_partials() rows");
+  if (rows == 0 && !sums) return TFB_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  const dim3 grid((unsigned)ceil_div(cols, 256), (unsigned)tfb_colsum_partials(rows, cols));
+  TFB_DISPATCH_16(dtype, T, {
+    launch_overlapped(grad_rows_kernel<T>, grid, dim3(256), 0, st, (const T*)dy, (const T*)act, (T*)dz, sums ? partials : nullptr,
+                      rows, (int)cols, dy_ld, act_ld, dz_ld);
+    const int rc = launched("grad_rows");
+    if (rc || !sums) return rc;
+    return finalize_partials<T>(partials, n_partials, (int)cols, (int)cols, sums, nullptr, st, 0);
+  })
+}
 
 extern "C" int tfb_relu_bwd(const void* dy, const void* act, void* dz, int64_t n, int dtype,
                             void* stream) {

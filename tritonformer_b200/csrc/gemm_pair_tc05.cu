@@ -16,11 +16,14 @@
 // Every wait is bounded (mbar_wait); the two cluster-wide barriers (after set-up, before exit) are
 // reached unconditionally by both CTAs.
 #include "gemm_sched.cuh"
+#include <string.h>
 #include <type_traits>
 
 namespace tfb {
 
 extern std::atomic<int> g_gemm_debug;
+bool gemm_needs_direct(const void* c, int64_t ldc, const void* bias, const void* addend, int64_t ld_addend, const void* mask,
+                       int64_t ld_mask);
 
 constexpr int GP_M = 128;    // rows per CTA
 constexpr int GP_N = 256;    // columns per pair tile
@@ -47,6 +50,7 @@ struct PairParams {
   int M, N, K;
   int64_t ldc, ld_addend, ld_mask;
   int relu;
+  int direct;          // C, addend, mask or bias cannot go through TMA boxes: element-wise coalesced stores (store_direct)
   int tiles_m, tiles_n;  // in 256 x 256 pair tiles
   int sk_tiles;          // pair tiles [0, sk_tiles) are split along K over all pairs; 0 = whole tiles only
   int* flags;            // per split tile: one arrival counter per (CTA of the pair, epilogue warp)
@@ -263,14 +267,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     uint8_t* stage_c = smem + GP_OFF_EPI_C + ew * 4096;
     uint8_t* stage_x = smem + GP_OFF_EPI_X + ew * 4096;
     const bool x_is_addend = p.addend != nullptr;
-    const bool use_x = (p.addend != nullptr || p.mask != nullptr);
+    const bool use_x = !p.direct && (p.addend != nullptr || p.mask != nullptr);
     const T* mask_direct = (p.addend != nullptr && p.mask != nullptr) ? reinterpret_cast<const T*>(p.mask) : nullptr;
     constexpr int STEPS = GP_N / 64 / (GP_EPI_WARPS / 4);  // 64-column steps per warp
     int buf = 0;
     uint32_t acc_phase = 0, x_phase = 0;
     bool ok = true;
     if (lane == 0) {
-      tma_prefetch_desc(&tmC);
+      if (!p.direct) tma_prefetch_desc(&tmC);
       if (use_x) tma_prefetch_desc(&tmX);
     }
     Segments segs(kblocks, num_tiles, p.sk_tiles, num_pairs, pair, dead);
@@ -362,6 +366,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
             r1[4 * e + 2] = __float_as_uint(__uint_as_float(r1[4 * e + 2]) + v[8 + e].z);
             r1[4 * e + 3] = __float_as_uint(__uint_as_float(r1[4 * e + 3]) + v[8 + e].w);
           }
+        }
+        if (p.direct) {
+          const DirectOut<T> out{reinterpret_cast<T*>(p.C), bias, reinterpret_cast<const T*>(p.addend),
+                                 reinterpret_cast<const T*>(p.mask), p.ldc, p.ld_addend, p.ld_mask, p.M, p.N, p.relu};
+          store_direct<T>(out, r0, reinterpret_cast<float*>(stage_c), row0, col0, lane);
+          store_direct<T>(out, r1, reinterpret_cast<float*>(stage_x), row0, col0 + 32, lane);
+          continue;
         }
         if (use_x) {
           if (!mbar_wait(&x_full[ew], x_phase, 0xb00 | ew, abort_flag)) { ok = false; break; }
@@ -502,11 +513,13 @@ int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, cons
   const bool a_mn = (a_sk != 1), b_mn = (b_sk != 1);
   CUtensorMap tmA, tmB, tmC, tmX;
   int rc;
+  const bool direct = gemm_needs_direct(c, ldc, bias, addend, ld_addend, mask, ld_mask);
   {
     uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, str[1] = {(uint64_t)ldc * 2};
     uint32_t box[2] = {64, 32};
-    if ((rc = encode_tmap_sw128(&tmC, c, dtype, 2, dims, str, box))) return rc;
-    const void* xp = addend ? addend : mask;
+    if (direct) memset(&tmC, 0, sizeof(tmC));
+    else if ((rc = encode_tmap_sw128(&tmC, c, dtype, 2, dims, str, box))) return rc;
+    const void* xp = direct ? nullptr : addend ? addend : mask;
     str[0] = (uint64_t)(addend ? ld_addend : ld_mask) * 2;
     if (xp) { if ((rc = encode_tmap_sw128(&tmX, xp, dtype, 2, dims, str, box))) return rc; }
     else tmX = tmC;
@@ -524,7 +537,7 @@ int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, cons
   PairParams p;
   p.C = c; p.bias = bias; p.addend = addend; p.mask = mask;
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.ldc = ldc; p.ld_addend = ld_addend; p.ld_mask = ld_mask;
-  p.relu = relu; p.debug = g_gemm_debug.load();
+  p.relu = relu; p.direct = direct; p.debug = g_gemm_debug.load();
   p.tiles_m = (int)ceil_div(M, 2 * GP_M); p.tiles_n = (int)ceil_div(N, GP_N);
   const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
   int64_t sk_tiles = 0;

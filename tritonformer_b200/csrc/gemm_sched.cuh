@@ -74,4 +74,41 @@ __device__ __forceinline__ bool flag_wait(const int* flag, int expect, int code,
   return false;
 }
 
+// Epilogue output that TMA boxes cannot carry (a row pitch that is no multiple of 16 bytes, an unaligned base): the
+// 32 x 32 block of fp32 accumulators of a warp (thread = row) is turned through a 4 KB swizzled box in shared memory, so
+// that a warp then touches consecutive elements of one row.  Bias, ReLU, addend and mask are applied there, coalesced as
+// well, and the value is rounded once.
+template <typename T> struct DirectOut {
+  T* c;
+  const T *bias, *addend, *mask;
+  int64_t ldc, ld_addend, ld_mask;
+  int M, N, relu;
+};
+template <typename T>
+__device__ __forceinline__ void store_direct(const DirectOut<T>& o, const uint32_t (&r)[32], float* box, int row0, int col0,
+                                             int lane) {
+#pragma unroll
+  for (int v = 0; v < 8; ++v)
+    *reinterpret_cast<uint4*>(box + lane * 32 + ((v ^ (lane & 7)) << 2)) =
+        make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+  __syncwarp();
+  const int col = col0 + lane;
+  const int rows = o.M - row0 < 32 ? o.M - row0 : 32;
+  if (col < o.N) {
+    const float b = o.bias ? Num<T>::to_f(o.bias[col]) : 0.f;
+    T* c = o.c + (int64_t)row0 * o.ldc + col;
+    const T* add = o.addend ? o.addend + (int64_t)row0 * o.ld_addend + col : nullptr;
+    const T* mask = o.mask ? o.mask + (int64_t)row0 * o.ld_mask + col : nullptr;
+#pragma unroll 8
+    for (int i = 0; i < rows; ++i) {
+      float f = box[i * 32 + (((lane >> 2) ^ (i & 7)) << 2) + (lane & 3)] + b;
+      if (o.relu) f = fmaxf(f, 0.f);
+      if (add) f += Num<T>::to_f(add[(int64_t)i * o.ld_addend]);
+      if (mask && !(Num<T>::to_f(mask[(int64_t)i * o.ld_mask]) > 0.f)) f = 0.f;
+      c[(int64_t)i * o.ldc] = Num<T>::from_f(f);
+    }
+  }
+  __syncwarp();  // the box may be overwritten
+}
+
 }  // namespace tfb

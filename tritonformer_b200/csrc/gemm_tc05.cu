@@ -20,6 +20,7 @@
 // product X·W, the input gradient dY·Wᵀ and the weight gradient Xᵀ·dY (contraction over every
 // token of the batch, i.e. the batch reduction fused into the product) are the same kernel.
 #include "gemm_sched.cuh"
+#include <string.h>
 #include <type_traits>
 
 namespace tfb {
@@ -27,6 +28,8 @@ namespace tfb {
 extern std::atomic<int> g_gemm_debug;
 extern std::atomic<int> g_gemm_free_sms;
 int64_t gemm_pair_tiles(int64_t M, int64_t N);
+bool gemm_needs_direct(const void* c, int64_t ldc, const void* bias, const void* addend, int64_t ld_addend, const void* mask,
+                       int64_t ld_mask);
 int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, const void* addend, int64_t ld_addend,
                    const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
                    int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, int sms, void* workspace,
@@ -59,6 +62,7 @@ struct GemmParams {
   int M, N, K;
   int64_t ldc, ld_addend, ld_mask;
   int relu;
+  int direct;          // C, addend, mask or bias cannot go through TMA boxes: element-wise coalesced stores (store_direct)
   int tiles_m, tiles_n;
   int sk_tiles;        // tiles [0, sk_tiles) are split along K over all CTAs; 0 = whole tiles only
 };
@@ -201,14 +205,14 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
     uint8_t* stage_x = smem + Cfg::OFF_EPI_X + ew * 4096;
     // at most one of addend / mask travels through the TMA box; a second one is read directly
     const bool x_is_addend = p.addend != nullptr;
-    const bool use_x = (p.addend != nullptr || p.mask != nullptr);
+    const bool use_x = !p.direct && (p.addend != nullptr || p.mask != nullptr);
     const T* mask_direct = (p.addend != nullptr && p.mask != nullptr) ? reinterpret_cast<const T*>(p.mask) : nullptr;
     constexpr int STEPS = BN / 64;
     int buf = 0;
     uint32_t acc_phase = 0, x_phase = 0;
     bool ok = true;
     if (lane == 0) {
-      tma_prefetch_desc(&tmC);
+      if (!p.direct) tma_prefetch_desc(&tmC);
       if (use_x) tma_prefetch_desc(&tmX);
     }
     Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x, dead);
@@ -295,6 +299,13 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
             r1[4 * e + 2] = __float_as_uint(__uint_as_float(r1[4 * e + 2]) + v[8 + e].z);
             r1[4 * e + 3] = __float_as_uint(__uint_as_float(r1[4 * e + 3]) + v[8 + e].w);
           }
+        }
+        if (p.direct) {
+          const DirectOut<T> out{reinterpret_cast<T*>(p.C), bias, reinterpret_cast<const T*>(p.addend),
+                                 reinterpret_cast<const T*>(p.mask), p.ldc, p.ld_addend, p.ld_mask, p.M, p.N, p.relu};
+          store_direct<T>(out, r0, reinterpret_cast<float*>(stage_c), row0, col0, lane);
+          store_direct<T>(out, r1, reinterpret_cast<float*>(stage_x), row0, col0 + 32, lane);
+          continue;
         }
         if (use_x) {
           if (!mbar_wait(&x_full[ew], x_phase, 0x500 | ew, abort_flag)) { ok = false; break; }
@@ -457,17 +468,22 @@ static int dispatch_major(bool a_mn, bool b_mn, const CUtensorMap& tmA, const CU
 // Whether (ptr, strides) can be described by a TMA tensor map of 16-bit elements.
 static bool tma_ok(const void* ptr, int64_t s_outer) { return aligned16(ptr) && s_outer % 8 == 0 && s_outer > 0; }
 
-bool gemm_tc05_eligible(const void* a, const void* b, const void* c, const void* bias, const void* addend,
-                        int64_t ld_addend, const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K,
-                        int64_t a_sm, int64_t a_sk, int64_t b_sk, int64_t b_sn, int64_t ldc) {
-  if (addend && !(aligned16(addend) && ld_addend % 8 == 0)) return false;
-  if (mask && !(aligned16(mask) && ld_mask % 8 == 0)) return false;
+bool gemm_tc05_eligible(const void* a, const void* b, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
+                        int64_t b_sk, int64_t b_sn) {
   if (M < 1 || N < 1 || K < 1) return false;
   if (M >= (1LL << 31) || N >= (1LL << 31) || K >= (1LL << 31)) return false;
   const bool a_ok = (a_sk == 1) ? tma_ok(a, a_sm) : (a_sm == 1 && tma_ok(a, a_sk));
   const bool b_ok = (b_sk == 1) ? tma_ok(b, b_sn) : (b_sn == 1 && tma_ok(b, b_sk));
   // A tensor of extent 1 along its strided dim still needs a legal stride; callers pass real strides.
-  return a_ok && b_ok && aligned16(c) && ldc % 8 == 0 && (bias == nullptr || aligned16(bias));
+  return a_ok && b_ok;
+}
+
+// Outputs (or epilogue operands) whose rows TMA cannot describe: the epilogue writes them element by element.
+bool gemm_needs_direct(const void* c, int64_t ldc, const void* bias, const void* addend, int64_t ld_addend, const void* mask,
+                       int64_t ld_mask) {
+  return !(aligned16(c) && ldc % 8 == 0 && (bias == nullptr || aligned16(bias)) &&
+           (addend == nullptr || (aligned16(addend) && ld_addend % 8 == 0)) &&
+           (mask == nullptr || (aligned16(mask) && ld_mask % 8 == 0)));
 }
 
 int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const void* addend, int64_t ld_addend,
@@ -519,12 +535,14 @@ int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const voi
 
   CUtensorMap tmA, tmB, tmC, tmX;
   int rc;
+  const bool direct = gemm_needs_direct(c, ldc, bias, addend, ld_addend, mask, ld_mask);
   {
-    // output and addend/mask: (N inner, M outer), boxes of 64 columns x 32 rows
+    // output and addend/mask: (N inner, M outer), boxes of 64 columns x 32 rows (direct stores use no map)
     uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, str[1] = {(uint64_t)ldc * 2};
     uint32_t box[2] = {64, 32};
-    if ((rc = encode_tmap_sw128(&tmC, c, dtype, 2, dims, str, box))) return rc;
-    const void* xp = addend ? addend : mask;
+    if (direct) memset(&tmC, 0, sizeof(tmC));
+    else if ((rc = encode_tmap_sw128(&tmC, c, dtype, 2, dims, str, box))) return rc;
+    const void* xp = direct ? nullptr : addend ? addend : mask;
     str[0] = (uint64_t)(addend ? ld_addend : ld_mask) * 2;
     if (xp) { if ((rc = encode_tmap_sw128(&tmX, xp, dtype, 2, dims, str, box))) return rc; }
     else tmX = tmC;
@@ -544,7 +562,7 @@ int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const voi
   p.flags = sk_tiles ? reinterpret_cast<int*>(workspace) : nullptr;
   p.partials = sk_tiles ? reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + kFlagBytes) : nullptr;
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.ldc = ldc; p.ld_addend = ld_addend; p.ld_mask = ld_mask;
-  p.relu = relu;
+  p.relu = relu; p.direct = direct;
   p.tiles_m = (int)tm; p.tiles_n = (int)ceil_div(N, BN); p.sk_tiles = (int)sk_tiles;
   TFB_DISPATCH_16(dtype, T, {
     if (BN == 256) return dispatch_major<T, 256>(a_mn, b_mn, tmA, tmB, tmC, tmX, p, (int)grid, st);

@@ -71,10 +71,12 @@ static std::vector<int64_t> with_last(const Tensor& x, int64_t n) {
   return s;
 }
 
-static Tensor linear_body(const Tensor& x, const Tensor& w, const Tensor& bias, bool relu) {
+static Tensor linear_body(const Tensor& x, const Tensor& w, const Tensor& bias, bool relu, Mat* mx, Mat* mw) {
   check_linear(x, w, bias);
-  const Mat mx = as_rows(x), mw = as_matrix(w);
-  Tensor y = at::empty(with_last(x, mw.cols), x.options());
+  const int dtype = dtype_code(x.scalar_type());
+  *mx = tma_fit(as_rows(x), x, dtype);
+  *mw = tma_fit(as_matrix(w), x, dtype);
+  Tensor y = at::empty(with_last(x, mw->cols), x.options());
   Epilogue e;
   Tensor bc;
   if (bias.defined()) {
@@ -82,8 +84,19 @@ static Tensor linear_body(const Tensor& x, const Tensor& w, const Tensor& bias, 
     e.bias = bc.data_ptr();
   }
   e.relu = relu;
-  gemm(mx, mw, y.data_ptr(), mw.cols, e, dtype_code(x.scalar_type()), x.device(), current_stream(x));
+  gemm(*mx, *mw, y.data_ptr(), mw->cols, e, dtype, x.device(), current_stream(x));
   return y;
+}
+
+// A saved operand: the tensor itself, or the copy with aligned rows that forward made of it.
+static Mat saved_operand(const Mat& plain, const Tensor& packed) {
+  if (!packed.defined()) return plain;
+  Mat m = plain;
+  const bool rows_first = plain.s1 == 1;
+  m.keep = packed;
+  m.p = packed.data_ptr();
+  (rows_first ? m.s0 : m.s1) = packed.size(1);
+  return m;
 }
 
 struct LinearFn : torch::autograd::Function<LinearFn> {
@@ -91,41 +104,48 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     Amp amp;
     BodyGuard guard;
     Tensor x = amp(x_), w = amp(w_);
-    Tensor y = linear_body(x, w, amp(val(bias_)), relu);
+    Mat mx, mw;
+    Tensor y = linear_body(x, w, amp(val(bias_)), relu, &mx, &mw);
     ctx->saved_data["bias"] = bias_.has_value();
-    ctx->save_for_backward(relu ? variable_list{x, w, y} : variable_list{x, w});
+    ctx->save_for_backward({x, w, relu ? y : Tensor(), mx.packed, mw.packed});
     return y;
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     BodyGuard guard;
     const variable_list saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &w = saved[1];
+    const Tensor &x = saved[0], &w = saved[1], &act = saved[2];
     const at::ScalarType type = x.scalar_type();
     const int dtype = dtype_code(type);
-    Tensor dz = grads[0].to(type);
-    if (saved.size() > 2) dz = relu_backward(dz, saved[2]);
     const bool has_bias = ctx->saved_data["bias"].toBool();
     const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
-    const Mat mdy = as_rows(dz), mw = as_matrix(w);
+    const bool need_db = has_bias && ctx->needs_input_grad(2);
     Tensor dx, dw, db;
+    // dz: the incoming gradient masked by the ReLU, with rows the products can read, and its column sums
+    const Tensor dy = grads[0].to(type);
+    Mat dz = as_rows(dy);
+    if (act.defined() || !tma_fits(dz)) {
+      dz = grad_rows(dz, act, need_db ? &db : nullptr, x, dtype);
+    } else if (need_db) {
+      db = column_sum(dy);
+    }
+    const Mat mw = saved_operand(as_matrix(w), saved[4]);
     GradTarget g;
     Mat mx;
     if (need_dx) dx = at::empty(x.sizes(), x.options());
     if (need_dw) {
       g = weight_target(w, type);
-      mx = as_rows(x);
+      mx = saved_operand(as_rows(x), saved[3]);
     }
     const bool fork = need_dx && need_dw && g.in_place && g_mode.fork.load(std::memory_order_relaxed);
     SideWork side(x, fork);
     side.mark();
-    if (need_dx) gemm(mdy, mw.t(), dx.data_ptr(), mw.rows, Epilogue{}, dtype, x.device(), side.main());
+    if (need_dx) gemm(dz, mw.t(), dx.data_ptr(), mw.rows, Epilogue{}, dtype, x.device(), side.main());
     if (need_dw) {
-      weight_grad(mx, mdy, g, dtype, x.device(), side.stream());
+      weight_grad(mx, dz, g, dtype, x.device(), side.stream());
       side.keep(mx.keep);
-      side.keep(mdy.keep);
+      side.keep(dz.keep);
       dw = g.fresh;
     }
-    if (has_bias && ctx->needs_input_grad(2)) db = column_sum(dz);
     side.join(g_mode.defer.load(std::memory_order_relaxed));
     return {dx, dw, db, Tensor()};
   }
@@ -142,7 +162,8 @@ Tensor linear(const Tensor& x, const Tensor& w, const Tensor& bias, bool relu) {
   if (any_requires_grad({&x, &w, &bias})) return LinearFn::apply(x, w, opt(bias), relu);
   Amp amp;
   BodyGuard guard;
-  return linear_body(amp(x), amp(w), amp(bias), relu);
+  Mat mx, mw;
+  return linear_body(amp(x), amp(w), amp(bias), relu, &mx, &mw);
 }
 
 // ----------------------------------------------------------------------------------------------------- LayerNorm
@@ -385,10 +406,13 @@ struct LmLossFn : torch::autograd::Function<LmLossFn> {
     const Tensor& logits = s[0];
     const int64_t b = logits.size(0), t = logits.size(1), v = logits.size(2);
     const Tensor g = grads[0].to(at::kFloat);
-    Tensor dlogits = at::empty(logits.sizes(), logits.options());
+    // rows of an odd vocabulary are padded to 16 bytes, as the head's products want to read them
+    const int64_t ld = (v + 7) / 8 * 8;
+    Tensor dlogits = at::empty({b, t, ld}, logits.options());
+    if (ld != v) dlogits = dlogits.slice(2, 0, v);
     check(tfb_lm_loss_bwd(logits.data_ptr(), static_cast<const int64_t*>(s[1].data_ptr()),
                           static_cast<const float*>(s[2].data_ptr()), static_cast<const float*>(g.data_ptr()), dlogits.data_ptr(),
-                          b, t, v, v, v, dtype_code(logits.scalar_type()), current_stream(logits)));
+                          b, t, v, v, ld, dtype_code(logits.scalar_type()), current_stream(logits)));
     return {dlogits, Tensor()};
   }
 };

@@ -90,13 +90,21 @@ int dtype_code(at::ScalarType t);
 // A matrix of 16-bit values with element strides; `keep` owns the memory where a copy was needed.
 struct Mat {
   Tensor keep;
+  Tensor packed;  // keep, where tma_fit made a copy
   const void* p = nullptr;
   int64_t rows = 0, cols = 0, s0 = 0, s1 = 0;
-  Mat t() const { return Mat{keep, p, cols, rows, s1, s0}; }
+  Mat t() const { return Mat{keep, packed, p, cols, rows, s1, s0}; }
 };
 Mat as_rows(const Tensor& x);                        // (.., d) -> (rows, d), one of the strides 1
 Mat as_matrix(const Tensor& w);                      // a 2-D weight, one of the strides 1
 Mat block(const void* p, int64_t rows, int64_t cols);  // contiguous
+
+// Whether the GEMM can read the matrix through TMA (16-byte aligned rows); tma_fit copies one that it cannot into rows
+// padded to a multiple of 16 bytes - a pass over the operand, against a kernel that runs at a twentieth of the rate.
+bool tma_fits(const Mat& m);
+Mat tma_fit(const Mat& m, const Tensor& like, int dtype);
+// dz = act > 0 ? dy : 0 (act undefined: dy) in aligned rows; sums: its column sums, unless null
+Mat grad_rows(const Mat& dy, const Tensor& act, Tensor* sums, const Tensor& like, int dtype);
 
 struct Epilogue {
   const void* bias = nullptr;
@@ -115,7 +123,6 @@ std::tuple<Tensor, Tensor> layernorm_forward(const Tensor& x, const Tensor& alph
 Tensor layernorm_backward(const Tensor& dy, const Tensor& x, const Tensor& alpha, const Tensor& stats, const Tensor& dres,
                           void* dalpha, void* dbeta, bool add);
 Tensor column_sum(const Tensor& x);
-Tensor relu_backward(const Tensor& dy, const Tensor& act);
 
 struct Bias {  // resolved form of the attention bias
   Tensor slopes;

@@ -224,6 +224,46 @@ Mat block(const void* p, int64_t rows, int64_t cols) {
   return m;
 }
 
+bool tma_fits(const Mat& m) {
+  const int64_t outer = m.s1 == 1 ? m.s0 : m.s1;
+  return (reinterpret_cast<uintptr_t>(m.p) & 15) == 0 && outer > 0 && outer % 8 == 0;
+}
+
+Mat grad_rows(const Mat& dy_, const Tensor& act, Tensor* sums, const Tensor& like, int dtype) {
+  Mat dy = dy_;
+  if (dy.s1 != 1) {  // a transposed gradient
+    Tensor c = dy.keep.contiguous();
+    dy = block(c.data_ptr(), dy.rows, dy.cols);
+    dy.keep = c;
+  }
+  const int64_t ld = (dy.cols + 7) / 8 * 8;
+  const Mat a = act.defined() ? as_rows(act) : Mat{};
+  Tensor out = at::empty({dy.rows, ld}, like.options()), partials;
+  int64_t n = 0;
+  if (sums) {
+    n = tfb_colsum_partials(dy.rows, dy.cols);
+    partials = at::empty({n, dy.cols}, like.options().dtype(at::kFloat));
+    *sums = at::empty({dy.cols}, like.options());
+  }
+  check(tfb_grad_rows(dy.p, a.p, out.data_ptr(), sums ? sums->data_ptr() : nullptr,
+                      sums ? static_cast<float*>(partials.data_ptr()) : nullptr, n, dy.rows, dy.cols,
+                      dy.rows > 1 ? dy.s0 : dy.cols, a.p ? a.s0 : 0, ld, dtype, current_stream(like)));
+  Mat m;
+  m.keep = m.packed = out;
+  m.p = out.data_ptr();
+  m.rows = dy.rows;
+  m.cols = dy.cols;
+  m.s0 = ld;
+  m.s1 = 1;
+  return m;
+}
+
+Mat tma_fit(const Mat& m, const Tensor& like, int dtype) {
+  if (tma_fits(m) || m.rows == 0 || m.cols == 0) return m;
+  if (m.s1 == 1) return grad_rows(m, Tensor(), nullptr, like, dtype);
+  return grad_rows(m.t(), Tensor(), nullptr, like, dtype).t();
+}
+
 void gemm(const Mat& a, const Mat& b, void* out, int64_t ldc, const Epilogue& e, int dtype, c10::Device device,
           cudaStream_t stream) {
   Tensor ws = gemm_workspace(device, stream);
@@ -293,13 +333,6 @@ Tensor column_sum(const Tensor& x) {
   check(tfb_colsum(m.p, out.data_ptr(), static_cast<float*>(partials.data_ptr()), n, m.rows, m.cols,
                    m.rows > 1 ? m.s0 : m.cols, dtype_code(x.scalar_type()), current_stream(x)));
   return out;
-}
-
-Tensor relu_backward(const Tensor& dy, const Tensor& act) {
-  Tensor g = dy.contiguous(), a = act.contiguous();
-  Tensor dz = at::empty(g.sizes(), g.options());
-  check(tfb_relu_bwd(g.data_ptr(), a.data_ptr(), dz.data_ptr(), g.numel(), dtype_code(g.scalar_type()), current_stream(g)));
-  return dz;
 }
 
 // --------------------------------------------------------------------------------------------------- attention

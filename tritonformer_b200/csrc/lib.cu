@@ -20,9 +20,8 @@ int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const voi
               const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
               int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, void* workspace,
               int64_t workspace_bytes, cudaStream_t st);
-bool gemm_tc05_eligible(const void* a, const void* b, const void* c, const void* bias, const void* addend,
-                        int64_t ld_addend, const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K,
-                        int64_t a_sm, int64_t a_sk, int64_t b_sk, int64_t b_sn, int64_t ldc);
+bool gemm_tc05_eligible(const void* a, const void* b, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
+                        int64_t b_sk, int64_t b_sn);
 int64_t gemm_tc05_workspace_bytes();
 int read_dev_status(int reset);
 int launch_wait_probe(unsigned long long limit_ns, int* waited_ok, cudaStream_t st);
@@ -84,8 +83,7 @@ extern "C" int tfb_gemm_fused(const void* a, const void* b, void* c, const void*
   TFB_REQUIRE(K > 0, "gemm: empty contraction");
   cudaStream_t st = (cudaStream_t)stream;
   const bool fast = !g_force_generic_gemm.load() &&
-                    gemm_tc05_eligible(a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk,
-                                       b_sn, ldc);
+                    gemm_tc05_eligible(a, b, M, N, K, a_sm, a_sk, b_sk, b_sn);
   if (path) *path = fast ? 1 : 0;
   if (fast)
     return gemm_tc05(a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk, b_sn, ldc, relu,
