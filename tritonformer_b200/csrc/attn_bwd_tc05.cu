@@ -1,4 +1,4 @@
-// Causal flash attention backward on tcgen05 / TMEM for sm_100a (head_dim 64 or 128, T % 128 == 0).
+// Causal flash attention backward on tcgen05 / TMEM for sm_100a (head_dim 32, 64 or 128).
 //
 // One CTA per (128-key tile, batch*head); it walks the query tiles at or below the diagonal.
 // Everything is computed transposed (rows = keys) so that the per-query statistics (log-sum-exp,
@@ -20,6 +20,9 @@
 // At head_dim 64 the scores of tile i+1 are issued as soon as the compute warps hold the scores of tile i in
 // registers, ahead of the gradient products of tile i, so the compute warps find them ready and work on tile
 // i+1 while the tensor core finishes tile i.
+// A sequence that is no multiple of 128: the rows past its end are zeros in shared memory (TMA fill) with statistics of
+// zero, so their dS and their shares of dV, dK and dQ vanish; their own rows are not stored.  head_dim 32 runs on the
+// head_dim 64 kernel with zero columns.
 // TMEM columns: [0,128) Sᵀ; [128,256) dPᵀ; [256,256+hd) dV; then dK; then dQ_i (at head_dim 128
 // dQ_i reuses the Sᵀ columns).
 #include "attn.cuh"
@@ -79,7 +82,7 @@ struct FbParams {
   float* dq_acc;  // (B,H,T,HD) fp32, zero on entry
   void *dk, *dv;
   int64_t sdk_b, sdk_h, sdk_t, sdv_b, sdv_h, sdv_t;
-  int H, T;
+  int H, T, hd;   // hd: the real head_dim, at most HD
   int BH, group;  // batch*heads; how many of them are walked together (their tiles share the L2)
   float scale;
   int bias_mode;
@@ -135,7 +138,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // CTAs are dispatched in block order: within a group of batch*head slices the key tiles with the
   // longest walk (tile 0) of EVERY slice come first, so the tail of the kernel is made of short CTAs
-  const int nq = p.T / FB_T;
+  const int nq = (p.T + FB_T - 1) / FB_T;
   int kt, bh;
   if (p.debug & 32) {  // per-slice order (test switch)
     kt = blockIdx.x % nq;
@@ -357,9 +360,10 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       // column l, fetched one tile ahead (so the global-memory latency is not part of the tile) and handed to the
       // other lanes through a slice of shared memory that belongs to this warp: no barrier across the warps.
       auto load_stat = [&](int it, float& l2, float& dl) {
-        const int64_t at = (int64_t)bh * p.T + (kt + it) * FB_T + cq * 32 + lane;
-        l2 = p.lse[at];  // converted to log2 units where it is used: nothing here may wait for the load
-        dl = p.delta[at];
+        const int i = (kt + it) * FB_T + cq * 32 + lane;
+        const int64_t at = (int64_t)bh * p.T + i;
+        l2 = i < p.T ? p.lse[at] : 0.f;  // converted to log2 units where it is used: nothing here may wait for the load
+        dl = i < p.T ? p.delta[at] : 0.f;
       };
       float lse_next, delta_next;
       load_stat(0, lse_next, delta_next);
@@ -488,12 +492,14 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
 #pragma unroll 1
         for (int c = 0; c < HD / 64; ++c) {  // this warp's HD / 4 columns in steps of 16
           const int col0 = cq * (HD / 4) + c * 16;
+          if (col0 >= p.hd) break;
           uint32_t v[16], w[16];
           tmem_ld16(lane_addr + Cfg::COL_DV + col0, v);
           tmem_ld16(lane_addr + Cfg::COL_DK + col0, w);
           tc_wait_ld();
 #pragma unroll
           for (int v4 = 0; v4 < 2; ++v4) {
+            if (j >= p.T) break;
             float g[8], d[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
@@ -591,20 +597,21 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
+            // (rows past the sequence's end hold exact zeros: added to the next slice's rows they change nothing)
             const int row0 = (int)((int64_t)bh * p.T) + i0 + qd * 32;
             tma_reduce_add_2d(&tmDQ, stage, 0, row0);
-            tma_reduce_add_2d(&tmDQ, stage + 4096, 32, row0);
+            if (p.hd > 32) tma_reduce_add_2d(&tmDQ, stage + 4096, 32, row0);
             tma_store_commit();
           }
         }
       } else {
-        float* dq_row = p.dq_acc + ((int64_t)bh * p.T + i0 + r) * HD;
+        float* dq_row = p.dq_acc + ((int64_t)bh * p.T + i0 + r) * p.hd;
 #pragma unroll 1
-        for (int c = 0; c < HD / 32; ++c) {
+        for (int c = 0; c < p.hd / 32; ++c) {
           uint32_t v[32];
           tmem_ld32(lane_addr + Cfg::COL_DQ + c * 32, v);
           tc_wait_ld();
-          if (!(p.debug & 1))
+          if (!(p.debug & 1) && i0 + r < p.T)
 #pragma unroll
             for (int e = 0; e < 32; e += 4)
               asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dq_row + c * 32 + e),
@@ -675,38 +682,36 @@ static int encode_bhtd(CUtensorMap* m, const void* ptr, const AttnStrides& s, in
   return encode_tmap_sw128(m, ptr, dtype, 4, dims, str, box);
 }
 
-bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd) {
-  return (hd == 64 || hd == 128) && a.T % 128 == 0 && a.bias_mode != 3;
-}
+bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd) { return hd <= 128 && a.bias_mode != 3; }
 
 template <typename T, int HD>
-static int bwd_tc05_launch(const AttnArgs& a, int dtype, cudaStream_t st) {
+static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   using Cfg = FbCfg<HD>;
   int rc;
   // the delta pass also clears the fp32 dQ accumulator (contiguous (B,H,T,HD), 16-byte aligned: checked by the
   // caller), so no fill sits between the kernels in the stream
-  if ((rc = attn_delta(a, HD, dtype, st, a.dq_acc))) return rc;
+  if ((rc = attn_delta(a, hd, dtype, st, a.dq_acc))) return rc;
   CUtensorMap tq, tk, tv, tdo, tdq;
   {
     // fp32 dQ accumulator as a (HD, B*H*T) matrix, boxes of 32 floats x 32 rows
-    const uint64_t dims[2] = {(uint64_t)HD, (uint64_t)a.B * a.H * a.T};
-    const uint64_t str[1] = {(uint64_t)HD * 4};
+    const uint64_t dims[2] = {(uint64_t)hd, (uint64_t)a.B * a.H * a.T};
+    const uint64_t str[1] = {(uint64_t)hd * 4};
     const uint32_t box[2] = {32, 32};
     if ((rc = encode_tmap_sw128(&tdq, a.dq_acc, TFB_F32, 2, dims, str, box))) return rc;
   }
-  if ((rc = encode_bhtd(&tq, a.q, a.sq, a.B, a.H, a.T, HD, dtype))) return rc;
-  if ((rc = encode_bhtd(&tk, a.k, a.sk, a.B, a.H, a.T, HD, dtype))) return rc;
-  if ((rc = encode_bhtd(&tv, a.v, a.sv, a.B, a.H, a.T, HD, dtype))) return rc;
-  if ((rc = encode_bhtd(&tdo, a.d_o, a.sdo, a.B, a.H, a.T, HD, dtype))) return rc;
+  if ((rc = encode_bhtd(&tq, a.q, a.sq, a.B, a.H, a.T, hd, dtype))) return rc;
+  if ((rc = encode_bhtd(&tk, a.k, a.sk, a.B, a.H, a.T, hd, dtype))) return rc;
+  if ((rc = encode_bhtd(&tv, a.v, a.sv, a.B, a.H, a.T, hd, dtype))) return rc;
+  if ((rc = encode_bhtd(&tdo, a.d_o, a.sdo, a.B, a.H, a.T, hd, dtype))) return rc;
   FbParams p;
   p.lse = a.lse; p.delta = a.delta; p.dq_acc = a.dq_acc; p.dk = a.dk; p.dv = a.dv;
   p.sdk_b = a.sdk.b; p.sdk_h = a.sdk.h; p.sdk_t = a.sdk.t;
   p.sdv_b = a.sdv.b; p.sdv_h = a.sdv.h; p.sdv_t = a.sdv.t;
-  p.H = a.H; p.T = a.T; p.scale = a.scale; p.bias_mode = a.bias_mode; p.slopes = a.slopes;
+  p.H = a.H; p.T = a.T; p.hd = hd; p.scale = a.scale; p.bias_mode = a.bias_mode; p.slopes = a.slopes;
   p.debug = g_attn_debug.load();
   p.BH = a.B * a.H;
   p.group = attn_slices_per_group(a.B * a.H, a.T, HD);
-  dim3 grid((a.T / FB_T) * a.B * a.H);
+  dim3 grid((unsigned)ceil_div(a.T, FB_T) * a.B * a.H);
   static std::atomic<uint64_t> done[4] = {{0}, {0}, {0}, {0}};
 #define FB_LAUNCH(MODE, SLOT)                                                                                       \
   {                                                                                                                 \
@@ -722,17 +727,17 @@ static int bwd_tc05_launch(const AttnArgs& a, int dtype, cudaStream_t st) {
   else FB_LAUNCH(4, 3)
 #undef FB_LAUNCH
   if ((rc = launched("attention_bwd(tcgen05)"))) return rc;
-  const int64_t nvec = (int64_t)a.B * a.H * a.T * HD / 8;
+  const int64_t nvec = (int64_t)a.B * a.H * a.T * hd / 8;
   const unsigned blocks = (unsigned)(ceil_div(nvec, 256) < 148 * 8 ? ceil_div(nvec, 256) : 148 * 8);
   launch_overlapped(attn_dq_convert_kernel<T>, dim3(blocks), dim3(256), 0, st, a.dq_acc, (T*)a.dq, a.sdq.b, a.sdq.h,
-                    a.sdq.t, a.H, a.T, HD, a.scale, nvec);
+                    a.sdq.t, a.H, a.T, hd, a.scale, nvec);
   return launched("attention_dq_convert");
 }
 
 int attn_tc05_bwd(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   TFB_DISPATCH_16(dtype, T, {
-    if (hd == 64) return bwd_tc05_launch<T, 64>(a, dtype, st);
-    return bwd_tc05_launch<T, 128>(a, dtype, st);
+    if (hd <= 64) return bwd_tc05_launch<T, 64>(a, hd, dtype, st);
+    return bwd_tc05_launch<T, 128>(a, hd, dtype, st);
   })
 }
 

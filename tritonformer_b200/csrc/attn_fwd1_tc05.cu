@@ -1,5 +1,5 @@
 // Causal flash attention forward on tcgen05 / TMEM: persistent CTAs, one 128-query tile at a time with its
-// score buffers doubled and eight softmax warps (head_dim 64 or 128, T % 128 == 0).
+// score buffers doubled and eight softmax warps (head_dim 32, 64 or 128).
 //
 //   warp 0      TMA producer (Q of each tile into one of two buffers, K_j / V_j tiles of 128 keys through rings)
 //   warp 1      MMA issuer (one elected lane, an event loop over non-blocking barrier probes)
@@ -30,6 +30,11 @@
 // P is stored 16-bit, two keys per 32-bit column, into tensor memory, over the first half of the score columns
 // it was computed from, and is the A operand of P·V.
 // TMEM columns: [0,128) S0 / P0, [128,256) S1 / P1, [256, 256 + 2 head_dim) the two accumulators.
+// A sequence that is no multiple of 128 leaves the last tile partly empty: TMA fills the rows past its end with zeros, the
+// causal mask keeps their keys from every real query, and nothing is stored for their queries.  head_dim 32 runs on the
+// head_dim 64 kernel the same way: the columns past 32 are zeros (twice the tensor work of a path that is bound by the
+// exponentials, which are per score).  Measured at B3 H11 T1472 hd64 bf16, forward: 106 us on the mma.sync kernel that such
+// sequences took before.
 // Barrier phases run on counters that continue across items: `g` counts the steps of the CTA (score and P
 // buffers alternate with g), `n` counts its items (Q buffers and accumulators alternate with n).
 #include "attn.cuh"
@@ -84,7 +89,7 @@ struct F1Params {
   void* out;
   float* lse;
   int64_t so_b, so_h, so_t;
-  int H, T;
+  int H, T, hd;   // hd: the real head_dim, at most HD
   int BH, group;  // batch*heads; how many of them are walked together (their K and V share the L2)
   int total;      // items: query tiles x batch*heads
   float scale;
@@ -139,7 +144,7 @@ __device__ __forceinline__ bool f1_item(const F1Params& p, int n, int& qt, int& 
   const int G = (int)gridDim.x, c = (int)blockIdx.x;
   const int v = n * G + ((n & 1) ? (G - 1 - c) : c);
   if (v >= p.total) return false;
-  const int nt = p.T / F1_TILE;
+  const int nt = (p.T + F1_TILE - 1) / F1_TILE;
   if (p.debug & 32) {  // per-slice order (test switch)
     qt = (nt - 1) - v % nt;
     bh = v / nt;
@@ -420,6 +425,7 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
 #pragma unroll
     for (int w = 0; w < F1_NW; ++w) pend_w[w] = 1.f;
     T* pend_row = nullptr;
+    bool pend_live = false, pend_store = false;  // the row exists; it does and so do this warp's output columns
     float* pend_lse = nullptr;
     auto finish_pending = [&]() {
       if (!pend) return;
@@ -450,13 +456,14 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
           if (lane == 0) mbar_arrive(&o_free[0]);
 #pragma unroll
           for (int v8 = 0; v8 < F1_OW / 8; ++v8) {
+            if (!pend_store) break;
             float o8[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) o8[e] = acc[v8 * 8 + e] * inv;
             *reinterpret_cast<uint4*>(pend_row + v8 * 8) = pack8<T>(o8);
           }
         }
-        if (ch == 0) *pend_lse = (pend_m + log2f(pend_l)) * kLn2_1;
+        if (ch == 0 && pend_live) *pend_lse = (pend_m + log2f(pend_l)) * kLn2_1;
       }
       if (prof) atomicAdd(&g_prof_f1[11], (unsigned long long)(clock64() - f0));
     };
@@ -701,6 +708,8 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
       pend_glast = g0 + jlast;
       pend_row = reinterpret_cast<T*>(p.out) + b * p.so_b + h * p.so_h + (int64_t)i * p.so_t + ch * F1_OW;
       pend_lse = p.lse + (int64_t)bh * p.T + i;
+      pend_live = i < p.T;
+      pend_store = pend_live && ch * F1_OW < p.hd;
       pend = true;
       g0 += jlast + 1;
       if (prof) atomicAdd(&g_prof_f1[5], 1ull);
@@ -740,12 +749,12 @@ int encode_tmap_sw128(CUtensorMap* out, const void* base, int dtype, int rank, c
                       const uint64_t* strides_bytes, const uint32_t* box);
 
 template <typename T, int HD>
-static int fwd1_launch(const AttnArgs& a, int dtype, cudaStream_t st) {
+static int fwd1_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   using Cfg = F1Cfg<HD>;
   CUtensorMap tq, tk, tv;
   int rc;
   const uint32_t box[4] = {64, 128, 1, 1};
-  const uint64_t dims[4] = {(uint64_t)HD, (uint64_t)a.T, (uint64_t)a.H, (uint64_t)a.B};
+  const uint64_t dims[4] = {(uint64_t)hd, (uint64_t)a.T, (uint64_t)a.H, (uint64_t)a.B};
   {
     const uint64_t s[3] = {(uint64_t)a.sq.t * 2, (uint64_t)a.sq.h * 2, (uint64_t)a.sq.b * 2};
     if ((rc = encode_tmap_sw128(&tq, a.q, dtype, 4, dims, s, box))) return rc;
@@ -760,11 +769,11 @@ static int fwd1_launch(const AttnArgs& a, int dtype, cudaStream_t st) {
   }
   F1Params p;
   p.out = a.out; p.lse = a.lse; p.so_b = a.so.b; p.so_h = a.so.h; p.so_t = a.so.t;
-  p.H = a.H; p.T = a.T; p.scale = a.scale; p.bias_mode = a.bias_mode; p.slopes = a.slopes;
+  p.H = a.H; p.T = a.T; p.hd = hd; p.scale = a.scale; p.bias_mode = a.bias_mode; p.slopes = a.slopes;
   p.debug = g_attn_debug.load();
   p.BH = a.B * a.H;
   p.group = attn_slices_per_group(a.B * a.H, a.T, HD);
-  p.total = (a.T / F1_TILE) * a.B * a.H;
+  p.total = (int)ceil_div(a.T, F1_TILE) * a.B * a.H;
   const int sms = sm_count();
   if (sms <= 0) return fail(TFB_ERR_LAUNCH, "attention_fwd(tcgen05): cannot read the SM count");
   dim3 grid(p.total < sms ? p.total : sms);  // one persistent CTA per SM
@@ -784,15 +793,13 @@ static int fwd1_launch(const AttnArgs& a, int dtype, cudaStream_t st) {
   return launched("attention_fwd(tcgen05, persistent)");
 }
 
-// The tcgen05 forward takes head_dim 64 / 128, whole 128-query tiles and no dense bias table.
-bool attn_tc05_fwd_eligible(const AttnArgs& a, int hd) {
-  return (hd == 64 || hd == 128) && a.T % 128 == 0 && a.bias_mode != 3;
-}
+// The tcgen05 kernels take everything but a dense bias table.
+bool attn_tc05_fwd_eligible(const AttnArgs& a, int hd) { return hd <= 128 && a.bias_mode != 3; }
 
 int attn_fwd1_tc05(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   TFB_DISPATCH_16(dtype, T, {
-    if (hd == 64) return fwd1_launch<T, 64>(a, dtype, st);
-    return fwd1_launch<T, 128>(a, dtype, st);
+    if (hd <= 64) return fwd1_launch<T, 64>(a, hd, dtype, st);
+    return fwd1_launch<T, 128>(a, hd, dtype, st);
   })
 }
 
