@@ -19,7 +19,7 @@
 // Either operand may be K-major (contraction index contiguous) or MN-major, so the forward
 // product X·W, the input gradient dY·Wᵀ and the weight gradient Xᵀ·dY (contraction over every
 // token of the batch, i.e. the batch reduction fused into the product) are the same kernel.
-#include "gemm_sched.cuh"
+#include "gemm_epi.cuh"
 #include <string.h>
 #include <type_traits>
 
@@ -204,9 +204,11 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
     uint8_t* stage_c = smem + Cfg::OFF_EPI_C + ew * 4096;
     uint8_t* stage_x = smem + Cfg::OFF_EPI_X + ew * 4096;
     // at most one of addend / mask travels through the TMA box; a second one is read directly
-    const bool x_is_addend = p.addend != nullptr;
     const bool use_x = !p.direct && (p.addend != nullptr || p.mask != nullptr);
-    const T* mask_direct = (p.addend != nullptr && p.mask != nullptr) ? reinterpret_cast<const T*>(p.mask) : nullptr;
+    const EpiArgs<T> epi{{reinterpret_cast<T*>(p.C), bias, reinterpret_cast<const T*>(p.addend), reinterpret_cast<const T*>(p.mask),
+                          p.ldc, p.ld_addend, p.ld_mask, p.M, p.N, p.relu},
+                         &tmC, &tmX, stage_c, stage_x, &x_full[ew], use_x, p.addend != nullptr, p.direct != 0,
+                         (p.addend != nullptr && p.mask != nullptr) ? reinterpret_cast<const T*>(p.mask) : nullptr};
     constexpr int STEPS = BN / 64;
     int buf = 0;
     uint32_t acc_phase = 0, x_phase = 0;
@@ -221,7 +223,6 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
       const int m0 = (tile % p.tiles_m) * TB_M;
       const int n0 = (tile / p.tiles_m) * BN;
       const int row0 = m0 + q * 32;       // first row of this warp's slice
-      const int row = row0 + lane;
       const bool contributes = kb0 > 0;                      // a later part of a split tile
       const bool finishes = kb0 == 0 && kb1 < kblocks_all;   // first part of a split tile: owns its epilogue
       if (use_x && !contributes && lane == 0) {  // box of step 0, in flight while the main loop still runs
@@ -234,22 +235,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
       if (contributes) {
         // fp32 partial of this warp's 32 rows into this CTA's slot, then one arrival on the tile's counter
         // slot layout [column group of 4][row]: the 32 lanes of a warp touch 512 contiguous bytes
-        float4* slot = reinterpret_cast<float4*>(p.partials + (int64_t)blockIdx.x * TB_M * BN) + q * 32 + lane;
-#pragma unroll 1
-        for (int st = 0; st < STEPS; ++st) {
-          uint32_t r0[32], r1[32];
-          tmem_ld32(taddr + st * 64, r0);
-          tmem_ld32(taddr + st * 64 + 32, r1);
-          tc_wait_ld();
-          float4* dst = slot + st * 16 * TB_M;
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            __stcg(dst + e * TB_M, make_float4(__uint_as_float(r0[4 * e]), __uint_as_float(r0[4 * e + 1]),
-                                        __uint_as_float(r0[4 * e + 2]), __uint_as_float(r0[4 * e + 3])));
-            __stcg(dst + (8 + e) * TB_M, make_float4(__uint_as_float(r1[4 * e]), __uint_as_float(r1[4 * e + 1]),
-                                            __uint_as_float(r1[4 * e + 2]), __uint_as_float(r1[4 * e + 3])));
-          }
-        }
+        store_partials<STEPS>(taddr, reinterpret_cast<float4*>(p.partials + (int64_t)blockIdx.x * TB_M * BN) + q * 32 + lane, TB_M);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
@@ -274,97 +260,10 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
         __syncwarp();  // lane 0's acquire orders the whole warp's reads of the partial tiles
         if (!fine) { ok = false; break; }
       }
-#pragma unroll 1
-      for (int st = 0; st < STEPS && ok; ++st) {
-        const int col0 = n0 + st * 64;
-        uint32_t r0[32], r1[32];
-        tmem_ld32(taddr + st * 64, r0);
-        tmem_ld32(taddr + st * 64 + 32, r1);
-        tc_wait_ld();
-        for (int c = 1; c <= n_parts; ++c) {
-          // all sixteen loads of this thread's 64 columns are issued before the first add
-          const float4* src = reinterpret_cast<const float4*>(p.partials + (int64_t)(blockIdx.x + c) * TB_M * BN) +
-                              st * 16 * TB_M + q * 32 + lane;
-          float4 v[16];
-#pragma unroll
-          for (int e = 0; e < 16; ++e) v[e] = __ldcg(src + e * TB_M);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            r0[4 * e] = __float_as_uint(__uint_as_float(r0[4 * e]) + v[e].x);
-            r0[4 * e + 1] = __float_as_uint(__uint_as_float(r0[4 * e + 1]) + v[e].y);
-            r0[4 * e + 2] = __float_as_uint(__uint_as_float(r0[4 * e + 2]) + v[e].z);
-            r0[4 * e + 3] = __float_as_uint(__uint_as_float(r0[4 * e + 3]) + v[e].w);
-            r1[4 * e] = __float_as_uint(__uint_as_float(r1[4 * e]) + v[8 + e].x);
-            r1[4 * e + 1] = __float_as_uint(__uint_as_float(r1[4 * e + 1]) + v[8 + e].y);
-            r1[4 * e + 2] = __float_as_uint(__uint_as_float(r1[4 * e + 2]) + v[8 + e].z);
-            r1[4 * e + 3] = __float_as_uint(__uint_as_float(r1[4 * e + 3]) + v[8 + e].w);
-          }
-        }
-        if (p.direct) {
-          const DirectOut<T> out{reinterpret_cast<T*>(p.C), bias, reinterpret_cast<const T*>(p.addend),
-                                 reinterpret_cast<const T*>(p.mask), p.ldc, p.ld_addend, p.ld_mask, p.M, p.N, p.relu};
-          store_direct<T>(out, r0, reinterpret_cast<float*>(stage_c), row0, col0, lane);
-          store_direct<T>(out, r1, reinterpret_cast<float*>(stage_x), row0, col0 + 32, lane);
-          continue;
-        }
-        if (use_x) {
-          if (!mbar_wait(&x_full[ew], x_phase, 0x500 | ew, abort_flag)) { ok = false; break; }
-          x_phase ^= 1;
-        }
-        // the staging box of the previous step must have been read by the TMA unit
-        if (lane == 0) tma_store_wait_read();
-        __syncwarp();
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {  // 16-byte chunks (8 columns) of this thread's row
-          const int col = col0 + v * 8;
-          float f[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v < 4 ? r0[v * 8 + j] : r1[(v - 4) * 8 + j]);
-          if (bias && col < p.N) {
-            if (col + 8 <= p.N) {
-              float b[8];
-              unpack8<T>(__ldg(reinterpret_cast<const uint4*>(bias + col)), b);
-#pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] += b[j];
-            } else {
-              for (int j = 0; j < 8 && col + j < p.N; ++j) f[j] += Num<T>::to_f(bias[col + j]);
-            }
-          }
-          if (p.relu) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = fmaxf(f[j], 0.f);
-          }
-          const uint32_t soff = lane * 128 + ((v ^ (lane & 7)) << 4);
-          if (use_x) {
-            float o[8];
-            unpack8<T>(*reinterpret_cast<const uint4*>(stage_x + soff), o);
-            if (x_is_addend) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] += o[j];
-            } else {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] = o[j] > 0.f ? f[j] : 0.f;
-            }
-          }
-          if (mask_direct && row < p.M) {
-            for (int j = 0; j < 8 && col + j < p.N; ++j)
-              if (!(Num<T>::to_f(mask_direct[(int64_t)row * p.ld_mask + col + j]) > 0.f)) f[j] = 0.f;
-          }
-          *reinterpret_cast<uint4*>(stage_c + soff) = pack8<T>(f);
-        }
-        fence_proxy_async_smem();  // staged output visible to the TMA unit; addend box reads are done
-        __syncwarp();
-        if (lane == 0) {
-          if (col0 < p.N && row0 < p.M) tma_store_2d(&tmC, stage_c, col0, row0);
-          tma_store_commit();
-          if (use_x) {  // next box: the next step of this tile, or nothing (step 0 of the next tile is issued above)
-            if (st + 1 < STEPS) {
-              mbar_expect_tx(&x_full[ew], 4096);
-              tma_load_2d(stage_x, &tmX, col0 + 64, row0, &x_full[ew]);
-            }
-          }
-        }
-      }
+      if (n_parts > 0)
+        add_partials<STEPS>(taddr, reinterpret_cast<const float4*>(p.partials + (int64_t)(blockIdx.x + 1) * TB_M * BN) + q * 32 + lane,
+                            TB_M * BN / 4, n_parts, TB_M);
+      epilogue_tile<T, STEPS>(epi, taddr, row0, n0, lane, x_phase, abort_flag, 0x500 | ew, ok);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[buf]);
