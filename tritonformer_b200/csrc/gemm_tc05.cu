@@ -30,6 +30,9 @@ extern std::atomic<int> g_gemm_free_sms;
 int64_t gemm_pair_tiles(int64_t M, int64_t N);
 bool gemm_needs_direct(const void* c, int64_t ldc, const void* bias, const void* addend, int64_t ld_addend, const void* mask,
                        int64_t ld_mask);
+int gemm_tile_tc05(const TilePlan& plan, const void* a, const void* b, void* c, const void* bias, const void* addend,
+                   int64_t ld_addend, const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K, int64_t a_sm,
+                   int64_t a_sk, int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, cudaStream_t st);
 int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, const void* addend, int64_t ld_addend,
                    const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
                    int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, int sms, void* workspace,
@@ -400,6 +403,12 @@ int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const voi
   const int dbg = g_gemm_debug.load();
   const bool can_split = !(dbg & 1) && workspace != nullptr && aligned16(workspace) &&
                          workspace_bytes >= gemm_tc05_workspace_bytes();
+  if (!(dbg & 128)) {
+    const TilePlan plan = gemm_tile_plan(M, N, K, sms);
+    if (plan.bn)
+      return gemm_tile_tc05(plan, a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk, b_sn, ldc, relu,
+                            dtype, st);
+  }
   // Outputs of at least 256 x 256 that can occupy the pairs of SMs run on CTA pairs (a third less
   // operand traffic per flop): either a 256 x 256 tile for every pair, or a tile for at least every
   // second pair and enough k-blocks to share.
