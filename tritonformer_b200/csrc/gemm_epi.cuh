@@ -113,12 +113,12 @@ __device__ __forceinline__ void finish16(const EpiArgs<T>& a, float (&f)[16], in
 }
 
 // The whole epilogue of a warp's share of a tile.  `ok` turns false when a bounded wait ran out.
-template <typename T, int STEPS>
-__device__ __forceinline__ void epilogue_tile(const EpiArgs<T>& a, uint32_t taddr, int row0, int n0, int lane, uint32_t& x_phase,
+template <typename T>
+__device__ __forceinline__ void epilogue_tile(const EpiArgs<T>& a, int steps, uint32_t taddr, int row0, int n0, int lane, uint32_t& x_phase,
                                               volatile int* abort_flag, int code, bool& ok) {
   if (a.direct) {
 #pragma unroll 1
-    for (int st = 0; st < STEPS * 2; ++st) {
+    for (int st = 0; st < steps * 2; ++st) {
       if (n0 + st * 32 >= a.out.N) break;
       uint32_t r[32];
       tmem_ld32(taddr + st * 32, r);
@@ -128,7 +128,7 @@ __device__ __forceinline__ void epilogue_tile(const EpiArgs<T>& a, uint32_t tadd
     return;
   }
 #pragma unroll 1
-  for (int st = 0; st < STEPS; ++st) {
+  for (int st = 0; st < steps; ++st) {
     const int col0 = n0 + st * 64;
     if (a.use_x) {
       if (!mbar_wait(a.x_full, x_phase, code, abort_flag)) { ok = false; return; }
@@ -171,7 +171,7 @@ __device__ __forceinline__ void epilogue_tile(const EpiArgs<T>& a, uint32_t tadd
     if (lane == 0) {
       if (col0 < a.out.N && row0 < a.out.M) tma_store_2d(a.tm_c, box, col0, row0);
       tma_store_commit();
-      if (a.use_x && st + 1 < STEPS) {  // next box: the next step of this tile (step 0 of the next tile is issued by the caller)
+      if (a.use_x && st + 1 < steps) {  // next box: the next step of this tile (step 0 of the next tile is issued by the caller)
         mbar_expect_tx(a.x_full, 4096);
         tma_load_2d(a.stage_x, a.tm_x, col0 + 64, row0, a.x_full);
       }

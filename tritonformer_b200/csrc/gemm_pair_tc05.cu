@@ -148,6 +148,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       mbar_init(&acc_empty[i], 2 * GP_EPI_WARPS);  // the epilogue warps of both CTAs
     }
     for (int i = 0; i < GP_EPI_WARPS; ++i) mbar_init(&x_full[i], 1);
+    *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -156,20 +157,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     __syncwarp();
     tmem_alloc_pair(tmem_holder, GP_TMEM_COLS);
   }
-  // set-up above is CTA-local and may overlap the previous kernel's tail; global memory comes after
-  grid_dependency_wait();
-  allow_dependents();
-  if (threadIdx.x == 0) *abort_flag = (*(volatile int*)&g_dev_status != 0) ? 1 : 0;
   tc_fence_before();
   __syncthreads();
   // the peer's barriers and tensor memory are ready before anything is signalled across the pair
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  const bool dead = *abort_flag != 0;
+  // set-up above is local to the pair and may overlap the previous kernel's tail; global memory comes after
+  grid_dependency_wait();
+  allow_dependents();
   if (prof && threadIdx.x == 0) pr[1] = (unsigned long long)(clock64() - t_entry);  // set-up
 
-  const int num_tiles = dead ? 0 : p.tiles_m * p.tiles_n;
+  const int num_tiles = p.tiles_m * p.tiles_n;
   const int kblocks = (p.K + GP_K - 1) / GP_K;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
 
@@ -179,7 +178,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      Segments segs(kblocks, num_tiles, p.sk_tiles, num_pairs, pair, dead);
+      Segments segs(kblocks, num_tiles, p.sk_tiles, num_pairs, pair, false);
       int tile, kb0, kb1;
       while (ok && segs.next(tile, kb0, kb1)) {
         const int m0 = (tile % p.tiles_m) * (2 * GP_M) + (int)rank * GP_M;  // this CTA's rows
@@ -213,46 +212,48 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------------- MMA issuer (leader only)
-    if (lane == 0 && leader) {
+    // The whole warp runs the loop and one elected lane issues each instruction: warp-uniform code keeps the operand
+    // descriptors in the uniform registers the tensor core reads them from.
+    if (leader) {
       constexpr uint32_t idesc = instr_desc_f16(2 * GP_M, GP_N, std::is_same<T, __nv_bfloat16>::value ? 1 : 0,
                                                 A_MN ? 1 : 0, B_MN ? 1 : 0);
+      const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0), s0 = smem_u32(smem);
+      const bool prof = p.debug & 64 && lane == 0 && blockIdx.x < 148;
       int stage = 0;
       uint32_t phase = 0;
       int buf = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      Segments segs(kblocks, num_tiles, p.sk_tiles, num_pairs, pair, dead);
+      Segments segs(kblocks, num_tiles, p.sk_tiles, num_pairs, pair, false);
       int tile, kb0, kb1;
       while (ok && segs.next(tile, kb0, kb1)) {
         const long long a0 = clock64();
-        if (!mbar_wait(&acc_empty[buf], acc_phase ^ 1, 0x800 | buf, abort_flag)) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], acc_phase ^ 1, 0x800 | buf, abort_flag))) { ok = false; break; }
         if (prof) pr[4] += (unsigned long long)(clock64() - a0);  // MMA waiting for a free accumulator
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * GP_N;
+        const uint32_t d_tmem = tb + buf * GP_N;
         for (int kb = kb0; kb < kb1; ++kb) {
           const long long f0 = clock64();
-          if (!mbar_wait(&full[stage], phase, 0x900 | stage, abort_flag)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, 0x900 | stage, abort_flag))) { ok = false; break; }
           if (prof) {
             const long long f1 = clock64();
             pr[5] += (unsigned long long)(f1 - f0);  // MMA waiting for operands
             if (pr[6] == 0) pr[6] = (unsigned long long)(f1 - t_entry);  // first operands landed
           }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * GP_STAGE_BYTES);
-          const uint32_t sb = sa + GP_A_BYTES;
+          const uint32_t sa = s0 + stage * GP_STAGE_BYTES, sb = sa + GP_A_BYTES;
+          const uint64_t ad = A_MN ? smem_desc_sw128(sa, 8192, 1024) : smem_desc_sw128(sa, 16, 1024);
+          const uint64_t bd = B_MN ? smem_desc_sw128(sb, 8192, 1024) : smem_desc_sw128(sb, 16, 1024);
+          // K-major: 16 elements = 32 bytes along the swizzled row; MN-major: 16 k-rows of 128 B
 #pragma unroll
           for (int k = 0; k < GP_K / 16; ++k) {
-            const uint64_t ad = A_MN ? smem_desc_sw128(sa + k * 2048, 8192, 1024)
-                                     : smem_desc_sw128(sa + k * 32, 16, 1024);
-            const uint64_t bd = B_MN ? smem_desc_sw128(sb + k * 2048, 8192, 1024)
-                                     : smem_desc_sw128(sb + k * 32, 16, 1024);
-            tc_mma_ss_pair(d_tmem, ad, bd, idesc, ((kb - kb0) | k) ? 1u : 0u);
+            const uint64_t ak = desc_advance(ad, k * (A_MN ? 2048 : 32)), bk = desc_advance(bd, k * (B_MN ? 2048 : 32));
+            if (elect_one()) tc_mma_ss_pair(d_tmem, ak, bk, idesc, ((kb - kb0) | k) ? 1u : 0u);
           }
-          tc_commit_pair(&empty[stage]);  // both producers may refill the slot once these MMAs have read it
+          if (elect_one()) tc_commit_pair(&empty[stage]);  // both producers may refill the slot once these MMAs have read it
           if (++stage == GP_STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        tc_commit_pair(&acc_full[buf]);  // both epilogues
+        if (elect_one()) tc_commit_pair(&acc_full[buf]);  // both epilogues
         buf ^= 1;
         if (buf == 0) acc_phase ^= 1;
       }
@@ -276,11 +277,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     int buf = 0;
     uint32_t acc_phase = 0, x_phase = 0;
     bool ok = true;
+    // an earlier kernel that gave up leaves the status set: then nothing is written, handed over or waited for
+    const bool dead = *(volatile int*)&g_dev_status != 0;
     if (lane == 0) {
       if (!p.direct) tma_prefetch_desc(&tmC);
       if (use_x) tma_prefetch_desc(&tmX);
     }
-    Segments segs(kblocks, num_tiles, p.sk_tiles, num_pairs, pair, dead);
+    Segments segs(kblocks, num_tiles, p.sk_tiles, num_pairs, pair, false);
     int tile, kb0, kb1;
     while (ok && segs.next(tile, kb0, kb1)) {
       const int m0 = (tile % p.tiles_m) * (2 * GP_M) + (int)rank * GP_M;
@@ -288,7 +291,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       const int row0 = m0 + q * 32;
       const bool contributes = kb0 > 0;                  // a later part of a split tile
       const bool finishes = kb0 == 0 && kb1 < kblocks;   // first part of a split tile: owns its epilogue
-      if (use_x && !contributes && lane == 0) {  // box of step 0, in flight while the main loop still runs
+      if (use_x && !contributes && !dead && lane == 0) {  // box of step 0, in flight while the main loop still runs
         mbar_expect_tx(&x_full[ew], 4096);
         tma_load_2d(stage_x, &tmX, n0, row0, &x_full[ew]);
       }
@@ -303,12 +306,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       const int64_t slot_f4 = (int64_t)GP_M * GP_N / 4;  // float4 per slot
       const int my_f4 = half * STEPS * 16 * GP_M + q * 32 + lane;
       if (contributes) {
-        store_partials<STEPS>(taddr, reinterpret_cast<float4*>(p.partials) + (int64_t)blockIdx.x * slot_f4 + my_f4, GP_M);
+        if (!dead) store_partials<STEPS>(taddr, reinterpret_cast<float4*>(p.partials) + (int64_t)blockIdx.x * slot_f4 + my_f4, GP_M);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
           __threadfence();  // the warp's partial rows are visible before the arrival
-          atomicAdd(p.flags + (tile * 2 + (int)rank) * GP_EPI_WARPS + ew, 1);
+          if (!dead) atomicAdd(p.flags + (tile * 2 + (int)rank) * GP_EPI_WARPS + ew, 1);
           mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
         }
         buf ^= 1;
@@ -316,7 +319,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
         continue;
       }
       int n_parts = 0;  // partial tiles to add: the pairs after this one whose ranges reach into the tile
-      if (finishes) {
+      if (finishes && !dead) {
         n_parts = partials_expected(tile, kblocks, p.sk_tiles, num_pairs, pair);
         int* flag = p.flags + (tile * 2 + (int)rank) * GP_EPI_WARPS + ew;
         int fine = 1;
@@ -331,7 +334,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       if (n_parts > 0)  // the same CTA rank of the pairs behind this one wrote the slots
         add_partials<STEPS>(taddr, reinterpret_cast<const float4*>(p.partials) + (int64_t)(blockIdx.x + 2) * slot_f4 + my_f4, 2 * slot_f4,
                             n_parts, GP_M);
-      epilogue_tile<T, STEPS>(epi, taddr, row0, n0, lane, x_phase, abort_flag, 0xb00 | ew, ok);
+      if (!dead) epilogue_tile<T>(epi, STEPS, taddr, row0, n0, lane, x_phase, abort_flag, 0xb00 | ew, ok);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
@@ -339,7 +342,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       buf ^= 1;
       if (buf == 0) acc_phase ^= 1;
     }
-    if (lane == 0) tma_store_wait_all();
+    if (lane == 0) tma_store_wait_read();  // the boxes have been read; the kernel's end completes the writes
     if (prof && ew == 0 && lane == 0) pr[11] = (unsigned long long)(clock64() - t_entry);  // epilogue done
   }
 
@@ -352,7 +355,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
   }
   // neither CTA leaves (or frees tensor memory) while the other may still signal its barriers or
   // have MMAs reading its shared memory
-  cluster_sync_all();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (warp == 1) {
     __syncwarp();
     tc_fence_after();

@@ -12,13 +12,14 @@
 
 namespace tfb {
 
-// Plan of the one-wave kernel (gemm_tile_tc05.cu): tile width (0: not for it), CTAs that share a tile's contraction, and the
+// Plan of the one-wave kernel (gemm_tile_tc05.cu): tile width (0: not for it), workers that share a tile's contraction, and the
 // cycles its model gives the product.
 struct TilePlan {
   int bn, split;
+  bool pair;  // on CTA pairs
   int64_t cycles;
 };
-TilePlan gemm_tile_plan(int64_t M, int64_t N, int64_t K, int sms);
+TilePlan gemm_tile_plan(int64_t M, int64_t N, int64_t K, bool b_mn, int sms);
 
 constexpr int kFlagBytes = 8192;  // head of the workspace: arrival counters, zero between kernels
 

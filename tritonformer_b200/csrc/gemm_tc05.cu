@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
       mbar_init(&acc_empty[i], 4);  // one arrival per epilogue warp
     }
     for (int i = 0; i < 4; ++i) mbar_init(&x_full[i], 1);
+    *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -109,19 +110,15 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
     __syncwarp();
     tmem_alloc(tmem_holder, Cfg::TMEM_COLS);
   }
-  // everything above touches only this CTA's shared memory, TMEM and kernel parameters, so it may
-  // run while the previous kernel of the stream is still finishing; global memory comes after this
-  grid_dependency_wait();
-  allow_dependents();
-  // an earlier kernel that gave up leaves the status set: then this one does nothing
-  if (threadIdx.x == 0) *abort_flag = (*(volatile int*)&g_dev_status != 0) ? 1 : 0;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-
   const int kblocks_all = (p.K + TB_K - 1) / TB_K;
-  const bool dead = *abort_flag != 0;
+  // everything above touches only this CTA's shared memory, TMEM and kernel parameters, so it may
+  // run while the previous kernel of the stream is still finishing; global memory comes after this
+  grid_dependency_wait();
+  allow_dependents();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -129,7 +126,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x, dead);
+      Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x, false);
       int tile, kb0, kb1;
       while (ok && segs.next(tile, kb0, kb1)) {
         const int m0 = (tile % p.tiles_m) * TB_M;
@@ -158,39 +155,39 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
+      // The whole warp runs the loop and one elected lane issues each instruction: warp-uniform code keeps the operand
+      // descriptors in the uniform registers the tensor core reads them from.
       constexpr uint32_t idesc = instr_desc_f16(TB_M, BN, sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1 : 0,
                                                 A_MN ? 1 : 0, B_MN ? 1 : 0);
+      const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0), s0 = smem_u32(smem);
       int stage = 0;
       uint32_t phase = 0;
       int buf = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x, dead);
+      Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x, false);
       int tile, kb0, kb1;
       while (ok && segs.next(tile, kb0, kb1)) {
-        if (!mbar_wait(&acc_empty[buf], acc_phase ^ 1, 0x300 | buf, abort_flag)) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], acc_phase ^ 1, 0x300 | buf, abort_flag))) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * BN;
+        const uint32_t d_tmem = tb + buf * BN;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full[stage], phase, 0x200 | stage, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES);
-          const uint32_t sb = sa + Cfg::A_BYTES;
+          if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, 0x200 | stage, abort_flag))) { ok = false; break; }
+          const uint32_t sa = s0 + stage * Cfg::STAGE_BYTES, sb = sa + Cfg::A_BYTES;
+          const uint64_t ad = A_MN ? smem_desc_sw128(sa, 8192, 1024) : smem_desc_sw128(sa, 16, 1024);
+          const uint64_t bd = B_MN ? smem_desc_sw128(sb, 8192, 1024) : smem_desc_sw128(sb, 16, 1024);
+          // K-major: 16 elements = 32 bytes along the swizzled row; MN-major: 16 k-rows of 128 B
 #pragma unroll
           for (int k = 0; k < TB_K / 16; ++k) {
-            // K-major: 16 elements = 32 bytes along the swizzled row; MN-major: 16 k-rows of 128 B
-            const uint64_t ad = A_MN ? smem_desc_sw128(sa + k * 2048, 8192, 1024)
-                                     : smem_desc_sw128(sa + k * 32, 16, 1024);
-            const uint64_t bd = B_MN ? smem_desc_sw128(sb + k * 2048, 8192, 1024)
-                                     : smem_desc_sw128(sb + k * 32, 16, 1024);
-            tc_mma_ss(d_tmem, ad, bd, idesc, ((kb - kb0) | k) ? 1u : 0u);
+            const uint64_t ak = desc_advance(ad, k * (A_MN ? 2048 : 32)), bk = desc_advance(bd, k * (B_MN ? 2048 : 32));
+            if (elect_one()) tc_mma_ss(d_tmem, ak, bk, idesc, ((kb - kb0) | k) ? 1u : 0u);
           }
-          tc_commit(&empty[stage]);  // slot reusable once these MMAs have read it
+          if (elect_one()) tc_commit(&empty[stage]);  // slot reusable once these MMAs have read it
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        tc_commit(&acc_full[buf]);  // accumulator complete
+        if (elect_one()) tc_commit(&acc_full[buf]);  // accumulator complete
         buf ^= 1;
         if (buf == 0) acc_phase ^= 1;
       }
@@ -216,11 +213,13 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
     int buf = 0;
     uint32_t acc_phase = 0, x_phase = 0;
     bool ok = true;
+    // an earlier kernel that gave up leaves the status set: then nothing is written, handed over or waited for
+    const bool dead = *(volatile int*)&g_dev_status != 0;
     if (lane == 0) {
       if (!p.direct) tma_prefetch_desc(&tmC);
       if (use_x) tma_prefetch_desc(&tmX);
     }
-    Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x, dead);
+    Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x, false);
     int tile, kb0, kb1;
     while (ok && segs.next(tile, kb0, kb1)) {
       const int m0 = (tile % p.tiles_m) * TB_M;
@@ -228,7 +227,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
       const int row0 = m0 + q * 32;       // first row of this warp's slice
       const bool contributes = kb0 > 0;                      // a later part of a split tile
       const bool finishes = kb0 == 0 && kb1 < kblocks_all;   // first part of a split tile: owns its epilogue
-      if (use_x && !contributes && lane == 0) {  // box of step 0, in flight while the main loop still runs
+      if (use_x && !contributes && !dead && lane == 0) {  // box of step 0, in flight while the main loop still runs
         mbar_expect_tx(&x_full[ew], 4096);
         tma_load_2d(stage_x, &tmX, n0, row0, &x_full[ew]);
       }
@@ -238,12 +237,12 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
       if (contributes) {
         // fp32 partial of this warp's 32 rows into this CTA's slot, then one arrival on the tile's counter
         // slot layout [column group of 4][row]: the 32 lanes of a warp touch 512 contiguous bytes
-        store_partials<STEPS>(taddr, reinterpret_cast<float4*>(p.partials + (int64_t)blockIdx.x * TB_M * BN) + q * 32 + lane, TB_M);
+        if (!dead) store_partials<STEPS>(taddr, reinterpret_cast<float4*>(p.partials + (int64_t)blockIdx.x * TB_M * BN) + q * 32 + lane, TB_M);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
           __threadfence();  // the warp's partial rows are visible before the arrival
-          atomicAdd(p.flags + tile * 4 + q, 1);
+          if (!dead) atomicAdd(p.flags + tile * 4 + q, 1);
           mbar_arrive(&acc_empty[buf]);
         }
         buf ^= 1;
@@ -251,7 +250,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
         continue;
       }
       int n_parts = 0;  // partial tiles to add: the CTAs after this one whose ranges reach into the tile
-      if (finishes) {
+      if (finishes && !dead) {
         n_parts = partials_expected(tile, kblocks_all, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x);
         int* flag = p.flags + tile * 4 + q;
         int fine = 1;
@@ -266,14 +265,14 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
       if (n_parts > 0)
         add_partials<STEPS>(taddr, reinterpret_cast<const float4*>(p.partials + (int64_t)(blockIdx.x + 1) * TB_M * BN) + q * 32 + lane,
                             TB_M * BN / 4, n_parts, TB_M);
-      epilogue_tile<T, STEPS>(epi, taddr, row0, n0, lane, x_phase, abort_flag, 0x500 | ew, ok);
+      if (!dead) epilogue_tile<T>(epi, STEPS, taddr, row0, n0, lane, x_phase, abort_flag, 0x500 | ew, ok);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[buf]);
       buf ^= 1;
       if (buf == 0) acc_phase ^= 1;
     }
-    if (lane == 0) tma_store_wait_all();  // global writes of this warp are complete before the CTA exits
+    if (lane == 0) tma_store_wait_read();  // the boxes have been read; the kernel's end completes the writes
   }
 
   // Unwind: every role has left its loop (normally or through a bounded wait).
@@ -404,7 +403,7 @@ int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const voi
   const bool can_split = !(dbg & 1) && workspace != nullptr && aligned16(workspace) &&
                          workspace_bytes >= gemm_tc05_workspace_bytes();
   if (!(dbg & 128)) {
-    const TilePlan plan = gemm_tile_plan(M, N, K, sms);
+    const TilePlan plan = gemm_tile_plan(M, N, K, b_mn, sms);
     if (plan.bn)
       return gemm_tile_tc05(plan, a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk, b_sn, ldc, relu,
                             dtype, st);

@@ -1,35 +1,46 @@
-// tcgen05 GEMM for outputs that one wave of CTAs covers: one 128 x BN tile per cluster of S CTAs, nothing persistent.
+// tcgen05 GEMM for outputs that one wave of CTAs covers: one output tile per cluster, nothing persistent.
 //
 //   C[M,N] = mask(act(A·B + bias) + addend), same contract as gemm_tc05.cu.
 //
-// What bounds these products is the chain of latencies of ONE tile (first operands, last product, epilogue, store), not
-// throughput, so the kernel is built to keep that chain short:
+// What bounds these products is the chain of latencies of ONE tile (first operands, last product, epilogue, store) and, for
+// longer contractions, the operand traffic from the L2 (about 10-15 TB/s for the whole chip), so the kernel is built to
+// keep that chain short and, where it matters, the tile wide:
 //   - set-up and the block barrier come before griddepcontrol.wait, and so does an L2 prefetch of the first B tiles (the
 //     weights, in a forward pass; a prefetch reads nothing that could be stale, L2 is where the writes land);
-//   - the contraction is cut over the S CTAs of a cluster (1, 2, 4 or 8), which exchange fp32 partial tiles through
-//     distributed shared memory: each CTA sums and finishes BN / S columns of the tile, in rank order (the sum does not
+//   - a worker is one CTA (tile 128 x 64 or 128 x 128) or a CTA pair (256 x 128, 192 or 256, tcgen05 with cta_group::2: half
+//     the operand bytes per flop at 256 x 256);
+//   - the contraction is cut over the workers of a cluster (1, 2, 4 or 8), which exchange fp32 partial tiles through
+//     distributed shared memory: each sums and finishes its share of the tile's columns, in rank order (the sum does not
 //     depend on timing).  Through a workspace in global memory with arrival counters the same exchange took 4-5 us;
 //   - short rolled code everywhere (see gemm_epi.cuh).
-// Warps: 0 TMA producer, 1 MMA issuer, 2-5 epilogue.  fp16 512 x 256 x 1024: see the table in the launch rule below.
+// Warps: 0 TMA producer, 1 MMA issuer (of the pair's first CTA), then the epilogue.
 #include "gemm_epi.cuh"
 #include <string.h>
 #include <type_traits>
 
 namespace tfb {
 
-constexpr int GT_M = 128;
+extern std::atomic<int> g_gemm_debug;
+
+constexpr int GT_M = 128;  // rows per CTA
 constexpr int GT_K = 64;
-constexpr int GT_THREADS = 192;
 
 bool gemm_needs_direct(const void* c, int64_t ldc, const void* bias, const void* addend, int64_t ld_addend, const void* mask,
                        int64_t ld_mask);
 
-template <int BN> struct TileCfg {
+template <int BN, bool PAIR, bool B_MN> struct TileCfg {
+  static constexpr int BC = PAIR ? BN / 2 : BN;         // columns of B that a CTA loads
+  static constexpr int CHUNKS = (BC + 63) / 64;         // in 64-column boxes where B is MN-major
   static constexpr int A_BYTES = GT_M * GT_K * 2;
-  static constexpr int B_BYTES = BN * GT_K * 2;
+  static constexpr int B_BYTES = CHUNKS * 8192;
+  static constexpr int LOAD_BYTES = A_BYTES + (B_MN ? B_BYTES : BC * 128);
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int MAX_STAGES = (BN == 64) ? 6 : 5;
-  static constexpr int BOX_BYTES = 8 * 4096;  // two staging boxes per epilogue warp
+  static constexpr int EPI_WARPS = PAIR ? 8 : 4;        // one or two per TMEM lane quarter
+  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+  static constexpr int BOX_BYTES = 2 * EPI_WARPS * 4096;
+  static constexpr int MAX_STAGES = 6;
+  static constexpr int SMEM_LIMIT = 227 * 1024 - 512;
+  static constexpr int TMEM_COLS = BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
 };
 
 struct TileParams {
@@ -39,7 +50,7 @@ struct TileParams {
   int64_t ldc, ld_addend, ld_mask;
   int relu, direct;
   int tiles_m;
-  int split;    // CTAs per cluster, each with a share of K
+  int split;    // workers per cluster, each with a share of K
   int stages;   // ring depth
 };
 
@@ -58,9 +69,35 @@ __device__ __forceinline__ void gt_store_remote(uint32_t addr, const uint32_t* v
                : "memory");
 }
 __device__ __forceinline__ void gt_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// no memory ordering: 1.0-1.3 k cycles less than the release form at this point
+__device__ __forceinline__ void gt_cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void gt_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void gt_cluster_sync() {
+  gt_cluster_arrive();
+  gt_cluster_wait();
+}
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int c0, int c1) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(m), "r"(c0), "r"(c1) : "memory");
+}
+// Pair forms: the load's bytes are counted on the barrier of the pair's first CTA; one commit arrives at both CTAs.
+__device__ __forceinline__ void gt_load_pair(void* dst, const CUtensorMap* m, int c0, int c1, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(m), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void gt_mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void gt_commit_pair(uint64_t* bar, uint16_t ctas) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                   smem_u32(bar)), "h"(ctas)
+               : "memory");
 }
 
 // Eight columns of one row straight to global memory (vectors where the pitches allow them).
@@ -106,29 +143,31 @@ __device__ __forceinline__ void finish_row8(const TileParams& p, float (&f)[8], 
   }
 }
 
-template <typename T, int BN, bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(GT_THREADS) gemm_tile_tc05_kernel(const __grid_constant__ CUtensorMap tmA,
-                                                                    const __grid_constant__ CUtensorMap tmB,
-                                                                    const __grid_constant__ CUtensorMap tmC,
-                                                                    const __grid_constant__ CUtensorMap tmX,
-                                                                    const TileParams p) {
-  using Cfg = TileCfg<BN>;
+template <typename T, int BN, bool PAIR, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
+    gemm_tile_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                          const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmX, const TileParams p) {
+  using Cfg = TileCfg<BN, PAIR, B_MN>;
+  constexpr int WIDTH = PAIR ? 2 : 1;  // CTAs per worker
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t bars[2 * Cfg::MAX_STAGES + 5];
+  __shared__ uint64_t bars[2 * Cfg::MAX_STAGES + 1 + Cfg::EPI_WARPS];
   __shared__ uint32_t tmem_holder;
   __shared__ int abort_word;
   uint64_t *full = bars, *empty = bars + Cfg::MAX_STAGES, *acc_full = bars + 2 * Cfg::MAX_STAGES, *x_full = acc_full + 1;
   volatile int* abort_flag = &abort_word;
-  uint8_t* boxes = smem + p.stages * Cfg::STAGE_BYTES;                  // [4 warps][2] staging boxes; with a split, the
-  float4* recv = reinterpret_cast<float4*>(boxes);                      // partials of the other CTAs instead
+  uint8_t* boxes = smem + p.stages * Cfg::STAGE_BYTES;  // [epilogue warp][2] staging boxes; with a split, the partial sums of
+  float4* recv = reinterpret_cast<float4*>(boxes);      // the other workers instead
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = p.split > 1 ? (int)gt_cluster_rank() : 0;
-  const int tile = (int)blockIdx.x / p.split;
-  const int m0 = (tile % p.tiles_m) * GT_M, n0 = (tile / p.tiles_m) * BN;
+  const int rank = (PAIR || p.split > 1) ? (int)gt_cluster_rank() : 0;
+  const int part = rank / WIDTH, side = rank % WIDTH;  // which worker of the cluster, which CTA of the worker
+  const int tile = (int)blockIdx.x / (WIDTH * p.split);
+  const int m0 = (tile % p.tiles_m) * (GT_M * WIDTH) + side * GT_M;  // this CTA's rows
+  const int n0 = (tile / p.tiles_m) * BN;
+  const int nb = n0 + side * Cfg::BC;                                // this CTA's columns of B
   const int kblocks = (p.K + GT_K - 1) / GT_K;
-  const int kb0 = kblocks * rank / p.split, kb1 = kblocks * (rank + 1) / p.split;
+  const int kb0 = kblocks * part / p.split, kb1 = kblocks * (part + 1) / p.split;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < p.stages; ++i) {
@@ -136,7 +175,7 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tile_tc05_kernel(const __grid
       mbar_init(&empty[i], 1);
     }
     mbar_init(acc_full, 1);
-    for (int i = 0; i < 4; ++i) mbar_init(&x_full[i], 1);
+    for (int i = 0; i < Cfg::EPI_WARPS; ++i) mbar_init(&x_full[i], 1);
     abort_word = 0;
     mbar_fence_init();
   }
@@ -147,23 +186,29 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tile_tc05_kernel(const __grid
     for (int kb = kb0; kb < kb1 && kb < kb0 + p.stages; ++kb) {
       if (B_MN) {
 #pragma unroll
-        for (int i = 0; i < BN / 64; ++i) tma_prefetch_2d(&tmB, n0 + i * 64, kb * GT_K);
+        for (int i = 0; i < Cfg::CHUNKS; ++i) tma_prefetch_2d(&tmB, nb + i * 64, kb * GT_K);
       } else {
-        tma_prefetch_2d(&tmB, kb * GT_K, n0);
+        tma_prefetch_2d(&tmB, kb * GT_K, nb);
       }
     }
   }
   if (warp == 1) {
     __syncwarp();
-    tmem_alloc(&tmem_holder, BN);
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
+                   "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      tmem_alloc(&tmem_holder, Cfg::TMEM_COLS);
+    }
   }
   tc_fence_before();
   __syncthreads();
+  // every CTA of the cluster runs, with its barriers and tensor memory ready, before another one signals or writes to it
+  if (PAIR || p.split > 1) gt_cluster_sync();
   tc_fence_after();
   const uint32_t tmem_base = tmem_holder;
-  // first use of the cluster barrier: every CTA of the cluster runs before another one writes to its shared memory
-  if (p.split > 1) gt_cluster_arrive();
-  // everything above touches only this CTA's shared memory, tensor memory and kernel parameters (and the L2)
+  // everything above touches only this cluster's shared memory, tensor memory and kernel parameters (and the L2)
   grid_dependency_wait();
   allow_dependents();
 
@@ -176,56 +221,76 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tile_tc05_kernel(const __grid
         if (!mbar_wait(&empty[stage], phase ^ 1, 0x100 | stage, abort_flag)) break;
         uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
         uint8_t* sb = sa + Cfg::A_BYTES;
-        mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
         const int k0 = kb * GT_K;
+        if (side == 0) mbar_expect_tx(&full[stage], WIDTH * Cfg::LOAD_BYTES);  // the first CTA's barrier counts both
+        const uint32_t bar = PAIR ? gt_map(smem_u32(&full[stage]), (uint32_t)(rank & ~1)) : 0u;
+        auto load = [&](void* dst, const CUtensorMap* m, int c0, int c1) {
+          if (PAIR) gt_load_pair(dst, m, c0, c1, bar);
+          else tma_load_2d(dst, m, c0, c1, &full[stage]);
+        };
         if (A_MN) {
 #pragma unroll
-          for (int i = 0; i < GT_M / 64; ++i) tma_load_2d(sa + i * 8192, &tmA, m0 + i * 64, k0, &full[stage]);
+          for (int i = 0; i < GT_M / 64; ++i) load(sa + i * 8192, &tmA, m0 + i * 64, k0);
         } else {
-          tma_load_2d(sa, &tmA, k0, m0, &full[stage]);
+          load(sa, &tmA, k0, m0);
         }
         if (B_MN) {
 #pragma unroll
-          for (int i = 0; i < BN / 64; ++i) tma_load_2d(sb + i * 8192, &tmB, n0 + i * 64, k0, &full[stage]);
+          for (int i = 0; i < Cfg::CHUNKS; ++i) load(sb + i * 8192, &tmB, nb + i * 64, k0);
         } else {
-          tma_load_2d(sb, &tmB, k0, n0, &full[stage]);
+          load(sb, &tmB, k0, nb);
         }
         if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    // the whole warp runs the loop and one elected lane issues: the descriptors stay in uniform registers
-    constexpr uint32_t idesc = instr_desc_f16(GT_M, BN, std::is_same<T, __nv_bfloat16>::value ? 1 : 0, A_MN ? 1 : 0, B_MN ? 1 : 0);
-    const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
-    const uint32_t s0 = smem_u32(smem);
-    int stage = 0;
-    uint32_t phase = 0;
-    bool ok = true;
+    if (side == 0) {
+      // the whole warp runs the loop and one elected lane issues: the descriptors stay in uniform registers
+      constexpr uint32_t idesc =
+          instr_desc_f16(GT_M * WIDTH, BN, std::is_same<T, __nv_bfloat16>::value ? 1 : 0, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
+      const uint32_t s0 = smem_u32(smem);
+      const uint16_t ctas = (uint16_t)(3u << (rank & ~1));
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
 #pragma unroll 1
-    for (int kb = kb0; kb < kb1; ++kb) {
-      if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, 0x200 | stage, abort_flag))) { ok = false; break; }
-      tc_fence_after();
-      const uint32_t sa = s0 + stage * Cfg::STAGE_BYTES, sb = sa + Cfg::A_BYTES;
-      const uint64_t ad = A_MN ? smem_desc_sw128(sa, 8192, 1024) : smem_desc_sw128(sa, 16, 1024);
-      const uint64_t bd = B_MN ? smem_desc_sw128(sb, 8192, 1024) : smem_desc_sw128(sb, 16, 1024);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, 0x200 | stage, abort_flag))) { ok = false; break; }
+        const uint32_t sa = s0 + stage * Cfg::STAGE_BYTES, sb = sa + Cfg::A_BYTES;
+        const uint64_t ad = A_MN ? smem_desc_sw128(sa, 8192, 1024) : smem_desc_sw128(sa, 16, 1024);
+        const uint64_t bd = B_MN ? smem_desc_sw128(sb, 8192, 1024) : smem_desc_sw128(sb, 16, 1024);
 #pragma unroll
-      for (int k = 0; k < GT_K / 16; ++k)
-        if (elect_one())
-          tc_mma_ss(tb, desc_advance(ad, k * (A_MN ? 2048 : 32)), desc_advance(bd, k * (B_MN ? 2048 : 32)), idesc,
-                    ((kb - kb0) | k) ? 1u : 0u);
-      if (elect_one()) tc_commit(&empty[stage]);
-      if (++stage == p.stages) { stage = 0; phase ^= 1; }
+        for (int k = 0; k < GT_K / 16; ++k) {
+          const uint64_t ak = desc_advance(ad, k * (A_MN ? 2048 : 32)), bk = desc_advance(bd, k * (B_MN ? 2048 : 32));
+          if (elect_one()) {
+            if (PAIR) gt_mma_pair(tb, ak, bk, idesc, ((kb - kb0) | k) ? 1u : 0u);
+            else tc_mma_ss(tb, ak, bk, idesc, ((kb - kb0) | k) ? 1u : 0u);
+          }
+        }
+        if (elect_one()) {
+          if (PAIR) gt_commit_pair(&empty[stage], ctas);
+          else tc_commit(&empty[stage]);
+        }
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+      if (ok && elect_one()) {
+        if (PAIR) gt_commit_pair(acc_full, ctas);
+        else tc_commit(acc_full);
+      }
     }
-    if (ok && elect_one()) tc_commit(acc_full);
     __syncwarp();
   } else {
-    const int q = warp & 3, ew = warp - 2;
+    constexpr int HALVES = Cfg::EPI_WARPS / 4;  // warps per TMEM lane quarter: they share the columns
+    const int q = warp & 3, ew = warp - 2, half = ew >> 2;
     const int row0 = m0 + q * 32;
     // an earlier kernel that gave up leaves the status set: then nothing is written
     const bool dead = *(volatile int*)&g_dev_status != 0;
     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
     if (p.split == 1) {
+      constexpr int FIRST = (BN / 64 + HALVES - 1) / HALVES;  // 64-column steps of the first half; the rest is the second's
+      const int col = half * FIRST * 64, steps = half == 0 ? FIRST : BN / 64 - FIRST;
       const bool use_x = !p.direct && (p.addend != nullptr || p.mask != nullptr);
       const EpiArgs<T> epi{{reinterpret_cast<T*>(p.C), reinterpret_cast<const T*>(p.bias), reinterpret_cast<const T*>(p.addend),
                             reinterpret_cast<const T*>(p.mask), p.ldc, p.ld_addend, p.ld_mask, p.M, p.N, p.relu},
@@ -233,29 +298,32 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tile_tc05_kernel(const __grid
                            p.direct != 0, (p.addend != nullptr && p.mask != nullptr) ? reinterpret_cast<const T*>(p.mask) : nullptr};
       if (use_x && lane == 0) {  // in flight while the main loop runs
         mbar_expect_tx(&x_full[ew], 4096);
-        tma_load_2d(epi.stage_x, &tmX, n0, row0, &x_full[ew]);
+        tma_load_2d(epi.stage_x, &tmX, n0 + col, row0, &x_full[ew]);
       }
-      bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
-      tc_fence_after();
       uint32_t x_phase = 0;
-      if (ok && !dead) epilogue_tile<T, BN / 64>(epi, taddr, row0, n0, lane, x_phase, abort_flag, 0x500 | ew, ok);
-      if (lane == 0) tma_store_wait_all();
+      bool ok = true;
+      ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
+      tc_fence_after();
+      __syncwarp();
+      if (PAIR) gt_cluster_arrive_relaxed();  // matched by the wait before the exit
+      if (ok && !dead) epilogue_tile<T>(epi, steps, taddr + col, row0, n0 + col, lane, x_phase, abort_flag, 0x500 | ew, ok);
+      if (lane == 0) tma_store_wait_read();  // the boxes have been read; the kernel's end completes the writes
     } else {
       bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
       tc_fence_after();
-      // column slice r of the tile goes to the CTA of rank r: [source][group of 4 columns][row], so that the 32 lanes of a
-      // warp write 512 contiguous bytes
-      const int slice = BN / p.split;
+      // Column slice r of the tile goes to worker r (the CTA of the same side): [source][group of 4 columns][row], so that the
+      // 32 lanes of a warp write 512 contiguous bytes.  Sources are numbered without the receiver itself.  The columns of a
+      // slice are shared by the HALVES warps of a lane quarter.
+      const int slice = BN / p.split, lo = half * (slice / HALVES), hi = lo + slice / HALVES;
       const int trow = q * 32 + lane;
-      __syncwarp();
-      gt_cluster_wait();
       if (ok) {
 #pragma unroll 1
         for (int i = 1; i < p.split; ++i) {
-          const int to = (rank + i) % p.split;
-          const uint32_t dst = gt_map(smem_u32(recv + (rank * (slice / 4)) * GT_M + trow), (uint32_t)to);
+          const int to = (part + i) % p.split;
+          const int slot = part < to ? part : part - 1;
+          const uint32_t dst = gt_map(smem_u32(recv + slot * (slice / 4) * GT_M + trow), (uint32_t)(to * WIDTH + side));
 #pragma unroll 1
-          for (int c = 0; c < slice; c += 8) {
+          for (int c = lo; c < hi; c += 8) {
             uint32_t v[8];
             tmem_ld8(taddr + to * slice + c, v);
             tc_wait_ld();
@@ -265,40 +333,38 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tile_tc05_kernel(const __grid
         }
       }
       __syncwarp();
-      gt_cluster_arrive();
-      gt_cluster_wait();
+      gt_cluster_sync();
       if (ok && !dead && *abort_flag == 0) {
 #pragma unroll 1
-        for (int c = 0; c < slice; c += 8) {
+        for (int c = lo; c < hi; c += 8) {
           uint32_t own[8];
-          tmem_ld8(taddr + rank * slice + c, own);
+          tmem_ld8(taddr + part * slice + c, own);
           tc_wait_ld();
           float f[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) f[j] = 0.f;
 #pragma unroll 1
           for (int r = 0; r < p.split; ++r) {
-            float4 lo, hi;
-            if (r == rank) {
-              lo = make_float4(__uint_as_float(own[0]), __uint_as_float(own[1]), __uint_as_float(own[2]), __uint_as_float(own[3]));
-              hi = make_float4(__uint_as_float(own[4]), __uint_as_float(own[5]), __uint_as_float(own[6]), __uint_as_float(own[7]));
+            float4 a, b;
+            if (r == part) {
+              a = make_float4(__uint_as_float(own[0]), __uint_as_float(own[1]), __uint_as_float(own[2]), __uint_as_float(own[3]));
+              b = make_float4(__uint_as_float(own[4]), __uint_as_float(own[5]), __uint_as_float(own[6]), __uint_as_float(own[7]));
             } else {
-              const float4* src = recv + (r * (slice / 4) + c / 4) * GT_M + trow;
-              lo = src[0];
-              hi = src[GT_M];
+              const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + c / 4) * GT_M + trow;
+              a = src[0];
+              b = src[GT_M];
             }
-            f[0] += lo.x; f[1] += lo.y; f[2] += lo.z; f[3] += lo.w;
-            f[4] += hi.x; f[5] += hi.y; f[6] += hi.z; f[7] += hi.w;
+            f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+            f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
           }
-          finish_row8<T>(p, f, row0 + lane, n0 + rank * slice + c);
+          finish_row8<T>(p, f, row0 + lane, n0 + part * slice + c);
         }
       }
     }
   }
-  if (p.split > 1 && warp < 2) {  // the epilogue warps passed both above
-    gt_cluster_wait();
-    gt_cluster_arrive();
-    gt_cluster_wait();
+  if (warp < 2) {  // the epilogue warps are in the middle of, or past, these
+    if (p.split > 1) gt_cluster_sync();
+    else if (PAIR) gt_cluster_arrive_relaxed();
   }
 
   tc_fence_before();
@@ -307,28 +373,35 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tile_tc05_kernel(const __grid
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
     __syncthreads();
   }
+  // A pair's CTAs leave when both have seen the accumulator complete: nothing reads or signals the other one after that.
+  // (With a split the exchange's barrier already says so.)
+  if (PAIR && p.split == 1) gt_cluster_wait();
   if (warp == 1) {
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc(tmem_base, BN);
+    if (PAIR)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)Cfg::TMEM_COLS) : "memory");
+    else tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
 }
 
 // ------------------------------------------------------------------------------- host side
-template <typename T, int BN, bool A_MN, bool B_MN>
+template <typename T, int BN, bool PAIR, bool A_MN, bool B_MN>
 static int launch_tile(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmX,
-                       const TileParams& p, int tiles, cudaStream_t st) {
-  using Cfg = TileCfg<BN>;
-  auto kern = gemm_tile_tc05_kernel<T, BN, A_MN, B_MN>;
+                       TileParams& p, int tiles, cudaStream_t st) {
+  using Cfg = TileCfg<BN, PAIR, B_MN>;
+  auto kern = gemm_tile_tc05_kernel<T, BN, PAIR, A_MN, B_MN>;
   static std::atomic<uint64_t> attr_done{0};
-  constexpr int most = Cfg::MAX_STAGES * Cfg::STAGE_BYTES + GT_M * BN * 4 + 1024;
-  static_assert(most <= 227 * 1024 - 512, "shared memory");
-  if (int rc0 = ensure_dynamic_smem(kern, most, attr_done, "gemm_tile_tc05")) return rc0;
-  // with a split the partials of split - 1 CTAs, BN / split columns each (slots of all ranks are laid out, one unused)
-  const int tail = p.split > 1 ? GT_M * BN * 4 : Cfg::BOX_BYTES;
+  if (int rc0 = ensure_dynamic_smem(kern, Cfg::SMEM_LIMIT, attr_done, "gemm_tile_tc05")) return rc0;
+  // behind the ring: the staging boxes, or the partial tiles of split - 1 workers, a slice of the columns each
+  const int tail = p.split > 1 ? GT_M * (BN / p.split) * (p.split - 1) * 4 : Cfg::BOX_BYTES;
+  const int room = (Cfg::SMEM_LIMIT - 1024 - tail) / Cfg::STAGE_BYTES;
+  if (p.stages > Cfg::MAX_STAGES) p.stages = Cfg::MAX_STAGES;
+  if (p.stages > room) p.stages = room;
+  const int workers = tiles * p.split, cluster = p.split * (PAIR ? 2 : 1);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tiles * p.split));
-  cfg.blockDim = dim3(GT_THREADS);
+  cfg.gridDim = dim3((unsigned)(workers * (PAIR ? 2 : 1)));
+  cfg.blockDim = dim3(Cfg::THREADS);
   cfg.dynamicSmemBytes = (size_t)(p.stages * Cfg::STAGE_BYTES + tail + 1024);
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -337,41 +410,85 @@ static int launch_tile(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n++].val.programmaticStreamSerializationAllowed = 1;
   }
-  if (p.split > 1) {
+  if (cluster > 1) {
     attr[n].id = cudaLaunchAttributeClusterDimension;
-    attr[n].val.clusterDim.x = (unsigned)p.split;
+    attr[n].val.clusterDim.x = (unsigned)cluster;
     attr[n].val.clusterDim.y = 1;
     attr[n++].val.clusterDim.z = 1;
   }
   cfg.attrs = attr;
   cfg.numAttrs = n;
-  (void)cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, tmX, p);
+  (void)cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, tmX, static_cast<const TileParams&>(p));
   return launched("gemm_tile_tc05");
 }
 
-template <typename T, int BN>
+template <typename T, int BN, bool PAIR>
 static int dispatch_tile(bool a_mn, bool b_mn, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
-                         const CUtensorMap& tmX, const TileParams& p, int tiles, cudaStream_t st) {
-  if (a_mn && b_mn) return launch_tile<T, BN, true, true>(tmA, tmB, tmC, tmX, p, tiles, st);
-  if (a_mn) return launch_tile<T, BN, true, false>(tmA, tmB, tmC, tmX, p, tiles, st);
-  if (b_mn) return launch_tile<T, BN, false, true>(tmA, tmB, tmC, tmX, p, tiles, st);
-  return launch_tile<T, BN, false, false>(tmA, tmB, tmC, tmX, p, tiles, st);
+                         const CUtensorMap& tmX, TileParams& p, int tiles, cudaStream_t st) {
+  if (a_mn && b_mn) return launch_tile<T, BN, PAIR, true, true>(tmA, tmB, tmC, tmX, p, tiles, st);
+  if (a_mn) return launch_tile<T, BN, PAIR, true, false>(tmA, tmB, tmC, tmX, p, tiles, st);
+  if (b_mn) return launch_tile<T, BN, PAIR, false, true>(tmA, tmB, tmC, tmX, p, tiles, st);
+  return launch_tile<T, BN, PAIR, false, false>(tmA, tmB, tmC, tmX, p, tiles, st);
 }
 
-// The tile kernel's plan for a product: BN and the split that the model below puts lowest, or bn = 0 when the output needs
-// more than one wave of CTAs.  Cycles of a CTA: a fixed chain of latencies, its k-blocks at the rate shared memory feeds the
-// tensor core (24 and 32 KB per k-block at 128 B/clk), the exchange of a split.
-TilePlan gemm_tile_plan(int64_t M, int64_t N, int64_t K, int sms) {
-  TilePlan best{0, 0, 0};
-  const int64_t tm = ceil_div(M, GT_M), kblocks = ceil_div(K, GT_K);
-  for (int bn = 64; bn <= 128; bn *= 2) {
-    const int64_t tiles = tm * ceil_div(N, bn);
-    if (tiles > sms) continue;
-    for (int split = 1; split <= 8; split *= 2) {
-      // clusters of 4 and 8 CTAs do not fill every GPC
-      if (tiles * split > (split <= 2 ? sms : split == 4 ? sms * 15 / 16 : sms * 7 / 8) || kblocks < split) break;
-      const int64_t cycles = 3000 + ceil_div(kblocks, split) * (bn == 64 ? 200 : 270) + (split > 1 ? 1000 + 100 * split : bn == 128 ? 600 : 0);
-      if (best.bn == 0 || cycles < best.cycles) best = TilePlan{bn, split, cycles};
+// Cycles of the one-wave kernel for a plan: a fixed chain of latencies, the k-blocks of a CTA, the exchange of a split.  What
+// a k-block costs is mostly what an SM can take in from the L2, about 62 bytes a cycle (measured over tiles, splits and
+// contraction lengths: 24 KB 400-430 cycles, 32 KB 480-540, whatever the tensor core would need).
+static int64_t tile_cycles(int bn, bool pair, int split, bool b_mn, int64_t kblocks) {
+  const int64_t bytes = 16384 + (pair ? (b_mn ? (bn / 2 + 63) / 64 * 8192 : bn / 2 * 128) : bn * 128);
+  const int64_t mma = pair ? bn * 2 : bn * 2 + 60;
+  const int64_t per = bytes / 60 > mma ? bytes / 60 : mma;
+  return 5000 + (pair ? 1000 : 0) + bn * 8 + ceil_div(kblocks, split) * per + (split > 1 ? 1800 + 200 * split + bn * 8 : 0);
+}
+
+// CTAs that run at the same time in clusters of `cluster`, one CTA per SM (clusters do not fill every GPC: 16 clusters of 8
+// took two waves here).  Asked from the runtime once per device and size.
+static int cluster_room(int cluster, int sms) {
+  if (cluster == 1) return sms;
+  static std::atomic<int> known[64][9] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  int room = known[dev][cluster].load(std::memory_order_relaxed);
+  if (room == 0) {
+    auto kern = gemm_tile_tc05_kernel<__half, 128, true, false, false>;
+    constexpr int smem = 160 * 1024;  // more than half of an SM's
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TileCfg<128, true, false>::SMEM_LIMIT);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)cluster * 64);
+    cfg.blockDim = dim3(TileCfg<128, true, false>::THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+      (void)cudaGetLastError();
+      n = sms * 3 / 4 / cluster;
+    }
+    room = n * cluster;
+    known[dev][cluster].store(room, std::memory_order_relaxed);
+  }
+  return room < sms ? room : sms;
+}
+
+TilePlan gemm_tile_plan(int64_t M, int64_t N, int64_t K, bool b_mn, int sms) {
+  TilePlan best{0, 0, false, 0};
+  const int64_t kblocks = ceil_div(K, GT_K);
+  const int forced = (g_gemm_debug.load() >> 16) & 0xfff;  // tuning switch: 1 + (bn / 64) * 2 + pair, 16 * split
+  for (int pair = 0; pair <= 1; ++pair) {
+    if (pair && (M <= GT_M || N < 64)) break;
+    for (int bn = pair ? 128 : 64; bn <= (pair ? 256 : 128); bn += 64) {
+      const int64_t tiles = ceil_div(M, pair ? 2 * GT_M : GT_M) * ceil_div(N, bn);
+      for (int split = 1; split <= (pair ? 4 : 8); split *= 2) {
+        const int cluster = split * (pair ? 2 : 1);
+        if (kblocks < split || tiles * cluster > cluster_room(cluster, sms)) break;
+        if (forced && forced != 1 + (bn / 64) * 2 + pair + 16 * split) continue;
+        const int64_t cycles = tile_cycles(bn, pair != 0, split, b_mn, kblocks);
+        if (best.bn == 0 || cycles < best.cycles) best = TilePlan{bn, split, pair != 0, cycles};
+      }
     }
   }
   return best;
@@ -403,22 +520,24 @@ int gemm_tile_tc05(const TilePlan& plan, const void* a, const void* b, void* c, 
     else      { dims[0] = (uint64_t)K; dims[1] = (uint64_t)M; str[0] = (uint64_t)a_sm * 2; box[0] = GT_K; box[1] = GT_M; }
     if ((rc = encode_tmap_sw128(&tmA, a, dtype, 2, dims, str, box))) return rc;
     if (b_mn) { dims[0] = (uint64_t)N; dims[1] = (uint64_t)K; str[0] = (uint64_t)b_sk * 2; box[0] = 64; box[1] = GT_K; }
-    else      { dims[0] = (uint64_t)K; dims[1] = (uint64_t)N; str[0] = (uint64_t)b_sn * 2; box[0] = GT_K; box[1] = (uint32_t)plan.bn; }
+    else      { dims[0] = (uint64_t)K; dims[1] = (uint64_t)N; str[0] = (uint64_t)b_sn * 2; box[0] = GT_K; box[1] = (uint32_t)(plan.pair ? plan.bn / 2 : plan.bn); }
     if ((rc = encode_tmap_sw128(&tmB, b, dtype, 2, dims, str, box))) return rc;
   }
   TileParams p;
   p.C = c; p.bias = bias; p.addend = addend; p.mask = mask;
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.ldc = ldc; p.ld_addend = ld_addend; p.ld_mask = ld_mask;
   p.relu = relu; p.direct = direct;
-  p.tiles_m = (int)ceil_div(M, GT_M);
+  p.tiles_m = (int)ceil_div(M, plan.pair ? 2 * GT_M : GT_M);
   p.split = plan.split;
   const int64_t per_cta = ceil_div(ceil_div(K, GT_K), plan.split);
   const int tiles = p.tiles_m * (int)ceil_div(N, plan.bn);
-  const int most = plan.bn == 64 ? TileCfg<64>::MAX_STAGES : TileCfg<128>::MAX_STAGES;
-  p.stages = (int)(per_cta < most ? per_cta : most);
+  p.stages = (int)(per_cta < 64 ? per_cta : 64);  // cut to the shared memory there is at launch
   TFB_DISPATCH_16(dtype, T, {
-    if (plan.bn == 64) return dispatch_tile<T, 64>(a_mn, b_mn, tmA, tmB, tmC, tmX, p, tiles, st);
-    return dispatch_tile<T, 128>(a_mn, b_mn, tmA, tmB, tmC, tmX, p, tiles, st);
+    if (!plan.pair && plan.bn == 64) return dispatch_tile<T, 64, false>(a_mn, b_mn, tmA, tmB, tmC, tmX, p, tiles, st);
+    if (!plan.pair) return dispatch_tile<T, 128, false>(a_mn, b_mn, tmA, tmB, tmC, tmX, p, tiles, st);
+    if (plan.bn == 128) return dispatch_tile<T, 128, true>(a_mn, b_mn, tmA, tmB, tmC, tmX, p, tiles, st);
+    if (plan.bn == 192) return dispatch_tile<T, 192, true>(a_mn, b_mn, tmA, tmB, tmC, tmX, p, tiles, st);
+    return dispatch_tile<T, 256, true>(a_mn, b_mn, tmA, tmB, tmC, tmX, p, tiles, st);
   })
 }
 
