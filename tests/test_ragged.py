@@ -87,3 +87,22 @@ def test_lm_loss_of_an_odd_vocabulary(cols, dtype):
     # exp2f of an fp32 difference: a few 1e-6 of the probability, then one rounding (or half a subnormal step)
     err = (logits.grad.double() - ref.grad).abs()
     assert (err <= (EPS[dtype] + 1e-5) * ref.grad.abs() + 1e-6 + 2.0 ** -25).all()
+
+
+@pytest.mark.parametrize("table_dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dtype,hd,t", [(torch.float16, 64, 192), (torch.bfloat16, 128, 2560)])
+def test_alibi_table_penalty_is_the_tables_entry(dtype, hd, t, table_dtype):
+    """Queries and keys of zero leave the scores to the bias alone, so an entry that is rounded otherwise than the table's
+    shows: the fp16 distances above 2048 and the bf16 ones above 256 are themselves rounded."""
+    from tritonformer_b200.attention import BiasedCausalAttention
+    from tritonformer_b200.transformer import generate_alibi_mask
+    h = 6  # slopes that are no powers of two among them
+    table = generate_alibi_mask(t, h, device="cuda", dtype=table_dtype)[0]
+    q = torch.zeros(1, h, t, hd, device="cuda", dtype=dtype)
+    v = (torch.rand(1, h, t, hd, device="cuda") * 2 - 1).to(dtype)
+    out = BiasedCausalAttention.apply(q, q, v, table)
+    want = torch.softmax(table.double(), -1) @ v[0].double()
+    # |v| <= 1 and the probabilities sum to one: half a unit of the 16-bit type for the probabilities, half for the output,
+    # and 7.5e-5 for the cubic exponential (twice: numerator and row sum)
+    tol = (2.0 ** -10 if dtype is torch.float16 else 2.0 ** -8) + 2e-4
+    assert (out[0].double() - want).abs().max().item() < tol

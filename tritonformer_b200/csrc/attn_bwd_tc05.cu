@@ -431,17 +431,21 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
               const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
               float pe[4], de[4];
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
+              for (int k = 0; k < 4; k += 2) {
                 const int e = e4 * 4 + k;
-                float x = fmaf(__uint_as_float(sv_[c & 1][e]), c2, -lv[k]);
+                float x0 = fmaf(__uint_as_float(sv_[c & 1][e]), c2, -lv[k]), x1 = fmaf(__uint_as_float(sv_[c & 1][e + 1]), c2, -lv[k + 1]);
                 if (plain) {
-                  pe[k] = ex2_approx_b(x);  // (one exponential in four on the FMA pipe, as in the forward, changed nothing here)
+                  pe[k] = ex2_approx_b(x0);  // (one exponential in four on the FMA pipe, as in the forward, changed nothing here)
+                  pe[k + 1] = ex2_approx_b(x1);
                 } else {
                   const int i = i0 + col0 + e;
-                  x = alibi.sub_from(x, d0 + (float)e);  // a key above the diagonal (negative distance) is masked below
-                  pe[k] = (j > i) ? 0.f : ex2_approx_b(x);
+                  // a key above the diagonal (negative distance) is masked below
+                  f2_unpack(alibi.sub_pair(f2_pack(x0, x1), d0 + (float)e, d0 + (float)(e + 1)), x0, x1);
+                  pe[k] = (j > i) ? 0.f : ex2_approx_b(x0);
+                  pe[k + 1] = (j > i + 1) ? 0.f : ex2_approx_b(x1);
                 }
                 de[k] = pe[k] * (__uint_as_float(dv_[c & 1][e]) - dl[k]);
+                de[k + 1] = pe[k + 1] * (__uint_as_float(dv_[c & 1][e + 1]) - dl[k + 1]);
               }
               pk[c * 4 + e4 * 2] = pack2<T>(pe[0], pe[1]);
               pk[c * 4 + e4 * 2 + 1] = pack2<T>(pe[2], pe[3]);

@@ -521,11 +521,7 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
             for (int e2 = 0; e2 < 16; ++e2) {  // pairs of keys
               uint64_t xp = f2_fma(f2_pack(__uint_as_float(v[2 * e2]), __uint_as_float(v[2 * e2 + 1])), c2p, negmp);
               float p0, p1;
-              if (BIAS) {
-                float x0, x1;
-                f2_unpack(xp, x0, x1);
-                xp = f2_pack(alibi.sub_from(x0, d0 - (float)(2 * e2)), alibi.sub_from(x1, d0 - (float)(2 * e2 + 1)));
-              }
+              if (BIAS) xp = alibi.sub_pair(xp, d0 - (float)(2 * e2), d0 - (float)(2 * e2 + 1));
               if ((e2 & 3) == 3) {  // one pair in four on the FMA pipe
                 ex2_fma2(xp, p0, p1);
               } else {
@@ -582,10 +578,14 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
               } else {
                 const float d0 = (float)(i - (kbase + c * 32));
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                  float x = alibi.sub_from(__uint_as_float(v[e]) * c2, d0 - (float)e);  // masked keys: overwritten
-                  if (e >= cnt[c]) x = -INFINITY;
-                  mx4[e & 3] = fmaxf(mx4[e & 3], x);
+                for (int e = 0; e < 32; e += 2) {
+                  float x0, x1;  // masked keys: overwritten
+                  f2_unpack(alibi.sub_pair(f2_pack(__uint_as_float(v[e]) * c2, __uint_as_float(v[e + 1]) * c2), d0 - (float)e,
+                                           d0 - (float)(e + 1)), x0, x1);
+                  if (e >= cnt[c]) x0 = -INFINITY;
+                  if (e + 1 >= cnt[c]) x1 = -INFINITY;
+                  mx4[e & 3] = fmaxf(mx4[e & 3], x0);
+                  mx4[(e + 1) & 3] = fmaxf(mx4[(e + 1) & 3], x1);
                 }
               }
             }
@@ -652,9 +652,12 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
                 } else {
                   const float d0 = (float)(i - (kbase + c * 32));
 #pragma unroll
-                  for (int e = 0; e < 32; ++e) {
-                    const float x = alibi.sub_from(fmaf(__uint_as_float(v[e]), c2, neg_m), d0 - (float)e);
-                    e_[e] = (e >= cnt[c]) ? 0.f : ex2_mufu(x);
+                  for (int e = 0; e < 32; e += 2) {
+                    float x0, x1;
+                    f2_unpack(alibi.sub_pair(f2_pack(fmaf(__uint_as_float(v[e]), c2, neg_m), fmaf(__uint_as_float(v[e + 1]), c2, neg_m)),
+                                             d0 - (float)e, d0 - (float)(e + 1)), x0, x1);
+                    e_[e] = (e >= cnt[c]) ? 0.f : ex2_mufu(x0);
+                    e_[e + 1] = (e + 1 >= cnt[c]) ? 0.f : ex2_mufu(x1);
                   }
                 }
 #pragma unroll
