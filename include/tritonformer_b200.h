@@ -277,6 +277,9 @@ int tfb_attention_bwd(const void* q, const void* k, const void* v, const void* o
  *
  * tfb_grad_check: sets *found_inf to 1 if any of the n gradients is inf or nan (leaves it alone otherwise).   */
 int tfb_grad_check(const void* grad, int64_t n, int dtype, int* found_inf, void* stream);
+/* The same over `count` buckets in one launch (host arrays of pointers and sizes).                             */
+int tfb_grad_check_many(const void* const* grads, const int64_t* n, int count, int dtype, int* found_inf,
+                        void* stream);
 /* tfb_adamw_step: AdamW on n elements with fp32 master weights (torch.optim.AdamW's arithmetic, operation by
  * operation): g = grad * *inv_scale; master *= 1 - lr*weight_decay; exp_avg, exp_avg_sq updated; master -=
  * lr / (1 - beta1^t) * exp_avg / (sqrt(exp_avg_sq) / sqrt(1 - beta2^t) + eps) with t = *steps_taken + 1;
@@ -287,6 +290,11 @@ int tfb_adamw_step(const void* grad, void* param, float* master, float* exp_avg,
                    int64_t n, int dtype, const float* inv_scale, const int* found_inf,
                    const float* steps_taken, double lr, double beta1, double beta2, double eps,
                    double weight_decay, void* stream);
+/* The same over `count` buckets in one launch (host arrays of pointers and sizes).                             */
+int tfb_adamw_step_many(const void* const* grads, void* const* params, float* const* masters,
+                        float* const* exp_avgs, float* const* exp_avg_sqs, const int64_t* n, int count, int dtype,
+                        const float* inv_scale, const int* found_inf, const float* steps_taken, double lr,
+                        double beta1, double beta2, double eps, double weight_decay, void* stream);
 /* tfb_loss_scale_update: after the step kernels of every bucket.  state4 (device) = {loss scale, 1 / scale,
  * good steps since the scale last changed, optimizer steps taken}.  If *found_inf: scale *= backoff, the
  * good-step count restarts; else the step counter advances and after `interval` good steps scale *= growth

@@ -136,3 +136,44 @@ def test_fused_adamw_trains_the_model_like_torch_adamw():
             assert torch.equal(p.detach().float().cpu(), s.detach().half().float()) or \
                 (p.detach().float().cpu() - s.detach()).abs().max().item() <= 2e-3 * s.detach().abs().max().item(), n
     assert float(scaler.state[3].item()) == 3.0
+
+
+@pytest.mark.parametrize("dtype,code", [(torch.float16, 0), (torch.bfloat16, 1)])
+def test_many_buckets_in_one_launch_match_one_at_a_time(dtype, code):
+    """More buckets than a launch takes, empty ones and the edges of vectors and chunks among them: bit for bit what a call
+    per bucket gives, and a value that is not finite is found wherever it is."""
+    import ctypes
+    dev = torch.device("cuda", 0)
+    sizes = [1, 7, 8, 9, 0, 2047, 2048, 2049, 8191, 8192, 8200, 100003] * 6
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    g = [torch.randn(n, device=dev, generator=gen).to(dtype) for n in sizes]
+    w = [torch.randn(n, device=dev, generator=gen) for n in sizes]
+    m = [torch.randn(n, device=dev, generator=gen) for n in sizes]
+    v = [torch.rand(n, device=dev, generator=gen) for n in sizes]
+    sides = []
+    for _ in range(2):
+        sides.append([[t.clone() for t in x] for x in ([a.to(dtype) for a in w], w, m, v)])
+    hyper = (1e-3, 0.9, 0.999, 1e-8, 0.1)
+    one, many = sides
+    for i, n in enumerate(sizes):
+        L.check(L.lib.tfb_adamw_step(g[i].data_ptr(), *(x[i].data_ptr() for x in one), n, code, None, None, None, *hyper,
+                                     L.stream_ptr(dev)))
+    count = len(sizes)
+    ptrs = lambda x: (ctypes.c_void_p * count)(*(t.data_ptr() for t in x))
+    ns = (ctypes.c_int64 * count)(*sizes)
+    L.check(L.lib.tfb_adamw_step_many(ptrs(g), *(ptrs(x) for x in many), ns, count, code, None, None, None, *hyper,
+                                      L.stream_ptr(dev)))
+    for a, b in zip(one, many):
+        for s, t in zip(a, b):
+            assert torch.equal(s, t)
+    found = torch.zeros(1, device=dev, dtype=torch.int32)
+    check = lambda: L.check(L.lib.tfb_grad_check_many(ptrs(g), ns, count, code, found.data_ptr(), L.stream_ptr(dev)))
+    check()
+    assert found.item() == 0
+    for i, n in enumerate(sizes[:12]):
+        for at in {0, n // 2, n - 1} if n else ():
+            keep, g[i + 60][at] = g[i + 60][at].clone(), float("inf")
+            check()
+            assert found.item() == 1, (i, at)
+            found.zero_()
+            g[i + 60][at] = keep

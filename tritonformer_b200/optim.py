@@ -4,11 +4,13 @@ the device.
 The reference ships no optimizer (its README trains with one); this is the step that follows forward+backward
 in a training loop.  `FusedAdamW` works on `dp.GradBuckets`: every bucket of 16-bit gradients gets a flat
 16-bit parameter buffer of the same layout (the model's parameters become views of it, names and values
-unchanged), and flat fp32 buffers for the master weights and the two moments.  A step is, per bucket, one pass
+unchanged), and flat fp32 buffers for the master weights and the two moments.  A step is one pass over all buckets
 that looks for inf / nan and one pass that updates; whether the step is taken, the loss scale and the step
 count live in device memory, so nothing synchronises the host and the step can be captured in a CUDA graph
 together with forward, backward and the gradient all-reduce.
 """
+import ctypes
+
 import torch
 
 from . import _lib
@@ -76,14 +78,19 @@ class FusedAdamW:
         device, if any gradient of any bucket is inf or nan."""
         s = self.scaler
         stream = _lib.stream_ptr(self.buckets.buckets[0].device)
-        for g in self.buckets.buckets:
-            _lib.check(_lib.lib.tfb_grad_check(g.data_ptr(), g.numel(), _lib.dtype_code(g.dtype),
-                                               s.found_inf.data_ptr(), stream))
-        for g, p16, w, m, v in zip(self.buckets.buckets, self.params16, self.master, self.exp_avg, self.exp_avg_sq):
-            _lib.check(_lib.lib.tfb_adamw_step(g.data_ptr(), p16.data_ptr(), w.data_ptr(), m.data_ptr(), v.data_ptr(),
-                                               g.numel(), _lib.dtype_code(g.dtype), s.inv_scale.data_ptr(),
-                                               s.found_inf.data_ptr(), s.steps_taken.data_ptr(), self.lr,
-                                               self.betas[0], self.betas[1], self.eps, self.weight_decay, stream))
+        lists = [self.buckets.buckets, self.params16, self.master, self.exp_avg, self.exp_avg_sq]
+        groups = []  # buckets of one dtype go into one launch
+        for dtype in dict.fromkeys(g.dtype for g in self.buckets.buckets):
+            at = [i for i, g in enumerate(self.buckets.buckets) if g.dtype is dtype]
+            ptrs = [(ctypes.c_void_p * len(at))(*(x[i].data_ptr() for i in at)) for x in lists]
+            sizes = (ctypes.c_int64 * len(at))(*(self.buckets.buckets[i].numel() for i in at))
+            groups.append((ptrs, sizes, len(at), _lib.dtype_code(dtype)))
+        for ptrs, sizes, count, code in groups:
+            _lib.check(_lib.lib.tfb_grad_check_many(ptrs[0], sizes, count, code, s.found_inf.data_ptr(), stream))
+        for ptrs, sizes, count, code in groups:
+            _lib.check(_lib.lib.tfb_adamw_step_many(*ptrs, sizes, count, code, s.inv_scale.data_ptr(), s.found_inf.data_ptr(),
+                                                    s.steps_taken.data_ptr(), self.lr, self.betas[0], self.betas[1], self.eps,
+                                                    self.weight_decay, stream))
         s.update()
 
     def bytes_per_step(self):
