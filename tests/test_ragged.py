@@ -106,3 +106,22 @@ def test_alibi_table_penalty_is_the_tables_entry(dtype, hd, t, table_dtype):
     # and 7.5e-5 for the cubic exponential (twice: numerator and row sum)
     tol = (2.0 ** -10 if dtype is torch.float16 else 2.0 ** -8) + 2e-4
     assert (out[0].double() - want).abs().max().item() < tol
+
+
+@pytest.mark.parametrize("heads,t,hd", [(300, 64, 64), (333, 128, 128), (333, 128, 32), (150, 192, 64), (120, 384, 128), (90, 640, 64)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_attention_backward_with_several_items_per_sm(heads, t, hd, dtype):
+    """More (key tile, head) items than SMs, walks of one tile among them: a CTA goes on to the blocks that have not started."""
+    from tritonformer_b200.attention import CausalAttention
+    torch.manual_seed(heads + t)
+    q, k, v = (torch.randn(1, heads, t, hd, device="cuda").to(dtype).requires_grad_() for _ in range(3))
+    g = torch.randn(1, heads, t, hd, device="cuda").to(dtype)
+    got = torch.autograd.grad(CausalAttention.apply(q, k, v), (q, k, v), g)
+    qd, kd, vd = (x.detach().double().requires_grad_() for x in (q, k, v))
+    s = (qd @ kd.transpose(-1, -2)) / hd ** 0.5
+    s = s.masked_fill(~torch.ones(t, t, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    want = torch.autograd.grad(torch.softmax(s, -1) @ vd, (qd, kd, vd), g.double())
+    for a, b in zip(got, want):
+        # per head, in the 2-norm: P, dS, the saved output (in delta) and the gradient itself are each rounded to 16 bits
+        err = (a.double() - b).flatten(2).norm(dim=2) / b.flatten(2).norm(dim=2)
+        assert err.max().item() < 4 * EPS[dtype]

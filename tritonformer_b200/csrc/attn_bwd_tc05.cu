@@ -1,6 +1,14 @@
 // Causal flash attention backward on tcgen05 / TMEM for sm_100a (head_dim 32, 64 or 128).
 //
-// One CTA per (128-key tile, batch*head); it walks the query tiles at or below the diagonal.
+// An item is a (128-key tile, batch*head); a CTA walks its query tiles at or below the diagonal.  The grid has one block per
+// item, but a CTA that is nearly done with its item takes over a block that has not been launched yet (cluster launch
+// control: that launch is cancelled and its block index handed over), so tensor memory, barriers and the ring stay set up
+// from item to item.  With a fresh CTA per item, 8.9 k of the 53 k cycles of an average item at T 2048 were spent outside the
+// walk.  A list dealt out in advance would do the same, but not beside the weight-gradient products of another stream, which
+// hold some of the SMs.  At head_dim 64, K and V are doubled as well, so that the next item's scores run ahead like those of
+// any next tile, and an item's dV and dK are written behind the arithmetic of the next item's first tile.
+// Backward with its two small passes, fp16: B4 H16 T2048 hd64 208 -> 194 us, B1 H12 T4096 hd128 265 -> 255, B2 H16 T2048
+// hd128 202 -> 188.
 // Everything is computed transposed (rows = keys) so that the per-query statistics (log-sum-exp,
 // delta) are per-column constants and no row reductions are needed:
 //   Sᵀ  = K Q_iᵀ                 dPᵀ = V dO_iᵀ                      (tensor cores -> TMEM)
@@ -48,20 +56,23 @@ template <int HD> struct FbCfg {
   // there, so its shared-memory buffer is not allocated and the third stage takes its place.  One stage at
   // head_dim 128 (shared memory).
   static constexpr int QSTAGES = (HD == 64) ? 3 : 1;
-  static constexpr int OFF_K = 0;
+  // K and V of two items at head_dim 64: the next item's scores run ahead of the current item's last products like those of
+  // any next tile.  (With one, the walk stood still for 7.9 k cycles from item to item.)
+  static constexpr int KVSTAGES = (HD == 64) ? 2 : 1;
+  static constexpr int OFF_K = 0;                                    // [KVSTAGES][K, V]
   static constexpr int OFF_V = TILE_BYTES;
-  static constexpr int OFF_Q = 2 * TILE_BYTES;                       // [QSTAGES]
+  static constexpr int OFF_Q = KVSTAGES * 2 * TILE_BYTES;            // [QSTAGES]
   static constexpr int OFF_DO = OFF_Q + QSTAGES * TILE_BYTES;        // [QSTAGES]
   static constexpr int OFF_P = OFF_DO + QSTAGES * TILE_BYTES;        // Pᵀ  128 x 128 x 2 B (head_dim 128 only)
   static constexpr int OFF_DS = OFF_P + ((256 + 3 * HD + 64 <= 512) ? 0 : 32768);  // dSᵀ 128 x 128 x 2 B
   static constexpr int OFF_STAT = OFF_DS + 32768;                    // [2 parities][16 compute warps][lse2[32], delta[32]] fp32
-  // dQ_i staging for the TMA reduction: boxes of 32 rows x 128 B, one per drain warp and 32-column chunk.  At
-  // head_dim 64 they have shared memory of their own (two per warp).  At head_dim 128 there is none left, and the
+  // dQ_i staging for the TMA reduction: boxes of 32 rows x 128 B (32 columns).  At head_dim 64 they have shared memory of
+  // their own, one per drain warp, which its two chunks pass through one after the other.  At head_dim 128 there is none left, and the
   // sixteen boxes are the Pᵀ / dSᵀ buffers themselves: between the last gradient product of a tile and the
   // compute warps' next write nothing else uses them.
   static constexpr bool DQ_TMA = true;
   static constexpr bool DQ_IN_PDS = (HD == 128);
-  static constexpr int DQ_BOXES = (HD == 64) ? 2 : 0;
+  static constexpr int DQ_BOXES = (HD == 64) ? 1 : 0;
   static constexpr int OFF_DQ = OFF_STAT + 8192;
   static constexpr int OFF_BAR = OFF_DQ + 4 * DQ_BOXES * 4096;
   static constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
@@ -118,43 +129,70 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
                                                                       const __grid_constant__ CUtensorMap tmDQ,
                                                                       const FbParams p) {
   using Cfg = FbCfg<HD>;
-  constexpr int QS = Cfg::QSTAGES;
+  constexpr int QS = Cfg::QSTAGES, KVS = Cfg::KVSTAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* s_stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);  // [2 parities][16 warps][lse2[32], delta[32]]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
-  uint64_t* kv_full = bars + 0;
-  uint64_t* q_full = bars + 1;    // [3] Q_i and dO_i landed
-  uint64_t* q_empty = bars + 4;   // [3] products reading them retired
-  uint64_t* s_full = bars + 7;    // Sᵀ and dPᵀ in TMEM
-  uint64_t* pds_full = bars + 8;  // Pᵀ and dSᵀ in smem (and Sᵀ, dPᵀ consumed)
-  uint64_t* dq_full = bars + 9;   // dV, dK, dQ_i products retired
-  uint64_t* dq_free = bars + 10;  // dQ_i read out of TMEM
-  uint64_t* s_free = bars + 11;   // Sᵀ and dPᵀ read out of TMEM (head_dim 64: the next scores may overwrite them)
-  uint64_t* stage_free = bars + 12;  // head_dim 128: the TMA unit has read dQ_i out of the Pᵀ / dSᵀ buffers
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 13);
+  uint64_t* q_full = bars + 0;       // [3] Q_i and dO_i landed
+  uint64_t* q_empty = bars + 3;      // [3] products reading them retired
+  uint64_t* s_full = bars + 6;       // Sᵀ and dPᵀ in TMEM
+  uint64_t* pds_full = bars + 7;     // Pᵀ and dSᵀ in smem (and Sᵀ, dPᵀ consumed)
+  uint64_t* dq_full = bars + 8;      // dV, dK, dQ_i products retired
+  uint64_t* dq_free = bars + 9;      // dQ_i read out of TMEM
+  uint64_t* s_free = bars + 10;      // Sᵀ and dPᵀ read out of TMEM (head_dim 64: the next scores may overwrite them)
+  uint64_t* stage_free = bars + 11;  // head_dim 128: the TMA unit has read dQ_i out of the Pᵀ / dSᵀ buffers
+  uint64_t* kv_full = bars + 12;     // [KVSTAGES] K and V of an item landed
+  uint64_t* kv_empty = bars + 14;    // [KVSTAGES] the item's last products have retired: K and V may be replaced
+  uint64_t* acc_free = bars + 16;    // dV and dK of an item have been read out of TMEM
+  uint64_t* next_full = bars + 17;   // the answer to the request for another item has landed
+  uint64_t* next_empty = bars + 18;  // every role has read it
+  uint8_t* next_item = reinterpret_cast<uint8_t*>(bars + 20);  // the answer, 16 bytes
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 22);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // CTAs are dispatched in block order: within a group of batch*head slices the key tiles with the
-  // longest walk (tile 0) of EVERY slice come first, so the tail of the kernel is made of short CTAs
+  // Items (key tile, batch*head) are numbered longest walk first: within a group of batch*head slices the key tiles with the
+  // longest walk (tile 0) of EVERY slice come first, so the tail of the kernel is made of short ones.
   const int nq = (p.T + FB_T - 1) / FB_T;
-  int kt, bh;
-  if (p.debug & 32) {  // per-slice order (test switch)
-    kt = blockIdx.x % nq;
-    bh = blockIdx.x / nq;
-  } else {
-    const int g = blockIdx.x / (nq * p.group), r = blockIdx.x % (nq * p.group);
-    const int gsz = min(p.group, p.BH - g * p.group);
-    kt = r / gsz;
-    bh = g * p.group + r % gsz;
-  }
-  const int b = bh / p.H, h = bh % p.H;
-  const int j0 = kt * FB_T;
-  const int iters = nq - kt;
+  struct Item {
+    int kt, bh;  // (the rest follows from these where it is needed: few registers live through the walk)
+  };
+  auto item_of = [&](int block) -> Item {
+    Item w;
+    if (p.debug & 32) {  // per-slice order (test switch)
+      w.kt = block % nq;
+      w.bh = block / nq;
+    } else {
+      const int g = block / (nq * p.group), r = block % (nq * p.group);
+      const int gsz = min(p.group, p.BH - g * p.group);
+      w.kt = r / gsz;
+      w.bh = g * p.group + r % gsz;
+    }
+    return w;
+  };
+  // The item after the CTA's n-th one: false when there is none.  Read by every role once per item; `alone`: by one lane.
+  auto next_of = [&](int n, Item& w, bool alone) -> bool {
+    bool ok = mbar_wait(next_full, n & 1, 0x2800, abort_flag);
+    if (!alone) ok = __all_sync(0xffffffffu, ok) != 0;
+    if (!ok) return false;
+    int block;
+    bool more = clc_answer(next_item, block);
+    fence_proxy_async_smem();  // read, before the next answer is written
+    if (!alone) {  // the same in every lane: tells the compiler so, and with it that the operand descriptors are uniform
+      more = __all_sync(0xffffffffu, more) != 0;
+      block = __shfl_sync(0xffffffffu, block, 0);
+    }
+    if (alone || lane == 0) mbar_arrive(next_empty);
+    if (more) w = item_of(block);
+    return more;
+  };
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
+    for (int i = 0; i < Cfg::KVSTAGES; ++i) {
+      mbar_init(&kv_full[i], 1);
+      mbar_init(&kv_empty[i], 1);
+    }
     for (int i = 0; i < 3; ++i) {
       mbar_init(&q_full[i], 1);
       mbar_init(&q_empty[i], 1);
@@ -165,6 +203,9 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
     mbar_init(dq_free, 4);
     mbar_init(s_free, FB_CWARPS);
     mbar_init(stage_free, 4);
+    mbar_init(acc_free, FB_CWARPS);
+    mbar_init(next_full, 1);
+    mbar_init(next_empty, 2 + FB_CWARPS + 4);  // producer, MMA issuer, compute warps, drain warps
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -188,23 +229,44 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
       tma_prefetch_desc(&tmDO);
-      mbar_expect_tx(kv_full, 2 * Cfg::TILE_BYTES);
-#pragma unroll
-      for (int c = 0; c < Cfg::PANELS; ++c) {
-        tma_load_4d(smem + Cfg::OFF_K + c * 16384, &tmK, c * 64, j0, h, b, kv_full);
-        tma_load_4d(smem + Cfg::OFF_V + c * 16384, &tmV, c * 64, j0, h, b, kv_full);
-      }
-      for (int it = 0; it < iters; ++it) {
-        const int st = it % QS;
-        const uint32_t ph = (it / QS) & 1;
-        if (!mbar_wait(&q_empty[st], ph ^ 1, 0x2100 | st, abort_flag)) break;
-        mbar_expect_tx(&q_full[st], 2 * Cfg::TILE_BYTES);
-        const int i0 = (kt + it) * FB_T;
+      Item w = item_of(blockIdx.x);
+      int g = 0;  // tiles of the CTA so far: the phases of every barrier run on across its items
+      bool ok = true;
+      // K and V of the CTA's n-th item
+      auto load_kv = [&](int n) -> bool {
+        const int ks = n % KVS, b = w.bh / p.H, h = w.bh % p.H;
+        if (n >= KVS && !mbar_wait(&kv_empty[ks], (n / KVS - 1) & 1, 0x2110 | ks, abort_flag)) return false;
+        mbar_expect_tx(&kv_full[ks], 2 * Cfg::TILE_BYTES);
+        uint8_t* dst = smem + Cfg::OFF_K + ks * 2 * Cfg::TILE_BYTES;
 #pragma unroll
         for (int c = 0; c < Cfg::PANELS; ++c) {
-          tma_load_4d(smem + Cfg::OFF_Q + st * Cfg::TILE_BYTES + c * 16384, &tmQ, c * 64, i0, h, b, &q_full[st]);
-          tma_load_4d(smem + Cfg::OFF_DO + st * Cfg::TILE_BYTES + c * 16384, &tmDO, c * 64, i0, h, b, &q_full[st]);
+          tma_load_4d(dst + c * 16384, &tmK, c * 64, w.kt * FB_T, h, b, &kv_full[ks]);
+          tma_load_4d(dst + Cfg::TILE_BYTES + c * 16384, &tmV, c * 64, w.kt * FB_T, h, b, &kv_full[ks]);
         }
+        return true;
+      };
+      for (int n = 0; ok; ++n) {
+        if (KVS > 1) ok = load_kv(n);
+        for (int it = 0; it < nq - w.kt && ok; ++it, ++g) {
+          const int st = g % QS;
+          const uint32_t ph = (g / QS) & 1;
+          if (!mbar_wait(&q_empty[st], ph ^ 1, 0x2100 | st, abort_flag)) { ok = false; break; }
+          mbar_expect_tx(&q_full[st], 2 * Cfg::TILE_BYTES);
+          const int i0 = (w.kt + it) * FB_T, b = w.bh / p.H, h = w.bh % p.H;
+#pragma unroll
+          for (int c = 0; c < Cfg::PANELS; ++c) {
+            tma_load_4d(smem + Cfg::OFF_Q + st * Cfg::TILE_BYTES + c * 16384, &tmQ, c * 64, i0, h, b, &q_full[st]);
+            tma_load_4d(smem + Cfg::OFF_DO + st * Cfg::TILE_BYTES + c * 16384, &tmDO, c * 64, i0, h, b, &q_full[st]);
+          }
+          if (KVS == 1 && it == 0) ok = load_kv(n);
+        }
+        // Asked for only now, with the item's last loads issued: asked for at its start, the CTAs with the longest items
+        // would take the first of the remaining ones.
+        if (ok && n > 0) ok = mbar_wait(next_empty, (n - 1) & 1, 0x2120, abort_flag);
+        if (!ok) break;
+        mbar_expect_tx(next_full, 16);
+        clc_request(next_item, next_full);
+        ok = next_of(n, w, true);
       }
     }
   } else if (warp == 1) {
@@ -243,12 +305,13 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         const bool r = mbar_wait(bar, parity, code, abort_flag);
         return WHOLE_WARP ? (__all_sync(0xffffffffu, r) != 0) : r;
       };
-      bool ok = wait(kv_full, 0, 0x2200);
+      bool ok = true;
       // Sᵀ = K Q_iᵀ and dPᵀ = V dO_iᵀ of query tile `it`
-      auto issue_scores = [&](int it) -> bool {
-        const int st = it % QS;
+      auto issue_scores = [&](int g, int n) -> bool {  // g: tiles of the CTA before this one, n: items
+        const uint32_t kv = (n % KVS) * 2 * Cfg::TILE_BYTES;
+        const int st = g % QS;
         PROF_T(a0);
-        if (!wait(&q_full[st], (it / QS) & 1, 0x2300 | st)) return false;
+        if (!wait(&q_full[st], (g / QS) & 1, 0x2300 | st)) return false;
         PROF_T(a1);
         PROF_ADD(7, a0, a1);
         tc_fence_after();
@@ -258,12 +321,12 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
 #pragma unroll
         for (int s = 0; s < HD / 16; ++s) {
           const uint32_t off = (s / 4) * 16384 + (s % 4) * 32;
-          if (leader()) tc_mma_ss(tb + Cfg::COL_S, desc_advance(dk_k, off), desc_advance(q_k, off), idesc_s, s ? 1u : 0u);
+          if (leader()) tc_mma_ss(tb + Cfg::COL_S, desc_advance(dk_k, kv + off), desc_advance(q_k, off), idesc_s, s ? 1u : 0u);
         }
 #pragma unroll
         for (int s = 0; s < HD / 16; ++s) {
           const uint32_t off = (s / 4) * 16384 + (s % 4) * 32;
-          if (leader()) tc_mma_ss(tb + Cfg::COL_DP, desc_advance(dv_k, off), desc_advance(do_k, off), idesc_s, s ? 1u : 0u);
+          if (leader()) tc_mma_ss(tb + Cfg::COL_DP, desc_advance(dv_k, kv + off), desc_advance(do_k, off), idesc_s, s ? 1u : 0u);
         }
         if (leader()) tc_commit(s_full);
         PROF_T(i1_);
@@ -271,13 +334,14 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         return true;
       };
       // dV += Pᵀ dO_i, dK += dSᵀ Q_i, dQ_i = dS K
-      auto issue_grads = [&](int it) -> bool {
-        const int st = it % QS;
+      auto issue_grads = [&](int g, int n, int it, bool last) -> bool {
+        const uint32_t kv = (n % KVS) * 2 * Cfg::TILE_BYTES;
+        const int st = g % QS;
         const uint64_t q_mn = smem_desc_sw128(s0 + Cfg::OFF_Q + st * Cfg::TILE_BYTES, 16384, 1024);
         const uint64_t do_mn = smem_desc_sw128(s0 + Cfg::OFF_DO + st * Cfg::TILE_BYTES, 16384, 1024);
         // the dQ columns still hold the previous tile's dQ until the drain warps are done with it
         PROF_T(a0);
-        if (it > 0 && !wait(dq_free, (it - 1) & 1, 0x2400)) return false;
+        if (g > 0 && !wait(dq_free, (g - 1) & 1, 0x2400)) return false;
         PROF_T(a1);
         PROF_ADD(8, a0, a1);
         tc_fence_after();
@@ -298,43 +362,59 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
 #pragma unroll
         for (int s = 0; s < FB_T / 16; ++s) {  // contraction over the 128 keys of this CTA
           const uint32_t moff = s * 2048;      // 16 key rows of 128 B in dSᵀ and in K
-          if (leader()) tc_mma_ss(tb + Cfg::COL_DQ, desc_advance(dds_mn, moff), desc_advance(dk_mn, moff), idesc_q, s ? 1u : 0u);
+          if (leader()) tc_mma_ss(tb + Cfg::COL_DQ, desc_advance(dds_mn, moff), desc_advance(dk_mn, kv + moff), idesc_q, s ? 1u : 0u);
         }
         if (leader()) {
           tc_commit(&q_empty[st]);
           tc_commit(dq_full);
+          if (last) tc_commit(&kv_empty[n % KVS]);
         }
         PROF_T(i1_);
         PROF_ADD(15, i0_, i1_);
         return true;
       };
-      if (ok) ok = issue_scores(0);
-      for (int it = 0; it < iters && ok; ++it) {
-        if (!Cfg::DQ_ALIASED && it + 1 < iters) {
-          // The compute warps hand Sᵀ / dPᵀ back as soon as they hold them in registers, about half-way through
-          // their work on the tile: the next tile's scores are issued then and have landed when the warps come
-          // back for them.  (Issued only once Pᵀ / dSᵀ were ready, they cost a round trip of 1.5 k cycles per
-          // tile that nothing hid: the score buffers cannot be doubled, tensor memory is full.)
-          if (!wait(s_free, it & 1, 0x2550)) { ok = false; break; }
-          if (!issue_scores(it + 1)) { ok = false; break; }
-        }
-        PROF_T(a0);
-        if (!wait(pds_full, it & 1, 0x2500)) { ok = false; break; }
-        PROF_T(a1);
-        PROF_ADD(6, a0, a1);
-        if (!Cfg::DQ_ALIASED) {
-          ok = issue_grads(it);
-        } else {
-          // dQ_i reuses the Sᵀ columns: the next scores may only follow once dQ_i has been drained
-          ok = issue_grads(it);
-          if (ok && it + 1 < iters) {
+      Item w = item_of(blockIdx.x);
+      int g = 0;
+      ok = wait(&kv_full[0], 0, 0x2200) && issue_scores(0, 0);
+      for (int n = 0; ok; ++n) {
+        Item wn = w;
+        bool more = false;
+        for (int it = 0; it < nq - w.kt && ok; ++it, ++g) {
+          const bool last = w.kt + it + 1 == nq;
+          if (KVS > 1 && last) {
+            more = next_of(n, wn, !WHOLE_WARP);
+            if (more && !wait(&kv_full[(n + 1) % KVS], ((n + 1) / KVS) & 1, 0x2200)) { ok = false; break; }
+          }
+          if (!Cfg::DQ_ALIASED && (!last || more)) {
+            // The compute warps hand Sᵀ / dPᵀ back as soon as they hold them in registers, about half-way through
+            // their work on the tile: the next tile's scores are issued then and have landed when the warps come
+            // back for them.  (Issued only once Pᵀ / dSᵀ were ready, they cost a round trip of 1.5 k cycles per
+            // tile that nothing hid: the score buffers cannot be doubled, tensor memory is full.)
+            if (!wait(s_free, g & 1, 0x2550)) { ok = false; break; }
+            if (!issue_scores(g + 1, last ? n + 1 : n)) { ok = false; break; }
+          }
+          PROF_T(a0);
+          if (!wait(pds_full, g & 1, 0x2500)) { ok = false; break; }
+          PROF_T(a1);
+          PROF_ADD(6, a0, a1);
+          // the first products of an item overwrite dV and dK of the one before
+          if (it == 0 && n > 0 && !wait(acc_free, (n - 1) & 1, 0x2560)) { ok = false; break; }
+          ok = issue_grads(g, n, it, last);
+          if (KVS == 1 && ok && last) {
+            more = next_of(n, wn, !WHOLE_WARP);
+            if (more && !wait(&kv_full[0], (n + 1) & 1, 0x2200)) { ok = false; break; }
+          }
+          if (Cfg::DQ_ALIASED && ok && (!last || more)) {
+            // dQ_i reuses the Sᵀ columns: the next scores may only follow once dQ_i has been drained
             PROF_T(b0);
-            ok = wait(dq_free, it & 1, 0x2450);
+            ok = wait(dq_free, g & 1, 0x2450);
             PROF_T(b1);
             PROF_ADD(8, b0, b1);
-            if (ok) ok = issue_scores(it + 1);
+            if (ok) ok = issue_scores(g + 1, last ? n + 1 : n);
           }
         }
+        if (!more) break;
+        w = wn;
       }
       PROF_T(tm_end);
       PROF_ADD(9, tm_start, tm_end);
@@ -350,8 +430,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       const int ct = threadIdx.x - 64;   // 0..255 within the compute group
       const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
       const float c2 = p.scale * kLog2eB;
-      const AlibiLog2<BIAS> alibi(BIAS ? p.slopes[h] : 0.f);
-      const int j = j0 + r;              // this thread's key
       uint8_t* sp = smem + Cfg::OFF_P;
       uint8_t* sds = smem + Cfg::OFF_DS;
       bool ok = true;
@@ -359,28 +437,65 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       // Per-query statistics of the warp's 32 query columns: lane l carries lse and delta of
       // column l, fetched one tile ahead (so the global-memory latency is not part of the tile) and handed to the
       // other lanes through a slice of shared memory that belongs to this warp: no barrier across the warps.
-      auto load_stat = [&](int it, float& l2, float& dl) {
-        const int i = (kt + it) * FB_T + cq * 32 + lane;
-        const int64_t at = (int64_t)bh * p.T + i;
+      auto load_stat = [&](const Item& w, int it, float& l2, float& dl) {
+        const int i = (w.kt + it) * FB_T + cq * 32 + lane;
+        const int64_t at = (int64_t)w.bh * p.T + i;
         l2 = i < p.T ? p.lse[at] : 0.f;  // converted to log2 units where it is used: nothing here may wait for the load
         dl = i < p.T ? p.delta[at] : 0.f;
       };
       float lse_next, delta_next;
-      load_stat(0, lse_next, delta_next);
-      for (int it = 0; it < iters; ++it) {
-        const int i0 = (kt + it) * FB_T;
+      Item w = item_of(blockIdx.x), wp = w;  // wp: the item before
+      load_stat(w, 0, lse_next, delta_next);
+      // dV and dK of an item whose products have all retired
+      auto store_item = [&](const Item& w) {
+        tc_fence_after();
+        const int j = w.kt * FB_T + r;
+        T* dvp = reinterpret_cast<T*>(p.dv) + (w.bh / p.H) * p.sdv_b + (w.bh % p.H) * p.sdv_h + (int64_t)j * p.sdv_t;
+        T* dkp = reinterpret_cast<T*>(p.dk) + (w.bh / p.H) * p.sdk_b + (w.bh % p.H) * p.sdk_h + (int64_t)j * p.sdk_t;
+#pragma unroll 1
+        for (int c = 0; c < HD / 32; ++c) {  // this warp's HD / 4 columns in steps of 8
+          const int col0 = cq * (HD / 4) + c * 8;
+          if (col0 >= p.hd) break;
+          uint32_t v[8], u[8];
+          tmem_ld8(lane_addr + Cfg::COL_DV + col0, v);
+          tmem_ld8(lane_addr + Cfg::COL_DK + col0, u);
+          tc_wait_ld();
+          if (j < p.T) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[e]);
+            *reinterpret_cast<uint4*>(dvp + col0) = pack8<T>(f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(u[e]) * p.scale;
+            *reinterpret_cast<uint4*>(dkp + col0) = pack8<T>(f);
+          }
+          __syncwarp();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_free);  // the next item's products may overwrite them
+      };
+      // With the next item's scores already there, an item is stored behind the arithmetic of the next one's first tile,
+      // which hides its last products.
+      constexpr bool LATE_STORE = KVS > 1;
+      int g = 0;  // tiles of the CTA before this one
+      for (int n = 0;; ++n) {
+      const AlibiLog2<BIAS> alibi(BIAS ? p.slopes[w.bh % p.H] : 0.f);
+      const int j = w.kt * FB_T + r;     // this thread's key
+      for (int it = 0; it < nq - w.kt; ++it, ++g) {
+        const int i0 = (w.kt + it) * FB_T;
         const bool diag = (it == 0);
         PROF_T(t0);
         // this tile's statistics, double buffered by iteration parity: a lane that is already here may share
         // the warp with one that still reads the previous tile's slice
-        float* s_lse2 = s_stat + ((it & 1) * FB_CWARPS + cw) * 64;
+        float* s_lse2 = s_stat + ((g & 1) * FB_CWARPS + cw) * 64;
         float* s_delta = s_lse2 + 32;
         s_lse2[lane] = lse_next * kLog2eB;
         s_delta[lane] = delta_next;
         __syncwarp();
         PROF_T(t1);
-        if (it + 1 < iters) load_stat(it + 1, lse_next, delta_next);  // after the warp barrier, which would wait for it
-        if (ok) ok = mbar_wait(s_full, it & 1, 0x2600, abort_flag);
+        if (it + 1 < nq - w.kt) load_stat(w, it + 1, lse_next, delta_next);  // after the warp barrier, which would wait for it
+        if (ok) ok = mbar_wait(s_full, g & 1, 0x2600, abort_flag);
         PROF_T(t2);
         PROF_ADD(5, t0, t1);
         PROF_ADD(1, t1, t2);
@@ -392,7 +507,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
 #pragma unroll
           for (int e = 0; e < 16; ++e) pk[e] = dk_[e] = 0u;
           if (!Cfg::DQ_ALIASED && lane == 0) mbar_arrive(s_free);
-          if (it > 0 && ok) ok = mbar_wait(dq_full, (it - 1) & 1, 0x2650, abort_flag);
+          if (g > 0 && ok) ok = mbar_wait(dq_full, (g - 1) & 1, 0x2650, abort_flag);
         }
         if (ok && !quiet) {
           tc_fence_after();
@@ -455,13 +570,14 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           }
           // Pᵀ / dSᵀ of the previous tile are still being read by its gradient products
           if (prof) t3 = clock64();
-          if (it > 0) ok = mbar_wait(dq_full, (it - 1) & 1, 0x2650, abort_flag);
+          if (g > 0) ok = mbar_wait(dq_full, (g - 1) & 1, 0x2650, abort_flag);
           // ... and, at head_dim 128, by the TMA reduction of its dQ, which was staged in them
-          if (Cfg::DQ_IN_PDS && it > 0 && ok) ok = mbar_wait(stage_free, (it - 1) & 1, 0x2660, abort_flag);
+          if (Cfg::DQ_IN_PDS && g > 0 && ok) ok = mbar_wait(stage_free, (g - 1) & 1, 0x2660, abort_flag);
           if (prof) t4 = clock64();
           PROF_ADD(2, t2, t3);
           PROF_ADD(3, t3, t4);
         }
+        if (LATE_STORE && it == 0 && n > 0 && ok) store_item(wp);  // (the wait for dq_full above was for its last tile)
         if (ok && quiet) {
           tc_fence_before();
           __syncwarp();
@@ -488,32 +604,16 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           PROF_ADD(13, t45, t5);
         }
       }
-      if (ok && mbar_wait(dq_full, (iters - 1) & 1, 0x2680, abort_flag)) {
-        // dV and dK are complete
-        tc_fence_after();
-        T* dvp = reinterpret_cast<T*>(p.dv) + b * p.sdv_b + h * p.sdv_h + (int64_t)j * p.sdv_t;
-        T* dkp = reinterpret_cast<T*>(p.dk) + b * p.sdk_b + h * p.sdk_h + (int64_t)j * p.sdk_t;
-#pragma unroll 1
-        for (int c = 0; c < HD / 64; ++c) {  // this warp's HD / 4 columns in steps of 16
-          const int col0 = cq * (HD / 4) + c * 16;
-          if (col0 >= p.hd) break;
-          uint32_t v[16], w[16];
-          tmem_ld16(lane_addr + Cfg::COL_DV + col0, v);
-          tmem_ld16(lane_addr + Cfg::COL_DK + col0, w);
-          tc_wait_ld();
-#pragma unroll
-          for (int v4 = 0; v4 < 2; ++v4) {
-            if (j >= p.T) break;
-            float g[8], d[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              g[e] = __uint_as_float(v[v4 * 8 + e]);
-              d[e] = __uint_as_float(w[v4 * 8 + e]) * p.scale;
-            }
-            *reinterpret_cast<uint4*>(dvp + col0 + v4 * 8) = pack8<T>(g);
-            *reinterpret_cast<uint4*>(dkp + col0 + v4 * 8) = pack8<T>(d);
-          }
-        }
+      Item wn = w;
+      const bool more = __all_sync(0xffffffffu, ok) != 0 && next_of(n, wn, false);
+      if (more) load_stat(wn, 0, lse_next, delta_next);  // on their way while this item is finished
+      if (!LATE_STORE || !more) {
+        if (ok) ok = mbar_wait(dq_full, (g - 1) & 1, 0x2680, abort_flag);
+        if (ok) store_item(w);
+      }
+      if (!more || !ok) break;
+      wp = w;
+      w = wn;
       }
     }
   } else if (!dead) {
@@ -528,10 +628,15 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
     const bool prof = (p.debug & 2) && warp == 2 + FB_CWARPS && lane == 0;
     uint8_t* stage = smem + Cfg::OFF_DQ + (warp - 2 - FB_CWARPS) * Cfg::DQ_BOXES * 4096;
     if (Cfg::DQ_TMA && lane == 0) tma_prefetch_desc(&tmDQ);
-    for (int it = 0; it < iters; ++it) {
-      const int i0 = (kt + it) * FB_T;
+    Item w = item_of(blockIdx.x);
+    int g = 0;
+    bool ok = true;
+    for (int n = 0; ok; ++n) {
+    const int bh = w.bh;
+    for (int it = 0; it < nq - w.kt; ++it, ++g) {
+      const int i0 = (w.kt + it) * FB_T;
       PROF_T(a0);
-      if (!mbar_wait(dq_full, it & 1, 0x2700, abort_flag)) break;
+      if (!mbar_wait(dq_full, g & 1, 0x2700, abort_flag)) { ok = false; break; }
       PROF_T(a1);
       PROF_ADD(10, a0, a1);
       tc_fence_after();
@@ -587,26 +692,28 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         tc_wait_ld();
         // TMEM is drained: the tensor core may overwrite dQ while the rows travel on
         tc_fence_before();
-        if (lane == 0) tma_store_wait_read();  // previous boxes have been read by the TMA unit
         __syncwarp();
         if (lane == 0) mbar_arrive(dq_free);
-        if (!(p.debug & 1)) {
+        // (rows past the sequence's end hold exact zeros: added to the next slice's rows they change nothing)
+        const int row0 = (int)((int64_t)bh * p.T) + i0 + qd * 32;
+        auto add_box = [&](const uint32_t (&v)[32], int col) {
+          if (lane == 0) tma_store_wait_read();  // the box has been read by the TMA unit
+          __syncwarp();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {  // 16-byte chunks (4 floats) of this row in each of the two boxes
+          for (int j = 0; j < 8; ++j) {  // 16-byte chunks (4 floats) of this row
             const uint32_t off = lane * 128 + ((j ^ (lane & 7)) << 4);
-            *reinterpret_cast<uint4*>(stage + off) = make_uint4(v0[4 * j], v0[4 * j + 1], v0[4 * j + 2], v0[4 * j + 3]);
-            *reinterpret_cast<uint4*>(stage + 4096 + off) =
-                make_uint4(v1[4 * j], v1[4 * j + 1], v1[4 * j + 2], v1[4 * j + 3]);
+            *reinterpret_cast<uint4*>(stage + off) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
           }
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            // (rows past the sequence's end hold exact zeros: added to the next slice's rows they change nothing)
-            const int row0 = (int)((int64_t)bh * p.T) + i0 + qd * 32;
-            tma_reduce_add_2d(&tmDQ, stage, 0, row0);
-            if (p.hd > 32) tma_reduce_add_2d(&tmDQ, stage + 4096, 32, row0);
+            tma_reduce_add_2d(&tmDQ, stage, col, row0);
             tma_store_commit();
           }
+        };
+        if (!(p.debug & 1)) {
+          add_box(v0, 0);
+          if (p.hd > 32) add_box(v1, 32);
         }
       } else {
         float* dq_row = p.dq_acc + ((int64_t)bh * p.T + i0 + r) * p.hd;
@@ -629,6 +736,8 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       }
       PROF_T(a2);
       PROF_ADD(11, a1, a2);
+    }
+    ok = __all_sync(0xffffffffu, ok) != 0 && next_of(n, w, false);
     }
     if (Cfg::DQ_TMA && lane == 0) tma_store_wait_all();  // every reduction has reached global memory
   }

@@ -121,6 +121,29 @@ __device__ __forceinline__ void tma_store_wait_read_but1() { asm volatile("cp.as
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// ---- cluster launch control: a running CTA takes over the block of one that has not been launched ---------------
+// One thread asks; the 16-byte answer is counted on the barrier.  Not to be asked again after an answer without a block.
+__device__ __forceinline__ void clc_request(void* answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(answer)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ bool clc_answer(const void* answer, int& block_x) {
+  uint32_t x = 0, got;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 a;\n\t"
+      "ld.shared.b128 a, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+      "selp.u32 %1, 1, 0, p;\n\t"
+      "mov.u32 %0, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, _, _, _}, a;\n\t}"
+      : "=&r"(x), "=r"(got)
+      : "r"(smem_u32(answer))
+      : "memory");
+  block_x = (int)x;
+  return got != 0;
+}
+
 // ---- tcgen05 / TMEM -------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* holder, uint32_t ncols) {  // whole warp
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)),
