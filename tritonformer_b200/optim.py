@@ -78,6 +78,15 @@ class FusedAdamW:
         device, if any gradient of any bucket is inf or nan."""
         s = self.scaler
         stream = _lib.stream_ptr(self.buckets.buckets[0].device)
+        if len(self.buckets.buckets) == 1:  # without the lists' host time: 22 against 29 us a step
+            (g,), (p16,), (w,), (m,), (v,) = self.buckets.buckets, self.params16, self.master, self.exp_avg, self.exp_avg_sq
+            n, code = g.numel(), _lib.dtype_code(g.dtype)
+            _lib.check(_lib.lib.tfb_grad_check(g.data_ptr(), n, code, s.found_inf.data_ptr(), stream))
+            _lib.check(_lib.lib.tfb_adamw_step(g.data_ptr(), p16.data_ptr(), w.data_ptr(), m.data_ptr(), v.data_ptr(), n, code,
+                                               s.inv_scale.data_ptr(), s.found_inf.data_ptr(), s.steps_taken.data_ptr(), self.lr,
+                                               self.betas[0], self.betas[1], self.eps, self.weight_decay, stream))
+            s.update()
+            return
         lists = [self.buckets.buckets, self.params16, self.master, self.exp_avg, self.exp_avg_sq]
         groups = []  # buckets of one dtype go into one launch
         for dtype in dict.fromkeys(g.dtype for g in self.buckets.buckets):
