@@ -28,8 +28,9 @@
 // At head_dim 64 the scores of tile i+1 are issued as soon as the compute warps hold the scores of tile i in
 // registers, ahead of the gradient products of tile i, so the compute warps find them ready and work on tile
 // i+1 while the tensor core finishes tile i.
-// A sequence that is no multiple of 128: the rows past its end are zeros in shared memory (TMA fill) with statistics of
-// zero, so their dS and their shares of dV, dK and dQ vanish; their own rows are not stored.  head_dim 32 runs on the
+// A sequence that is no multiple of 128: the rows past its end are zeros in shared memory (TMA fill); as queries they get
+// exact zeros for P and dS and their rows of dQ are left out (the accumulator's next rows are another slice's), as keys the
+// mask keeps them from every query and their rows are not stored.  head_dim 32 runs on the
 // head_dim 64 kernel with zero columns.
 // TMEM columns: [0,128) Sᵀ; [128,256) dPᵀ; [256,256+hd) dV; then dK; then dQ_i (at head_dim 128
 // dQ_i reuses the Sᵀ columns).
@@ -121,7 +122,9 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-template <typename T, int HD, int BIAS>
+// RAGGED: T is no multiple of 128 (a run-time branch in the compute and drain loops cost whole tiles 1 %: B4 H16 T2048 hd64
+// fp16 193 against 191 us, spilled registers).
+template <typename T, int HD, int BIAS, bool RAGGED>
 __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                       const __grid_constant__ CUtensorMap tmK,
                                                                       const __grid_constant__ CUtensorMap tmV,
@@ -577,6 +580,12 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           PROF_ADD(2, t2, t3);
           PROF_ADD(3, t3, t4);
         }
+        // T is a multiple of 64, so a warp's 32 queries are all real or all past the sequence's end.  The latter get exact
+        // zeros: what was worked out from the zero-filled rows is NaN where K or V holds an infinity.
+        if (RAGGED && i0 + cq * 32 >= p.T) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) pk[e] = dk_[e] = 0u;
+        }
         if (LATE_STORE && it == 0 && n > 0 && ok) store_item(wp);  // (the wait for dq_full above was for its last tile)
         if (ok && quiet) {
           tc_fence_before();
@@ -677,7 +686,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          if (!(p.debug & 1)) {
+          if ((!RAGGED || i0 + qd * 32 < p.T) && !(p.debug & 1)) {  // the rows past the end are the next slice's
 #pragma unroll
             for (int c = 0; c < HD / 32; ++c) tma_reduce_add_2d(&tmDQ, boxes + c * 4096, c * 32, row0);
             tma_store_commit();
@@ -694,7 +703,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(dq_free);
-        // (rows past the sequence's end hold exact zeros: added to the next slice's rows they change nothing)
         const int row0 = (int)((int64_t)bh * p.T) + i0 + qd * 32;
         auto add_box = [&](const uint32_t (&v)[32], int col) {
           if (lane == 0) tma_store_wait_read();  // the box has been read by the TMA unit
@@ -707,7 +715,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            tma_reduce_add_2d(&tmDQ, stage, col, row0);
+            if (!RAGGED || i0 + qd * 32 < p.T) tma_reduce_add_2d(&tmDQ, stage, col, row0);  // the rows past the end are the next slice's
             tma_store_commit();
           }
         };
@@ -797,7 +805,7 @@ static int encode_bhtd(CUtensorMap* m, const void* ptr, const AttnStrides& s, in
 
 bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd) { return hd <= 128 && a.bias_mode != 3; }
 
-template <typename T, int HD>
+template <typename T, int HD, bool RAGGED>
 static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   using Cfg = FbCfg<HD>;
   int rc;
@@ -828,11 +836,11 @@ static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st
   static std::atomic<uint64_t> done[4] = {{0}, {0}, {0}, {0}};
 #define FB_LAUNCH(MODE, SLOT)                                                                                       \
   {                                                                                                                 \
-    if ((rc = ensure_dynamic_smem(attn_bwd_tc05_kernel<T, HD, MODE>, Cfg::SMEM_BYTES, done[SLOT],                   \
+    if ((rc = ensure_dynamic_smem(attn_bwd_tc05_kernel<T, HD, MODE, RAGGED>, Cfg::SMEM_BYTES, done[SLOT],                   \
                                   "attention_bwd(tcgen05)")))                                                       \
       return rc;                                                                                                    \
-    launch_overlapped(attn_bwd_tc05_kernel<T, HD, MODE>, grid, dim3(FB_THREADS), Cfg::SMEM_BYTES, st, tq, tk, tv, tdo, \
-                      tdq, p);                                                                                      \
+    launch_overlapped(attn_bwd_tc05_kernel<T, HD, MODE, RAGGED>, grid, dim3(FB_THREADS), Cfg::SMEM_BYTES, st, tq, tk, \
+                      tv, tdo, tdq, p);                                                                             \
   }
   if (a.bias_mode == 0) FB_LAUNCH(0, 0)
   else if (a.bias_mode == 1) FB_LAUNCH(1, 1)
@@ -849,8 +857,9 @@ static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st
 
 int attn_tc05_bwd(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   TFB_DISPATCH_16(dtype, T, {
-    if (hd <= 64) return bwd_tc05_launch<T, 64>(a, hd, dtype, st);
-    return bwd_tc05_launch<T, 128>(a, hd, dtype, st);
+    const bool ragged = a.T % FB_T != 0;
+    if (hd <= 64) return ragged ? bwd_tc05_launch<T, 64, true>(a, hd, dtype, st) : bwd_tc05_launch<T, 64, false>(a, hd, dtype, st);
+    return ragged ? bwd_tc05_launch<T, 128, true>(a, hd, dtype, st) : bwd_tc05_launch<T, 128, false>(a, hd, dtype, st);
   })
 }
 
