@@ -43,3 +43,34 @@ def test_attention_backward_of_a_key_that_no_query_reaches(t, hd):
     assert torch.equal(dv[0, 0, t - 3], torch.zeros_like(dv[0, 0, t - 3]))
     assert torch.equal(dk[0, 0, t - 3], torch.zeros_like(dk[0, 0, t - 3]))
     assert dv.isfinite().all() and dk.isfinite().all()
+
+
+@pytest.mark.parametrize("t,hd", [(64, 64), (192, 64), (192, 128), (128, 32), (192, 32)])
+@pytest.mark.parametrize("dtype", HALF)
+def test_attention_passes_nan_on(t, hd, dtype):
+    """A NaN in any key reaches every query that sees it, at the sizes that are no whole tiles of the full width."""
+    from tritonformer_b200.attention import CausalAttention
+    q, k, v, _ = _heads(t - 1, t, hd, dtype)  # head i: NaN in key i
+    for i in range(t - 1):
+        k[0, i, i, 0] = float("nan")
+    out = CausalAttention.apply(q, k, v)
+    seen = torch.ones(t, t, dtype=torch.bool, device="cuda").tril()[:, : t - 1].t()  # (key, query)
+    assert torch.equal(out[0].isnan().all(-1), seen)
+    assert torch.equal(out[0].isnan().any(-1), seen)
+
+
+@pytest.mark.parametrize("t,hd", [(192, 64), (704, 128), (320, 64), (512, 32), (192, 32)])
+def test_attention_statistics_are_those_of_exact_exponentials(t, hd):
+    """The log-sum-exp of the sizes that are no whole tiles of the full width: fp32 sums of exponentials that are good to a
+    few units in the last place (2^-21 relative with 2^-22 for the sums), scores from fp32 products of 16-bit values."""
+    from tritonformer_b200 import _lib as L
+    h = 4
+    q, k, v, _ = _heads(h, t, hd, torch.float16)
+    out, lse = torch.empty_like(q), torch.empty(1, h, t, device="cuda")
+    L.check(L.lib.tfb_attention_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), 1, h, t, hd,
+                                    *(L.strides3(x) for x in (q, k, v, out)), None, 0, None, 0, 0, 0, L.stream_ptr(q.device), None))
+    s = (q.double() @ k.double().transpose(-1, -2)) / hd ** 0.5
+    s = s.masked_fill(~torch.ones(t, t, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    want = torch.logsumexp(s, -1)
+    # |score| <= about 8: 2^-22 of it for the product's sum and the scaling, as much for the result itself
+    assert (lse.double() - want).abs().max().item() <= 2.0 ** -21 + 3 * 2.0 ** -22 * max(8.0, want.abs().max().item())

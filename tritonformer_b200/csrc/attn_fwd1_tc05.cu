@@ -165,7 +165,8 @@ __device__ __forceinline__ bool f1_item(const F1Params& p, int n, int& qt, int& 
 static __device__ unsigned long long g_prof_f1[16];
 #define F1_PROF(idx, t0, t1) do { if (prof) atomicAdd(&g_prof_f1[idx], (unsigned long long)((t1) - (t0))); } while (0)
 
-template <typename T, int HD, int BIAS>
+// POLY: one pair of exponentials in four on the FMA pipe (see fwd1_launch).
+template <typename T, int HD, int BIAS, bool POLY>
 __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                        const __grid_constant__ CUtensorMap tmK,
                                                                        const __grid_constant__ CUtensorMap tmV,
@@ -522,7 +523,7 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
               uint64_t xp = f2_fma(f2_pack(__uint_as_float(v[2 * e2]), __uint_as_float(v[2 * e2 + 1])), c2p, negmp);
               float p0, p1;
               if (BIAS) xp = alibi.sub_pair(xp, d0 - (float)(2 * e2), d0 - (float)(2 * e2 + 1));
-              if ((e2 & 3) == 3) {  // one pair in four on the FMA pipe
+              if (POLY && (e2 & 3) == 3) {
                 ex2_fma2(xp, p0, p1);
               } else {
                 float x0, x1;
@@ -751,7 +752,10 @@ int attn_fwd1_tc05_counters(unsigned long long* out) {
 int encode_tmap_sw128(CUtensorMap* out, const void* base, int dtype, int rank, const uint64_t* dims,
                       const uint64_t* strides_bytes, const uint32_t* box);
 
-template <typename T, int HD>
+// Whole tiles of the full width take one pair of exponentials in four from the cubic (POLY).  The shapes that came here from
+// the mma.sync kernel keep its precision, in P and in the row sums, and its NaN (the cubic clamps its argument, which makes a
+// NaN score a probability of nearly zero): every exponential on the SFU.  B3 H11 T1472 hd64 bf16: 29.3 us, with the cubic 28.9; B1 H12 T4032 hd128 fp16: 62.8, 61.1.
+template <typename T, int HD, bool POLY>
 static int fwd1_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   using Cfg = F1Cfg<HD>;
   CUtensorMap tq, tk, tv;
@@ -783,10 +787,10 @@ static int fwd1_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   static std::atomic<uint64_t> done[4] = {{0}, {0}, {0}, {0}};
 #define F1_LAUNCH(MODE, SLOT)                                                                                        \
   {                                                                                                                  \
-    if ((rc = ensure_dynamic_smem(attn_fwd1_tc05_kernel<T, HD, MODE>, Cfg::SMEM_BYTES, done[SLOT],                   \
+    if ((rc = ensure_dynamic_smem(attn_fwd1_tc05_kernel<T, HD, MODE, POLY>, Cfg::SMEM_BYTES, done[SLOT],                   \
                                   "attention_fwd(tcgen05)")))                                                        \
       return rc;                                                                                                     \
-    launch_overlapped(attn_fwd1_tc05_kernel<T, HD, MODE>, grid, dim3(Cfg::THREADS), Cfg::SMEM_BYTES, st, tq, tk, tv, p); \
+    launch_overlapped(attn_fwd1_tc05_kernel<T, HD, MODE, POLY>, grid, dim3(Cfg::THREADS), Cfg::SMEM_BYTES, st, tq, tk, tv, p); \
   }
   if (a.bias_mode == 0) F1_LAUNCH(0, 0)
   else if (a.bias_mode == 1) F1_LAUNCH(1, 1)
@@ -801,8 +805,10 @@ bool attn_tc05_fwd_eligible(const AttnArgs& a, int hd) { return hd <= 128 && a.b
 
 int attn_fwd1_tc05(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   TFB_DISPATCH_16(dtype, T, {
-    if (hd <= 64) return fwd1_launch<T, 64>(a, hd, dtype, st);
-    return fwd1_launch<T, 128>(a, hd, dtype, st);
+    if (hd < 64 || (hd == 64 && a.T % F1_TILE)) return fwd1_launch<T, 64, false>(a, hd, dtype, st);
+    if (hd == 64) return fwd1_launch<T, 64, true>(a, hd, dtype, st);
+    if (a.T % F1_TILE) return fwd1_launch<T, 128, false>(a, hd, dtype, st);
+    return fwd1_launch<T, 128, true>(a, hd, dtype, st);
   })
 }
 
