@@ -74,3 +74,20 @@ def test_attention_statistics_are_those_of_exact_exponentials(t, hd):
     want = torch.logsumexp(s, -1)
     # |score| <= about 8: 2^-22 of it for the product's sum and the scaling, as much for the result itself
     assert (lse.double() - want).abs().max().item() <= 2.0 ** -21 + 3 * 2.0 ** -22 * max(8.0, want.abs().max().item())
+
+
+@pytest.mark.parametrize("cols", [1, 7, 9, 17, 257, 2047, 50257])
+@pytest.mark.parametrize("dtype", HALF)
+def test_cross_entropy_of_an_odd_vocabulary_passes_nan_on(cols, dtype):
+    """A NaN logit in any column of a row makes its loss NaN; columns of -inf are left out of the sum."""
+    from tritonformer_b200.crossentropy import CrossEntropyLossFP32
+    at = sorted({c for c in (*range(9), cols // 2, cols - 9, cols - 2, cols - 1) if 0 <= c < cols})
+    logits = torch.randn(len(at) * 8, cols, device="cuda").to(dtype)  # eight rows of each: every alignment of a row
+    for i, c in enumerate(at):
+        logits[i::len(at), c] = float("nan")
+    labels = torch.zeros(logits.shape[0], dtype=torch.int64, device="cuda")
+    assert CrossEntropyLossFP32.apply(logits, labels).isnan().all()
+    masked = torch.randn(8, cols, device="cuda").to(dtype)
+    masked[:, : cols - 1] = -float("inf")
+    loss = CrossEntropyLossFP32.apply(masked, torch.full((8,), cols - 1, device="cuda"))
+    assert loss.abs().max().item() <= 1e-6 * masked[:, -1].float().abs().max().item() + 1e-6

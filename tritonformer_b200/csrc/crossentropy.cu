@@ -75,6 +75,13 @@ __global__ void __launch_bounds__(CE_THREADS) ce_fwd_kernel(
       if (m != -INFINITY) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) s += exp2f(fmaf(f[j], kLog2e, -m));
+      } else {  // nothing but -inf so far, or NaN, which fmaxf passes over: a NaN sum under a finite maximum outlives the merges
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (f[j] != f[j]) {
+            m = 0.f;
+            s = f[j];
+          }
       }
     }
   }
