@@ -91,3 +91,54 @@ def test_cross_entropy_of_an_odd_vocabulary_passes_nan_on(cols, dtype):
     masked[:, : cols - 1] = -float("inf")
     loss = CrossEntropyLossFP32.apply(masked, torch.full((8,), cols - 1, device="cuda"))
     assert loss.abs().max().item() <= 1e-6 * masked[:, -1].float().abs().max().item() + 1e-6
+
+
+def _layer(dtype=torch.float16, seed=0, **kw):
+    from tritonformer_b200.transformer import TransformerConfig, TransformerLayer
+    cfg = dict(vocab_size=64, hidden_size=128, max_position_embeddings=128, num_attention_heads=2, head_dim=64, ffn_dim=192,
+               num_hidden_layers=1, use_linear_bias=True, attn_bias=False)
+    cfg.update(kw)
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    layer = TransformerLayer(TransformerConfig(**cfg), device="cuda").to(dtype)
+    with torch.no_grad():
+        for n, p in layer.named_parameters():
+            p.copy_(torch.randn(p.shape, device="cuda", generator=gen) * (0.05 if "layernorm" not in n else 0.2)
+                    + (1.0 if n.endswith("layernorm.weight") else 0.0))
+    return layer
+
+
+def _fuse_projections(layer):
+    """The q, k and v weights as column blocks of one matrix (Transformer.fuse_projection_weights)."""
+    att = layer.attention
+    parts = [att.q_proj, att.k_proj, att.v_proj]
+    buf = torch.cat([p.weight.detach() for p in parts], 1)
+    d = buf.shape[0]
+    for i, p in enumerate(parts):
+        p.weight = torch.nn.Parameter(buf[:, i * d:(i + 1) * d])
+    return layer
+
+
+class _ContiguousCopies(torch.autograd.graph.saved_tensors_hooks):
+    """What saving on the host does to a saved tensor: a copy comes back, contiguous whatever the tensor was."""
+
+    def __init__(self):
+        super().__init__(lambda t: t.detach().clone(memory_format=torch.contiguous_format), lambda t: t.clone())
+
+
+@pytest.mark.parametrize("hooks", [_ContiguousCopies, torch.autograd.graph.save_on_cpu])
+@pytest.mark.parametrize("fused", [True, False])
+def test_layer_backward_from_copies_of_the_saved_tensors(hooks, fused):
+    import contextlib
+    layer = _layer()
+    if fused:
+        _fuse_projections(layer)
+    x = torch.randn(2, 128, 128, device="cuda").half()
+    g = torch.randn_like(x)
+    grads = []
+    for context in (contextlib.nullcontext, hooks):
+        xi = x.clone().requires_grad_()
+        with context():
+            y = layer(xi)
+        grads.append(torch.autograd.grad(y, [xi] + list(layer.parameters()), g))
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)

@@ -55,15 +55,15 @@ static const void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nu
 
 // [Wq | Wk | Wv]: in place if the three already are the column blocks of one matrix (Transformer.fuse_projection_weights),
 // else concatenated.
-static Mat qkv_matrix(const LayerWeights& w, Tensor* cat) {
-  const int64_t d = w.wq.size(1);
-  const Tensor* parts[3] = {&w.wq, &w.wk, &w.wv};
+static Mat qkv_matrix(const Tensor& wq, const Tensor& wk, const Tensor& wv, Tensor* cat) {
+  const int64_t d = wq.size(1);
+  const Tensor* parts[3] = {&wq, &wk, &wv};
   if (adjacent_columns(parts, 3, 3 * d)) {
-    Mat m = block(w.wq.data_ptr(), w.wq.size(0), 3 * d);
-    m.keep = w.wq;
+    Mat m = block(wq.data_ptr(), wq.size(0), 3 * d);
+    m.keep = wq;
     return m;
   }
-  *cat = at::cat({w.wq, w.wk, w.wv}, 1);
+  *cat = at::cat({wq, wk, wv}, 1);
   return as_matrix(*cat);
 }
 
@@ -111,7 +111,7 @@ static Tensor layer_forward(const Tensor& x, const LayerWeights& w, const Bias& 
   if (rows == 0) return y;
 
   norm_forward(x.data_ptr(), w.ln1_w, w.ln1_b, s.slab[s.normed1], s.floats(s.stats1), rows, d, eps1, dtype, st);
-  gemm(block(s.slab[s.normed1], rows, d), qkv_matrix(w, wcat), s.slab[s.qkv], 3 * d, Epilogue{}, dtype, dev, st);
+  gemm(block(s.slab[s.normed1], rows, d), qkv_matrix(w.wq, w.wk, w.wv, wcat), s.slab[s.qkv], 3 * d, Epilogue{}, dtype, dev, st);
   const int64_t es = x.element_size(), hd = shape.hd;
   auto in = [&](int i) { return Heads{s.slab[s.qkv] + i * d * es, {t * 3 * d, hd, 3 * d}}; };
   const Heads out{s.slab[s.ctx], {t * d, hd, d}};
@@ -154,9 +154,11 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
 
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     BodyGuard guard;
+    // Saved-tensor hooks may hand back copies with strides of their own, so nothing that forward found out about the layout
+    // of a saved tensor holds here: it is asked again, or the tensor made contiguous.
     const variable_list v = ctx->get_saved_variables();
-    const Tensor &x = v[0], &ln1_w = v[1], &ln1_b = v[2], &wq = v[3], &wk = v[4], &wv = v[5], &wo = v[6], &ln2_w = v[7],
-                 &ln2_b = v[8], &w1 = v[9], &w2 = v[10], &wcat = v[11];
+    const Tensor x = v[0].contiguous(), &ln1_w = v[1], &ln1_b = v[2], &wq = v[3], &wk = v[4], &wv = v[5], &wo = v[6],
+                 &ln2_w = v[7], &ln2_b = v[8], &w1 = v[9], &w2 = v[10], &wcat = v[11];
     const std::vector<int64_t> ints = ctx->saved_data["i"].toIntVector();
     const int64_t heads = ints[0];
     const bool has_b1 = ints[2] != 0, has_b2 = ints[3] != 0;
@@ -275,7 +277,8 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     const bool need_dx = need(0) || need(1) || need(2);
     side.mark();
     if (need_dx) {
-      const Mat wqkv = wcat.defined() ? as_matrix(wcat) : block(wq.data_ptr(), d, 3 * d);
+      Tensor cat;
+      const Mat wqkv = wcat.defined() ? as_matrix(wcat) : qkv_matrix(wq, wk, wv, &cat);
       gemm(mdqkv, wqkv.t(), k[chain_at], d, Epilogue{}, dtype, dev, st);
     }
     if (one_product) {
