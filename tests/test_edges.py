@@ -142,3 +142,25 @@ def test_layer_backward_from_copies_of_the_saved_tensors(hooks, fused):
         grads.append(torch.autograd.grad(y, [xi] + list(layer.parameters()), g))
     for a, b in zip(*grads):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("hooks", [_ContiguousCopies, torch.autograd.graph.save_on_cpu])
+@pytest.mark.parametrize("transposed", ["neither", "x", "w", "both"])
+@pytest.mark.parametrize("m,k,n", [(5, 9, 13), (33, 33, 33), (40, 64, 24), (130, 257, 71)])
+def test_linear_backward_from_copies_of_the_saved_tensors(hooks, transposed, m, k, n):
+    import contextlib
+    from tritonformer_b200.linear import LinearBias, LinearNoBiasReLU
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    mk = lambda r, c, t: (torch.randn(c, r, device="cuda", generator=gen).half().t() if t
+                          else torch.randn(r, c, device="cuda", generator=gen).half())
+    x, w = mk(m, k, transposed in ("x", "both")), mk(k, n, transposed in ("w", "both"))
+    b, g = mk(1, n, False)[0], mk(m, n, False)
+    for fn, extra in ((LinearBias, (b,)), (LinearNoBiasReLU, ())):
+        grads = []
+        for context in (contextlib.nullcontext, hooks):
+            args = [t.detach().requires_grad_() for t in (x, w, *extra)]
+            with context():
+                y = fn.apply(*args)
+            grads.append(torch.autograd.grad(y, args, g))
+        for a, c in zip(*grads):
+            assert torch.equal(a, c)

@@ -88,14 +88,15 @@ static Tensor linear_body(const Tensor& x, const Tensor& w, const Tensor& bias, 
   return y;
 }
 
-// A saved operand: the tensor itself, or the copy with aligned rows that forward made of it.
-static Mat saved_operand(const Mat& plain, const Tensor& packed) {
+// A saved operand: the tensor itself, or the copy with aligned rows that forward made of it, by rows or by columns.  Which of
+// the two forward says: a saved-tensor hook may have handed the plain tensor back with other strides.
+static Mat saved_operand(const Mat& plain, const Tensor& packed, bool by_rows) {
   if (!packed.defined()) return plain;
   Mat m = plain;
-  const bool rows_first = plain.s1 == 1;
   m.keep = packed;
   m.p = packed.data_ptr();
-  (rows_first ? m.s0 : m.s1) = packed.size(1);
+  m.s0 = by_rows ? packed.size(1) : 1;
+  m.s1 = by_rows ? 1 : packed.size(1);
   return m;
 }
 
@@ -106,7 +107,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     Tensor x = amp(x_), w = amp(w_);
     Mat mx, mw;
     Tensor y = linear_body(x, w, amp(val(bias_)), relu, &mx, &mw);
-    ctx->saved_data["bias"] = bias_.has_value();
+    ctx->saved_data["flags"] = int64_t(bias_.has_value() | (mx.s1 == 1) << 1 | (mw.s1 == 1) << 2);
     ctx->save_for_backward({x, w, relu ? y : Tensor(), mx.packed, mw.packed});
     return y;
   }
@@ -116,7 +117,8 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     const Tensor &x = saved[0], &w = saved[1], &act = saved[2];
     const at::ScalarType type = x.scalar_type();
     const int dtype = dtype_code(type);
-    const bool has_bias = ctx->saved_data["bias"].toBool();
+    const int64_t flags = ctx->saved_data["flags"].toInt();
+    const bool has_bias = flags & 1;
     const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
     const bool need_db = has_bias && ctx->needs_input_grad(2);
     Tensor dx, dw, db;
@@ -128,13 +130,13 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     } else if (need_db) {
       db = column_sum(dy);
     }
-    const Mat mw = saved_operand(as_matrix(w), saved[4]);
+    const Mat mw = saved_operand(as_matrix(w), saved[4], flags & 4);
     GradTarget g;
     Mat mx;
     if (need_dx) dx = at::empty(x.sizes(), x.options());
     if (need_dw) {
       g = weight_target(w, type);
-      mx = saved_operand(as_rows(x), saved[3]);
+      mx = saved_operand(as_rows(x), saved[3], flags & 2);
     }
     const bool fork = need_dx && need_dw && g.in_place && g_mode.fork.load(std::memory_order_relaxed);
     SideWork side(x, fork);
