@@ -164,3 +164,44 @@ def test_linear_backward_from_copies_of_the_saved_tensors(hooks, transposed, m, 
             grads.append(torch.autograd.grad(y, args, g))
         for a, c in zip(*grads):
             assert torch.equal(a, c)
+
+
+def _calls(dtype=torch.float16):
+    """(name, function of one floating tensor, that tensor) for every operator."""
+    from tritonformer_b200.attention import BiasedCausalAttention, CausalAttention
+    from tritonformer_b200.crossentropy import CrossEntropyLoss, CrossEntropyLossFP32, lm_loss
+    from tritonformer_b200.embedding import Embedding
+    from tritonformer_b200.layernorm import LayerNorm
+    from tritonformer_b200.linear import LinearBias, LinearBiasReLU, LinearNoBias, LinearNoBiasReLU
+    from tritonformer_b200.softmax import Softmax
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=gen).to(dtype)
+    x, w, b, q = r(2, 64, 128), r(128, 64), r(64), r(2, 2, 64, 64)
+    one, ids = r(128), torch.randint(0, 64, (2, 64), device="cuda", generator=gen)
+    layer = _layer(dtype).requires_grad_(False)
+    return [("linear", lambda t: LinearNoBias.apply(t, w), x), ("linear_weight", lambda t: LinearBias.apply(x, t, b), w),
+            ("linear_relu", lambda t: LinearNoBiasReLU.apply(t, w), x),
+            ("linear_bias_relu", lambda t: LinearBiasReLU.apply(x, w, t), b),
+            ("layernorm", lambda t: LayerNorm.apply(t, one, one, 1e-5), x), ("softmax", lambda t: Softmax.apply(t), x),
+            ("attention", lambda t: CausalAttention.apply(t, q, q), q),
+            ("attention_slopes", lambda t: BiasedCausalAttention.apply(q, q, t, torch.tensor([0.5, 0.25], device="cuda")), q),
+            ("cross_entropy", lambda t: CrossEntropyLoss.apply(t[0], ids[0]), x),
+            ("cross_entropy_fp32", lambda t: CrossEntropyLossFP32.apply(t[0], ids[0]), x),
+            ("lm_loss", lambda t: lm_loss(t, ids), x), ("embedding", lambda t: Embedding.apply(ids, t, None), w),
+            ("layer", lambda t: layer(t), x)]
+
+
+def test_forward_mode_and_transforms_are_refused():
+    """Not implemented, and said so: a result without its tangent would pass for a constant."""
+    import torch.autograd.forward_ad as fwd
+    for name, fn, x in _calls():
+        for grad in (False, True):
+            with torch.set_grad_enabled(grad), fwd.dual_level():
+                dual = fwd.make_dual(x.clone().requires_grad_(grad), torch.ones_like(x))
+                with pytest.raises(NotImplementedError):
+                    fn(dual)
+                fn(x)
+        with pytest.raises(RuntimeError):
+            torch.func.grad(lambda t: fn(t).float().sum())(x)
+        with torch.no_grad(), pytest.raises(RuntimeError):
+            torch.func.vmap(fn)(torch.stack([x, x]))

@@ -1,8 +1,10 @@
 // Autograd functions of the single operators.
 #include "functions.h"
 
+#include <ATen/FuncTorchTLS.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
+#include <torch/csrc/autograd/forward_grad.h>
 
 namespace tfb_host {
 
@@ -50,6 +52,18 @@ bool adjacent_columns(const Tensor* const* parts, int n, int64_t width) {
       return false;
   }
   return true;
+}
+
+bool needs_node(std::initializer_list<const Tensor*> inputs) {
+  if (const auto& functorch = at::functorch::functorchTLSAccessor()) functorch->checkSupportsCppAutogradFunction();
+  if (torch::autograd::ForwardADLevel::try_get_by_idx(0))
+    for (const Tensor* t : inputs)
+      TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(0).defined(),
+                                  "the operators of tritonformer_b200 have no forward-mode derivative");
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : inputs)
+    if (t->defined() && t->requires_grad()) return true;
+  return false;
 }
 
 // -------------------------------------------------------------------------------------------------------- linear
@@ -153,15 +167,8 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
   }
 };
 
-static bool any_requires_grad(std::initializer_list<const Tensor*> ts) {
-  if (!at::GradMode::is_enabled()) return false;
-  for (const Tensor* t : ts)
-    if (t->defined() && t->requires_grad()) return true;
-  return false;
-}
-
 Tensor linear(const Tensor& x, const Tensor& w, const Tensor& bias, bool relu) {
-  if (any_requires_grad({&x, &w, &bias})) return LinearFn::apply(x, w, opt(bias), relu);
+  if (needs_node({&x, &w, &bias})) return LinearFn::apply(x, w, opt(bias), relu);
   Amp amp;
   BodyGuard guard;
   Mat mx, mw;
@@ -189,7 +196,7 @@ struct LayerNormFn : torch::autograd::Function<LayerNormFn> {
 };
 
 Tensor layernorm(const Tensor& x, const Tensor& alpha, const Tensor& beta, double eps) {
-  if (any_requires_grad({&x, &alpha, &beta})) return LayerNormFn::apply(x, alpha, beta, eps);
+  if (needs_node({&x, &alpha, &beta})) return LayerNormFn::apply(x, alpha, beta, eps);
   Amp amp;
   BodyGuard guard;
   return std::get<0>(layernorm_forward(amp(x), amp(alpha), amp(beta), eps));
@@ -273,7 +280,7 @@ struct AttentionFn : torch::autograd::Function<AttentionFn> {
 
 Tensor attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& slopes, int64_t rounded, const Tensor& table,
                  bool with_amp) {
-  if (any_requires_grad({&q, &k, &v})) return AttentionFn::apply(q, k, v, opt(slopes), rounded, opt(table), with_amp);
+  if (needs_node({&q, &k, &v, &slopes, &table})) return AttentionFn::apply(q, k, v, opt(slopes), rounded, opt(table), with_amp);
   Amp amp;
   if (!with_amp) amp.on = false;
   BodyGuard guard;
@@ -321,7 +328,7 @@ struct SoftmaxFn : torch::autograd::Function<SoftmaxFn> {
 };
 
 Tensor softmax(const Tensor& x) {
-  if (any_requires_grad({&x})) return SoftmaxFn::apply(x);
+  if (needs_node({&x})) return SoftmaxFn::apply(x);
   BodyGuard guard;
   return softmax_body(x);
 }
@@ -370,7 +377,7 @@ struct CrossEntropyFn : torch::autograd::Function<CrossEntropyFn> {
 };
 
 Tensor cross_entropy(const Tensor& logits, const Tensor& labels, bool f32) {
-  if (any_requires_grad({&logits})) return CrossEntropyFn::apply(logits, labels, f32);
+  if (needs_node({&logits})) return CrossEntropyFn::apply(logits, labels, f32);
   Amp amp;
   BodyGuard guard;
   return cross_entropy_body(amp(logits), labels, f32).loss;
@@ -420,7 +427,7 @@ struct LmLossFn : torch::autograd::Function<LmLossFn> {
 };
 
 Tensor lm_loss(const Tensor& logits, const Tensor& labels) {
-  if (any_requires_grad({&logits})) return LmLossFn::apply(logits, labels);
+  if (needs_node({&logits})) return LmLossFn::apply(logits, labels);
   Amp amp;
   BodyGuard guard;
   Tensor l = amp(logits);
@@ -486,7 +493,7 @@ struct EmbeddingFn : torch::autograd::Function<EmbeddingFn> {
 };
 
 Tensor embedding(const Tensor& ids, const Tensor& tok, const Tensor& pos) {
-  if (any_requires_grad({&tok, &pos})) return EmbeddingFn::apply(ids, tok, opt(pos));
+  if (needs_node({&tok, &pos})) return EmbeddingFn::apply(ids, tok, opt(pos));
   Amp amp;
   BodyGuard guard;
   return embedding_body(ids, amp(tok), amp(pos));

@@ -19,6 +19,10 @@ struct BodyGuard {
   c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::autocast_dispatch_keyset};
 };
 
+// Whether a call needs an autograd node.  Without one the body runs below autograd, where a tangent would be lost and a
+// transform's wrapper has no memory, so what the nodes do not implement - forward mode, function transforms - is refused here.
+bool needs_node(std::initializer_list<const Tensor*> inputs);
+
 // Where a weight gradient goes: into the parameter's existing .grad (added, or written in overwrite mode), when a block of
 // linear.accumulate_into_grad is in force and the buffer fits, or into a new tensor that is returned to autograd.
 struct GradTarget {

@@ -310,13 +310,8 @@ Tensor layer(const Tensor& x, const LayerWeights& w, const Bias& bias_, int64_t 
     const Amp amp;
     bias.table = bias.table.to(amp.on ? amp.type : x.scalar_type());
   }
-  bool grad = at::GradMode::is_enabled();
-  if (grad) {
-    grad = false;
-    for (const Tensor* t : {&x, &w.ln1_w, &w.ln1_b, &w.wq, &w.wk, &w.wv, &w.wo, &w.ln2_w, &w.ln2_b, &w.w1, &w.b1, &w.w2, &w.b2})
-      grad = grad || (t->defined() && t->requires_grad());
-  }
-  if (grad)
+  if (needs_node({&x, &w.ln1_w, &w.ln1_b, &w.wq, &w.wk, &w.wv, &w.wo, &w.ln2_w, &w.ln2_b, &w.w1, &w.b1, &w.w2, &w.b2,
+                  &bias.slopes, &bias.table}))
     return LayerFn::apply(x, w.ln1_w, w.ln1_b, w.wq, w.wk, w.wv, w.wo, w.ln2_w, w.ln2_b, w.w1, w.w2, opt(w.b1), opt(w.b2), &bias,
                           heads, eps1, eps2);
   Amp a;
