@@ -205,3 +205,43 @@ def test_forward_mode_and_transforms_are_refused():
             torch.func.grad(lambda t: fn(t).float().sum())(x)
         with torch.no_grad(), pytest.raises(RuntimeError):
             torch.func.vmap(fn)(torch.stack([x, x]))
+
+
+def test_traced_operators_replay():
+    """A traced call gives on new inputs what the operator gives, and differentiates."""
+    for name, fn, x in _calls():
+        example = x.clone()
+        traced = torch.jit.trace(fn, example, check_trace=False)
+        new = torch.randn_like(x).flip(0)
+        with torch.no_grad():
+            assert torch.equal(traced(new), fn(new)), name
+        both = []
+        for f in (fn, traced):
+            t = new.clone().requires_grad_()
+            y = f(t)
+            both.append(torch.autograd.grad(y, t, torch.ones_like(y) * 0.5)[0])
+        assert torch.equal(*both), name
+
+
+@pytest.mark.parametrize("alibi", [False, True])
+def test_traced_model_replays(alibi):
+    from tritonformer_b200.transformer import Transformer, TransformerConfig
+    torch.manual_seed(0)
+    model = Transformer(TransformerConfig(vocab_size=96, hidden_size=128, max_position_embeddings=64, num_attention_heads=2,
+                                          head_dim=64, ffn_dim=256, num_hidden_layers=2, use_linear_bias=True,
+                                          attn_bias=alibi), device="cuda")
+    with torch.no_grad():
+        model.logits_out.weight.normal_(0.0, 0.02)
+    ids = torch.randint(0, 96, (2, 2, 64), device="cuda")
+
+    class Logits(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.model = model
+
+        def forward(self, t):
+            return self.model(t, None)
+
+    traced = torch.jit.trace(Logits(), ids[0], check_trace=False)
+    with torch.no_grad():
+        assert torch.equal(traced(ids[1]), model(ids[1], None))

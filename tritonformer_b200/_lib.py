@@ -82,6 +82,8 @@ try:
 except ImportError as e:
     raise RuntimeError("tritonformer_b200: the native host path _host.so is missing or does not load (%s). Build it with "
                        "`python tritonformer_b200/build.py`; there is no fallback implementation." % e) from e
+from . import _trace  # noqa: E402,F401  (registers itself with the host path)
+
 if os.environ.get("TFB_FORCE_GENERIC_GEMM") == "1":  # test switch, see tfb_debug_set
     lib.tfb_debug_set(0, 1)
 if os.environ.get("TFB_FORCE_GENERIC_ATTN") == "1":

@@ -1,6 +1,7 @@
 // Python binding of the native host path: plain CPython calls on positional arguments, the interpreter lock released
 // while kernels are enqueued (the backward pass runs on another thread).
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include "functions.h"
@@ -64,10 +65,32 @@ PyObject* tensor_result(F body) {
   return THPVariable_Wrap(out);
 }
 
-#define TFB_PY(name) PyObject* name(PyObject*, PyObject* const* argv, Py_ssize_t argc)
+#define TFB_PY(name) PyObject* name(PyObject* self, PyObject* const* argv, Py_ssize_t argc)
+
+PyObject* g_recorder = nullptr;  // what an operator's call goes to while torch.jit.trace records (_trace.py)
+
+// An operator: the call itself, or while a trace is being recorded recorder(operator, *arguments).
+template <typename F>
+PyObject* traceable(PyObject* self, const char* name, PyObject* const* argv, Py_ssize_t argc, F body) {
+  if (C10_LIKELY(!torch::jit::tracer::isTracing() || !g_recorder)) return guarded(body);
+  PyObject* args = PyTuple_New(argc + 1);
+  if (!args) return nullptr;
+  PyObject* op = PyObject_GetAttrString(self, name);
+  PyObject* out = nullptr;
+  if (op) {
+    PyTuple_SET_ITEM(args, 0, op);
+    for (Py_ssize_t i = 0; i < argc; ++i) {
+      Py_INCREF(argv[i]);
+      PyTuple_SET_ITEM(args, i + 1, argv[i]);
+    }
+    out = PyObject_Call(g_recorder, args, nullptr);
+  }
+  Py_DECREF(args);
+  return out;
+}
 
 TFB_PY(py_linear) {
-  return guarded([&] {
+  return traceable(self, "linear", argv, argc, [&] {
     Args a(argv, argc, 4, "linear");
     const Tensor &x = a.tensor(), &w = a.tensor(), &b = a.tensor();
     const bool relu = a.truth();
@@ -75,7 +98,7 @@ TFB_PY(py_linear) {
   });
 }
 TFB_PY(py_layernorm) {
-  return guarded([&] {
+  return traceable(self, "layernorm", argv, argc, [&] {
     Args a(argv, argc, 4, "layernorm");
     const Tensor &x = a.tensor(), &w = a.tensor(), &b = a.tensor();
     const double eps = a.real();
@@ -83,7 +106,7 @@ TFB_PY(py_layernorm) {
   });
 }
 TFB_PY(py_attention) {  // q, k, v, slopes, rounded, table, amp
-  return guarded([&] {
+  return traceable(self, "attention", argv, argc, [&] {
     Args a(argv, argc, 7, "attention");
     const Tensor &q = a.tensor(), &k = a.tensor(), &v = a.tensor(), &slopes = a.tensor();
     const int64_t rounded = a.integer();
@@ -93,14 +116,14 @@ TFB_PY(py_attention) {  // q, k, v, slopes, rounded, table, amp
   });
 }
 TFB_PY(py_softmax) {
-  return guarded([&] {
+  return traceable(self, "softmax", argv, argc, [&] {
     Args a(argv, argc, 1, "softmax");
     const Tensor& x = a.tensor();
     return tensor_result([&] { return softmax(x); });
   });
 }
 TFB_PY(py_cross_entropy) {  // logits, labels, fp32 losses
-  return guarded([&] {
+  return traceable(self, "cross_entropy", argv, argc, [&] {
     Args a(argv, argc, 3, "cross_entropy");
     const Tensor &x = a.tensor(), &y = a.tensor();
     const bool f32 = a.truth();
@@ -108,14 +131,14 @@ TFB_PY(py_cross_entropy) {  // logits, labels, fp32 losses
   });
 }
 TFB_PY(py_lm_loss) {
-  return guarded([&] {
+  return traceable(self, "lm_loss", argv, argc, [&] {
     Args a(argv, argc, 2, "lm_loss");
     const Tensor &x = a.tensor(), &y = a.tensor();
     return tensor_result([&] { return lm_loss(x, y); });
   });
 }
 TFB_PY(py_embedding) {
-  return guarded([&] {
+  return traceable(self, "embedding", argv, argc, [&] {
     Args a(argv, argc, 3, "embedding");
     const Tensor &ids = a.tensor(), &tok = a.tensor(), &pos = a.tensor();
     return tensor_result([&] { return embedding(ids, tok, pos); });
@@ -123,7 +146,7 @@ TFB_PY(py_embedding) {
 }
 // x, ln1_w, ln1_b, wq, wk, wv, wo, ln2_w, ln2_b, w1, b1, w2, b2, slopes, rounded, table, heads, eps1, eps2
 TFB_PY(py_layer) {
-  return guarded([&] {
+  return traceable(self, "layer", argv, argc, [&] {
     Args a(argv, argc, 19, "layer");
     const Tensor& x = a.tensor();
     LayerWeights w;
@@ -172,6 +195,14 @@ TFB_PY(py_gemm_workspace) {  // device index, stream handle
     });
   });
 }
+TFB_PY(py_set_recorder) {
+  return guarded([&]() -> PyObject* {
+    if (argc != 1) throw ArgumentError("set_recorder: wrong number of arguments");
+    Py_INCREF(argv[0]);
+    Py_XDECREF(std::exchange(g_recorder, argv[0]));
+    Py_RETURN_NONE;
+  });
+}
 TFB_PY(py_reset_workspaces) {
   return guarded([&]() -> PyObject* {
     reset_workspaces();
@@ -183,7 +214,7 @@ TFB_PY(py_reset_workspaces) {
 PyMethodDef methods[] = {TFB_METHOD(linear), TFB_METHOD(layernorm), TFB_METHOD(attention), TFB_METHOD(softmax),
                          TFB_METHOD(cross_entropy), TFB_METHOD(lm_loss), TFB_METHOD(embedding), TFB_METHOD(layer),
                          TFB_METHOD(set_grad_mode), TFB_METHOD(take_written), TFB_METHOD(join_weight_grads),
-                         TFB_METHOD(gemm_workspace), TFB_METHOD(reset_workspaces), {nullptr, nullptr, 0, nullptr}};
+                         TFB_METHOD(gemm_workspace), TFB_METHOD(reset_workspaces), TFB_METHOD(set_recorder), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Native host path of tritonformer_b200.", -1, methods,
                       nullptr, nullptr, nullptr, nullptr};
 
