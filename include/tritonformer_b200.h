@@ -162,7 +162,7 @@ int tfb_colsum(const void* x, void* out, float* partials, int64_t n_partials,
 
 /* What the backward of a linear layer needs before its products, in one pass: dz = act > 0 ? dy : 0 (act may be NULL: a
  * copy) and, unless `sums` is NULL, sums[j] = sum_i dz[i,j] (scratch: tfb_colsum_partials() rows of `cols` floats).  dy and
- * act may have any row pitch and any base; dz has 16-byte aligned rows (dz_ld a multiple of 8, at least cols rounded up
+ * act may have any row pitch (0 and overlapping rows too) and any base; dz has 16-byte aligned rows (dz_ld a multiple of 8, at least cols rounded up
  * to one; the padding is written with zeros), as the tcgen05 GEMM wants its operands.                          */
 int tfb_grad_rows(const void* dy, const void* act, void* dz, void* sums, float* partials, int64_t n_partials,
                   int64_t rows, int64_t cols, int64_t dy_ld, int64_t act_ld, int64_t dz_ld, int dtype,

@@ -245,3 +245,38 @@ def test_traced_model_replays(alibi):
     traced = torch.jit.trace(Logits(), ids[0], check_trace=False)
     with torch.no_grad():
         assert torch.equal(traced(ids[1]), model(ids[1], None))
+
+
+@pytest.mark.parametrize("form", ["LinearNoBias", "LinearBias", "LinearNoBiasReLU", "LinearBiasReLU"])
+@pytest.mark.parametrize("k,n", [(128, 64), (77, 51)])
+@pytest.mark.parametrize("dtype", HALF)
+def test_linear_takes_broadcast_and_overlapping_rows(form, k, n, dtype):
+    """Rows that repeat (stride 0) or overlap, as an input and as a gradient, give what their copies give."""
+    import tritonformer_b200.linear as L
+    fn, bias = getattr(L, form), "NoBias" not in form
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=gen).to(dtype)
+    w, b = r(k, n), r(n)
+    inputs = [r(1, k).expand(9, k), r(k + 30).unfold(0, k, 3), r(2, 1, k).expand(2, 5, k), r(1, 1, k).expand(2, 5, k), r(6, k)]
+    for x in inputs:
+        rows = x.shape[:-1]
+        for g in (r(n).expand(*rows, n), r(n + len(rows) * 16).unfold(0, n, 1)[: rows[-1]].expand(*rows, n), r(*rows, n)):
+            sides = []
+            for xi, gi in ((x, g), (x.contiguous(), g.contiguous())):
+                args = [t.detach().requires_grad_() for t in ((xi, w, b) if bias else (xi, w))]
+                y = fn.apply(*args)
+                sides.append((y.detach(),) + torch.autograd.grad(y, args, gi))
+            for one, two in zip(*sides):
+                assert torch.equal(one, two)
+
+
+@pytest.mark.parametrize("form", ["LinearNoBias", "LinearBias", "LinearNoBiasReLU", "LinearBiasReLU"])
+def test_linear_gradient_of_a_sum_over_rows(form):
+    import tritonformer_b200.linear as L
+    x, w, b = (torch.randn(*s, device="cuda").half() for s in ((2, 7, 64), (64, 40), (40,)))
+    args = [t.requires_grad_() for t in ((x, w, b) if "NoBias" not in form else (x, w))]
+    y = getattr(L, form).apply(*args)
+    got = torch.autograd.grad(y.sum((0, 1)), args, torch.ones(40, device="cuda").half())
+    want = torch.autograd.grad(getattr(L, form).apply(*args), args, torch.ones_like(y))
+    for a, c in zip(got, want):
+        assert torch.equal(a, c)

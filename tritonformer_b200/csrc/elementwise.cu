@@ -146,7 +146,7 @@ extern "C" int tfb_grad_rows(const void* dy, const void* act, void* dz, void* su
                              int64_t rows, int64_t cols, int64_t dy_ld, int64_t act_ld, int64_t dz_ld, int dtype,
                              void* stream) {
   TFB_REQUIRE(rows >= 0 && cols > 0 && cols < (1LL << 31) - 256, "grad_rows: bad shape");
-  TFB_REQUIRE(dy_ld >= cols && (!act || act_ld >= cols), "grad_rows: row stride smaller than cols");
+  TFB_REQUIRE(dy_ld >= 0 && (!act || act_ld >= 0), "grad_rows: negative row stride");  // rows may repeat or overlap: only read
   TFB_REQUIRE(aligned16(dz) && dz_ld % 8 == 0 && dz_ld >= ceil_div(cols, 8) * 8, "grad_rows: dz rows must be 16-byte aligned");
   TFB_REQUIRE(!sums || (partials && n_partials == tfb_colsum_partials(rows, cols)),
               "grad_rows: scratch must hold tfb_colsum_partials() rows");
