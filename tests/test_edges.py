@@ -280,3 +280,27 @@ def test_linear_gradient_of_a_sum_over_rows(form):
     want = torch.autograd.grad(getattr(L, form).apply(*args), args, torch.ones_like(y))
     for a, c in zip(got, want):
         assert torch.equal(a, c)
+
+
+@pytest.mark.parametrize("t,hd", [(64, 64), (192, 64), (192, 128), (128, 32), (192, 32)])
+@pytest.mark.parametrize("which", ["q", "k", "v", "grad_heads", "grad_batch", "grad_rows"])
+def test_attention_takes_broadcast_operands(t, hd, which):
+    """One head's operand for all heads, or a gradient that repeats over heads, batch or positions."""
+    from tritonformer_b200.attention import CausalAttention
+    gen = torch.Generator(device="cuda").manual_seed(t + hd)
+    q, k, v, g = (torch.randn(2, 3, t, hd, device="cuda", generator=gen).half() for _ in range(4))
+    if which in "qkv":
+        one = {"q": q, "k": k, "v": v}[which][:1, :1].expand(2, 3, t, hd)
+        q, k, v = (one if n == which else x for n, x in (("q", q), ("k", k), ("v", v)))
+    else:
+        g = {"grad_heads": g[:, :1], "grad_batch": g[:1], "grad_rows": g[:, :, :1]}[which].expand(2, 3, t, hd)
+    args = [x.detach().requires_grad_() for x in (q, k, v)]
+    out = CausalAttention.apply(*args)
+    got = (out.detach(),) + torch.autograd.grad(out, args, g)
+    qd, kd, vd = (x.detach().double().requires_grad_() for x in (q, k, v))
+    s = (qd @ kd.transpose(-1, -2)) / hd ** 0.5
+    s = s.masked_fill(~torch.ones(t, t, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    ref = torch.softmax(s, -1) @ vd
+    want = (ref.detach(),) + torch.autograd.grad(ref, (qd, kd, vd), g.double())
+    for a, b in zip(got, want):  # P, dS, the output in delta and the result are each rounded to 16 bits
+        assert ((a.double() - b).norm() / b.norm()).item() < 4 * 2.0 ** -11

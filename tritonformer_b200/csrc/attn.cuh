@@ -21,6 +21,9 @@ struct AttnArgs {
   int64_t bias_sh, bias_si;
 };
 
+// Whole tiles of the full width: 128-row tiles and a head_dim that fills its panels.
+inline bool attn_whole_tiles(const AttnArgs& a, int hd) { return hd >= 64 && a.T % 128 == 0; }
+inline bool attn_strides_positive(const AttnStrides& s) { return s.b > 0 && s.h > 0 && s.t > 0; }
 
 // The tcgen05 kernels order their CTAs longest walk first ACROSS batch*head slices.  The slices walked
 // together keep their K and V (forward) or Q, K, V, dO (backward) live in the L2 at the same time; this

@@ -803,7 +803,10 @@ static int encode_bhtd(CUtensorMap* m, const void* ptr, const AttnStrides& s, in
   return encode_tmap_sw128(m, ptr, dtype, 4, dims, str, box);
 }
 
-bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd) { return hd <= 128 && a.bias_mode != 3; }
+bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd) {  // as in the forward
+  return a.bias_mode != 3 && (attn_whole_tiles(a, hd) || (attn_strides_positive(a.sq) && attn_strides_positive(a.sk) &&
+                                                          attn_strides_positive(a.sv) && attn_strides_positive(a.sdo)));
+}
 
 template <typename T, int HD, bool RAGGED>
 static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {

@@ -800,15 +800,19 @@ static int fwd1_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   return launched("attention_fwd(tcgen05, persistent)");
 }
 
-// The tcgen05 kernels take everything but a dense bias table.
-bool attn_tc05_fwd_eligible(const AttnArgs& a, int hd) { return hd <= 128 && a.bias_mode != 3; }
+// The tcgen05 kernels take everything but a dense bias table.  An operand that repeats itself (stride 0: one head's keys for
+// all, the gradient of a sum) has no tensor map that is certain to be encodable, and outside of whole tiles of the full width
+// such calls have always run on the generic kernel.
+bool attn_tc05_fwd_eligible(const AttnArgs& a, int hd) {
+  return a.bias_mode != 3 && (attn_whole_tiles(a, hd) || (attn_strides_positive(a.sq) && attn_strides_positive(a.sk) &&
+                                                          attn_strides_positive(a.sv)));
+}
 
 int attn_fwd1_tc05(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   TFB_DISPATCH_16(dtype, T, {
-    if (hd < 64 || (hd == 64 && a.T % F1_TILE)) return fwd1_launch<T, 64, false>(a, hd, dtype, st);
-    if (hd == 64) return fwd1_launch<T, 64, true>(a, hd, dtype, st);
-    if (a.T % F1_TILE) return fwd1_launch<T, 128, false>(a, hd, dtype, st);
-    return fwd1_launch<T, 128, true>(a, hd, dtype, st);
+    const bool whole = attn_whole_tiles(a, hd);
+    if (hd <= 64) return whole ? fwd1_launch<T, 64, true>(a, hd, dtype, st) : fwd1_launch<T, 64, false>(a, hd, dtype, st);
+    return whole ? fwd1_launch<T, 128, true>(a, hd, dtype, st) : fwd1_launch<T, 128, false>(a, hd, dtype, st);
   })
 }
 
