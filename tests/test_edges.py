@@ -304,3 +304,26 @@ def test_attention_takes_broadcast_operands(t, hd, which):
     want = (ref.detach(),) + torch.autograd.grad(ref, (qd, kd, vd), g.double())
     for a, b in zip(got, want):  # P, dS, the output in delta and the result are each rounded to 16 bits
         assert ((a.double() - b).norm() / b.norm()).item() < 4 * 2.0 ** -11
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 64, 64), (256, 256, 256), (300, 248, 640), (640, 1000, 512)])
+def test_one_wave_product_with_an_epilogue_operand_after_an_expired_wait(m, n, k):
+    """While the status word is set a product writes nothing and leaves no load of its addend or mask on the way; the
+    products behind it are right again once the word is cleared."""
+    from tritonformer_b200 import _lib as L, linear as LIN
+    assert L.device_status() == 0
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    a, b, add, mask = (torch.randn(*s, device="cuda", generator=gen).half() for s in ((m, k), (k, n), (m, n), (m, n)))
+    b *= k ** -0.5
+    L.check(L.lib.tfb_debug_wait_probe(1_000_000, None, L.stream_ptr(a.device)))
+    out = torch.full((m, n), 777.0, device="cuda", dtype=torch.float16)
+    for _ in range(20):
+        LIN.gemm(a, k, 1, b, n, 1, m, n, k, addend=add, out=out)
+        LIN.gemm(a, k, 1, b, n, 1, m, n, k, mask=mask, out=out)
+    assert bool((out == 777.0).all())
+    assert L.device_status(reset=True) == 0x7E00
+    want = a.double() @ b.double()
+    for _ in range(5):
+        got = LIN.gemm(a, k, 1, b, n, 1, m, n, k, addend=add)
+        assert (got.double() - (want + add.double())).abs().max().item() <= 2.0 ** -10 * (want.abs().max().item() + 8)
+    assert L.device_status() == 0

@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
                             reinterpret_cast<const T*>(p.mask), p.ldc, p.ld_addend, p.ld_mask, p.M, p.N, p.relu},
                            &tmC, &tmX, boxes + ew * 8192, boxes + ew * 8192 + 4096, &x_full[ew], use_x, p.addend != nullptr,
                            p.direct != 0, (p.addend != nullptr && p.mask != nullptr) ? reinterpret_cast<const T*>(p.mask) : nullptr};
-      if (use_x && lane == 0) {  // in flight while the main loop runs
+      if (use_x && !dead && lane == 0) {  // in flight while the main loop runs; waited for by epilogue_tile, or below
         mbar_expect_tx(&x_full[ew], 4096);
         tma_load_2d(epi.stage_x, &tmX, n0 + col, row0, &x_full[ew]);
       }
@@ -306,7 +306,13 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
       tc_fence_after();
       __syncwarp();
       if (PAIR) gt_cluster_arrive_relaxed();  // matched by the wait before the exit
-      if (ok && !dead) epilogue_tile<T>(epi, steps, taddr + col, row0, n0 + col, lane, x_phase, abort_flag, 0x500 | ew, ok);
+      if (ok && !dead) {
+        epilogue_tile<T>(epi, steps, taddr + col, row0, n0 + col, lane, x_phase, abort_flag, 0x500 | ew, ok);
+      } else if (use_x && !dead) {  // no CTA leaves with a load into its shared memory on the way (a millisecond at most)
+        const uint64_t t0 = global_ns();
+        while (!mbar_try_wait(&x_full[ew], 0) && global_ns() - t0 < 1000000) {
+        }
+      }
       if (lane == 0) tma_store_wait_read();  // the boxes have been read; the kernel's end completes the writes
     } else {
       bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
