@@ -327,3 +327,14 @@ def test_one_wave_product_with_an_epilogue_operand_after_an_expired_wait(m, n, k
         got = LIN.gemm(a, k, 1, b, n, 1, m, n, k, addend=add)
         assert (got.double() - (want + add.double())).abs().max().item() <= 2.0 ** -10 * (want.abs().max().item() + 8)
     assert L.device_status() == 0
+
+
+def test_what_a_backward_refuses_is_an_assertion_error():
+    from tritonformer_b200.attention import CausalAttention
+    args = [torch.randn(1, 2, 128, 64, device="cuda").half().requires_grad_() for _ in range(3)]
+    out = CausalAttention.apply(*args)
+    unaligned = torch.randn(out.numel() + 1, device="cuda").half()[1:].view_as(out)
+    with pytest.raises(AssertionError, match="grad_out needs a 16-byte aligned base"):
+        out.backward(unaligned)
+    with pytest.raises(AssertionError, match="multiple of 64"):
+        CausalAttention.apply(*(a[:, :, :100] for a in args))

@@ -10,6 +10,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
+#include <torch/csrc/Exceptions.h>
 
 #include <atomic>
 #include <mutex>
@@ -24,9 +25,11 @@ namespace tfb_host {
 
 using at::Tensor;
 
-// Raised for a bad argument; becomes an AssertionError in Python, like the reference's asserts.
-struct ArgumentError : std::runtime_error {
-  using std::runtime_error::runtime_error;
+// Raised for a bad argument; becomes an AssertionError in Python, like the reference's asserts, also where a backward raises it
+// on a thread of the autograd engine (which hands the exception on and knows this base class).
+struct ArgumentError : torch::PyTorchError {
+  using torch::PyTorchError::PyTorchError;
+  PyObject* python_type() override { return PyExc_AssertionError; }
 };
 #define TFB_ASSERT(cond, msg) \
   do {                        \

@@ -46,12 +46,7 @@ class Args {
 template <typename F>
 PyObject* guarded(F body) {
   HANDLE_TH_ERRORS
-  try {
-    return body();
-  } catch (const ArgumentError& e) {
-    PyErr_SetString(PyExc_AssertionError, e.what());
-    return nullptr;
-  }
+  return body();
   END_HANDLE_TH_ERRORS
 }
 
