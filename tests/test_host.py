@@ -28,3 +28,33 @@ def test_a_traced_call_replays_and_differentiates():
         assert torch.allclose(a, b, rtol=1e-6, atol=1e-6)
     with torch.no_grad():
         assert torch.allclose(traced(x), model(x))
+
+
+def test_overlap_switches_act_when_they_are_set(monkeypatch):
+    from tritonformer_b200 import linear
+    told = []
+    real = linear._host
+
+    class Host:
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+        def set_grad_mode(self, *mode):
+            told.append(mode)
+            real.set_grad_mode(*mode)
+
+    monkeypatch.setattr(linear, "_host", Host())
+    before = linear.FORK_WEIGHT_GRAD
+    try:
+        linear.FORK_WEIGHT_GRAD = False
+        assert told[-1] == (False, False, False, False)
+        linear.FORK_WEIGHT_GRAD = True
+        assert told[-1] == (False, False, False, True)
+        with linear.accumulate_into_grad(overwrite=True):
+            assert told[-1] == (True, True, False, True)
+            linear.FORK_WEIGHT_GRAD = False
+            assert told[-1] == (True, True, False, False)
+        assert told[-1] == (False, False, False, False)
+    finally:
+        linear.FORK_WEIGHT_GRAD = before
+    assert told[-1][3] == before

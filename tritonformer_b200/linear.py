@@ -13,6 +13,8 @@ The incoming gradient is never modified (the reference masks it in place).
 import os
 import contextlib
 import ctypes
+import sys
+import types
 
 import torch
 from torch.autograd import Function
@@ -246,7 +248,6 @@ def weight_grad(x, dy, w):
 # blocks of `transformer.py` are such a graph (the residual sums happen inside kernels, into fresh tensors).
 FORK_WEIGHT_GRAD = os.environ.get("TFB_FORK_DW", "1") != "0"
 DEFER_WEIGHT_GRAD_JOIN = False  # set by the accumulate_into_grad block in force
-_tell_host()
 _side_streams = {}
 _unjoined = {}  # (device index, compute stream handle) -> (compute stream, side stream) with work not yet joined
 
@@ -433,3 +434,16 @@ class LinearBiasReLU(Function):
     @amp_backward
     def backward(ctx, grad_output):
         return _backward(ctx, grad_output, True, True)
+
+
+class _Switches(types.ModuleType):
+    """This module's class: the native host path hears of a switch when it is set, not when the next block begins."""
+
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        if name in ("FORK_WEIGHT_GRAD", "DEFER_WEIGHT_GRAD_JOIN"):
+            _tell_host()
+
+
+sys.modules[__name__].__class__ = _Switches
+_tell_host()
