@@ -338,3 +338,11 @@ def test_what_a_backward_refuses_is_an_assertion_error():
         out.backward(unaligned)
     with pytest.raises(AssertionError, match="multiple of 64"):
         CausalAttention.apply(*(a[:, :, :100] for a in args))
+
+
+def test_a_layer_refuses_an_empty_batch_where_it_comes_in():
+    layer = _layer()
+    for shape in ((0, 64, 128), (2, 0, 128)):
+        for grad in (False, True):
+            with torch.set_grad_enabled(grad), pytest.raises(AssertionError, match="attention: bad shape"):
+                layer(torch.empty(shape, device="cuda", dtype=torch.float16))

@@ -80,6 +80,9 @@ static void check_layer(const Tensor& x, LayerWeights& w, int64_t heads) {
     TFB_ASSERT(p->size(0) == d && p->size(1) == d, "Dimension mismatch in the attention projections");
   TFB_ASSERT(w.w1.size(0) == d && w.w2.size(0) == f && w.w2.size(1) == d, "Dimension mismatch in the MLP");
   TFB_ASSERT(heads > 0 && d % heads == 0, "the number of heads must divide the hidden size");
+  if (x.size(0) == 0 || x.size(1) == 0)
+    throw ArgumentError("attention: bad shape B=" + std::to_string(x.size(0)) + " H=" + std::to_string(heads) +
+                        " T=" + std::to_string(x.size(1)));
   check_attention({x.size(0), heads, x.size(1), d / heads}, x.scalar_type());
   for (Tensor* p : {&w.ln1_w, &w.ln1_b, &w.ln2_w, &w.ln2_b}) {
     TFB_ASSERT(p->scalar_type() == x.scalar_type(), "LayerNorm parameters must match the input dtype");
@@ -108,7 +111,6 @@ static Tensor layer_forward(const Tensor& x, const LayerWeights& w, const Bias& 
   cudaStream_t st = current_stream(x);
   s.slab.allocate(x);
   Tensor y = at::empty(x.sizes(), x.options());
-  if (rows == 0) return y;
 
   norm_forward(x.data_ptr(), w.ln1_w, w.ln1_b, s.slab[s.normed1], s.floats(s.stats1), rows, d, eps1, dtype, st);
   gemm(block(s.slab[s.normed1], rows, d), qkv_matrix(w.wq, w.wk, w.wv, wcat), s.slab[s.qkv], 3 * d, Epilogue{}, dtype, dev, st);
@@ -175,7 +177,6 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     const Tensor dy = grads[0].to(type).contiguous();
     const Mat mdy = block(dy.data_ptr(), rows, d);
     Tensor db1, db2;
-    TORCH_CHECK(rows > 0, "the layer has no backward for an empty batch");
 
     // where the weight gradients go (all targets exist before the side stream starts)
     GradTarget gw1, gw2, gwo, gq[3], gqkv;
