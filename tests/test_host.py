@@ -58,3 +58,15 @@ def test_overlap_switches_act_when_they_are_set(monkeypatch):
     finally:
         linear.FORK_WEIGHT_GRAD = before
     assert told[-1][3] == before
+
+
+def test_a_table_that_was_used_can_be_saved(tmp_path):
+    from tritonformer_b200.attention import _resolve_bias
+    from tritonformer_b200.transformer import generate_alibi_mask
+    table = generate_alibi_mask(64, 4, device="cpu")[0]
+    found = _resolve_bias(table, 4, 64, torch.float16)
+    assert found.table is None and found.rounded == 1
+    torch.save(table, tmp_path / "table.pt")
+    again = torch.load(tmp_path / "table.pt")  # weights only
+    assert torch.equal(again, table)
+    assert torch.equal(_resolve_bias(again, 4, 64, torch.float16).slopes, found.slopes)

@@ -72,15 +72,14 @@ def _resolve_bias(attn_bias, heads, seq, dtype):
     assert attn_bias.shape[1] >= seq, "attention bias is smaller than the sequence"
     # The verdict is remembered ON the tensor object (with the version counter it was taken at), so it dies
     # with the tensor: another table that later lands at the same address is a different object and is
-    # examined afresh.  In-place writes bump the counter; writes through `.data` do not and are not seen.
+    # examined afresh.  In-place writes bump the counter; writes through `.data` do not and are not seen.  It is kept as
+    # plain values, because it is saved with the tensor.
     memo = getattr(attn_bias, "_tfb_alibi", None)
     if memo is None or memo[0] != attn_bias._version:
-        slopes = _detect_alibi(attn_bias)
-        found = _Bias(slopes=slopes, rounded=1 if attn_bias.dtype is torch.float16 else 2) if slopes is not False else None
-        memo = (attn_bias._version, found)
+        memo = (attn_bias._version, _detect_alibi(attn_bias))
         attn_bias._tfb_alibi = memo
-    if memo[1] is not None:
-        return memo[1]
+    if memo[1] is not False:
+        return _Bias(slopes=memo[1], rounded=1 if attn_bias.dtype is torch.float16 else 2)
     table = attn_bias if attn_bias.dtype == dtype else attn_bias.to(dtype)
     return _Bias(table=_unit_inner(table))
 
