@@ -51,6 +51,7 @@ Tensor embedding(const Tensor& ids, const Tensor& tok, const Tensor& pos);
 struct LayerWeights {
   Tensor ln1_w, ln1_b, wq, wk, wv, wo, ln2_w, ln2_b, w1, b1, w2, b2;
 };
-Tensor layer(const Tensor& x, const LayerWeights& w, const Bias& bias, int64_t heads, double eps1, double eps2);
+// act: where wanted, the hidden activations that the layer keeps (a view of what its node has saved)
+Tensor layer(const Tensor& x, const LayerWeights& w, const Bias& bias, int64_t heads, double eps1, double eps2, Tensor* act);
 
 }  // namespace tfb_host

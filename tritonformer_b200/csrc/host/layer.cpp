@@ -49,6 +49,10 @@ struct Saved {
     act = slab.add(rows * f * 2);
   }
   float* floats(size_t at) const { return reinterpret_cast<float*>(slab[at]); }
+  Tensor activations(const Tensor& x, int64_t f) const {  // relu(LN2(h) W1 + b1) as a tensor
+    const int64_t rows = x.size(0) * x.size(1);
+    return slab.buf.narrow(0, (int64_t)act, rows * f * 2).view(x.scalar_type()).view({x.size(0), x.size(1), f});
+  }
 };
 
 static const void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
@@ -139,7 +143,7 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x_, const Tensor& ln1_w, const Tensor& ln1_b, const Tensor& wq,
                         const Tensor& wk, const Tensor& wv, const Tensor& wo, const Tensor& ln2_w, const Tensor& ln2_b,
                         const Tensor& w1, const Tensor& w2, const OptTensor& b1, const OptTensor& b2, const Bias* bias,
-                        int64_t heads, double eps1, double eps2) {
+                        int64_t heads, double eps1, double eps2, Tensor* act) {
     Amp a;
     BodyGuard guard;
     LayerWeights w{a(ln1_w), a(ln1_b), a(wq), a(wk), a(wv), a(wo), a(ln2_w), a(ln2_b), a(w1), a(val(b1)), a(w2), a(val(b2))};
@@ -148,6 +152,7 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     Saved s(x.size(0) * x.size(1), x.size(2), w.w1.size(1), heads);
     Tensor wcat;
     Tensor y = layer_forward(x, w, *bias, heads, eps1, eps2, s, &wcat);
+    if (act) *act = s.activations(x, w.w1.size(1));
     ctx->save_for_backward({x, w.ln1_w, w.ln1_b, w.wq, w.wk, w.wv, w.wo, w.ln2_w, w.ln2_b, w.w1, w.w2, wcat, s.slab.buf,
                             bias->slopes, bias->table});
     ctx->saved_data["i"] = std::vector<int64_t>{heads, bias->rounded, b1.has_value(), b2.has_value()};
@@ -301,11 +306,11 @@ struct LayerFn : torch::autograd::Function<LayerFn> {
     for (const Tensor& kept : {dy, s.slab.buf, k.buf}) side.keep(kept);
     side.join(all_in_place && g_mode.defer.load(std::memory_order_relaxed));
     return {need_dx ? dx : Tensor(), da1, db1n, gq[0].fresh, gq[1].fresh, gq[2].fresh, gwo.fresh, da2, db2n, gw1.fresh, gw2.fresh, db1, db2,
-            Tensor(), Tensor(), Tensor(), Tensor()};
+            Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
-Tensor layer(const Tensor& x, const LayerWeights& w, const Bias& bias_, int64_t heads, double eps1, double eps2) {
+Tensor layer(const Tensor& x, const LayerWeights& w, const Bias& bias_, int64_t heads, double eps1, double eps2, Tensor* act) {
   Bias bias = bias_;
   if (bias.table.defined()) {  // the attention reads the table in the type it computes in
     const Amp amp;
@@ -314,7 +319,7 @@ Tensor layer(const Tensor& x, const LayerWeights& w, const Bias& bias_, int64_t 
   if (needs_node({&x, &w.ln1_w, &w.ln1_b, &w.wq, &w.wk, &w.wv, &w.wo, &w.ln2_w, &w.ln2_b, &w.w1, &w.b1, &w.w2, &w.b2,
                   &bias.slopes, &bias.table}))
     return LayerFn::apply(x, w.ln1_w, w.ln1_b, w.wq, w.wk, w.wv, w.wo, w.ln2_w, w.ln2_b, w.w1, w.w2, opt(w.b1), opt(w.b2), &bias,
-                          heads, eps1, eps2);
+                          heads, eps1, eps2, act);
   Amp a;
   BodyGuard guard;
   LayerWeights c{a(w.ln1_w), a(w.ln1_b), a(w.wq), a(w.wk), a(w.wv), a(w.wo), a(w.ln2_w), a(w.ln2_b), a(w.w1), a(w.b1), a(w.w2),
@@ -323,7 +328,9 @@ Tensor layer(const Tensor& x, const LayerWeights& w, const Bias& bias_, int64_t 
   check_layer(xc, c, heads);
   Saved s(xc.size(0) * xc.size(1), xc.size(2), c.w1.size(1), heads);
   Tensor wcat;
-  return layer_forward(xc, c, bias, heads, eps1, eps2, s, &wcat);
+  Tensor y = layer_forward(xc, c, bias, heads, eps1, eps2, s, &wcat);
+  if (act) *act = s.activations(xc, c.w1.size(1));
+  return y;
 }
 
 }  // namespace tfb_host

@@ -140,20 +140,28 @@ TFB_PY(py_embedding) {
   });
 }
 // x, ln1_w, ln1_b, wq, wk, wv, wo, ln2_w, ln2_b, w1, b1, w2, b2, slopes, rounded, table, heads, eps1, eps2
+PyObject* layer_call(PyObject* const* argv, Py_ssize_t argc, Tensor* act) {
+  Args a(argv, argc, 19, "layer");
+  const Tensor& x = a.tensor();
+  LayerWeights w;
+  for (Tensor* t : {&w.ln1_w, &w.ln1_b, &w.wq, &w.wk, &w.wv, &w.wo, &w.ln2_w, &w.ln2_b, &w.w1, &w.b1, &w.w2, &w.b2})
+    *t = a.tensor();
+  Bias bias;
+  bias.slopes = a.tensor();
+  bias.rounded = (int)a.integer();
+  bias.table = a.tensor();
+  const int64_t heads = a.integer();
+  const double eps1 = a.real(), eps2 = a.real();
+  return tensor_result([&] { return layer(x, w, bias, heads, eps1, eps2, act); });
+}
 TFB_PY(py_layer) {
-  return traceable(self, "layer", argv, argc, [&] {
-    Args a(argv, argc, 19, "layer");
-    const Tensor& x = a.tensor();
-    LayerWeights w;
-    for (Tensor* t : {&w.ln1_w, &w.ln1_b, &w.wq, &w.wk, &w.wv, &w.wo, &w.ln2_w, &w.ln2_b, &w.w1, &w.b1, &w.w2, &w.b2})
-      *t = a.tensor();
-    Bias bias;
-    bias.slopes = a.tensor();
-    bias.rounded = (int)a.integer();
-    bias.table = a.tensor();
-    const int64_t heads = a.integer();
-    const double eps1 = a.real(), eps2 = a.real();
-    return tensor_result([&] { return layer(x, w, bias, heads, eps1, eps2); });
+  return traceable(self, "layer", argv, argc, [&] { return layer_call(argv, argc, nullptr); });
+}
+TFB_PY(py_layer_and_activations) {  // (output, hidden activations): what the model's tests look at
+  return guarded([&]() -> PyObject* {
+    Tensor act;
+    PyObject* y = layer_call(argv, argc, &act);
+    return Py_BuildValue("(NN)", y, THPVariable_Wrap(act));
   });
 }
 TFB_PY(py_set_grad_mode) {  // accumulating, overwrite, defer, fork
@@ -208,6 +216,7 @@ TFB_PY(py_reset_workspaces) {
 #define TFB_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {TFB_METHOD(linear), TFB_METHOD(layernorm), TFB_METHOD(attention), TFB_METHOD(softmax),
                          TFB_METHOD(cross_entropy), TFB_METHOD(lm_loss), TFB_METHOD(embedding), TFB_METHOD(layer),
+                         TFB_METHOD(layer_and_activations),
                          TFB_METHOD(set_grad_mode), TFB_METHOD(take_written), TFB_METHOD(join_weight_grads),
                          TFB_METHOD(gemm_workspace), TFB_METHOD(reset_workspaces), TFB_METHOD(set_recorder), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Native host path of tritonformer_b200.", -1, methods,

@@ -17,8 +17,8 @@ from ._amp import amp_backward, amp_forward
 from .layernorm import layernorm_backward, layernorm_forward
 
 
-# Test hook: when set to a list, MLPResidual.forward appends the boolean activation pattern (act > 0)
-# of every call, so a reference can be evaluated with the same pattern.
+# Test hook: when set to a list, every layer (the native one, and MLPResidual.forward) appends its boolean activation
+# pattern (act > 0), so a reference can be evaluated with the same pattern.
 CAPTURE_ACTIVATION_PATTERN = None
 
 

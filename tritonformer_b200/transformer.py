@@ -154,8 +154,7 @@ class TransformerLayer(nn.Module):
         if not USE_FUSED_BLOCKS or not hidden_states.is_cuda:
             hidden_states = hidden_states + self.attention(self.input_layernorm(hidden_states), attn_bias)
             return hidden_states + self.mlp(self.post_attention_layernorm(hidden_states))
-        if not (_linear.instrumented() or _attention.TIMING is not None
-                or _fused.CAPTURE_ACTIVATION_PATTERN is not None):
+        if not (_linear.instrumented() or _attention.TIMING is not None):
             return self._native(hidden_states, attn_bias)
         att, mlp = self.attention, self.mlp
         ln1, ln2 = self.input_layernorm, self.post_attention_layernorm
@@ -185,10 +184,15 @@ class TransformerLayer(nn.Module):
             bias = _NO_BIAS
         else:
             bias = _attention._resolve_bias(attn_bias, heads, hidden_states.shape[1], hidden_states.dtype)
-        return _host.layer(
+        args = (
             hidden_states, ln1.weight, ln1.bias, att["q_proj"].weight, att["k_proj"].weight, att["v_proj"].weight,
             att["out_proj"].weight, ln2.weight, ln2.bias, fc1.weight, fc1.bias, fc2.weight, fc2.bias,
             bias.slopes, bias.rounded, bias.table, heads, ln1.eps, ln2.eps)
+        if _fused.CAPTURE_ACTIVATION_PATTERN is None:
+            return _host.layer(*args)
+        out, act = _host.layer_and_activations(*args)
+        _fused.CAPTURE_ACTIVATION_PATTERN.append(act > 0)
+        return out
 
 
 _NO_BIAS = _attention._Bias()
