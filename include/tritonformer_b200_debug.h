@@ -20,12 +20,17 @@ extern "C" {
  *   key 3: value 1 launches every kernel fully serialised (no programmatic dependent launch: a
  *          kernel's set-up no longer overlaps its predecessor's tail).
  *   key 4: GEMM: bit 0 whole tiles only (no sharing of a tile's contraction between SMs), bit 5 (32)
- *          no CTA-pair kernel, bit 6 (64) per-CTA timeline counters of the CTA-pair kernel.
+ *          no persistent CTA-pair kernel, bit 6 (64) per-CTA timeline counters of that kernel, bit 7 (128)
+ *          no one-wave kernel, bits 16-27 the one plan the one-wave kernel may use (tfb_debug_gemm_plan).
  *   key 5: which counters tfb_debug_counters returns: -1 attention backward, -3 attention forward,
  *          n >= 0 the CTA-pair GEMM timeline of CTA n.
  *   key 6: how many SMs the persistent GEMM grids leave free (for a collective that runs beside
  *          them on another stream); 0 by default.                                */
 void tfb_debug_set(int key, int value);
+/* What the one-wave GEMM kernel does with an M x N x K product (b_mn: B is contiguous along N) under the switches in force:
+ * 0 if the product goes to the persistent kernels, else 1 + tile width / 64 * 2 + (on CTA pairs ? 1 : 0) + 16 * the number
+ * of workers that share a tile's contraction.                                              */
+int tfb_debug_gemm_plan(long long M, long long N, long long K, int b_mn);
 /* Timing counters of the attention backward kernel (16 cycle sums, filled while tfb_debug_set(2, 2)
  * is in effect); copies and clears them.  Synchronises the device.                        */
 int tfb_debug_counters(unsigned long long* out16);

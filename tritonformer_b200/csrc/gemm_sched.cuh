@@ -18,8 +18,10 @@ struct TilePlan {
   int bn, split;
   bool pair;  // on CTA pairs
   int64_t cycles;
+  int code() const { return bn ? 1 + (bn / 64) * 2 + (pair ? 1 : 0) + 16 * split : 0; }  // for the debug interface
 };
 TilePlan gemm_tile_plan(int64_t M, int64_t N, int64_t K, bool b_mn, int sms);
+TilePlan gemm_plan(int64_t M, int64_t N, int64_t K, bool b_mn);  // with the switches in force
 
 constexpr int kFlagBytes = 8192;  // head of the workspace: arrival counters, zero between kernels
 

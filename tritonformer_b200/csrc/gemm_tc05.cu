@@ -387,6 +387,19 @@ bool gemm_needs_direct(const void* c, int64_t ldc, const void* bias, const void*
            (mask == nullptr || (aligned16(mask) && ld_mask % 8 == 0)));
 }
 
+// SMs left to a collective that runs beside the GEMMs: a persistent grid sized for every SM would have its
+// last CTAs wait for one the collective holds, and the whole product would take two rounds
+static int gemm_sms() {
+  const int sms = sm_count() - g_gemm_free_sms.load();
+  return sms < 2 ? 2 : sms & ~1;
+}
+
+// The one-wave kernel's plan for a product; width 0: it goes to the persistent kernels.
+TilePlan gemm_plan(int64_t M, int64_t N, int64_t K, bool b_mn) {
+  if (g_gemm_debug.load() & 128) return TilePlan{0, 0, false, 0};
+  return gemm_tile_plan(M, N, K, b_mn, gemm_sms());
+}
+
 int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const void* addend, int64_t ld_addend,
               const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
               int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, void* workspace,
@@ -394,20 +407,14 @@ int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const voi
   const bool a_mn = (a_sk != 1);  // M contiguous
   const bool b_mn = (b_sk != 1);  // N contiguous
   const int64_t tm = ceil_div(M, TB_M);
-  // SMs left to a collective that runs beside the GEMMs: a persistent grid sized for every SM would have its
-  // last CTAs wait for one the collective holds, and the whole product would take two rounds
-  int sms = sm_count() - g_gemm_free_sms.load();
-  sms = sms < 2 ? 2 : sms & ~1;
+  const int sms = gemm_sms();
   const int64_t kblocks = ceil_div(K, TB_K);
   const int dbg = g_gemm_debug.load();
   const bool can_split = !(dbg & 1) && workspace != nullptr && aligned16(workspace) &&
                          workspace_bytes >= gemm_tc05_workspace_bytes();
-  if (!(dbg & 128)) {
-    const TilePlan plan = gemm_tile_plan(M, N, K, b_mn, sms);
-    if (plan.bn)
-      return gemm_tile_tc05(plan, a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk, b_sn, ldc, relu,
-                            dtype, st);
-  }
+  if (const TilePlan plan = gemm_plan(M, N, K, b_mn); plan.bn)
+    return gemm_tile_tc05(plan, a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk, b_sn, ldc, relu,
+                          dtype, st);
   // Outputs of at least 256 x 256 that can occupy the pairs of SMs run on CTA pairs (a third less
   // operand traffic per flop): either a 256 x 256 tile for every pair, or a tile for at least every
   // second pair and enough k-blocks to share.

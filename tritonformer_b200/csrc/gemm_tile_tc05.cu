@@ -483,17 +483,17 @@ static int cluster_room(int cluster, int sms) {
 TilePlan gemm_tile_plan(int64_t M, int64_t N, int64_t K, bool b_mn, int sms) {
   TilePlan best{0, 0, false, 0};
   const int64_t kblocks = ceil_div(K, GT_K);
-  const int forced = (g_gemm_debug.load() >> 16) & 0xfff;  // tuning switch: 1 + (bn / 64) * 2 + pair, 16 * split
+  const int dbg = g_gemm_debug.load(), forced = (dbg >> 16) & 0xfff;  // tuning switch: a plan's code
   for (int pair = 0; pair <= 1; ++pair) {
     if (pair && (M <= GT_M || N < 64)) break;
     for (int bn = pair ? 128 : 64; bn <= (pair ? 256 : 128); bn += 64) {
       const int64_t tiles = ceil_div(M, pair ? 2 * GT_M : GT_M) * ceil_div(N, bn);
       for (int split = 1; split <= (pair ? 4 : 8); split *= 2) {
         const int cluster = split * (pair ? 2 : 1);
-        if (kblocks < split || tiles * cluster > cluster_room(cluster, sms)) break;
-        if (forced && forced != 1 + (bn / 64) * 2 + pair + 16 * split) continue;
-        const int64_t cycles = tile_cycles(bn, pair != 0, split, b_mn, kblocks);
-        if (best.bn == 0 || cycles < best.cycles) best = TilePlan{bn, split, pair != 0, cycles};
+        if (kblocks < split || tiles * cluster > cluster_room(cluster, sms) || ((dbg & 1) && split > 1)) break;
+        const TilePlan plan{bn, split, pair != 0, tile_cycles(bn, pair != 0, split, b_mn, kblocks)};
+        if (forced && forced != plan.code()) continue;
+        if (best.bn == 0 || plan.cycles < best.cycles) best = plan;
       }
     }
   }

@@ -1,6 +1,6 @@
 // Library-wide state of the tritonformer_b200 C ABI: version, last error, launch counter,
 // test switches, and the GEMM entry point that picks between the two GEMM kernels.
-#include "common.cuh"
+#include "gemm_sched.cuh"
 #include "../../include/tritonformer_b200_debug.h"
 
 namespace tfb {
@@ -61,6 +61,10 @@ extern "C" void tfb_debug_set(int key, int value) {
   if (key == 4) g_gemm_debug.store(value);
   if (key == 6) g_gemm_free_sms.store(value < 0 ? 0 : value);
   if (key == 5) g_counter_select.store(value);
+}
+
+extern "C" int tfb_debug_gemm_plan(long long M, long long N, long long K, int b_mn) {
+  return gemm_plan(M, N, K, b_mn != 0).code();
 }
 
 extern "C" int64_t tfb_gemm_workspace_bytes(void) { return gemm_tc05_workspace_bytes(); }
