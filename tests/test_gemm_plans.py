@@ -123,3 +123,13 @@ def test_persistent_split_that_is_reached_by_default(m, n, k):
     assert int(ws[8192:].count_nonzero()) > 0, "no partial tile went through the workspace"
     assert int(ws[:8192].count_nonzero()) == 0
     _check_all_epilogues(m, n, k, "kk")
+
+
+def test_fewer_pair_tiles_than_pairs_run_on_the_one_wave_kernel():
+    """The persistent pair kernel hands its tiles out whole, so it is left with products that fill the pairs of SMs."""
+    from tritonformer_b200 import _lib
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    for tm in range(1, pairs):
+        for tn in range(1, (pairs - 1) // tm + 1):
+            for k in (64, 8192):
+                assert _lib.lib.tfb_debug_gemm_plan(256 * tm, 256 * tn, k, tn & 1) != 0, (tm, tn, k)

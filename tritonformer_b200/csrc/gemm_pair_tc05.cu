@@ -52,9 +52,6 @@ struct PairParams {
   int relu;
   int direct;          // C, addend, mask or bias cannot go through TMA boxes: element-wise coalesced stores (store_direct)
   int tiles_m, tiles_n;  // in 256 x 256 pair tiles
-  int sk_tiles;          // pair tiles [0, sk_tiles) are split along K over all pairs; 0 = whole tiles only
-  int* flags;            // per split tile: one arrival counter per (CTA of the pair, epilogue warp)
-  float* partials;       // one fp32 128 x 256 slot per CTA
   int debug;             // bit 6 (64): per-CTA timeline into g_pair_prof (tfb_debug_set key 4)
 };
 
@@ -178,12 +175,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      Segments segs(kblocks, num_tiles, p.sk_tiles, num_pairs, pair, false);
-      int tile, kb0, kb1;
-      while (ok && segs.next(tile, kb0, kb1)) {
+      for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
         const int m0 = (tile % p.tiles_m) * (2 * GP_M) + (int)rank * GP_M;  // this CTA's rows
         const int n0 = (tile / p.tiles_m) * GP_N + (int)rank * GP_NH;       // this CTA's half of B
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = 0; kb < kblocks; ++kb) {
           const long long w0 = clock64();
           if (!mbar_wait(&empty[stage], phase ^ 1, 0x700 | stage, abort_flag)) { ok = false; break; }
           if (prof) pr[2] += (unsigned long long)(clock64() - w0);  // producer waiting for a free slot
@@ -224,15 +219,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       int buf = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      Segments segs(kblocks, num_tiles, p.sk_tiles, num_pairs, pair, false);
-      int tile, kb0, kb1;
-      while (ok && segs.next(tile, kb0, kb1)) {
+      for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
         const long long a0 = clock64();
         if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], acc_phase ^ 1, 0x800 | buf, abort_flag))) { ok = false; break; }
         if (prof) pr[4] += (unsigned long long)(clock64() - a0);  // MMA waiting for a free accumulator
         tc_fence_after();
         const uint32_t d_tmem = tb + buf * GP_N;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = 0; kb < kblocks; ++kb) {
           const long long f0 = clock64();
           if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, 0x900 | stage, abort_flag))) { ok = false; break; }
           if (prof) {
@@ -247,7 +240,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
 #pragma unroll
           for (int k = 0; k < GP_K / 16; ++k) {
             const uint64_t ak = desc_advance(ad, k * (A_MN ? 2048 : 32)), bk = desc_advance(bd, k * (B_MN ? 2048 : 32));
-            if (elect_one()) tc_mma_ss_pair(d_tmem, ak, bk, idesc, ((kb - kb0) | k) ? 1u : 0u);
+            if (elect_one()) tc_mma_ss_pair(d_tmem, ak, bk, idesc, (kb | k) ? 1u : 0u);
           }
           if (elect_one()) tc_commit_pair(&empty[stage]);  // both producers may refill the slot once these MMAs have read it
           if (++stage == GP_STAGES) { stage = 0; phase ^= 1; }
@@ -277,21 +270,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     int buf = 0;
     uint32_t acc_phase = 0, x_phase = 0;
     bool ok = true;
-    // an earlier kernel that gave up leaves the status set: then nothing is written, handed over or waited for
+    // an earlier kernel that gave up leaves the status set: then nothing is written
     const bool dead = *(volatile int*)&g_dev_status != 0;
     if (lane == 0) {
       if (!p.direct) tma_prefetch_desc(&tmC);
       if (use_x) tma_prefetch_desc(&tmX);
     }
-    Segments segs(kblocks, num_tiles, p.sk_tiles, num_pairs, pair, false);
-    int tile, kb0, kb1;
-    while (ok && segs.next(tile, kb0, kb1)) {
+    for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
       const int m0 = (tile % p.tiles_m) * (2 * GP_M) + (int)rank * GP_M;
       const int n0 = (tile / p.tiles_m) * GP_N + half * STEPS * 64;  // first column of this warp's share
       const int row0 = m0 + q * 32;
-      const bool contributes = kb0 > 0;                  // a later part of a split tile
-      const bool finishes = kb0 == 0 && kb1 < kblocks;   // first part of a split tile: owns its epilogue
-      if (use_x && !contributes && !dead && lane == 0) {  // box of step 0, in flight while the main loop still runs
+      if (use_x && !dead && lane == 0) {  // box of step 0, in flight while the main loop still runs
         mbar_expect_tx(&x_full[ew], 4096);
         tma_load_2d(stage_x, &tmX, n0, row0, &x_full[ew]);
       }
@@ -301,39 +290,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       if (prof && ew == 0 && lane == 0) pr[8] += (unsigned long long)(e1 - e0);  // epilogue waiting for an accumulator
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * GP_N + half * STEPS * 64;
-      // partial tiles: slot layout [group of 4 columns][row], so the 32 lanes of a warp touch 512
-      // contiguous bytes; this warp's share starts at column group half * STEPS * 16
-      const int64_t slot_f4 = (int64_t)GP_M * GP_N / 4;  // float4 per slot
-      const int my_f4 = half * STEPS * 16 * GP_M + q * 32 + lane;
-      if (contributes) {
-        if (!dead) store_partials<STEPS>(taddr, reinterpret_cast<float4*>(p.partials) + (int64_t)blockIdx.x * slot_f4 + my_f4, GP_M);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          __threadfence();  // the warp's partial rows are visible before the arrival
-          if (!dead) atomicAdd(p.flags + (tile * 2 + (int)rank) * GP_EPI_WARPS + ew, 1);
-          mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
-        }
-        buf ^= 1;
-        if (buf == 0) acc_phase ^= 1;
-        continue;
-      }
-      int n_parts = 0;  // partial tiles to add: the pairs after this one whose ranges reach into the tile
-      if (finishes && !dead) {
-        n_parts = partials_expected(tile, kblocks, p.sk_tiles, num_pairs, pair);
-        int* flag = p.flags + (tile * 2 + (int)rank) * GP_EPI_WARPS + ew;
-        int fine = 1;
-        if (lane == 0) {
-          fine = flag_wait(flag, n_parts, 0xc00 | ew, abort_flag) ? 1 : 0;
-          if (fine) *flag = 0;  // this warp is the counter's only reader: hand it back cleared
-        }
-        fine = __shfl_sync(0xffffffffu, fine, 0);
-        __syncwarp();  // lane 0's acquire orders the whole warp's reads of the partial tiles
-        if (!fine) { ok = false; break; }
-      }
-      if (n_parts > 0)  // the same CTA rank of the pairs behind this one wrote the slots
-        add_partials<STEPS>(taddr, reinterpret_cast<const float4*>(p.partials) + (int64_t)(blockIdx.x + 2) * slot_f4 + my_f4, 2 * slot_f4,
-                            n_parts, GP_M);
       if (!dead) epilogue_tile<T>(epi, STEPS, taddr, row0, n0, lane, x_phase, abort_flag, 0xb00 | ew, ok);
       tc_fence_before();
       __syncwarp();
@@ -394,28 +350,9 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
 // Pair tiles the output offers; the caller takes this kernel when they fill the pairs of SMs.
 int64_t gemm_pair_tiles(int64_t M, int64_t N) { return ceil_div(M, 2 * GP_M) * ceil_div(N, GP_N); }
 
-// Work split of the pair kernel.  `workspace` may be null (whole tiles only).  Returns the number of
-// pairs to launch and sets *sk_tiles.
-static int64_t pair_schedule(int64_t tiles, int64_t kblocks, int64_t pairs, bool can_split, int64_t* sk_tiles) {
-  *sk_tiles = 0;
-  if (!can_split) return tiles < pairs ? tiles : pairs;
-  // With at least one tile per pair the tiles are handed out whole: cutting the tiles of a partial
-  // last wave along K (tried, also with the cut tiles done first) balances the pairs but does not
-  // shorten the kernel - with fewer pairs busy in the last wave each runs its k-blocks faster, and
-  // the partial tiles add traffic.
-  if (tiles >= pairs) return pairs;
-  // fewer tiles than pairs: as many pairs as leave each at least 8 k-blocks and each tile about 8 parts
-  int64_t g = tiles * kblocks / 8;
-  if (g > pairs) g = pairs;
-  if (g > tiles * 8) g = tiles * 8;
-  if (g * 4 >= tiles * 5 && tiles * 16 * 4 <= kFlagBytes) { *sk_tiles = tiles; return g; }
-  return tiles;
-}
-
 int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, const void* addend, int64_t ld_addend,
                    const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
-                   int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, int sms, void* workspace,
-                   cudaStream_t st) {
+                   int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, int sms, cudaStream_t st) {
   const bool a_mn = (a_sk != 1), b_mn = (b_sk != 1);
   CUtensorMap tmA, tmB, tmC, tmX;
   int rc;
@@ -446,11 +383,10 @@ int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, cons
   p.relu = relu; p.direct = direct; p.debug = g_gemm_debug.load();
   p.tiles_m = (int)ceil_div(M, 2 * GP_M); p.tiles_n = (int)ceil_div(N, GP_N);
   const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
-  int64_t sk_tiles = 0;
-  const int64_t pairs = pair_schedule(tiles, ceil_div(K, GP_K), sms / 2, workspace != nullptr && !(p.debug & 1), &sk_tiles);
-  p.sk_tiles = (int)sk_tiles;
-  p.flags = reinterpret_cast<int*>(workspace);
-  p.partials = workspace ? reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + kFlagBytes) : nullptr;
+  // The tiles are handed out whole: cutting the tiles of a partial last wave along K (tried, also with the cut tiles done
+  // first) balances the pairs but does not shorten the kernel - with fewer pairs busy in the last wave each runs its
+  // k-blocks faster, and the partial tiles add traffic.  Products with fewer tiles than pairs run on the one-wave kernel.
+  const int64_t pairs = tiles < sms / 2 ? tiles : sms / 2;
   const int grid = (int)(2 * pairs);
   TFB_DISPATCH_16(dtype, T, {
     if (a_mn && b_mn) return launch_pair<T, true, true>(tmA, tmB, tmC, tmX, p, grid, st);

@@ -1,6 +1,7 @@
-// Work distribution shared by the tcgen05 GEMM kernels ("stream-K").
+// What the tcgen05 GEMM kernels share: the one-wave kernel's plan, element-wise output, and the one-CTA kernel's work
+// distribution ("stream-K").
 //
-// A worker is a persistent CTA (or CTA pair).  The first sk_tiles output tiles are cut along K into
+// A worker is a persistent CTA.  The first sk_tiles output tiles are cut along K into
 // one equal, contiguous range of k-blocks per worker; the remaining tiles are handed out whole,
 // round-robin, after that.  A worker whose range starts inside a tile computes a partial tile: it
 // writes it (fp32) to its own workspace slot and raises the tile's arrival counter.  The worker that
@@ -29,11 +30,11 @@ struct Segments {
   int kblocks, tiles, workers;
   int64_t it, hi;  // cursor and end of this worker's k-block range in the split region
   int next_tile;   // next whole tile
-  __device__ Segments(int kblocks_, int tiles_, int sk_tiles, int workers_, int worker, bool dead) {
+  __device__ Segments(int kblocks_, int tiles_, int sk_tiles, int workers_, int worker) {
     kblocks = kblocks_;
-    tiles = dead ? 0 : tiles_;
+    tiles = tiles_;
     workers = workers_;
-    const int64_t sk_iters = dead ? 0 : (int64_t)sk_tiles * kblocks;
+    const int64_t sk_iters = (int64_t)sk_tiles * kblocks;
     it = sk_iters * worker / workers;
     hi = sk_iters * (worker + 1) / workers;
     next_tile = sk_tiles + worker;

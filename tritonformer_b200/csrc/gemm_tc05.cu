@@ -35,8 +35,7 @@ int gemm_tile_tc05(const TilePlan& plan, const void* a, const void* b, void* c, 
                    int64_t a_sk, int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, cudaStream_t st);
 int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, const void* addend, int64_t ld_addend,
                    const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
-                   int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, int sms, void* workspace,
-                   cudaStream_t st);
+                   int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, int sms, cudaStream_t st);
 
 constexpr int TB_M = 128;
 constexpr int TB_K = 64;  // 64 sixteen-bit elements = one 128-byte swizzle row
@@ -126,7 +125,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x, false);
+      Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x);
       int tile, kb0, kb1;
       while (ok && segs.next(tile, kb0, kb1)) {
         const int m0 = (tile % p.tiles_m) * TB_M;
@@ -166,7 +165,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
       int buf = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x, false);
+      Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x);
       int tile, kb0, kb1;
       while (ok && segs.next(tile, kb0, kb1)) {
         if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], acc_phase ^ 1, 0x300 | buf, abort_flag))) { ok = false; break; }
@@ -219,7 +218,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) gemm_tc05_kernel(const __grid_c
       if (!p.direct) tma_prefetch_desc(&tmC);
       if (use_x) tma_prefetch_desc(&tmX);
     }
-    Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x, false);
+    Segments segs(kblocks_all, p.tiles_m * p.tiles_n, p.sk_tiles, (int)gridDim.x, (int)blockIdx.x);
     int tile, kb0, kb1;
     while (ok && segs.next(tile, kb0, kb1)) {
       const int m0 = (tile % p.tiles_m) * TB_M;
@@ -415,16 +414,10 @@ int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const voi
   if (const TilePlan plan = gemm_plan(M, N, K, b_mn); plan.bn)
     return gemm_tile_tc05(plan, a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk, b_sn, ldc, relu,
                           dtype, st);
-  // Outputs of at least 256 x 256 that can occupy the pairs of SMs run on CTA pairs (a third less
-  // operand traffic per flop): either a 256 x 256 tile for every pair, or a tile for at least every
-  // second pair and enough k-blocks to share.
-  {
-    const int64_t pt = gemm_pair_tiles(M, N);
-    if (!(dbg & 32) && M >= 256 && N >= 256 &&
-        (pt >= sms / 2 || (can_split && pt * 2 >= sms / 2 && pt * kblocks >= (int64_t)(sms / 2) * 8)))
-      return gemm_pair_tc05(a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk, b_sn, ldc,
-                            relu, dtype, sms, can_split ? workspace : nullptr, st);
-  }
+  // Outputs with a 256 x 256 tile for every pair of SMs run on CTA pairs (a third less operand traffic per flop).
+  if (!(dbg & 32) && M >= 256 && N >= 256 && gemm_pair_tiles(M, N) >= sms / 2)
+    return gemm_pair_tc05(a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk, b_sn, ldc, relu, dtype,
+                          sms, st);
   // Tile width: fewest "waves x tile cost" over the SMs; the wide tile moves fewer operand bytes per
   // flop, so the narrow one has to win by a clear margin.
   const int64_t cost256 = ceil_div(tm * ceil_div(N, 256), sms) * 256;
