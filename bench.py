@@ -431,7 +431,8 @@ def run_b200_arm(args):
                    "algorithmic_bytes_read": 2.0 * (8192 * 1024 + 1024 * 4096),
                    "algorithmic_bytes_written": 2.0 * 8192 * 4096}
         roof = {"bound": "tensor",
-                "kernel": "gemm_pair_tc05_kernel + gemm_tc05_kernel (all linear fwd/dX/dW products of one step)",
+                "kernel": "gemm_pair_tc05_kernel + gemm_tile_tc05_kernel + gemm_tc05_kernel (all linear fwd/dX/dW products "
+                          "of one step)",
                 "achieved": achieved, "peak": peaks["tflops"], "unit": "TFLOP/s", "frac": achieved / peaks["tflops"],
                 "traffic": traffic["dram_bytes_read"] + traffic["dram_bytes_written"], "traffic_detail": traffic,
                 "launches": len(recs), "tcgen05_launches": sum(1 for r in recs if r["path"] == 1),
@@ -439,7 +440,8 @@ def run_b200_arm(args):
                 "flops_per_step": gflop, "sm_mhz": mhz(clk_step),
                 "ms_x_ghz": in_step_s * 1e3 * (mhz(clk_step) or 0) * 1e-3,
                 "how": "CUDA events around every GEMM call of eager steps (median of 10), on the step's own operands, "
-                       "one kernel at a time (in the timed step the weight-gradient products run beside the others "
+                       "one kernel at a time, the layers as the Python blocks that issue the same products one by one (in "
+                       "the timed step they are one native call each, and the weight-gradient products run beside the others "
                        "on a side stream)",
                 # the same calls back to back on dense random operands inside a CUDA graph: the kernels alone in
                 # the power-capped regime; ms_x_ghz (time x median SM clock, i.e. giga-cycles) separates what the
@@ -584,9 +586,10 @@ def run_kernel_bench(args):
             a_sm, a_sk = (1, m) if a_mn else (k, 1)
             b_sk, b_sn = (n, 1) if b_mn else (1, k)
             fn = lambda: LIN.gemm(a, a_sm, a_sk, b, b_sk, b_sn, m, n, k, out=c)
-            # outputs with a 256 x 256 tile for at least every second pair of SMs run on the CTA-pair kernel
-            pair = m >= 256 and n >= 256 and -(-m // 256) * -(-n // 256) >= 37
-            emit("gemm_pair_tc05_kernel" if pair else "gemm_tc05_kernel", f"{name} M{m} N{n} K{k}",
+            # one wave of CTAs, else 256 x 256 tiles on pairs of SMs, else one-CTA tiles
+            one_wave = L.lib.tfb_debug_gemm_plan(m, n, k, int(b_mn)) != 0
+            emit("gemm_tile_tc05_kernel" if one_wave else
+                 "gemm_pair_tc05_kernel" if m >= 256 and n >= 256 else "gemm_tc05_kernel", f"{name} M{m} N{n} K{k}",
                  _time_cuda(fn, iters, warmup), 2.0 * m * n * k, "TFLOP/s", "tensor")
     if which in ("attn", "all"):
         cases = [("B4 H16 T2048 hd64 fp16", 4, 16, 2048, 64, torch.float16, False),
