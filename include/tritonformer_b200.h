@@ -219,9 +219,10 @@ int tfb_gemm(const void* a, const void* b, void* c, const void* bias,
  * gradient).  workspace (may be NULL) is scratch of at least tfb_gemm_workspace_bytes() bytes, 16-byte
  * aligned, whose first 8192 bytes are ZERO on entry; they are zero again when the kernel has finished,
  * so one buffer cleared once serves every call on a stream (calls that share a workspace must be
- * stream-ordered).  With a workspace, when the output tiles do not fill whole waves of SMs, the
- * contraction of some tiles is shared between SMs ("stream-K": fp32 partial tiles, summed in a fixed
- * order, so the result does not depend on timing).                                                 */
+ * stream-ordered).  With a workspace, an output of at most 128 rows whose tiles do not fill the SMs
+ * shares the contraction of its tiles between SMs through it ("stream-K"); outputs that one wave of
+ * thread blocks covers share theirs within a cluster and need none.  Either way the fp32 partial tiles
+ * are summed in a fixed order, so the result does not depend on timing.                             */
 int64_t tfb_gemm_workspace_bytes(void);
 int tfb_gemm_fused(const void* a, const void* b, void* c, const void* bias,
                    const void* addend, int64_t ld_addend, const void* mask, int64_t ld_mask,

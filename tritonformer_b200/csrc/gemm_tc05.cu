@@ -10,8 +10,10 @@
 //                             bias / ReLU / addend / mask in fp32, round once into a swizzled smem
 //                             box, TMA store (the addend / mask box arrives by TMA load); overlaps
 //                             the next tile's main loop through the second accumulator buffer
-// Work split ("stream-K"): when there are fewer tiles than SMs, the tiles are cut along K into one
-// equal, contiguous range of k-blocks per CTA (the scheduler also handles a split region followed by
+// What comes here: products with fewer than 256 rows or columns and more tiles than one wave (the rest runs in
+// gemm_tile_tc05.cu and gemm_pair_tc05.cu).
+// Work split ("stream-K"): when there are fewer tiles than SMs (one tile row, 19 to 30 thousand columns), the tiles are cut
+// along K into one equal, contiguous range of k-blocks per CTA (the scheduler also handles a split region followed by
 // whole tiles).  A CTA whose range starts inside a tile writes that fp32 partial tile to its
 // own workspace slot and raises the tile's flags; the CTA that owns the tile's first k-blocks (its
 // last piece of the range, so the others are long done) adds the partials in CTA order and runs the
@@ -423,11 +425,9 @@ int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const voi
   const int64_t cost256 = ceil_div(tm * ceil_div(N, 256), sms) * 256;
   const int64_t cost128 = ceil_div(tm * ceil_div(N, 128), sms) * 128;
   int BN = (N <= 128 || cost128 * 10 < cost256 * 9) ? 128 : 256;
-  // Outputs with fewer tiles than SMs (weight gradients: small M x N, contraction over every token)
-  // share the K range of each tile between CTAs.  This pays only here: with more tiles than SMs the
-  // kernel is bound by operand traffic rather than by idle SMs in the last wave (measured), and the
-  // partial tiles would add to that traffic.  Very small outputs take the narrow tile so that a tile
-  // has fewer partials to add.
+  // Outputs with fewer tiles than SMs that the one-wave kernel left (one tile row whose 128-column tiles are more than a
+  // wave) share the K range of each tile between CTAs.  This pays only here: with more tiles than SMs the kernel is bound by
+  // operand traffic rather than by idle SMs in the last wave (measured), and the partial tiles would add to that traffic.
   if (can_split && N > 128 && tm * ceil_div(N, 256) < sms) BN = (tm * ceil_div(N, 256) * 3 <= sms) ? 128 : 256;
   const int64_t tiles = tm * ceil_div(N, BN);
   int64_t grid = tiles < sms ? tiles : sms;
