@@ -45,6 +45,31 @@ def test_attention_backward_of_a_key_that_no_query_reaches(t, hd):
     assert dv.isfinite().all() and dk.isfinite().all()
 
 
+@pytest.mark.parametrize("t,hd", [(64, 64), (192, 64), (448, 64), (192, 128), (256, 32), (448, 32), (320, 128)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_attention_with_keys_at_minus_infinity(t, hd, bias):
+    """A key whose score is -inf for every query counts for nothing, wherever in a tile it lies: at its start the first query
+    that sees it has no other key there.  Only queries with no other key at all have no result."""
+    from tritonformer_b200.attention import BiasedCausalAttention, CausalAttention
+    at = sorted({p for p in (1, 31, 32, 63, 64, 65, 127, 128, 129, 191, 192, 255, 256, 319, 320, t - 1) if p < t})
+    sets = [[p] for p in at] + [[p, p + 1] for p in at if p + 1 < t] + [at, list(range(64, t)), [0], [0, 1, 2]]
+    q, k, v, _ = _heads(len(sets), t, hd, torch.float16)
+    q = q.abs() + 0.125
+    for h, keys in enumerate(sets):
+        k[0, h, keys, 0] = -float("inf")
+    slopes = torch.tensor([2.0 ** -(1 + h % 6) for h in range(len(sets))], device="cuda")
+    out = BiasedCausalAttention.apply(q, k, v, slopes) if bias else CausalAttention.apply(q, k, v)
+    s = (q.double() @ k.double().transpose(-1, -2)) / hd ** 0.5
+    if bias:
+        i = torch.arange(t, device="cuda")
+        s = s - slopes.double()[:, None, None] * (i[:, None] - i[None, :])
+    s = s.masked_fill(~torch.ones(t, t, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    want = torch.softmax(s, -1) @ v.double()
+    assert torch.equal(out.isnan(), want.isnan())
+    # P and the result are rounded to 16 bits; values of about one
+    assert (out.double() - want).nan_to_num(0.0).abs().max().item() <= 2.0 ** -11 * 8
+
+
 @pytest.mark.parametrize("t,hd", [(64, 64), (192, 64), (192, 128), (128, 32), (192, 32)])
 @pytest.mark.parametrize("dtype", HALF)
 def test_attention_passes_nan_on(t, hd, dtype):
@@ -346,3 +371,19 @@ def test_a_layer_refuses_an_empty_batch_where_it_comes_in():
         for grad in (False, True):
             with torch.set_grad_enabled(grad), pytest.raises(AssertionError, match="attention: bad shape"):
                 layer(torch.empty(shape, device="cuda", dtype=torch.float16))
+
+
+@pytest.mark.parametrize("reentrant", [False, True])
+def test_layer_under_checkpointing(reentrant):
+    from torch.utils.checkpoint import checkpoint
+    layer = _fuse_projections(_layer())
+    x = torch.randn(2, 128, 128, device="cuda").half()
+    g = torch.randn_like(x)
+    grads = []
+    for run in (layer, lambda t: checkpoint(layer, t, use_reentrant=reentrant)):
+        layer.zero_grad(set_to_none=True)
+        xi = x.clone().requires_grad_()
+        run(xi).backward(g)
+        grads.append([xi.grad] + [p.grad for p in layer.parameters()])
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)

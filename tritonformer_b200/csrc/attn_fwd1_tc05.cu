@@ -633,7 +633,9 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
           // ---- pass 2: p = 2^(s - m_used), partial row sum, P into tensor memory
           float ls4[4] = {0.f, 0.f, 0.f, 0.f};
           {
-            const float neg_m = -m_used;
+            // a row whose keys so far are all at -inf has probabilities of zero; the next tile's single pass then comes out
+            // as not a number and is redone in two, which finds the first maximum
+            const float neg_m = (!POLY && m_used == -INFINITY) ? 0.f : -m_used;
             uint32_t buf[2][32];
             tmem_ld32(s_addr, buf[0]);
 #pragma unroll
@@ -753,8 +755,9 @@ int encode_tmap_sw128(CUtensorMap* out, const void* base, int dtype, int rank, c
                       const uint64_t* strides_bytes, const uint32_t* box);
 
 // Whole tiles of the full width take one pair of exponentials in four from the cubic (POLY).  The shapes that came here from
-// the mma.sync kernel keep its precision, in P and in the row sums, and its NaN (the cubic clamps its argument, which makes a
-// NaN score a probability of nearly zero): every exponential on the SFU.  B3 H11 T1472 hd64 bf16: 29.3 us, with the cubic 28.9; B1 H12 T4032 hd128 fp16: 62.8, 61.1.
+// the mma.sync kernel keep its exponentials, in P and in the row sums, and its NaN (the cubic clamps its argument, which
+// makes a NaN score a probability of nearly zero): all of them on the SFU.  B3 H11 T1472 hd64 bf16: 29.3 us, with the
+// cubic 28.9; B1 H12 T4032 hd128 fp16: 62.8, 61.1.
 template <typename T, int HD, bool POLY>
 static int fwd1_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   using Cfg = F1Cfg<HD>;
