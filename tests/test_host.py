@@ -70,3 +70,18 @@ def test_a_table_that_was_used_can_be_saved(tmp_path):
     again = torch.load(tmp_path / "table.pt")  # weights only
     assert torch.equal(again, table)
     assert torch.equal(_resolve_bias(again, 4, 64, torch.float16).slopes, found.slopes)
+
+
+def test_tensors_without_data_are_refused_before_anything_is_launched():
+    import pytest
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from tritonformer_b200.attention import CausalAttention
+    from tritonformer_b200.layernorm import LayerNorm
+    from tritonformer_b200.linear import LinearNoBias
+    from tritonformer_b200.softmax import Softmax
+    with FakeTensorMode():
+        x, w, q = (torch.empty(s, device="cuda", dtype=torch.float16) for s in ((4, 64), (64, 64), (1, 2, 64, 64)))
+        for call in (lambda: Softmax.apply(x), lambda: LinearNoBias.apply(x, w), lambda: CausalAttention.apply(q, q, q),
+                     lambda: LayerNorm.apply(x, w[0], w[0], 1e-5), lambda: LinearNoBias.apply(x, w.requires_grad_())):
+            with pytest.raises(NotImplementedError):
+                call()

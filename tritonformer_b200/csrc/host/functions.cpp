@@ -54,7 +54,16 @@ bool adjacent_columns(const Tensor* const* parts, int n, int64_t width) {
   return true;
 }
 
+// A tensor that only stands for one (fake tensors, wrapper subclasses): a kernel would read from address zero.
+static bool has_no_memory(const Tensor& t) {
+  if (!t.unsafeGetTensorImpl()->is_python_dispatch() || t.numel() == 0) return false;
+  return !t.has_storage() || t.storage().unsafeGetStorageImpl()->_mutable_data_ptr_no_checks().get() == nullptr;
+}
+
 bool needs_node(std::initializer_list<const Tensor*> inputs) {
+  for (const Tensor* t : inputs)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !has_no_memory(*t),
+                                "the operators of tritonformer_b200 run on tensors that hold data");
   if (const auto& functorch = at::functorch::functorchTLSAccessor()) functorch->checkSupportsCppAutogradFunction();
   if (torch::autograd::ForwardADLevel::try_get_by_idx(0))
     for (const Tensor* t : inputs)

@@ -20,7 +20,8 @@ struct BodyGuard {
 };
 
 // Whether a call needs an autograd node.  Without one the body runs below autograd, where a tangent would be lost and a
-// transform's wrapper has no memory, so what the nodes do not implement - forward mode, function transforms - is refused here.
+// transform's wrapper has no memory, so what the nodes do not implement - forward mode, function transforms - is refused here,
+// and so are tensors without data.
 bool needs_node(std::initializer_list<const Tensor*> inputs);
 
 // Where a weight gradient goes: into the parameter's existing .grad (added, or written in overwrite mode), when a block of
