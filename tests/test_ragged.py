@@ -70,6 +70,14 @@ def test_grad_rows(rows, cols, dtype, offset):
     assert torch.equal(dz[:, :cols], dy)
 
 
+@pytest.mark.parametrize("cols", [247, 248, 249, 495, 496, 497])
+@pytest.mark.parametrize("rows", [1, 31, 1300])
+def test_grad_rows_at_the_edges_of_a_warps_columns(rows, cols):
+    """A warp writes 248 columns; what it reads beside them is its neighbour's first vector, or nothing."""
+    for offset in range(8):
+        test_grad_rows(rows, cols, torch.float16, offset)
+
+
 @pytest.mark.parametrize("cols", [1, 7, 9, 2047, 2049, 50257])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_lm_loss_of_an_odd_vocabulary(cols, dtype):

@@ -77,62 +77,85 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, fl
 // dz = act > 0 ? dy : 0 (act may be null: a copy) with the column sums of dz on the way: what the backward of a linear
 // layer needs before its two products, in one pass over dy and act.  dy and act may have any alignment and pitch; dz has
 // 16-byte aligned rows, so that the products can read it through TMA whatever the layer's width (a copy with act and
-// sums null packs an operand the same way).  The work of a CTA is the one of colsum_kernel, four rows of a thread in
-// flight.  Measured with a cold L2, fp16: 46 us for 5015 x 2930 with mask and sums and their fold (1.9 TB/s of dy, act and dz),
-// 16.4 us for a copy of 5015 x 1477 (1.8 TB/s), 63.5 us for one of 1024 x 50257 (3.2 TB/s): short of the copy rate of 6.5, two
-// aligned loads and a funnel shift per eight elements.
-constexpr int GR_ROWS = 4;
+// sums null packs an operand the same way).
+// A warp takes 31 output vectors (248 columns) of a row.  All lanes of a row share one misalignment: lane l loads the aligned
+// vector that the l-th output begins in, and the rest of that output is in its neighbour's, so a row is loaded once.  Bound by
+// the loads: a thread requests its vectors of GR_ROWS rows before it uses the first.  (Each lane fetching both of its aligned vectors
+// itself made every row two dependent loads deep per lane.)  Cold L2, fp16: 5015 x 2930 with mask and sums and their fold
+// 39.6 -> 25.6 us (3.4 TB/s of dy, act and dz), a copy of 5015 x 1477 12.0 -> 8.7, of 1477 x 2930 7.4 -> 5.9, of 1024 x 50257
+// 57.5 -> 43.1 (4.8 TB/s).
+constexpr int GR_ROWS = 4, GR_COLS = 248;
+// Loads that vector.  One that holds no wanted byte is not touched; one that does never crosses the end of an allocation.
 template <typename T>
-__global__ void __launch_bounds__(256) grad_rows_kernel(const T* __restrict__ dy, const T* __restrict__ act,
-                                                        T* __restrict__ dz, float* __restrict__ partials, int64_t rows,
-                                                        int cols, int64_t dy_ld, int64_t act_ld, int64_t dz_ld) {
+__device__ __forceinline__ uint4 load_row_vec(const T* row, int c0, int cols) {
+  const uintptr_t v = reinterpret_cast<uintptr_t>(row + c0) & ~uintptr_t(15);
+  return v < reinterpret_cast<uintptr_t>(row + cols) ? ld_stream16(reinterpret_cast<const void*>(v)) : make_uint4(0, 0, 0, 0);
+}
+// The eight elements that begin `off` bytes into this lane's vector (nothing of use in lane 31).
+__device__ __forceinline__ uint4 shift_row_vec(const uint4& v, uint32_t off) {
+  uint32_t w[8] = {v.x, v.y, v.z, v.w, __shfl_down_sync(0xffffffffu, v.x, 1), __shfl_down_sync(0xffffffffu, v.y, 1),
+                   __shfl_down_sync(0xffffffffu, v.z, 1), __shfl_down_sync(0xffffffffu, v.w, 1)};
+  if (off & 8) {
+#pragma unroll
+    for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
+  }
+  if (off & 4) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
+  }
+  const uint32_t bits = (off & 2) * 8;
+  return make_uint4(__funnelshift_r(w[0], w[1], bits), __funnelshift_r(w[1], w[2], bits), __funnelshift_r(w[2], w[3], bits),
+                    __funnelshift_r(w[3], w[4], bits));
+}
+template <typename T, bool ACT>
+__global__ void __launch_bounds__(256, ACT ? 3 : 4) grad_rows_kernel(const T* __restrict__ dy, const T* __restrict__ act,
+                                                           T* __restrict__ dz, float* __restrict__ partials, int64_t rows,
+                                                           int cols, int64_t dy_ld, int64_t act_ld, int64_t dz_ld) {
   grid_dependency_wait();
   allow_dependents();
   __shared__ float sm[8][32][9];
   const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5;
-  const int c0 = (blockIdx.x * 32 + cl) * 8;
-  const int n = min(8, cols - c0);
+  const int c0 = blockIdx.x * GR_COLS + cl * 8;
+  const int n = cl == 31 ? 0 : min(8, cols - c0);  // columns this lane writes, none where not positive
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  if (n > 0) {
-    const int64_t step = (int64_t)gridDim.y * 8;
-    for (int64_t r0 = (int64_t)blockIdx.y * 8 + rl; r0 < rows; r0 += step * GR_ROWS) {
-      uint4 g[GR_ROWS], a[GR_ROWS];
+  const int64_t step = (int64_t)gridDim.y * 8;
+  for (int64_t r0 = (int64_t)blockIdx.y * 8 + rl; r0 < rows; r0 += step * GR_ROWS) {  // the same for all lanes of a warp
+    uint4 g[GR_ROWS], a[ACT ? GR_ROWS : 1];
 #pragma unroll
-      for (int i = 0; i < GR_ROWS; ++i) {
-        const int64_t r = r0 + i * step;
-        if (r >= rows) continue;
-        g[i] = load8_any(dy + r * dy_ld + c0, n);
-        if (act) a[i] = load8_any(act + r * act_ld + c0, n);
+    for (int i = 0; i < GR_ROWS; ++i) {
+      const int64_t r = r0 + i * step;
+      if (r >= rows) break;
+      g[i] = load_row_vec(dy + r * dy_ld, c0, cols);
+      if (ACT) a[i] = load_row_vec(act + r * act_ld, c0, cols);
+    }
+#pragma unroll
+    for (int i = 0; i < GR_ROWS; ++i) {
+      const int64_t r = r0 + i * step;
+      if (r >= rows) break;
+      float f[8];
+      unpack8<T>(shift_row_vec(g[i], (uint32_t)reinterpret_cast<uintptr_t>(dy + r * dy_ld) & 15), f);
+      if (ACT) {
+        float m[8];
+        unpack8<T>(shift_row_vec(a[i], (uint32_t)reinterpret_cast<uintptr_t>(act + r * act_ld) & 15), m);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = m[j] > 0.f ? f[j] : 0.f;
       }
 #pragma unroll
-      for (int i = 0; i < GR_ROWS; ++i) {
-        const int64_t r = r0 + i * step;
-        if (r >= rows) continue;
-        float f[8];
-        unpack8<T>(g[i], f);
-        if (act) {
-          float m[8];
-          unpack8<T>(a[i], m);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) f[j] = m[j] > 0.f ? f[j] : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (j >= n) f[j] = 0.f;  // the padding of a row
-          acc[j] += f[j];
-        }
-        *reinterpret_cast<uint4*>(dz + r * dz_ld + c0) = pack8<T>(f);
+      for (int j = 0; j < 8; ++j) {
+        if (j >= n) f[j] = 0.f;  // the padding of a row
+        acc[j] += f[j];
       }
+      if (n > 0) *reinterpret_cast<uint4*>(dz + r * dz_ld + c0) = pack8<T>(f);
     }
   }
   if (!partials) return;
 #pragma unroll
   for (int j = 0; j < 8; ++j) sm[rl][cl][j] = acc[j];
   __syncthreads();
-  const int cc = threadIdx.x, col = blockIdx.x * 256 + cc;
-  if (col < cols) {
+  const int cc = threadIdx.x, col = blockIdx.x * GR_COLS + cc;
+  if (cc < GR_COLS && col < cols) {
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) s += sm[i][cc >> 3][cc & 7];
@@ -154,10 +177,12 @@ extern "C" int tfb_grad_rows(const void* dy, const void* act, void* dz, void* su
               "grad_rows: scratch must hold tfb_colsum_partials() rows");
   if (rows == 0 && !sums) return TFB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const dim3 grid((unsigned)ceil_div(cols, 256), (unsigned)tfb_colsum_partials(rows, cols));
+  const dim3 grid((unsigned)ceil_div(cols, GR_COLS), (unsigned)tfb_colsum_partials(rows, cols));
   TFB_DISPATCH_16(dtype, T, {
-    launch_overlapped(grad_rows_kernel<T>, grid, dim3(256), 0, st, (const T*)dy, (const T*)act, (T*)dz, sums ? partials : nullptr,
-                      rows, (int)cols, dy_ld, act_ld, dz_ld);
+    if (act) launch_overlapped(grad_rows_kernel<T, true>, grid, dim3(256), 0, st, (const T*)dy, (const T*)act, (T*)dz, sums ? partials : nullptr,
+                               rows, (int)cols, dy_ld, act_ld, dz_ld);
+    else launch_overlapped(grad_rows_kernel<T, false>, grid, dim3(256), 0, st, (const T*)dy, (const T*)act, (T*)dz, sums ? partials : nullptr,
+                           rows, (int)cols, dy_ld, act_ld, dz_ld);
     const int rc = launched("grad_rows");
     if (rc || !sums) return rc;
     return finalize_partials<T>(partials, n_partials, (int)cols, (int)cols, sums, nullptr, st, 0);
