@@ -133,3 +133,14 @@ def test_fewer_pair_tiles_than_pairs_run_on_the_one_wave_kernel():
         for tn in range(1, (pairs - 1) // tm + 1):
             for k in (64, 8192):
                 assert _lib.lib.tfb_debug_gemm_plan(256 * tm, 256 * tn, k, tn & 1) != 0, (tm, tn, k)
+
+
+@pytest.mark.parametrize("layout", ["kn", "kk", "mn", "mk"])
+@pytest.mark.parametrize("m,n,k,dtype", [(3328, 1536, 136, torch.float16), (3304, 1528, 1000, torch.bfloat16)])
+def test_narrow_tiles_of_the_pair_kernel(m, n, k, dtype, layout):
+    """A little more than a wave of 256 x 256 tiles: 256 x 192 ones, with B in boxes of 32 columns where it is contiguous along N."""
+    from tritonformer_b200 import _lib
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    wide, narrow = (-(-(-(-m // 256) * -(-n // bn)) // pairs) for bn in (256, 192))
+    assert wide == narrow == 2 and _lib.lib.tfb_debug_gemm_plan(m, n, k, int(layout[1] == "n")) == 0
+    _check_all_epilogues(m, n, k, layout, dtype)

@@ -1,4 +1,4 @@
-// tcgen05 GEMM on CTA pairs (cta_group::2) for sm_100a: one 256 x 256 output tile per pair of SMs.
+// tcgen05 GEMM on CTA pairs (cta_group::2) for sm_100a: one 256 x 256 or 256 x 192 output tile per pair of SMs.
 //
 // Same contract as gemm_tc05.cu (C = mask(act(A·B + bias) + addend), either operand K- or MN-major),
 // for outputs large enough to give every pair of SMs tiles.  Why a second kernel: the one-CTA kernel
@@ -7,11 +7,11 @@
 // tile (32 KB per CTA for the same work), and the pair's tensor cores read B from both halves.
 //
 // Per CTA (both CTAs of the pair run the same code; "leader" = cluster rank 0):
-//   warp 0   : TMA producer - its A rows and its half of B into a 6-stage ring; the copies signal the
+//   warp 0   : TMA producer - its A rows and its half of B into a 5-stage ring; the copies signal the
 //              LEADER's full barrier (cp.async.bulk.tensor with .cta_group::2, no multicast)
-//   warp 1   : leader only: issues tcgen05.mma.cta_group::2 (M 256 over the pair, N 256, K 16) and
+//   warp 1   : leader only: issues tcgen05.mma.cta_group::2 (M 256 over the pair, N 256 or 192, K 16) and
 //              commits ring slots / finished accumulators to the barriers of BOTH CTAs
-//   warps 2-5: epilogue of this CTA's 128 rows from its own TMEM (two accumulator buffers), as in the
+//   warps 2-9: epilogue of this CTA's 128 rows from its own TMEM (two accumulator buffers), as in the
 //              one-CTA kernel; the buffer is handed back by an arrival on the leader's barrier
 // Every wait is bounded (mbar_wait); the two cluster-wide barriers (after set-up, before exit) are
 // reached unconditionally by both CTAs.
@@ -26,20 +26,26 @@ bool gemm_needs_direct(const void* c, int64_t ldc, const void* bias, const void*
                        int64_t ld_mask);
 
 constexpr int GP_M = 128;    // rows per CTA
-constexpr int GP_N = 256;    // columns per pair tile
-constexpr int GP_NH = 128;   // B rows loaded per CTA
 constexpr int GP_K = 64;
 constexpr int GP_EPI_WARPS = 8;  // 4, or 8 (two warps per TMEM lane quarter, half of the columns each)
 constexpr int GP_THREADS = 64 + 32 * GP_EPI_WARPS;
-constexpr int GP_STAGES = GP_EPI_WARPS == 8 ? 5 : 6;  // the staging boxes of eight warps take a ring slot's room
 constexpr int GP_A_BYTES = GP_M * GP_K * 2;
-constexpr int GP_B_BYTES = GP_NH * GP_K * 2;
-constexpr int GP_STAGE_BYTES = GP_A_BYTES + GP_B_BYTES;
 constexpr int GP_EPI_BYTES = GP_EPI_WARPS * 4096;  // one staging box per epilogue warp
-constexpr int GP_OFF_EPI_C = GP_STAGES * GP_STAGE_BYTES;
-constexpr int GP_OFF_EPI_X = GP_OFF_EPI_C + GP_EPI_BYTES;
-constexpr int GP_OFF_BAR = GP_OFF_EPI_X + GP_EPI_BYTES;
-constexpr int GP_SMEM_BYTES = GP_OFF_BAR + 1024 + 256;
+template <int BN> struct PairCfg {   // BN: columns per pair tile, 192 or 256
+  static constexpr int NH = BN / 2;  // columns of B loaded per CTA
+  static constexpr int STAGES = 5;
+  static constexpr int B_BYTES = NH * GP_K * 2;
+  static constexpr int STAGE_BYTES = GP_A_BYTES + B_BYTES;
+  // B contiguous along N comes in boxes of BOX columns by GP_K rows.  Half of 192 columns is no multiple of 64, so its boxes
+  // are 32 columns (64 bytes) wide, with the 64-byte swizzle.
+  static constexpr int BOX = NH % 64 == 0 ? 64 : 32;
+  static constexpr int FIRST = (BN / 64 + 1) / 2;  // 64-column steps of the first half of the epilogue warps
+  static constexpr int OFF_EPI_C = STAGES * STAGE_BYTES;
+  static constexpr int OFF_EPI_X = OFF_EPI_C + GP_EPI_BYTES;
+  static constexpr int OFF_BAR = OFF_EPI_X + GP_EPI_BYTES;
+  static constexpr int SMEM_BYTES = OFF_BAR + 1024 + 256;
+  static_assert(NH % BOX == 0 && STAGE_BYTES % 1024 == 0 && SMEM_BYTES <= 227 * 1024, "tile width");
+};
 constexpr int GP_TMEM_COLS = 512;
 
 struct PairParams {
@@ -51,7 +57,7 @@ struct PairParams {
   int64_t ldc, ld_addend, ld_mask;
   int relu;
   int direct;          // C, addend, mask or bias cannot go through TMA boxes: element-wise coalesced stores (store_direct)
-  int tiles_m, tiles_n;  // in 256 x 256 pair tiles
+  int tiles_m, tiles_n;  // in 256 x BN pair tiles
   int debug;             // bit 6 (64): per-CTA timeline into g_pair_prof (tfb_debug_set key 4)
 };
 
@@ -112,14 +118,16 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
       : "memory");
 }
 
-template <typename T, bool A_MN, bool B_MN>
+template <typename T, int BN, bool A_MN, bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     gemm_pair_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                           const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmX,
                           const PairParams p) {
+  using Cfg = PairCfg<BN>;
+  constexpr int GP_STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GP_OFF_BAR);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
   uint64_t* full = bars;                       // [STAGES] both producers -> leader's MMA (leader's copy is used)
   uint64_t* empty = bars + GP_STAGES;          // [STAGES] leader's MMA -> each CTA's producer
   uint64_t* acc_full = bars + 2 * GP_STAGES;   // [2] leader's MMA -> each CTA's epilogue
@@ -177,15 +185,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       bool ok = true;
       for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
         const int m0 = (tile % p.tiles_m) * (2 * GP_M) + (int)rank * GP_M;  // this CTA's rows
-        const int n0 = (tile / p.tiles_m) * GP_N + (int)rank * GP_NH;       // this CTA's half of B
+        const int n0 = (tile / p.tiles_m) * BN + (int)rank * Cfg::NH;       // this CTA's half of B
         for (int kb = 0; kb < kblocks; ++kb) {
           const long long w0 = clock64();
           if (!mbar_wait(&empty[stage], phase ^ 1, 0x700 | stage, abort_flag)) { ok = false; break; }
           if (prof) pr[2] += (unsigned long long)(clock64() - w0);  // producer waiting for a free slot
-          uint8_t* sa = smem + stage * GP_STAGE_BYTES;
+          uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + GP_A_BYTES;
           // the leader's barrier counts the bytes of both CTAs
-          if (leader) mbar_expect_tx(&full[stage], 2 * GP_STAGE_BYTES);
+          if (leader) mbar_expect_tx(&full[stage], 2 * Cfg::STAGE_BYTES);
           const uint32_t bar = map_to_cta(smem_u32(&full[stage]), 0);
           const int k0 = kb * GP_K;
           if (A_MN) {
@@ -196,7 +204,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
           }
           if (B_MN) {
 #pragma unroll
-            for (int i = 0; i < GP_NH / 64; ++i) tma_load_2d_pair(sb + i * 8192, &tmB, n0 + i * 64, k0, bar);
+            for (int i = 0; i < Cfg::NH / Cfg::BOX; ++i)
+              tma_load_2d_pair(sb + i * (Cfg::BOX * GP_K * 2), &tmB, n0 + i * Cfg::BOX, k0, bar);
           } else {
             tma_load_2d_pair(sb, &tmB, k0, n0, bar);
           }
@@ -210,7 +219,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     // The whole warp runs the loop and one elected lane issues each instruction: warp-uniform code keeps the operand
     // descriptors in the uniform registers the tensor core reads them from.
     if (leader) {
-      constexpr uint32_t idesc = instr_desc_f16(2 * GP_M, GP_N, std::is_same<T, __nv_bfloat16>::value ? 1 : 0,
+      constexpr uint32_t idesc = instr_desc_f16(2 * GP_M, BN, std::is_same<T, __nv_bfloat16>::value ? 1 : 0,
                                                 A_MN ? 1 : 0, B_MN ? 1 : 0);
       const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0), s0 = smem_u32(smem);
       const bool prof = p.debug & 64 && lane == 0 && blockIdx.x < 148;
@@ -224,7 +233,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
         if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], acc_phase ^ 1, 0x800 | buf, abort_flag))) { ok = false; break; }
         if (prof) pr[4] += (unsigned long long)(clock64() - a0);  // MMA waiting for a free accumulator
         tc_fence_after();
-        const uint32_t d_tmem = tb + buf * GP_N;
+        const uint32_t d_tmem = tb + buf * 256;
         for (int kb = 0; kb < kblocks; ++kb) {
           const long long f0 = clock64();
           if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, 0x900 | stage, abort_flag))) { ok = false; break; }
@@ -233,13 +242,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
             pr[5] += (unsigned long long)(f1 - f0);  // MMA waiting for operands
             if (pr[6] == 0) pr[6] = (unsigned long long)(f1 - t_entry);  // first operands landed
           }
-          const uint32_t sa = s0 + stage * GP_STAGE_BYTES, sb = sa + GP_A_BYTES;
+          const uint32_t sa = s0 + stage * Cfg::STAGE_BYTES, sb = sa + GP_A_BYTES;
           const uint64_t ad = A_MN ? smem_desc_sw128(sa, 8192, 1024) : smem_desc_sw128(sa, 16, 1024);
-          const uint64_t bd = B_MN ? smem_desc_sw128(sb, 8192, 1024) : smem_desc_sw128(sb, 16, 1024);
-          // K-major: 16 elements = 32 bytes along the swizzled row; MN-major: 16 k-rows of 128 B
+          const uint64_t bd = !B_MN ? smem_desc_sw128(sb, 16, 1024)
+                              : Cfg::BOX == 64 ? smem_desc_sw128(sb, 8192, 1024) : smem_desc_sw64(sb, 4096, 512);
+          // K-major: 16 elements = 32 bytes along the swizzled row; MN-major: 16 k-rows of a box
 #pragma unroll
           for (int k = 0; k < GP_K / 16; ++k) {
-            const uint64_t ak = desc_advance(ad, k * (A_MN ? 2048 : 32)), bk = desc_advance(bd, k * (B_MN ? 2048 : 32));
+            const uint64_t ak = desc_advance(ad, k * (A_MN ? 2048 : 32)), bk = desc_advance(bd, k * (B_MN ? Cfg::BOX * 32 : 32));
             if (elect_one()) tc_mma_ss_pair(d_tmem, ak, bk, idesc, (kb | k) ? 1u : 0u);
           }
           if (elect_one()) tc_commit_pair(&empty[stage]);  // both producers may refill the slot once these MMAs have read it
@@ -258,15 +268,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     const int ew = warp - 2;  // 0 .. EPI_WARPS-1
     const int half = ew >> 2; // with eight epilogue warps: which half of the tile's columns
     const T* bias = reinterpret_cast<const T*>(p.bias);
-    uint8_t* stage_c = smem + GP_OFF_EPI_C + ew * 4096;
-    uint8_t* stage_x = smem + GP_OFF_EPI_X + ew * 4096;
+    uint8_t* stage_c = smem + Cfg::OFF_EPI_C + ew * 4096;
+    uint8_t* stage_x = smem + Cfg::OFF_EPI_X + ew * 4096;
     // at most one of addend / mask travels through the TMA box; a second one is read directly
     const bool use_x = !p.direct && (p.addend != nullptr || p.mask != nullptr);
     const EpiArgs<T> epi{{reinterpret_cast<T*>(p.C), bias, reinterpret_cast<const T*>(p.addend), reinterpret_cast<const T*>(p.mask),
                           p.ldc, p.ld_addend, p.ld_mask, p.M, p.N, p.relu},
                          &tmC, &tmX, stage_c, stage_x, &x_full[ew], use_x, p.addend != nullptr, p.direct != 0,
                          (p.addend != nullptr && p.mask != nullptr) ? reinterpret_cast<const T*>(p.mask) : nullptr};
-    constexpr int STEPS = GP_N / 64 / (GP_EPI_WARPS / 4);  // 64-column steps per warp
+    const int first = half * Cfg::FIRST * 64;                             // first column of this warp's share of a tile
+    const int steps = half == 0 ? Cfg::FIRST : BN / 64 - Cfg::FIRST;      // of 64 columns
     int buf = 0;
     uint32_t acc_phase = 0, x_phase = 0;
     bool ok = true;
@@ -278,7 +289,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     }
     for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
       const int m0 = (tile % p.tiles_m) * (2 * GP_M) + (int)rank * GP_M;
-      const int n0 = (tile / p.tiles_m) * GP_N + half * STEPS * 64;  // first column of this warp's share
+      const int n0 = (tile / p.tiles_m) * BN + first;
       const int row0 = m0 + q * 32;
       if (use_x && !dead && lane == 0) {  // box of step 0, in flight while the main loop still runs
         mbar_expect_tx(&x_full[ew], 4096);
@@ -289,8 +300,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       const long long e1 = clock64();
       if (prof && ew == 0 && lane == 0) pr[8] += (unsigned long long)(e1 - e0);  // epilogue waiting for an accumulator
       tc_fence_after();
-      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * GP_N + half * STEPS * 64;
-      if (!dead) epilogue_tile<T>(epi, STEPS, taddr, row0, n0, lane, x_phase, abort_flag, 0xb00 | ew, ok);
+      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256 + first;
+      if (!dead) epilogue_tile<T>(epi, steps, taddr, row0, n0, lane, x_phase, abort_flag, 0xb00 | ew, ok);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
@@ -334,26 +345,44 @@ int gemm_pair_counters(int cta, unsigned long long* out) {
 }
 
 
-int encode_tmap_sw128(CUtensorMap* out, const void* base, int dtype, int rank, const uint64_t* dims,
-                      const uint64_t* strides_bytes, const uint32_t* box);
-
-template <typename T, bool A_MN, bool B_MN>
+template <typename T, int BN, bool A_MN, bool B_MN>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmX,
                        const PairParams& p, int grid, cudaStream_t st) {
-  auto kern = gemm_pair_tc05_kernel<T, A_MN, B_MN>;
+  auto kern = gemm_pair_tc05_kernel<T, BN, A_MN, B_MN>;
   static std::atomic<uint64_t> attr_done{0};
-  if (int rc0 = ensure_dynamic_smem(kern, GP_SMEM_BYTES, attr_done, "gemm_pair_tc05")) return rc0;
-  launch_overlapped(kern, dim3(grid), dim3(GP_THREADS), GP_SMEM_BYTES, st, tmA, tmB, tmC, tmX, p);
+  if (int rc0 = ensure_dynamic_smem(kern, PairCfg<BN>::SMEM_BYTES, attr_done, "gemm_pair_tc05")) return rc0;
+  launch_overlapped(kern, dim3(grid), dim3(GP_THREADS), PairCfg<BN>::SMEM_BYTES, st, tmA, tmB, tmC, tmX, p);
   return launched("gemm_pair_tc05");
 }
 
-// Pair tiles the output offers; the caller takes this kernel when they fill the pairs of SMs.
-int64_t gemm_pair_tiles(int64_t M, int64_t N) { return ceil_div(M, 2 * GP_M) * ceil_div(N, GP_N); }
+template <typename T, int BN>
+static int dispatch_pair(bool a_mn, bool b_mn, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
+                         const CUtensorMap& tmX, const PairParams& p, int grid, cudaStream_t st) {
+  if (a_mn && b_mn) return launch_pair<T, BN, true, true>(tmA, tmB, tmC, tmX, p, grid, st);
+  if (a_mn) return launch_pair<T, BN, true, false>(tmA, tmB, tmC, tmX, p, grid, st);
+  if (b_mn) return launch_pair<T, BN, false, true>(tmA, tmB, tmC, tmX, p, grid, st);
+  return launch_pair<T, BN, false, false>(tmA, tmB, tmC, tmX, p, grid, st);
+}
+
+// 256 x 256 tiles the output offers; the caller takes this kernel when they fill the pairs of SMs.
+int64_t gemm_pair_tiles(int64_t M, int64_t N) { return ceil_div(M, 2 * GP_M) * ceil_div(N, 256); }
+
+// Tile width.  A k-block of a 256 x 256 tile takes 528 cycles of its pair and one of a 256 x 192 tile 462 (what an SM takes in
+// from the L2, 32 and 28 KB at 62 bytes a cycle), so the narrow tile, which moves an eighth more operand bytes for the
+// same product, is for outputs whose last wave of wide tiles is mostly empty: as many waves of narrow ones.  M 4096 N 1536, two
+// waves of either: K 4608 (B contiguous along K) 49.2 us wide, 45.4 narrow, K 6144 65.6 and 62.1; B contiguous along N:
+// K 1536 20.8 and 19.8, K 6144 65.2 and 64.6.  M 2112 N 3072 K 1024: 15.9 and 15.6.
+int gemm_pair_width(int64_t M, int64_t N, int sms) {
+  const int64_t pairs = sms / 2, tm = ceil_div(M, 2 * GP_M);
+  const int64_t wide = ceil_div(tm * ceil_div(N, 256), pairs) * 528, narrow = ceil_div(tm * ceil_div(N, 192), pairs) * 462;
+  return narrow * 100 < wide * 95 ? 192 : 256;
+}
 
 int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, const void* addend, int64_t ld_addend,
                    const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
                    int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, int sms, cudaStream_t st) {
   const bool a_mn = (a_sk != 1), b_mn = (b_sk != 1);
+  const int width = gemm_pair_width(M, N, sms);
   CUtensorMap tmA, tmB, tmC, tmX;
   int rc;
   const bool direct = gemm_needs_direct(c, ldc, bias, addend, ld_addend, mask, ld_mask);
@@ -373,15 +402,17 @@ int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, cons
     if (a_mn) { dims[0] = (uint64_t)M; dims[1] = (uint64_t)K; str[0] = (uint64_t)a_sk * 2; box[0] = 64; box[1] = GP_K; }
     else      { dims[0] = (uint64_t)K; dims[1] = (uint64_t)M; str[0] = (uint64_t)a_sm * 2; box[0] = GP_K; box[1] = GP_M; }
     if ((rc = encode_tmap_sw128(&tmA, a, dtype, 2, dims, str, box))) return rc;
-    if (b_mn) { dims[0] = (uint64_t)N; dims[1] = (uint64_t)K; str[0] = (uint64_t)b_sk * 2; box[0] = 64; box[1] = GP_K; }
-    else      { dims[0] = (uint64_t)K; dims[1] = (uint64_t)N; str[0] = (uint64_t)b_sn * 2; box[0] = GP_K; box[1] = GP_NH; }
-    if ((rc = encode_tmap_sw128(&tmB, b, dtype, 2, dims, str, box))) return rc;
+    const bool narrow = width == 192;
+    if (b_mn) { dims[0] = (uint64_t)N; dims[1] = (uint64_t)K; str[0] = (uint64_t)b_sk * 2; box[0] = narrow ? 32 : 64; box[1] = GP_K; }
+    else      { dims[0] = (uint64_t)K; dims[1] = (uint64_t)N; str[0] = (uint64_t)b_sn * 2; box[0] = GP_K; box[1] = (uint32_t)(width / 2); }
+    if ((rc = b_mn && narrow ? encode_tmap_sw64(&tmB, b, dtype, 2, dims, str, box) : encode_tmap_sw128(&tmB, b, dtype, 2, dims, str, box)))
+      return rc;
   }
   PairParams p;
   p.C = c; p.bias = bias; p.addend = addend; p.mask = mask;
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.ldc = ldc; p.ld_addend = ld_addend; p.ld_mask = ld_mask;
   p.relu = relu; p.direct = direct; p.debug = g_gemm_debug.load();
-  p.tiles_m = (int)ceil_div(M, 2 * GP_M); p.tiles_n = (int)ceil_div(N, GP_N);
+  p.tiles_m = (int)ceil_div(M, 2 * GP_M); p.tiles_n = (int)ceil_div(N, width);
   const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
   // The tiles are handed out whole: cutting the tiles of a partial last wave along K (tried, also with the cut tiles done
   // first) balances the pairs but does not shorten the kernel - with fewer pairs busy in the last wave each runs its
@@ -389,10 +420,8 @@ int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, cons
   const int64_t pairs = tiles < sms / 2 ? tiles : sms / 2;
   const int grid = (int)(2 * pairs);
   TFB_DISPATCH_16(dtype, T, {
-    if (a_mn && b_mn) return launch_pair<T, true, true>(tmA, tmB, tmC, tmX, p, grid, st);
-    if (a_mn) return launch_pair<T, true, false>(tmA, tmB, tmC, tmX, p, grid, st);
-    if (b_mn) return launch_pair<T, false, true>(tmA, tmB, tmC, tmX, p, grid, st);
-    return launch_pair<T, false, false>(tmA, tmB, tmC, tmX, p, grid, st);
+    if (width == 192) return dispatch_pair<T, 192>(a_mn, b_mn, tmA, tmB, tmC, tmX, p, grid, st);
+    return dispatch_pair<T, 256>(a_mn, b_mn, tmA, tmB, tmC, tmX, p, grid, st);
   })
 }
 

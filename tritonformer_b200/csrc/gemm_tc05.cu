@@ -341,7 +341,10 @@ int encode_tmap_sw128(CUtensorMap* out, const void* base, int dtype, int rank, c
                       const uint64_t* strides_bytes, const uint32_t* box) {
   return encode_tmap(out, base, dtype, rank, dims, strides_bytes, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
-
+int encode_tmap_sw64(CUtensorMap* out, const void* base, int dtype, int rank, const uint64_t* dims,
+                     const uint64_t* strides_bytes, const uint32_t* box) {
+  return encode_tmap(out, base, dtype, rank, dims, strides_bytes, box, CU_TENSOR_MAP_SWIZZLE_64B);
+}
 
 // Arrival counters plus one fp32 128 x 256 partial tile per SM.
 int64_t gemm_tc05_workspace_bytes() { return kFlagBytes + (int64_t)sm_count() * TB_M * 256 * (int64_t)sizeof(float); }

@@ -179,6 +179,12 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr, uint32_t lbo
   return d;
 }
 
+// The same for an MN-major operand with the 64-byte swizzle: k-rows of 64 B (32 MN elements); sbo = bytes between 8-k-row
+// groups, lbo = bytes between consecutive 32-element MN chunks.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return (smem_desc_sw128(saddr, lbo_bytes, sbo_bytes) & ~((uint64_t)7 << 61)) | (uint64_t)4 << 61;
+}
+
 // Descriptor of the same layout `byte_off` bytes further on (the start-address field is the low 14
 // bits in 16-byte units; operands live below 256 KB, so the sum never leaves the field).  One 32-bit
 // add per MMA instead of rebuilding the descriptor keeps the single issuing thread off the critical path.
@@ -281,5 +287,8 @@ __device__ __forceinline__ bool elect_one() {
 // dims[0] is the contiguous dimension; strides_bytes[i] is the byte stride of dims[i+1].
 int encode_tmap_sw128(CUtensorMap* out, const void* base, int dtype, int rank, const uint64_t* dims,
                       const uint64_t* strides_bytes, const uint32_t* box);
+// The same with 64-byte swizzle: boxes whose rows are 64 bytes in shared memory.
+int encode_tmap_sw64(CUtensorMap* out, const void* base, int dtype, int rank, const uint64_t* dims,
+                     const uint64_t* strides_bytes, const uint32_t* box);
 
 }  // namespace tfb
