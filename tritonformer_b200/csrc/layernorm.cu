@@ -241,193 +241,156 @@ __global__ void __launch_bounds__(MAXT) ln_bwd_kernel(
 
 // Backward for vectorisable rows of at most 2048 elements: G warps share a row, a lane owns ONE
 // 16-byte vector of it, so a thread keeps only 8 columns of alpha and of the dalpha / dbeta sums in
-// registers.  Each step handles two rows of the row group.  The vectors of the following steps are
-// already on their way: every lane copies its own 16-byte pieces into a private slot of a
-// shared-memory ring with cp.async (LN_DEPTH steps deep, no registers held, no barrier needed since
-// a lane reads back only what it copied itself), which keeps about 100 KB per SM in flight - what
-// the HBM latency needs at this bandwidth.  The two row sums are reduced by warp shuffles and
-// exchanged between the G warps through shared memory behind a named barrier (double-buffered).
-constexpr int LN_DEPTH = 4;
-constexpr int LN_RING_BYTES = 8 * LN_DEPTH * 2 * 3 * 32 * 16;  // warps x steps x rows x tensors x lanes x 16 B
-
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)),
-               "l"(gsrc)
-               : "memory");
+// registers.  RG such groups make a CTA; a group takes one row at a time, with the next row's vectors on their way in
+// registers.  The two row sums are reduced by warp shuffles and exchanged between the G warps through shared memory behind
+// a named barrier (double-buffered).
+// What bounds it: the instructions a warp issues per row, one in 7 cycles at four warps per scheduler.  So the arithmetic is
+// packed (two columns an instruction), nothing is copied through shared memory, and six warps fit a scheduler.  With a
+// cp.async ring per lane, G a power of two and four warps per scheduler: 31 instructions per element.  With the residual
+// gradient and the fold of the partials, cold L2, fp16: 8192 x 1024 22.8 -> 18.0 us, 4096 x 1536 24.1 -> 15.5, 2048 x 768
+// 10.2 -> 7.7, 512 x 256 8.0 -> 4.2, 4096 x 2048 25.9 -> 23.0, 32768 x 1024 58.3 -> 50.6 (5.3 TB/s).
+constexpr int LN_WARPS = 12;  // of a CTA, at most
+constexpr int ln_groups(int g) { return LN_WARPS / g; }
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+template <typename T>
+__device__ __forceinline__ void unpack8_pairs(const uint4& raw, uint64_t (&v)[4]) {
+  float f[8];
+  unpack8<T>(raw, f);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = f2_pack(f[2 * i], f[2 * i + 1]);
 }
 
-template <typename T, int G>
-__global__ void __launch_bounds__(256, 2) ln_bwd_split_kernel(
+template <typename T, int G, bool RES>
+__global__ void __launch_bounds__(32 * G * ln_groups(G), LN_WARPS * 2 / (G * ln_groups(G))) ln_bwd_split_kernel(
     const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ alpha,
     const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
-    float* __restrict__ partials, int64_t rows, int d, int64_t dy_ld, int64_t x_ld, int64_t dx_ld,
-    const T* __restrict__ dres, int64_t dres_ld) {
+    float* __restrict__ partials, uint32_t rows, int d, uint32_t dy_ld, uint32_t x_ld, uint32_t dx_ld,
+    const T* __restrict__ dres, uint32_t dres_ld) {  // (32 bits: no registers for what walks down the tensors)
   grid_dependency_wait();
   allow_dependents();
-  constexpr int RG = 8 / G;  // row groups per CTA
+  constexpr int RG = ln_groups(G);
   extern __shared__ __align__(16) uint8_t ln_smem[];
-  uint4* ring = reinterpret_cast<uint4*>(ln_smem);                  // [warp][step][row][tensor][lane]
-  float* fold = reinterpret_cast<float*>(ln_smem + LN_RING_BYTES);  // [2][d]
-  __shared__ float4 xch[RG][2][G];
+  float* fold = reinterpret_cast<float*>(ln_smem);  // [RG][2][d]
+  __shared__ float2 xch[RG][2][G];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int part = warp % G, rg = warp / G;
-  const int nvec = d >> 3;
-  const int per = (nvec + G - 1) / G;  // vectors per warp, at most 32
-  const int c = part * per + lane;
-  const bool has = lane < per && c < nvec;
-  for (int i = threadIdx.x; i < 2 * d; i += blockDim.x) fold[i] = 0.f;
-  __syncthreads();
+  const int c = part * 32 + lane;
+  const bool has = c < (d >> 3);
 
-  float a[8], acc_a[8], acc_b[8];
+  uint64_t a[4], acc_a[4], acc_b[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) a[j] = acc_a[j] = acc_b[j] = 0.f;
-  if (has) unpack8<T>(__ldg(reinterpret_cast<const uint4*>(alpha) + c), a);
+  for (int j = 0; j < 4; ++j) a[j] = acc_a[j] = acc_b[j] = 0ull;
+  if (has) unpack8_pairs<T>(__ldg(reinterpret_cast<const uint4*>(alpha) + c), a);
   const float inv_d = 1.f / (float)d;
-  const int64_t stride = (int64_t)gridDim.x * RG;  // rows between the two rows of a step
-  const int64_t step_rows = 2 * stride;
-  int64_t row = (int64_t)blockIdx.x * RG + rg;
-  uint4* mine = ring + (size_t)warp * LN_DEPTH * 2 * 3 * 32 + lane;
-
-  // One commit group per step, issued by every lane (empty groups keep the count uniform).  The source pointers
-  // of the step being issued walk down the tensors (one 64-bit add per tensor and step; the row strides are
-  // multiples of eight elements on this path); `ileft` counts the rows from the first row of that step to the end.
-  const uint4* ix = reinterpret_cast<const uint4*>(x + row * x_ld) + c;
-  const uint4* idy = reinterpret_cast<const uint4*>(dy + row * dy_ld) + c;
-  const uint4* idr = dres ? reinterpret_cast<const uint4*>(dres + row * dres_ld) + c : nullptr;
-  const int64_t x_k = stride * (x_ld >> 3), dy_k = stride * (dy_ld >> 3), dr_k = stride * (dres_ld >> 3);  // second row
-  int64_t ileft = rows - row;
-  auto issue = [&](int slot) {
-    uint4* dst = mine + (slot * 2 * 3) * 32;
-    if (has && ileft > 0) {
-      cp_async16(dst, ix);
-      cp_async16(dst + 32, idy);
-      if (dres) cp_async16(dst + 64, idr);
+  const uint32_t stride = gridDim.x * RG;
+  uint32_t row = blockIdx.x * RG + rg;
+  auto at = [&](uint32_t r, uint32_t ld) -> uint64_t { return (uint64_t)r * ld + (uint32_t)(c * 8); };
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  uint4 nx = zero, ny = zero, nr = zero;
+  float n_mu = 0.f, n_rs = 0.f;
+  auto fetch = [&](uint32_t r) {
+    if (r >= rows) return;
+    if (has) {
+      nx = ld_stream16(x + at(r, x_ld));
+      ny = ld_stream16(dy + at(r, dy_ld));
+      if (RES) nr = ld_stream16(dres + at(r, dres_ld));
     }
-    if (has && ileft > stride) {
-      cp_async16(dst + 96, ix + x_k);
-      cp_async16(dst + 128, idy + dy_k);
-      if (dres) cp_async16(dst + 160, idr + dr_k);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    ix += 2 * x_k;
-    idy += 2 * dy_k;
-    if (dres) idr += 2 * dr_k;
-    ileft -= step_rows;
+    n_mu = __ldg(mean + r);
+    n_rs = __ldg(rstd + r);
   };
+  fetch(row);
+  int parity = 0;
+  for (; row < rows; row += stride) {
+    uint64_t h[4], g[4];
+    unpack8_pairs<T>(nx, h);
+    unpack8_pairs<T>(ny, g);
+    const uint4 raw = nr;
+    const float mu = n_mu, rs = n_rs;
+    fetch(row + stride);
+    // a lane without columns holds zeros, which contribute nothing
+    const uint64_t rs2 = has ? f2_pack(rs, rs) : 0ull, sh2 = has ? f2_pack(-mu * rs, -mu * rs) : 0ull;
+    uint64_t s1 = 0ull, s2 = 0ull;
+    const uint64_t one = f2_pack(1.f, 1.f);
 #pragma unroll
-  for (int s = 0; s < LN_DEPTH - 1; ++s) issue(s);
-  // the row statistics travel one step ahead in registers (a dependent load per step otherwise)
-  float mu_next[2], rs_next[2];
-  auto fetch_stats = [&](int64_t r0) {
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int64_t r = r0 + k * stride;
-      mu_next[k] = r < rows ? __ldg(mean + r) : 0.f;
-      rs_next[k] = r < rows ? __ldg(rstd + r) : 0.f;
+    for (int j = 0; j < 4; ++j) {
+      h[j] = f2_fma(h[j], rs2, sh2);          // normalised input
+      acc_a[j] = f2_fma(g[j], h[j], acc_a[j]);
+      acc_b[j] = f2_fma(g[j], one, acc_b[j]);
+      g[j] = f2_mul(g[j], a[j]);              // alpha-scaled gradient
+      s1 = f2_fma(g[j], h[j], s1);
+      s2 = f2_add(g[j], s2);
     }
-  };
-  fetch_stats(row);
-  int slot = 0, parity = 0;
-  for (; row < rows; row += step_rows) {
-    issue((slot + LN_DEPTH - 1) % LN_DEPTH);
-    const float mu_cur[2] = {mu_next[0], mu_next[1]}, rs_cur[2] = {rs_next[0], rs_next[1]};
-    fetch_stats(row + step_rows);
-    asm volatile("cp.async.wait_group %0;" ::"n"(LN_DEPTH - 1) : "memory");  // this step's copies have landed
-    uint4 cr[2];
-    float rs[2], s1[2], s2[2];
-    float h[2][8], gg[2][8];  // normalised input and alpha-scaled gradient, kept for the second pass
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int64_t r = row + k * stride;
-      const bool live = r < rows;
-      const float mu = mu_cur[k];
-      rs[k] = rs_cur[k];
-      const float shift = -mu * rs[k];
-      s1[k] = s2[k] = 0.f;
-      if (has && live) {
-        const uint4* src = mine + ((slot * 2 + k) * 3) * 32;
-        float xv[8], dv[8];
-        unpack8<T>(src[0], xv);
-        unpack8<T>(src[32], dv);
-        if (dres) cr[k] = src[64];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          h[k][j] = fmaf(xv[j], rs[k], shift);
-          gg[k][j] = dv[j] * a[j];
-          acc_a[j] = fmaf(dv[j], h[k][j], acc_a[j]);
-          acc_b[j] += dv[j];
-          s1[k] = fmaf(gg[k][j], h[k][j], s1[k]);
-          s2[k] += gg[k][j];
-        }
-      }
-    }
-    // The four sums of the step are reduced together: after the exchanges over 16 and over 8 lanes each lane
-    // carries ONE of them (which one: bits 4 and 3 of its lane number), so three more exchanges finish all four -
-    // six shuffles instead of twenty.  Lanes 0, 8, 16, 24 end up with s1[0], s2[0], s1[1], s2[1].
-    float red;
+    float t1, t2;
     {
-      const bool hi = lane & 16, mid = lane & 8;
-      float k0 = hi ? s1[1] : s1[0], k1 = hi ? s2[1] : s2[0];
-      k0 += __shfl_xor_sync(0xffffffffu, hi ? s1[0] : s1[1], 16);
-      k1 += __shfl_xor_sync(0xffffffffu, hi ? s2[0] : s2[1], 16);
-      red = (mid ? k1 : k0) + __shfl_xor_sync(0xffffffffu, mid ? k0 : k1, 8);
-      red += __shfl_xor_sync(0xffffffffu, red, 4);
-      red += __shfl_xor_sync(0xffffffffu, red, 2);
-      red += __shfl_xor_sync(0xffffffffu, red, 1);
-    }
-    if (G == 1) {
-      s1[0] = __shfl_sync(0xffffffffu, red, 0);
-      s2[0] = __shfl_sync(0xffffffffu, red, 8);
-      s1[1] = __shfl_sync(0xffffffffu, red, 16);
-      s2[1] = __shfl_sync(0xffffffffu, red, 24);
-    }
-    if (G > 1) {
-      // all G warps of the row group run the same number of steps, so the barrier counts match
-      if ((lane & 7) == 0) reinterpret_cast<float*>(&xch[rg][parity][part])[lane >> 3] = red;
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + rg), "r"(32 * G) : "memory");
-      float4 t = xch[rg][parity][0];
+      float lo, hi;
+      f2_unpack(s1, lo, hi);
+      t1 = lo + hi;
+      f2_unpack(s2, lo, hi);
+      t2 = lo + hi;
+      // both sums in five exchanges: after the first, the lower half of the warp carries t1 and the upper half t2
+      const bool up = lane & 16;
+      float v = (up ? t2 : t1) + __shfl_xor_sync(0xffffffffu, up ? t1 : t2, 16);
+      v += __shfl_xor_sync(0xffffffffu, v, 8);
+      v += __shfl_xor_sync(0xffffffffu, v, 4);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      if (G == 1) {
+        t1 = __shfl_sync(0xffffffffu, v, 0);
+        t2 = __shfl_sync(0xffffffffu, v, 16);
+      } else {
+        // all G warps of the group take the same number of rows, so the barrier counts match
+        if ((lane & 15) == 0) reinterpret_cast<float*>(&xch[rg][parity][part])[lane >> 4] = v;
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + rg), "r"(32 * G) : "memory");
+        t1 = t2 = 0.f;
 #pragma unroll
-      for (int g = 1; g < G; ++g) {
-        const float4 u = xch[rg][parity][g];
-        t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
-      }
-      s1[0] = t.x; s2[0] = t.y; s1[1] = t.z; s2[1] = t.w;
-      parity ^= 1;
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int64_t r = row + k * stride;
-      if (has && r < rows) {
-        // dx = rstd * (g - h * mean(g h) - mean(g)) as two fused multiply-adds per element
-        const float k1 = -rs[k] * s1[k] * inv_d, k2 = -rs[k] * s2[k] * inv_d;
-        float o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = fmaf(rs[k], gg[k][j], fmaf(k1, h[k][j], k2));
-        if (dres) {
-          float e[8];
-          unpack8<T>(cr[k], e);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += e[j];
+        for (int i = 0; i < G; ++i) {
+          const float2 u = xch[rg][parity][i];
+          t1 += u.x;
+          t2 += u.y;
         }
-        st_stream16(reinterpret_cast<uint4*>(dx + r * dx_ld) + c, pack8<T>(o));
+        parity ^= 1;
       }
     }
-    slot = (slot + 1) % LN_DEPTH;
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  // the row groups add their sums one after the other: a fixed order, so the result does not depend on timing
-  for (int g = 0; g < RG; ++g) {
-    if (has && rg == g) {
+    // dx = rstd * (g - h * mean(g h) - mean(g)) as two fused multiply-adds per element
+    const float k1 = -rs * t1 * inv_d, k2 = -rs * t2 * inv_d;
+    const uint64_t k1p = f2_pack(k1, k1), k2p = f2_pack(k2, k2);
+    uint64_t res[4];
+    if (RES) unpack8_pairs<T>(raw, res);
+    float o[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        fold[c * 8 + j] += acc_a[j];
-        fold[d + c * 8 + j] += acc_b[j];
-      }
+    for (int j = 0; j < 4; ++j) {
+      uint64_t v = f2_fma(rs2, g[j], f2_fma(k1p, h[j], k2p));
+      if (RES) v = f2_add(v, res[j]);  // gradient arriving through the residual branch that forked at this LayerNorm's input
+      f2_unpack(v, o[2 * j], o[2 * j + 1]);
     }
-    __syncthreads();
+    if (has) st_stream16(dx + at(row, dx_ld), pack8<T>(o));
   }
+  // the groups' sums are added in their order, so the result does not depend on timing
+  if (has) {
+    uint64_t* f = reinterpret_cast<uint64_t*>(fold + (size_t)rg * 2 * d + c * 8);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      f[j] = acc_a[j];
+      f[d / 2 + j] = acc_b[j];
+    }
+  }
+  __syncthreads();
   float* pa = partials + (int64_t)blockIdx.x * 2 * d;
-  for (int i = threadIdx.x; i < 2 * d; i += blockDim.x) pa[i] = fold[i];
+  for (int i = threadIdx.x; i < 2 * d; i += blockDim.x) {
+    float t = fold[i];
+#pragma unroll 4
+    for (int k = 1; k < RG; ++k) t += fold[(size_t)k * 2 * d + i];
+    pa[i] = t;
+  }
 }
 
 // 32 columns per CTA; the rows are spread over the CTA's warps (32 for many partial rows, 8 otherwise), so
@@ -476,24 +439,31 @@ static int ln_bwd_launch(const void* dy, const void* x, const void* alpha, const
   launch_overlapped(ln_bwd_kernel<T, V, MT>, dim3((unsigned)n_partials), dim3(threads), 0, st, \
       (const T*)dy, (const T*)x, (const T*)alpha, mean, rstd, (T*)dx, partials, rows, d, dy_ld, \
       x_ld, dx_ld, (const T*)dres, dres_ld)
-  if (vec && d <= 2048 && aligned16(alpha)) {
-    const size_t sm = (size_t)LN_RING_BYTES + (size_t)2 * d * sizeof(float);
+  constexpr int64_t kWide = 1LL << 31;
+  if (vec && d <= 2048 && aligned16(alpha) && rows < kWide && dy_ld < kWide && x_ld < kWide && dx_ld < kWide && dres_ld < kWide) {
     const T *gp = (const T*)dy, *xp = (const T*)x, *ap = (const T*)alpha, *rp = (const T*)dres;
     T* op = (T*)dx;
-    const dim3 grid((unsigned)n_partials), block(256);
-#define TFB_LN_SPLIT(G)                                                                                         \
-  do {                                                                                                          \
-    static std::atomic<uint64_t> attr_done{0};                                                                  \
-    if (int rc0 = ensure_dynamic_smem(ln_bwd_split_kernel<T, G>, (int)(LN_RING_BYTES + 2 * 2048 * sizeof(float)), \
-                                      attr_done, "layernorm_bwd"))                                              \
-      return rc0;                                                                                               \
-    launch_overlapped(ln_bwd_split_kernel<T, G>, grid, block, sm, st, gp, xp, ap, mean, rstd, op, partials, rows, d, \
-                      dy_ld, x_ld, dx_ld, rp, dres_ld);                                                         \
-  } while (0)
-    if (d <= 256) TFB_LN_SPLIT(1);
-    else if (d <= 512) TFB_LN_SPLIT(2);
-    else if (d <= 1024) TFB_LN_SPLIT(4);
-    else TFB_LN_SPLIT(8);
+    const dim3 grid((unsigned)n_partials);
+    // at most LN_WARPS / G groups of 2 d <= 512 G floats each: 24 KB
+#define TFB_LN_SPLIT(G, RES)                                                                                             \
+  launch_overlapped(ln_bwd_split_kernel<T, G, RES>, grid, dim3(32 * G * ln_groups(G)), (size_t)ln_groups(G) * 2 * d * 4, st, gp, xp, ap, \
+                    mean, rstd, op, partials, (uint32_t)rows, d, (uint32_t)dy_ld, (uint32_t)x_ld, (uint32_t)dx_ld, rp, (uint32_t)dres_ld)
+#define TFB_LN_GROUP(G)                                                                                                  \
+  case G:                                                                                                                \
+    if (dres) TFB_LN_SPLIT(G, true);                                                                                     \
+    else TFB_LN_SPLIT(G, false);                                                                                         \
+    break
+    switch ((d + 255) / 256) {
+      TFB_LN_GROUP(1);
+      TFB_LN_GROUP(2);
+      TFB_LN_GROUP(3);
+      TFB_LN_GROUP(4);
+      TFB_LN_GROUP(5);
+      TFB_LN_GROUP(6);
+      TFB_LN_GROUP(7);
+      TFB_LN_GROUP(8);
+    }
+#undef TFB_LN_GROUP
 #undef TFB_LN_SPLIT
   } else if (vec && threads <= 256) TFB_LN_BWD(true, 256);
   else if (vec) TFB_LN_BWD(true, 1024);
