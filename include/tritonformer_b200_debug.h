@@ -13,7 +13,8 @@ extern "C" {
 /* Test and tuning switches.
  *   key 0: value 1 sends every GEMM to the generic-stride kernel.
  *   key 1: value 1 sends every attention call to the mma.sync kernels.
- *   key 2: attention: bit 0 skips the dQ accumulation, bit 1 turns the cycle counters on, bit 5 (32) walks the
+ *   key 2: attention (bits 0, 1, 6 and 7 in the backward: head_dim 32 and 64): bit 0 skips the dQ accumulation, bit 1 turns the
+ *          cycle counters on, bit 5 (32) walks the
  *          (tile, batch*head) items slice by slice instead of longest first, bit 6 (64) adds dQ with vector
  *          atomics instead of the TMA reduction, bit 7 (128) keeps only the barriers of the backward's compute
  *          warps going (timing experiments: results are then meaningless).

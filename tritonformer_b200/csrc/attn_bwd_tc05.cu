@@ -1,14 +1,13 @@
-// Causal flash attention backward on tcgen05 / TMEM for sm_100a (head_dim 32, 64 or 128).
+// Causal flash attention backward on tcgen05 / TMEM for sm_100a (head_dim 32 or 64; 128: attn_bwd128_tc05.cu).
 //
 // An item is a (128-key tile, batch*head); a CTA walks its query tiles at or below the diagonal.  The grid has one block per
 // item, but a CTA that is nearly done with its item takes over a block that has not been launched yet (cluster launch
 // control: that launch is cancelled and its block index handed over), so tensor memory, barriers and the ring stay set up
 // from item to item.  With a fresh CTA per item, 8.9 k of the 53 k cycles of an average item at T 2048 were spent outside the
 // walk.  A list dealt out in advance would do the same, but not beside the weight-gradient products of another stream, which
-// hold some of the SMs.  At head_dim 64, K and V are doubled as well, so that the next item's scores run ahead like those of
+// hold some of the SMs.  K and V are doubled as well, so that the next item's scores run ahead like those of
 // any next tile, and an item's dV and dK are written behind the arithmetic of the next item's first tile.
-// Backward with its two small passes, fp16: B4 H16 T2048 hd64 208 -> 194 us, B1 H12 T4096 hd128 265 -> 255, B2 H16 T2048
-// hd128 202 -> 188.
+// Backward with its two small passes, fp16: B4 H16 T2048 hd64 208 -> 194 us.
 // Everything is computed transposed (rows = keys) so that the per-query statistics (log-sum-exp,
 // delta) are per-column constants and no row reductions are needed:
 //   Sᵀ  = K Q_iᵀ                 dPᵀ = V dO_iᵀ                      (tensor cores -> TMEM)
@@ -23,17 +22,19 @@
 //
 // Roles: warp 0 TMA producer, warp 1 MMA issuer, warps 2-17 compute (thread = TMEM lane, four
 // warps per lane quarter, each taking a quarter of the columns), warps 18-21 drain dQ_i.
-// At head_dim 64, Pᵀ goes into the 64 TMEM columns that are left instead of shared memory and is
+// Pᵀ goes into the 64 TMEM columns that are left instead of shared memory and is
 // the A operand of the dV product.
-// At head_dim 64 the scores of tile i+1 are issued as soon as the compute warps hold the scores of tile i in
+// The scores of tile i+1 are issued as soon as the compute warps hold the scores of tile i in
 // registers, ahead of the gradient products of tile i, so the compute warps find them ready and work on tile
 // i+1 while the tensor core finishes tile i.
 // A sequence that is no multiple of 128: the rows past its end are zeros in shared memory (TMA fill); as queries they get
 // exact zeros for P and dS and their rows of dQ are left out (the accumulator's next rows are another slice's), as keys the
 // mask keeps them from every query and their rows are not stored.  head_dim 32 runs on the
 // head_dim 64 kernel with zero columns.
-// TMEM columns: [0,128) Sᵀ; [128,256) dPᵀ; [256,256+hd) dV; then dK; then dQ_i (at head_dim 128
-// dQ_i reuses the Sᵀ columns).
+// (Sub-tiles of 64 queries on two CTAs per SM with half of tensor and shared memory each, tried here as well: 205-218 us against
+// 191 at B4 H16 T2048 fp16, 165 against 89 at B1 H8 T4096.  A sub-tile's chain takes 4.3 k cycles even alone on an SM, nearly as
+// long as a whole tile's 5.5 k, and the two CTAs share what it waits for.)
+// TMEM columns: [0,128) Sᵀ; [128,256) dPᵀ; [256,320) dV; then dK; then dQ_i; then Pᵀ.
 #include "attn.cuh"
 #include "tc05.cuh"
 #include <type_traits>
@@ -48,45 +49,30 @@ constexpr int FB_CWARPS = 16;        // compute warps: 4 TMEM lane quarters x 4 
 constexpr int FB_THREADS = 64 + 32 * FB_CWARPS + 128;  // TMA, MMA, compute warps, 4 dQ-drain warps
 constexpr int FB_COMPUTE = 256;     // threads in the compute warps
 
-template <int HD> struct FbCfg {
-  static constexpr int PANELS = HD / 64;
-  static constexpr int TILE_BYTES = PANELS * 16384;   // 128 rows x HD x 2 B
-  // Query-side ring depth.  head_dim 64 needs three stages: the gradient products of tile i-1 still read their
-  // Q / dO while the scores of tile i+1 are issued (with two, the load of tile i+1 could only start when tile
-  // i-1 had retired, and its latency showed up as a wait for scores on every tile).  Pᵀ lives in tensor memory
-  // there, so its shared-memory buffer is not allocated and the third stage takes its place.  One stage at
-  // head_dim 128 (shared memory).
-  static constexpr int QSTAGES = (HD == 64) ? 3 : 1;
-  // K and V of two items at head_dim 64: the next item's scores run ahead of the current item's last products like those of
-  // any next tile.  (With one, the walk stood still for 7.9 k cycles from item to item.)
-  static constexpr int KVSTAGES = (HD == 64) ? 2 : 1;
-  static constexpr int OFF_K = 0;                                    // [KVSTAGES][K, V]
-  static constexpr int OFF_V = TILE_BYTES;
-  static constexpr int OFF_Q = KVSTAGES * 2 * TILE_BYTES;            // [QSTAGES]
-  static constexpr int OFF_DO = OFF_Q + QSTAGES * TILE_BYTES;        // [QSTAGES]
-  static constexpr int OFF_P = OFF_DO + QSTAGES * TILE_BYTES;        // Pᵀ  128 x 128 x 2 B (head_dim 128 only)
-  static constexpr int OFF_DS = OFF_P + ((256 + 3 * HD + 64 <= 512) ? 0 : 32768);  // dSᵀ 128 x 128 x 2 B
-  static constexpr int OFF_STAT = OFF_DS + 32768;                    // [2 parities][16 compute warps][lse2[32], delta[32]] fp32
-  // dQ_i staging for the TMA reduction: boxes of 32 rows x 128 B (32 columns).  At head_dim 64 they have shared memory of
-  // their own, one per drain warp, which its two chunks pass through one after the other.  At head_dim 128 there is none left, and the
-  // sixteen boxes are the Pᵀ / dSᵀ buffers themselves: between the last gradient product of a tile and the
-  // compute warps' next write nothing else uses them.
-  static constexpr bool DQ_TMA = true;
-  static constexpr bool DQ_IN_PDS = (HD == 128);
-  static constexpr int DQ_BOXES = (HD == 64) ? 1 : 0;
-  static constexpr int OFF_DQ = OFF_STAT + 8192;
-  static constexpr int OFF_BAR = OFF_DQ + 4 * DQ_BOXES * 4096;
-  static constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
-  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
-  static constexpr int COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 256 + HD;
-  // dQ_i has columns of its own when they fit (hd 64); otherwise it reuses the Sᵀ columns
-  static constexpr bool DQ_ALIASED = (256 + 3 * HD > 512);
-  static constexpr int COL_DQ = DQ_ALIASED ? 0 : 256 + 2 * HD;
-  // Pᵀ (16-bit, two queries per column) lives in tensor memory when 64 columns are left for it (hd 64):
-  // it is the A operand of the dV product, which then reads only dO from shared memory
-  static constexpr bool P_TMEM = (256 + 3 * HD + 64 <= 512);
-  static constexpr int COL_PT = 256 + 3 * HD;
-};
+constexpr int HD = 64;
+constexpr int TILE_BYTES = FB_T * 128;   // 128 rows x 64 x 2 B
+// Query-side ring depth: the gradient products of tile i-1 still read their Q / dO while the scores of tile i+1 are issued
+// (with two, the load of tile i+1 could only start when tile i-1 had retired, and its latency showed up as a wait for scores on
+// every tile).
+constexpr int QS = 3;
+// K and V of two items: the next item's scores run ahead of the current item's last products like those of
+// any next tile.  (With one, the walk stood still for 7.9 k cycles from item to item.)
+constexpr int KVS = 2;
+constexpr int OFF_K = 0;                              // [KVS][K, V]
+constexpr int OFF_V = TILE_BYTES;
+constexpr int OFF_Q = KVS * 2 * TILE_BYTES;           // [QS]
+constexpr int OFF_DO = OFF_Q + QS * TILE_BYTES;       // [QS]
+constexpr int OFF_DS = OFF_DO + QS * TILE_BYTES;      // dSᵀ 128 x 128 x 2 B
+constexpr int OFF_STAT = OFF_DS + 32768;              // [2 parities][16 compute warps][lse2[32], delta[32]] fp32
+// dQ_i staging for the TMA reduction: a box of 32 rows x 128 B (32 columns) per drain warp, which its two chunks pass through
+// one after the other.
+constexpr int OFF_DQ = OFF_STAT + 8192;
+constexpr int OFF_BAR = OFF_DQ + 4 * 4096;
+constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
+static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
+constexpr int COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 256 + HD, COL_DQ = 256 + 2 * HD;
+// Pᵀ (16-bit, two queries per column): the A operand of the dV product, which then reads only dO from shared memory
+constexpr int COL_PT = 256 + 3 * HD;
 
 struct FbParams {
   const float* lse;
@@ -94,7 +80,7 @@ struct FbParams {
   float* dq_acc;  // (B,H,T,HD) fp32, zero on entry
   void *dk, *dv;
   int64_t sdk_b, sdk_h, sdk_t, sdv_b, sdv_h, sdv_t;
-  int H, T, hd;   // hd: the real head_dim, at most HD
+  int H, T, hd;   // hd: the real head_dim, 32 or 64
   int BH, group;  // batch*heads; how many of them are walked together (their tiles share the L2)
   float scale;
   int bias_mode;
@@ -124,29 +110,26 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 
 // RAGGED: T is no multiple of 128 (a run-time branch in the compute and drain loops cost whole tiles 1 %: B4 H16 T2048 hd64
 // fp16 193 against 191 us, spilled registers).
-template <typename T, int HD, int BIAS, bool RAGGED>
+template <typename T, int BIAS, bool RAGGED>
 __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                       const __grid_constant__ CUtensorMap tmK,
                                                                       const __grid_constant__ CUtensorMap tmV,
                                                                       const __grid_constant__ CUtensorMap tmDO,
                                                                       const __grid_constant__ CUtensorMap tmDQ,
                                                                       const FbParams p) {
-  using Cfg = FbCfg<HD>;
-  constexpr int QS = Cfg::QSTAGES, KVS = Cfg::KVSTAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* s_stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);  // [2 parities][16 warps][lse2[32], delta[32]]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
+  float* s_stat = reinterpret_cast<float*>(smem + OFF_STAT);  // [2 parities][16 warps][lse2[32], delta[32]]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* q_full = bars + 0;       // [3] Q_i and dO_i landed
   uint64_t* q_empty = bars + 3;      // [3] products reading them retired
   uint64_t* s_full = bars + 6;       // Sᵀ and dPᵀ in TMEM
   uint64_t* pds_full = bars + 7;     // Pᵀ and dSᵀ in smem (and Sᵀ, dPᵀ consumed)
   uint64_t* dq_full = bars + 8;      // dV, dK, dQ_i products retired
   uint64_t* dq_free = bars + 9;      // dQ_i read out of TMEM
-  uint64_t* s_free = bars + 10;      // Sᵀ and dPᵀ read out of TMEM (head_dim 64: the next scores may overwrite them)
-  uint64_t* stage_free = bars + 11;  // head_dim 128: the TMA unit has read dQ_i out of the Pᵀ / dSᵀ buffers
-  uint64_t* kv_full = bars + 12;     // [KVSTAGES] K and V of an item landed
-  uint64_t* kv_empty = bars + 14;    // [KVSTAGES] the item's last products have retired: K and V may be replaced
+  uint64_t* s_free = bars + 10;      // Sᵀ and dPᵀ read out of TMEM: the next scores may overwrite them
+  uint64_t* kv_full = bars + 12;     // [KVS] K and V of an item landed
+  uint64_t* kv_empty = bars + 14;    // [KVS] the item's last products have retired: K and V may be replaced
   uint64_t* acc_free = bars + 16;    // dV and dK of an item have been read out of TMEM
   uint64_t* next_full = bars + 17;   // the answer to the request for another item has landed
   uint64_t* next_empty = bars + 18;  // every role has read it
@@ -192,7 +175,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
   };
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < Cfg::KVSTAGES; ++i) {
+    for (int i = 0; i < KVS; ++i) {
       mbar_init(&kv_full[i], 1);
       mbar_init(&kv_empty[i], 1);
     }
@@ -205,7 +188,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
     mbar_init(dq_full, 1);
     mbar_init(dq_free, 4);
     mbar_init(s_free, FB_CWARPS);
-    mbar_init(stage_free, 4);
     mbar_init(acc_free, FB_CWARPS);
     mbar_init(next_full, 1);
     mbar_init(next_empty, 2 + FB_CWARPS + 4);  // producer, MMA issuer, compute warps, drain warps
@@ -239,29 +221,22 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       auto load_kv = [&](int n) -> bool {
         const int ks = n % KVS, b = w.bh / p.H, h = w.bh % p.H;
         if (n >= KVS && !mbar_wait(&kv_empty[ks], (n / KVS - 1) & 1, 0x2110 | ks, abort_flag)) return false;
-        mbar_expect_tx(&kv_full[ks], 2 * Cfg::TILE_BYTES);
-        uint8_t* dst = smem + Cfg::OFF_K + ks * 2 * Cfg::TILE_BYTES;
-#pragma unroll
-        for (int c = 0; c < Cfg::PANELS; ++c) {
-          tma_load_4d(dst + c * 16384, &tmK, c * 64, w.kt * FB_T, h, b, &kv_full[ks]);
-          tma_load_4d(dst + Cfg::TILE_BYTES + c * 16384, &tmV, c * 64, w.kt * FB_T, h, b, &kv_full[ks]);
-        }
+        mbar_expect_tx(&kv_full[ks], 2 * TILE_BYTES);
+        uint8_t* dst = smem + OFF_K + ks * 2 * TILE_BYTES;
+        tma_load_4d(dst, &tmK, 0, w.kt * FB_T, h, b, &kv_full[ks]);
+        tma_load_4d(dst + TILE_BYTES, &tmV, 0, w.kt * FB_T, h, b, &kv_full[ks]);
         return true;
       };
       for (int n = 0; ok; ++n) {
-        if (KVS > 1) ok = load_kv(n);
+        ok = load_kv(n);
         for (int it = 0; it < nq - w.kt && ok; ++it, ++g) {
           const int st = g % QS;
           const uint32_t ph = (g / QS) & 1;
           if (!mbar_wait(&q_empty[st], ph ^ 1, 0x2100 | st, abort_flag)) { ok = false; break; }
-          mbar_expect_tx(&q_full[st], 2 * Cfg::TILE_BYTES);
+          mbar_expect_tx(&q_full[st], 2 * TILE_BYTES);
           const int i0 = (w.kt + it) * FB_T, b = w.bh / p.H, h = w.bh % p.H;
-#pragma unroll
-          for (int c = 0; c < Cfg::PANELS; ++c) {
-            tma_load_4d(smem + Cfg::OFF_Q + st * Cfg::TILE_BYTES + c * 16384, &tmQ, c * 64, i0, h, b, &q_full[st]);
-            tma_load_4d(smem + Cfg::OFF_DO + st * Cfg::TILE_BYTES + c * 16384, &tmDO, c * 64, i0, h, b, &q_full[st]);
-          }
-          if (KVS == 1 && it == 0) ok = load_kv(n);
+          tma_load_4d(smem + OFF_Q + st * TILE_BYTES, &tmQ, 0, i0, h, b, &q_full[st]);
+          tma_load_4d(smem + OFF_DO + st * TILE_BYTES, &tmDO, 0, i0, h, b, &q_full[st]);
         }
         // Asked for only now, with the item's last loads issued: asked for at its start, the CTAs with the longest items
         // would take the first of the remaining ones.
@@ -279,39 +254,32 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
     // them to the uniform registers the tensor core reads (measured: 63 cycles per M128 N64 K16 instruction
     // against 49 with warp-uniform code, and 80-120 in this kernel, where it made the issue of a tile's 32
     // instructions the longest item of the step).
-    // At head_dim 128 every instruction is 64 cycles of tensor work, the single lane keeps up, and the faster
-    // bursts only took tensor-memory bandwidth from the compute warps (373 against 349 us at T 4096): there the
-    // loop stays in lane 0.
-    constexpr bool WHOLE_WARP = (HD == 64);
-    if (!dead && (WHOLE_WARP || lane == 0)) {
+    if (!dead) {
       constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
       constexpr uint32_t idesc_s = instr_desc_f16(128, 128, fmt, 0, 0);   // Sᵀ, dPᵀ : both K-major
       constexpr uint32_t idesc_kv = instr_desc_f16(128, HD, fmt, 0, 1);   // dV, dK  : A K-major, B MN-major
       constexpr uint32_t idesc_q = instr_desc_f16(128, HD, fmt, 1, 1);    // dQ      : both MN-major
       // read from shared memory: tell the compiler it is uniform
-      const uint32_t tb = WHOLE_WARP ? __shfl_sync(0xffffffffu, tmem_base, 0) : tmem_base;
-      auto leader = [&]() -> bool { return WHOLE_WARP ? elect_one() : true; };
+      const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0);
       // operand descriptors of every buffer in both roles; each MMA only advances the start address
       // (K-major: lbo unused, 8-row groups 1024 B apart; MN-major: 64-element chunks one 16 KB panel apart,
       // 8-row groups 1024 B apart)
       const uint32_t s0 = smem_u32(smem);
-      const uint64_t dk_k = smem_desc_sw128(s0 + Cfg::OFF_K, 16, 1024);
-      const uint64_t dk_mn = smem_desc_sw128(s0 + Cfg::OFF_K, 16384, 1024);
-      const uint64_t dv_k = smem_desc_sw128(s0 + Cfg::OFF_V, 16, 1024);
-      const uint64_t dp_k = smem_desc_sw128(s0 + Cfg::OFF_P, 16, 1024);
-      const uint64_t dds_k = smem_desc_sw128(s0 + Cfg::OFF_DS, 16, 1024);
-      const uint64_t dds_mn = smem_desc_sw128(s0 + Cfg::OFF_DS, 16384, 1024);
+      const uint64_t dk_k = smem_desc_sw128(s0 + OFF_K, 16, 1024);
+      const uint64_t dk_mn = smem_desc_sw128(s0 + OFF_K, 16384, 1024);
+      const uint64_t dv_k = smem_desc_sw128(s0 + OFF_V, 16, 1024);
+      const uint64_t dds_k = smem_desc_sw128(s0 + OFF_DS, 16, 1024);
+      const uint64_t dds_mn = smem_desc_sw128(s0 + OFF_DS, 16384, 1024);
       const bool prof = (p.debug & 2) && lane == 0;
       PROF_T(tm_start);
       // every lane waits; the verdict is made uniform so that the warp stays converged
       auto wait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
-        const bool r = mbar_wait(bar, parity, code, abort_flag);
-        return WHOLE_WARP ? (__all_sync(0xffffffffu, r) != 0) : r;
+        return __all_sync(0xffffffffu, mbar_wait(bar, parity, code, abort_flag)) != 0;
       };
       bool ok = true;
       // Sᵀ = K Q_iᵀ and dPᵀ = V dO_iᵀ of query tile `it`
       auto issue_scores = [&](int g, int n) -> bool {  // g: tiles of the CTA before this one, n: items
-        const uint32_t kv = (n % KVS) * 2 * Cfg::TILE_BYTES;
+        const uint32_t kv = (n % KVS) * 2 * TILE_BYTES;
         const int st = g % QS;
         PROF_T(a0);
         if (!wait(&q_full[st], (g / QS) & 1, 0x2300 | st)) return false;
@@ -319,29 +287,29 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         PROF_ADD(7, a0, a1);
         tc_fence_after();
         PROF_T(i0_);
-        const uint64_t q_k = smem_desc_sw128(s0 + Cfg::OFF_Q + st * Cfg::TILE_BYTES, 16, 1024);
-        const uint64_t do_k = smem_desc_sw128(s0 + Cfg::OFF_DO + st * Cfg::TILE_BYTES, 16, 1024);
+        const uint64_t q_k = smem_desc_sw128(s0 + OFF_Q + st * TILE_BYTES, 16, 1024);
+        const uint64_t do_k = smem_desc_sw128(s0 + OFF_DO + st * TILE_BYTES, 16, 1024);
 #pragma unroll
         for (int s = 0; s < HD / 16; ++s) {
           const uint32_t off = (s / 4) * 16384 + (s % 4) * 32;
-          if (leader()) tc_mma_ss(tb + Cfg::COL_S, desc_advance(dk_k, kv + off), desc_advance(q_k, off), idesc_s, s ? 1u : 0u);
+          if (elect_one()) tc_mma_ss(tb + COL_S, desc_advance(dk_k, kv + off), desc_advance(q_k, off), idesc_s, s ? 1u : 0u);
         }
 #pragma unroll
         for (int s = 0; s < HD / 16; ++s) {
           const uint32_t off = (s / 4) * 16384 + (s % 4) * 32;
-          if (leader()) tc_mma_ss(tb + Cfg::COL_DP, desc_advance(dv_k, kv + off), desc_advance(do_k, off), idesc_s, s ? 1u : 0u);
+          if (elect_one()) tc_mma_ss(tb + COL_DP, desc_advance(dv_k, kv + off), desc_advance(do_k, off), idesc_s, s ? 1u : 0u);
         }
-        if (leader()) tc_commit(s_full);
+        if (elect_one()) tc_commit(s_full);
         PROF_T(i1_);
         PROF_ADD(12, i0_, i1_);
         return true;
       };
       // dV += Pᵀ dO_i, dK += dSᵀ Q_i, dQ_i = dS K
       auto issue_grads = [&](int g, int n, int it, bool last) -> bool {
-        const uint32_t kv = (n % KVS) * 2 * Cfg::TILE_BYTES;
+        const uint32_t kv = (n % KVS) * 2 * TILE_BYTES;
         const int st = g % QS;
-        const uint64_t q_mn = smem_desc_sw128(s0 + Cfg::OFF_Q + st * Cfg::TILE_BYTES, 16384, 1024);
-        const uint64_t do_mn = smem_desc_sw128(s0 + Cfg::OFF_DO + st * Cfg::TILE_BYTES, 16384, 1024);
+        const uint64_t q_mn = smem_desc_sw128(s0 + OFF_Q + st * TILE_BYTES, 16384, 1024);
+        const uint64_t do_mn = smem_desc_sw128(s0 + OFF_DO + st * TILE_BYTES, 16384, 1024);
         // the dQ columns still hold the previous tile's dQ until the drain warps are done with it
         PROF_T(a0);
         if (g > 0 && !wait(dq_free, (g - 1) & 1, 0x2400)) return false;
@@ -354,20 +322,17 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         for (int s = 0; s < FB_T / 16; ++s) {  // contraction over the 128 queries of this tile
           const uint32_t koff = (s / 4) * 16384 + (s % 4) * 32;  // K-major A: 16 queries = 32 B along the row
           const uint32_t moff = s * 2048;                         // MN-major B: 16 query rows of 128 B
-          if (leader()) {
-            if (Cfg::P_TMEM)
-              tc_mma_ts(tb + Cfg::COL_DV, tb + Cfg::COL_PT + s * 8, desc_advance(do_mn, moff), idesc_kv, s ? 1u : acc);
-            else
-              tc_mma_ss(tb + Cfg::COL_DV, desc_advance(dp_k, koff), desc_advance(do_mn, moff), idesc_kv, s ? 1u : acc);
-            tc_mma_ss(tb + Cfg::COL_DK, desc_advance(dds_k, koff), desc_advance(q_mn, moff), idesc_kv, s ? 1u : acc);
+          if (elect_one()) {
+            tc_mma_ts(tb + COL_DV, tb + COL_PT + s * 8, desc_advance(do_mn, moff), idesc_kv, s ? 1u : acc);
+            tc_mma_ss(tb + COL_DK, desc_advance(dds_k, koff), desc_advance(q_mn, moff), idesc_kv, s ? 1u : acc);
           }
         }
 #pragma unroll
         for (int s = 0; s < FB_T / 16; ++s) {  // contraction over the 128 keys of this CTA
           const uint32_t moff = s * 2048;      // 16 key rows of 128 B in dSᵀ and in K
-          if (leader()) tc_mma_ss(tb + Cfg::COL_DQ, desc_advance(dds_mn, moff), desc_advance(dk_mn, kv + moff), idesc_q, s ? 1u : 0u);
+          if (elect_one()) tc_mma_ss(tb + COL_DQ, desc_advance(dds_mn, moff), desc_advance(dk_mn, kv + moff), idesc_q, s ? 1u : 0u);
         }
-        if (leader()) {
+        if (elect_one()) {
           tc_commit(&q_empty[st]);
           tc_commit(dq_full);
           if (last) tc_commit(&kv_empty[n % KVS]);
@@ -384,11 +349,11 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         bool more = false;
         for (int it = 0; it < nq - w.kt && ok; ++it, ++g) {
           const bool last = w.kt + it + 1 == nq;
-          if (KVS > 1 && last) {
-            more = next_of(n, wn, !WHOLE_WARP);
+          if (last) {
+            more = next_of(n, wn, false);
             if (more && !wait(&kv_full[(n + 1) % KVS], ((n + 1) / KVS) & 1, 0x2200)) { ok = false; break; }
           }
-          if (!Cfg::DQ_ALIASED && (!last || more)) {
+          if (!last || more) {
             // The compute warps hand Sᵀ / dPᵀ back as soon as they hold them in registers, about half-way through
             // their work on the tile: the next tile's scores are issued then and have landed when the warps come
             // back for them.  (Issued only once Pᵀ / dSᵀ were ready, they cost a round trip of 1.5 k cycles per
@@ -403,18 +368,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           // the first products of an item overwrite dV and dK of the one before
           if (it == 0 && n > 0 && !wait(acc_free, (n - 1) & 1, 0x2560)) { ok = false; break; }
           ok = issue_grads(g, n, it, last);
-          if (KVS == 1 && ok && last) {
-            more = next_of(n, wn, !WHOLE_WARP);
-            if (more && !wait(&kv_full[0], (n + 1) & 1, 0x2200)) { ok = false; break; }
-          }
-          if (Cfg::DQ_ALIASED && ok && (!last || more)) {
-            // dQ_i reuses the Sᵀ columns: the next scores may only follow once dQ_i has been drained
-            PROF_T(b0);
-            ok = wait(dq_free, g & 1, 0x2450);
-            PROF_T(b1);
-            PROF_ADD(8, b0, b1);
-            if (ok) ok = issue_scores(g + 1, last ? n + 1 : n);
-          }
         }
         if (!more) break;
         w = wn;
@@ -430,11 +383,9 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       const int qd = warp & 3;           // TMEM lane quarter
       const int cq = cw >> 2;            // which quarter (32) of the 128 query columns
       const int r = qd * 32 + lane;      // TMEM lane = key row
-      const int ct = threadIdx.x - 64;   // 0..255 within the compute group
       const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
       const float c2 = p.scale * kLog2eB;
-      uint8_t* sp = smem + Cfg::OFF_P;
-      uint8_t* sds = smem + Cfg::OFF_DS;
+      uint8_t* sds = smem + OFF_DS;
       bool ok = true;
       const bool prof = (p.debug & 2) && threadIdx.x == 64;
       // Per-query statistics of the warp's 32 query columns: lane l carries lse and delta of
@@ -460,8 +411,8 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           const int col0 = cq * (HD / 4) + c * 8;
           if (col0 >= p.hd) break;
           uint32_t v[8], u[8];
-          tmem_ld8(lane_addr + Cfg::COL_DV + col0, v);
-          tmem_ld8(lane_addr + Cfg::COL_DK + col0, u);
+          tmem_ld8(lane_addr + COL_DV + col0, v);
+          tmem_ld8(lane_addr + COL_DK + col0, u);
           tc_wait_ld();
           if (j < p.T) {
             float f[8];
@@ -480,7 +431,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       };
       // With the next item's scores already there, an item is stored behind the arithmetic of the next one's first tile,
       // which hides its last products.
-      constexpr bool LATE_STORE = KVS > 1;
       int g = 0;  // tiles of the CTA before this one
       for (int n = 0;; ++n) {
       const AlibiLog2<BIAS> alibi(BIAS ? p.slopes[w.bh % p.H] : 0.f);
@@ -509,7 +459,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         if (quiet) {
 #pragma unroll
           for (int e = 0; e < 16; ++e) pk[e] = dk_[e] = 0u;
-          if (!Cfg::DQ_ALIASED && lane == 0) mbar_arrive(s_free);
+          if (lane == 0) mbar_arrive(s_free);
           if (g > 0 && ok) ok = mbar_wait(dq_full, (g - 1) & 1, 0x2650, abort_flag);
         }
         if (ok && !quiet) {
@@ -522,17 +472,17 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           // than it saved, 230 against 210 us.)
           uint32_t sv_[2][8], dv_[2][8];
           PROF_T(tl0);
-          tmem_ld8(lane_addr + Cfg::COL_S + cq * 32, sv_[0]);
-          tmem_ld8(lane_addr + Cfg::COL_DP + cq * 32, dv_[0]);
+          tmem_ld8(lane_addr + COL_S + cq * 32, sv_[0]);
+          tmem_ld8(lane_addr + COL_DP + cq * 32, dv_[0]);
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             const int col0 = cq * 32 + c * 8;
             const float d0 = (float)(i0 + col0 - j);  // distance of the chunk's first query to this thread's key
             tc_wait_ld();
             if (c + 1 < 4) {
-              tmem_ld8(lane_addr + Cfg::COL_S + col0 + 8, sv_[(c + 1) & 1]);
-              tmem_ld8(lane_addr + Cfg::COL_DP + col0 + 8, dv_[(c + 1) & 1]);
-            } else if (!Cfg::DQ_ALIASED) {  // this warp's share of Sᵀ and dPᵀ is in registers
+              tmem_ld8(lane_addr + COL_S + col0 + 8, sv_[(c + 1) & 1]);
+              tmem_ld8(lane_addr + COL_DP + col0 + 8, dv_[(c + 1) & 1]);
+            } else {  // this warp's share of Sᵀ and dPᵀ is in registers
               tc_fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive(s_free);
@@ -574,8 +524,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           // Pᵀ / dSᵀ of the previous tile are still being read by its gradient products
           if (prof) t3 = clock64();
           if (g > 0) ok = mbar_wait(dq_full, (g - 1) & 1, 0x2650, abort_flag);
-          // ... and, at head_dim 128, by the TMA reduction of its dQ, which was staged in them
-          if (Cfg::DQ_IN_PDS && g > 0 && ok) ok = mbar_wait(stage_free, (g - 1) & 1, 0x2660, abort_flag);
           if (prof) t4 = clock64();
           PROF_ADD(2, t2, t3);
           PROF_ADD(3, t3, t4);
@@ -586,23 +534,21 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
 #pragma unroll
           for (int e = 0; e < 16; ++e) pk[e] = dk_[e] = 0u;
         }
-        if (LATE_STORE && it == 0 && n > 0 && ok) store_item(wp);  // (the wait for dq_full above was for its last tile)
+        if (it == 0 && n > 0 && ok) store_item(wp);  // (the wait for dq_full above was for its last tile)
         if (ok && quiet) {
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(pds_full);
         }
         if (ok && !quiet) {
-          if (Cfg::P_TMEM) tmem_st16(lane_addr + Cfg::COL_PT + cq * 16, pk);  // this thread's 32 queries of Pᵀ
+          tmem_st16(lane_addr + COL_PT + cq * 16, pk);  // this thread's 32 queries of Pᵀ
 #pragma unroll
           for (int v4 = 0; v4 < 4; ++v4) {
             const int cc = cq * 4 + v4;  // 16-byte chunk index along the 128 queries
             const uint32_t off = (cc >> 3) * 16384 + r * 128 + (((cc & 7) ^ (r & 7)) << 4);
-            if (!Cfg::P_TMEM)
-              *reinterpret_cast<uint4*>(sp + off) = make_uint4(pk[v4 * 4], pk[v4 * 4 + 1], pk[v4 * 4 + 2], pk[v4 * 4 + 3]);
             *reinterpret_cast<uint4*>(sds + off) = make_uint4(dk_[v4 * 4], dk_[v4 * 4 + 1], dk_[v4 * 4 + 2], dk_[v4 * 4 + 3]);
           }
-          if (Cfg::P_TMEM) tc_wait_st();
+          tc_wait_st();
           PROF_T(t45);
           tc_fence_before();
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -616,7 +562,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       Item wn = w;
       const bool more = __all_sync(0xffffffffu, ok) != 0 && next_of(n, wn, false);
       if (more) load_stat(wn, 0, lse_next, delta_next);  // on their way while this item is finished
-      if (!LATE_STORE || !more) {
+      if (!more) {
         if (ok) ok = mbar_wait(dq_full, (g - 1) & 1, 0x2680, abort_flag);
         if (ok) store_item(w);
       }
@@ -628,15 +574,14 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
   } else if (!dead) {
     // ---------------------------------------------------------------------------- dQ drain
     // the last four warps: lanes are query rows here; each warp adds its 32 rows of dQ_i to the fp32 accumulator.
-    // head_dim 64: the rows go through swizzled shared-memory boxes and the TMA unit performs the
-    // reduction (cp.reduce.async.bulk.tensor), which keeps the load/store path free for the compute
-    // warps; head_dim 128: vector red.global.add.
+    // The rows go through swizzled shared-memory boxes and the TMA unit performs the
+    // reduction (cp.reduce.async.bulk.tensor), which keeps the load/store path free for the compute warps.
     const int qd = warp & 3;
     const int r = qd * 32 + lane;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
     const bool prof = (p.debug & 2) && warp == 2 + FB_CWARPS && lane == 0;
-    uint8_t* stage = smem + Cfg::OFF_DQ + (warp - 2 - FB_CWARPS) * Cfg::DQ_BOXES * 4096;
-    if (Cfg::DQ_TMA && lane == 0) tma_prefetch_desc(&tmDQ);
+    uint8_t* stage = smem + OFF_DQ + (warp - 2 - FB_CWARPS) * 4096;
+    if (lane == 0) tma_prefetch_desc(&tmDQ);
     Item w = item_of(blockIdx.x);
     int g = 0;
     bool ok = true;
@@ -649,55 +594,10 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       PROF_T(a1);
       PROF_ADD(10, a0, a1);
       tc_fence_after();
-      if (HD == 128 && !(p.debug & 64)) {
-        // The warp's four chunks of 32 columns go into four boxes inside the Pᵀ / dSᵀ buffers (idle until the
-        // compute warps write the next tile's Pᵀ / dSᵀ), so tensor memory is free after four loads and the next
-        // scores - dQ reuses their columns - start while the TMA unit adds the boxes to the accumulator.  (Through
-        // one box per warp with a wait between chunks the drain took 4.3 k cycles per tile, all of it ahead of the
-        // next scores; vector atomics from registers 4.9 k.)
-        const int row0 = (int)((int64_t)bh * p.T) + i0 + qd * 32;
-        uint8_t* boxes = smem + Cfg::OFF_P + (warp - 2 - FB_CWARPS) * 4 * 4096;
-        // two loads in flight at a time; the columns are handed back as soon as the last load has landed, before
-        // the last stores and the proxy fence
-        auto store_box = [&](int c, const uint32_t (&v)[32]) {
-          if (p.debug & 1) return;
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const uint32_t off = lane * 128 + ((q ^ (lane & 7)) << 4);
-            *reinterpret_cast<uint4*>(boxes + c * 4096 + off) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-          }
-        };
-        {
-          uint32_t va[32], vb[32];
-          tmem_ld32(lane_addr + Cfg::COL_DQ, va);
-          tmem_ld32(lane_addr + Cfg::COL_DQ + 32, vb);
-          tc_wait_ld();
-          store_box(0, va);
-          store_box(1, vb);
-          tmem_ld32(lane_addr + Cfg::COL_DQ + 64, va);
-          tmem_ld32(lane_addr + Cfg::COL_DQ + 96, vb);
-          tc_wait_ld();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(dq_free);  // tensor memory is drained: the next scores may overwrite the columns
-          store_box(2, va);
-          store_box(3, vb);
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          if ((!RAGGED || i0 + qd * 32 < p.T) && !(p.debug & 1)) {  // the rows past the end are the next slice's
-#pragma unroll
-            for (int c = 0; c < HD / 32; ++c) tma_reduce_add_2d(&tmDQ, boxes + c * 4096, c * 32, row0);
-            tma_store_commit();
-            tma_store_wait_read();  // the boxes have been read: Pᵀ / dSᵀ may be written again
-          }
-          mbar_arrive(stage_free);
-        }
-      } else if (HD == 64 && !(p.debug & 64)) {
+      if (!(p.debug & 64)) {
         uint32_t v0[32], v1[32];
-        tmem_ld32(lane_addr + Cfg::COL_DQ, v0);
-        tmem_ld32(lane_addr + Cfg::COL_DQ + 32, v1);
+        tmem_ld32(lane_addr + COL_DQ, v0);
+        tmem_ld32(lane_addr + COL_DQ + 32, v1);
         tc_wait_ld();
         // TMEM is drained: the tensor core may overwrite dQ while the rows travel on
         tc_fence_before();
@@ -728,7 +628,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
 #pragma unroll 1
         for (int c = 0; c < p.hd / 32; ++c) {
           uint32_t v[32];
-          tmem_ld32(lane_addr + Cfg::COL_DQ + c * 32, v);
+          tmem_ld32(lane_addr + COL_DQ + c * 32, v);
           tc_wait_ld();
           if (!(p.debug & 1) && i0 + r < p.T)
 #pragma unroll
@@ -747,7 +647,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
     }
     ok = __all_sync(0xffffffffu, ok) != 0 && next_of(n, w, false);
     }
-    if (Cfg::DQ_TMA && lane == 0) tma_store_wait_all();  // every reduction has reached global memory
+    if (lane == 0) tma_store_wait_all();  // every reduction has reached global memory
   }
 
   tc_fence_before();
@@ -808,13 +708,11 @@ bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd) {  // as in the forward
                                                           attn_strides_positive(a.sv) && attn_strides_positive(a.sdo)));
 }
 
-template <typename T, int HD, bool RAGGED>
-static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
-  using Cfg = FbCfg<HD>;
+int attn_bwd128_tc05(const AttnArgs& a, int dtype, cudaStream_t st);
+
+template <typename T, bool RAGGED>
+static int bwd64_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   int rc;
-  // the delta pass also clears the fp32 dQ accumulator (contiguous (B,H,T,HD), 16-byte aligned: checked by the
-  // caller), so no fill sits between the kernels in the stream
-  if ((rc = attn_delta(a, hd, dtype, st, a.dq_acc))) return rc;
   CUtensorMap tq, tk, tv, tdo, tdq;
   {
     // fp32 dQ accumulator as a (HD, B*H*T) matrix, boxes of 32 floats x 32 rows
@@ -839,10 +737,10 @@ static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st
   static std::atomic<uint64_t> done[4] = {{0}, {0}, {0}, {0}};
 #define FB_LAUNCH(MODE, SLOT)                                                                                       \
   {                                                                                                                 \
-    if ((rc = ensure_dynamic_smem(attn_bwd_tc05_kernel<T, HD, MODE, RAGGED>, Cfg::SMEM_BYTES, done[SLOT],                   \
+    if ((rc = ensure_dynamic_smem(attn_bwd_tc05_kernel<T, MODE, RAGGED>, SMEM_BYTES, done[SLOT],                   \
                                   "attention_bwd(tcgen05)")))                                                       \
       return rc;                                                                                                    \
-    launch_overlapped(attn_bwd_tc05_kernel<T, HD, MODE, RAGGED>, grid, dim3(FB_THREADS), Cfg::SMEM_BYTES, st, tq, tk, \
+    launch_overlapped(attn_bwd_tc05_kernel<T, MODE, RAGGED>, grid, dim3(FB_THREADS), SMEM_BYTES, st, tq, tk, \
                       tv, tdo, tdq, p);                                                                             \
   }
   if (a.bias_mode == 0) FB_LAUNCH(0, 0)
@@ -850,7 +748,18 @@ static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st
   else if (a.bias_mode == 2) FB_LAUNCH(2, 2)
   else FB_LAUNCH(4, 3)
 #undef FB_LAUNCH
-  if ((rc = launched("attention_bwd(tcgen05)"))) return rc;
+  return launched("attention_bwd(tcgen05)");
+}
+
+template <typename T>
+static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
+  // the delta pass also clears the fp32 dQ accumulator (contiguous (B,H,T,hd), 16-byte aligned: checked by the
+  // caller), so no fill sits between the kernels in the stream
+  int rc = attn_delta(a, hd, dtype, st, a.dq_acc);
+  if (!rc)
+    rc = hd == 128 ? attn_bwd128_tc05(a, dtype, st)
+                   : a.T % FB_T ? bwd64_launch<T, true>(a, hd, dtype, st) : bwd64_launch<T, false>(a, hd, dtype, st);
+  if (rc) return rc;
   const int64_t nvec = (int64_t)a.B * a.H * a.T * hd / 8;
   const unsigned blocks = (unsigned)(ceil_div(nvec, 256) < 148 * 8 ? ceil_div(nvec, 256) : 148 * 8);
   launch_overlapped(attn_dq_convert_kernel<T>, dim3(blocks), dim3(256), 0, st, a.dq_acc, (T*)a.dq, a.sdq.b, a.sdq.h,
@@ -860,9 +769,7 @@ static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st
 
 int attn_tc05_bwd(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   TFB_DISPATCH_16(dtype, T, {
-    const bool ragged = a.T % FB_T != 0;
-    if (hd <= 64) return ragged ? bwd_tc05_launch<T, 64, true>(a, hd, dtype, st) : bwd_tc05_launch<T, 64, false>(a, hd, dtype, st);
-    return ragged ? bwd_tc05_launch<T, 128, true>(a, hd, dtype, st) : bwd_tc05_launch<T, 128, false>(a, hd, dtype, st);
+    return bwd_tc05_launch<T>(a, hd, dtype, st);
   })
 }
 
