@@ -663,25 +663,36 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
   }
 }
 
-// dq = round(scale * dq_acc), written with the caller's strides
+// dq = round(scale * dq_acc), written with the caller's strides.  Bound by memory; one slice per grid row, vectors of eight
+// columns, 1 << vshift of them per row (no 64-bit divisions to find a vector's row; figures at attn_delta_kernel).
+constexpr int DQ_VECS = 2;  // of a thread
 template <typename T>
 __global__ void __launch_bounds__(256) attn_dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq,
-                                                              int64_t sb, int64_t sh, int64_t st, int H, int T_,
-                                                              int hd, float scale, int64_t nvec) {
+                                                              int64_t sb, int64_t sh, int64_t st, int H, int rows, int vshift,
+                                                              float scale) {
   grid_dependency_wait();
   allow_dependents();
-  const int vpr = hd / 8;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < nvec;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(idx % vpr);
-    const int64_t row = idx / vpr;
-    const int i = (int)(row % T_);
-    const int64_t bh = row / T_;
-    const int b = (int)(bh / H), h = (int)(bh % H);
-    const float4 x = *reinterpret_cast<const float4*>(acc + idx * 8);
-    const float4 y = *reinterpret_cast<const float4*>(acc + idx * 8 + 4);
-    float f[8] = {x.x * scale, x.y * scale, x.z * scale, x.w * scale, y.x * scale, y.y * scale, y.z * scale, y.w * scale};
-    *reinterpret_cast<uint4*>(dq + b * sb + h * sh + (int64_t)i * st + c * 8) = pack8<T>(f);
+  const int bh = blockIdx.y, b = bh / H, h = bh % H;
+  const int total = rows << vshift;
+  const float4* src = reinterpret_cast<const float4*>(acc) + (int64_t)bh * total * 2;
+  T* dst = dq + b * sb + h * sh;
+  float4 x[DQ_VECS], y[DQ_VECS];
+#pragma unroll
+  for (int u = 0; u < DQ_VECS; ++u) {
+    const int v = (blockIdx.x * DQ_VECS + u) * 256 + threadIdx.x;
+    if (v < total) {
+      x[u] = __ldcs(src + 2 * (int64_t)v);
+      y[u] = __ldcs(src + 2 * (int64_t)v + 1);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < DQ_VECS; ++u) {
+    const int v = (blockIdx.x * DQ_VECS + u) * 256 + threadIdx.x;
+    if (v < total) {
+      const float f[8] = {x[u].x * scale, x[u].y * scale, x[u].z * scale, x[u].w * scale,
+                          y[u].x * scale, y[u].y * scale, y[u].z * scale, y[u].w * scale};
+      *reinterpret_cast<uint4*>(dst + (int64_t)(v >> vshift) * st + (v & ((1 << vshift) - 1)) * 8) = pack8<T>(f);
+    }
   }
 }
 
@@ -760,10 +771,10 @@ static int bwd_tc05_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st
     rc = hd == 128 ? attn_bwd128_tc05(a, dtype, st)
                    : a.T % FB_T ? bwd64_launch<T, true>(a, hd, dtype, st) : bwd64_launch<T, false>(a, hd, dtype, st);
   if (rc) return rc;
-  const int64_t nvec = (int64_t)a.B * a.H * a.T * hd / 8;
-  const unsigned blocks = (unsigned)(ceil_div(nvec, 256) < 148 * 8 ? ceil_div(nvec, 256) : 148 * 8);
-  launch_overlapped(attn_dq_convert_kernel<T>, dim3(blocks), dim3(256), 0, st, a.dq_acc, (T*)a.dq, a.sdq.b, a.sdq.h,
-                    a.sdq.t, a.H, a.T, hd, a.scale, nvec);
+  const int vshift = hd == 32 ? 2 : hd == 64 ? 3 : 4;
+  const dim3 grid((unsigned)ceil_div((int64_t)a.T << vshift, 256 * DQ_VECS), (unsigned)(a.B * a.H));
+  launch_overlapped(attn_dq_convert_kernel<T>, grid, dim3(256), 0, st, a.dq_acc, (T*)a.dq, a.sdq.b, a.sdq.h, a.sdq.t, a.H, a.T,
+                    vshift, a.scale);
   return launched("attention_dq_convert");
 }
 

@@ -223,37 +223,50 @@ __global__ void __launch_bounds__(AT_THREADS) attn_fwd_kernel(const AttnArgs a) 
 
 // delta[b,h,i] = sum_d dO[i,d] * O[i,d]; hd/8 lanes per row, one 16-byte load of each operand per lane.
 // `clear` (may be null): contiguous fp32 (B,H,T,HD) buffer; each lane zeroes the eight floats under its chunk.
+// Bound by memory: DELTA_ROWS rows of a thread in flight, one slice per grid row, no 64-bit divisions (four of them per
+// thread before).  Backward with this and the conversion's new form: B4 H16 T2048 hd64 fp16 191.5 -> 189.6 us, B3 H11 T1472 hd64 bf16
+// 69.0 -> 67.0, B1 H12 T4096 hd128 226.5 -> 222.7.
+constexpr int DELTA_ROWS = 2;
 template <typename T, int HD>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const AttnArgs a, float* __restrict__ clear) {
   grid_dependency_wait();
   allow_dependents();
   constexpr int LPR = HD / 8;          // lanes per row
-  constexpr int RPW = 32 / LPR;        // rows per warp
-  const int lane = threadIdx.x & 31;
-  const int sub = lane % LPR;
-  const int64_t row = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * RPW + lane / LPR;
-  const int64_t total = (int64_t)a.B * a.H * a.T;
-  float s = 0.f;
-  if (row < total) {
-    const int i = (int)(row % a.T);
-    const int64_t bh = row / a.T;
-    const int b = (int)(bh / a.H), h = (int)(bh % a.H);
-    const T* op = (const T*)a.o + b * a.so.b + h * a.so.h + (int64_t)i * a.so.t + sub * 8;
-    const T* gp = (const T*)a.d_o + b * a.sdo.b + h * a.sdo.h + (int64_t)i * a.sdo.t + sub * 8;
-    float x[8], y[8];
-    unpack8<T>(ld_stream16(op), x);
-    unpack8<T>(ld_stream16(gp), y);
+  constexpr int RPB = 256 / LPR;       // rows of a block at a time
+  const int sub = threadIdx.x % LPR, r0 = blockIdx.x * (RPB * DELTA_ROWS) + threadIdx.x / LPR;
+  const int bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
+  const T* op = (const T*)a.o + b * a.so.b + h * a.so.h + sub * 8;
+  const T* gp = (const T*)a.d_o + b * a.sdo.b + h * a.sdo.h + sub * 8;
+  uint4 x[DELTA_ROWS], y[DELTA_ROWS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s += x[j] * y[j];
-    if (clear) {
-      float4* z = reinterpret_cast<float4*>(clear + row * HD + sub * 8);
-      z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-      z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int u = 0; u < DELTA_ROWS; ++u) {
+    const int i = r0 + u * RPB;
+    if (i < a.T) {
+      x[u] = ld_stream16(op + i * a.so.t);
+      y[u] = ld_stream16(gp + i * a.sdo.t);
     }
   }
 #pragma unroll
-  for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (row < total && sub == 0) a.delta[row] = s;
+  for (int u = 0; u < DELTA_ROWS; ++u) {
+    const int i = r0 + u * RPB;
+    const int64_t row = (int64_t)bh * a.T + i;
+    float s = 0.f;
+    if (i < a.T) {
+      float p[8], q[8];
+      unpack8<T>(x[u], p);
+      unpack8<T>(y[u], q);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += p[j] * q[j];
+      if (clear) {
+        float4* z = reinterpret_cast<float4*>(clear + row * HD + sub * 8);
+        z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+        z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (i < a.T && sub == 0) a.delta[row] = s;
+  }
 }
 
 // --------------------------------------------------------------------------- backward: dK, dV
@@ -543,11 +556,11 @@ static int bwd_launch(const AttnArgs& a, cudaStream_t st) {
 }
 
 int attn_delta(const AttnArgs& a, int hd, int dtype, cudaStream_t st, float* clear) {
-  const int64_t rows = (int64_t)a.B * a.H * a.T;
+  const dim3 grid((unsigned)ceil_div(a.T, 256 / (hd / 8) * DELTA_ROWS), (unsigned)(a.B * a.H));
   TFB_DISPATCH_16(dtype, T, {
-    if (hd == 32) launch_overlapped(attn_delta_kernel<T, 32>, dim3((unsigned)ceil_div(rows, 8 * 8)), dim3(256), 0, st, a, clear);
-    else if (hd == 64) launch_overlapped(attn_delta_kernel<T, 64>, dim3((unsigned)ceil_div(rows, 8 * 4)), dim3(256), 0, st, a, clear);
-    else launch_overlapped(attn_delta_kernel<T, 128>, dim3((unsigned)ceil_div(rows, 8 * 2)), dim3(256), 0, st, a, clear);
+    if (hd == 32) launch_overlapped(attn_delta_kernel<T, 32>, grid, dim3(256), 0, st, a, clear);
+    else if (hd == 64) launch_overlapped(attn_delta_kernel<T, 64>, grid, dim3(256), 0, st, a, clear);
+    else launch_overlapped(attn_delta_kernel<T, 128>, grid, dim3(256), 0, st, a, clear);
   })
   return launched("attention_delta");
 }
