@@ -13,18 +13,12 @@ extern "C" {
 /* Test and tuning switches.
  *   key 0: value 1 sends every GEMM to the generic-stride kernel.
  *   key 1: value 1 sends every attention call to the mma.sync kernels.
- *   key 2: attention (bits 0, 1, 6 and 7 in the backward: head_dim 32 and 64): bit 0 skips the dQ accumulation, bit 1 turns the
- *          cycle counters on, bit 5 (32) walks the
- *          (tile, batch*head) items slice by slice instead of longest first, bit 6 (64) adds dQ with vector
- *          atomics instead of the TMA reduction, bit 7 (128) keeps only the barriers of the backward's compute
- *          warps going (timing experiments: results are then meaningless).
+ *   key 2: attention: bit 5 (32) walks the (tile, batch*head) items slice by slice instead of longest first.
  *   key 3: value 1 launches every kernel fully serialised (no programmatic dependent launch: a
  *          kernel's set-up no longer overlaps its predecessor's tail).
  *   key 4: GEMM: bit 0 whole tiles only (no sharing of a tile's contraction between SMs), bit 5 (32)
- *          no persistent CTA-pair kernel, bit 6 (64) per-CTA timeline counters of that kernel, bit 7 (128)
- *          no one-wave kernel, bits 16-27 the one plan the one-wave kernel may use (tfb_debug_gemm_plan).
- *   key 5: which counters tfb_debug_counters returns: -1 attention backward, -3 attention forward,
- *          n >= 0 the CTA-pair GEMM timeline of CTA n.
+ *          no persistent CTA-pair kernel, bit 7 (128) no one-wave kernel, bits 16-27 the one plan the one-wave kernel
+ *          may use (tfb_debug_gemm_plan).
  *   key 6: how many SMs the persistent GEMM grids leave free (for a collective that runs beside
  *          them on another stream); 0 by default.                                */
 void tfb_debug_set(int key, int value);
@@ -32,10 +26,6 @@ void tfb_debug_set(int key, int value);
  * 0 if the product goes to the persistent kernels, else 1 + tile width / 64 * 2 + (on CTA pairs ? 1 : 0) + 16 * the number
  * of workers that share a tile's contraction.                                              */
 int tfb_debug_gemm_plan(long long M, long long N, long long K, int b_mn);
-/* Timing counters of the attention backward kernel (16 cycle sums, filled while tfb_debug_set(2, 2)
- * is in effect); copies and clears them.  Synchronises the device.                        */
-int tfb_debug_counters(unsigned long long* out16);
-
 /* Launches a one-warp kernel that takes tensor memory, waits `limit_ns` nanoseconds on an mbarrier
  * that nothing arrives at, gives up, records 0x7e00 in the device status word, frees its tensor memory
  * and returns: the expiry path of the library's bounded waits, without a fault, a trap or an unbounded

@@ -19,7 +19,14 @@
 // per step that nothing hides).  A thread owns 64 keys of one query row; the two warps of a row each keep
 // an accumulator, a reference maximum and a row sum for THEIR keys and meet only twice per item, through
 // shared memory (an mbarrier with one arrival per warp and lane quarter, so the wait is bounded): for the
-// row maximum of the diagonal step and when the accumulators are merged.
+// row maximum of the diagonal step and when the accumulators are merged, which happens a step into the next item, so that
+// neither waits for the other at an item's end.
+// A step is 1.0 k cycles of arithmetic for the two warps of a scheduler, and what lies between two steps counts: with time
+// stamps for tuning in it (four reads of the clock a step, unused) and two hand-shakes at the end of each item, B4 H16 T2048
+// hd64 fp16 took 73.9 us and takes 69.4, with exact slopes 81.1 and 74.6, B3 H11 T1472 hd64 bf16 29.6 and 27.4, B3 H16 T704 with
+// the rounded table 18.1 and 17.1, B2 H16 T2048 hd128 bf16 with the table 57.6 and 53.0.
+// Tried and slower: whole key tiles for each of two groups of four warps (three score buffers; 80.9), two CTAs per SM
+// with one score buffer each (85.7).
 // An item walks its key tiles from the diagonal outwards.  The diagonal tile takes two passes (row maximum,
 // then probabilities) with the causal mask applied per 32-key chunk, which for a whole warp is either
 // untouched, cut by the diagonal or fully masked (then nothing is computed).  Every later tile is a single
@@ -70,9 +77,10 @@ template <int HD> struct F1Cfg {
   static constexpr int OFF_Q = 0;                                  // [2]
   static constexpr int OFF_K = 2 * TILE_BYTES;                     // [STAGES]
   static constexpr int OFF_V = OFF_K + STAGES * TILE_BYTES;        // [STAGES]
-  static constexpr int OFF_X = OFF_V + STAGES * TILE_BYTES;        // row exchange: [2 parities][warps per row][128 rows] floats
-  static constexpr int OFF_BAR = OFF_X + 2 * NW * 128 * 4;
-  static constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
+  static constexpr int OFF_X = OFF_V + STAGES * TILE_BYTES;        // [item parity][warps per row][128 rows] row maxima of a diagonal
+  static constexpr int OFF_ML = OFF_X + 2 * NW * 128 * 4;          // step, and [item parity][warps per row][128 rows] (maximum, row sum)
+  static constexpr int OFF_BAR = OFF_ML + 2 * NW * 128 * 8;
+  static constexpr int SMEM_BYTES = OFF_BAR + 512 + 1024;
   static_assert(OW % 16 == 0, "a softmax warp handles whole 16-column chunks of the accumulator");
   static_assert(COL_O + NW * HD <= 512, "tensor memory");
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
@@ -85,7 +93,7 @@ constexpr float kRescale1 = 8.0f;  // log2 units
 constexpr float kSinglePassLimit = 32768.f;
 
 struct F1Params {
-  int debug;  // bit 1: cycle counters of one softmax warp (tfb_debug_set key 2); bit 5: per-slice item order
+  int debug;  // bit 5: per-slice item order (tfb_debug_set key 2)
   void* out;
   float* lse;
   int64_t so_b, so_h, so_t;
@@ -159,12 +167,6 @@ __device__ __forceinline__ bool f1_item(const F1Params& p, int n, int& qt, int& 
 
 }  // namespace
 
-// [0] steps, [1] wait for scores, [2] pass, [3] row-pair exchange, [4] store fence + arrive (warp 2, lane 0);
-// per CTA: [5] items, [6] lifetime of the CTA, [7] entry -> set-up done, [8] first (diagonal) step of an item,
-// [9] its second step, [10] single passes that had to be redone, [11] normalisation and store of an item, [12] lifetime in ns
-static __device__ unsigned long long g_prof_f1[16];
-#define F1_PROF(idx, t0, t1) do { if (prof) atomicAdd(&g_prof_f1[idx], (unsigned long long)((t1) - (t0))); } while (0)
-
 // POLY: one pair of exponentials in four on the FMA pipe (see fwd1_launch).
 template <typename T, int HD, int BIAS, bool POLY>
 __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(const __grid_constant__ CUtensorMap tmQ,
@@ -190,14 +192,14 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
   uint64_t* p_full = s_full + 2;                 // [2 buffers] probabilities stored, score buffer read (8 warps)
   uint64_t* pv_done = p_full + 2;                // [2 buffers] the P·V that read the P buffer has retired
   uint64_t* o_free = pv_done + 2;                // [2 accumulators] the finished tile has been read out (8 warps)
-  uint64_t* pair_bar = o_free + 2;               // [4 lane quarters] both warps of the row pair have published
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(pair_bar + 4);
+  uint64_t* pair_bar = o_free + 2;               // [4 lane quarters] both warps of the row pair have published their row maxima,
+  uint64_t* part_bar = pair_bar + 4;             // [4] and their maxima and row sums of an item
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(part_bar + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
   float* xch = reinterpret_cast<float*>(smem + F1_OFF_X);
+  float2* parts = reinterpret_cast<float2*>(smem + Cfg::OFF_ML);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long t_entry = clock64();
-  const uint64_t ns_entry = global_ns();
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -214,7 +216,10 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
     }
-    for (int i = 0; i < 4; ++i) mbar_init(&pair_bar[i], F1_NW);
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(&pair_bar[i], F1_NW);
+      mbar_init(&part_bar[i], F1_NW);
+    }
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -376,65 +381,47 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
     const int r = qd * 32 + lane;       // row within the tile == TMEM lane
     const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
     const float c2 = p.scale * kLog2e1;
-    uint32_t pair_phase = 0;
-    int xpar = 0;
     bool ok = true;
-    long long xw_total = 0;
-    // Row exchange: publish a value for this row and combine the values of the other warps that share
-    // the row (maximum, or sum when `add`).  All warps of a row take the same path through a step, so
-    // they make the same number of exchanges.  Bounded wait; double-buffered by exchange parity.
-    auto exchange = [&](float mine, bool& fine, bool add) -> float {
-      const long long x0 = clock64();
-      float* slot = xch + xpar * (F1_NW * 128);
+    // Row exchange, once per item: publish this warp's row maximum and take the larger of it and the other warp's.  Bounded
+    // wait.  Two slots per row are enough: the scores of an item two further on wait for this step's probabilities.
+    auto exchange_max = [&](float mine, int n) -> float {
+      float* slot = xch + (n & 1) * (F1_NW * 128);
       slot[ch * 128 + r] = mine;
       __syncwarp();
       if (lane == 0) mbar_arrive(&pair_bar[qd]);
-      if (fine) fine = mbar_wait(&pair_bar[qd], pair_phase, 0x5c00 | qd, abort_flag);
-      pair_phase ^= 1;
-      float acc = mine;
+      if (ok) ok = mbar_wait(&pair_bar[qd], n & 1, 0x5c00 | qd, abort_flag);
+      float m = mine;
 #pragma unroll
-      for (int w = 1; w < F1_NW; ++w) {
-        const float other = slot[((ch + w) % F1_NW) * 128 + r];
-        acc = add ? acc + other : fmaxf(acc, other);
-      }
-      xpar ^= 1;
-      xw_total += clock64() - x0;
-      return acc;
+      for (int w = 1; w < F1_NW; ++w) m = fmaxf(m, slot[((ch + w) % F1_NW) * 128 + r]);
+      return m;
     };
-    // the same hand-shake, returning the value of every warp of the row, in warp order
-    auto gather = [&](float mine, bool& fine, float (&all)[F1_NW]) {
-      float* slot = xch + xpar * (F1_NW * 128);
-      slot[ch * 128 + r] = mine;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&pair_bar[qd]);
-      if (fine) fine = mbar_wait(&pair_bar[qd], pair_phase, 0x5d00 | qd, abort_flag);
-      pair_phase ^= 1;
-#pragma unroll
-      for (int w = 0; w < F1_NW; ++w) all[w] = slot[w * 128 + r];
-      xpar ^= 1;
-    };
-    const bool prof = (p.debug & 2) && warp == 2 + ((p.debug >> 8) & 15) && lane == 0;  // bits 8-11: which softmax warp
-    if (prof) atomicAdd(&g_prof_f1[7], (unsigned long long)(clock64() - t_entry));
     int g0 = 0;  // steps of the CTA before this item
-    long long last_w3 = clock64();
     // Normalisation and store of a finished tile, run one step late: after the first (diagonal) step of the NEXT
     // item, whose scores are already there, so that the wait for the tile's last P·V is hidden behind that step.
     bool pend = false;
-    int pend_glast = 0;
-    float pend_l = 1.f, pend_m = 0.f;
-    float pend_w[F1_NW];  // (split accumulators: their weights)
-#pragma unroll
-    for (int w = 0; w < F1_NW; ++w) pend_w[w] = 1.f;
+    int pend_glast = 0, pend_n = 0;
     T* pend_row = nullptr;
     bool pend_live = false, pend_store = false;  // the row exists; it does and so do this warp's output columns
     float* pend_lse = nullptr;
     auto finish_pending = [&]() {
       if (!pend) return;
       pend = false;
-      const long long f0 = clock64();
       if (ok) ok = mbar_wait(&pv_done[pend_glast & 1], (pend_glast >> 1) & 1, 0x5900, abort_flag);
+      if (ok) ok = mbar_wait(&part_bar[qd], pend_n & 1, 0x5d00 | qd, abort_flag);
       if (ok) {
         tc_fence_after();
+        // merge the row's warps: common maximum, each one's weight against it, common row sum
+        float2 ml[F1_NW];
+#pragma unroll
+        for (int w = 0; w < F1_NW; ++w) ml[w] = parts[((pend_n & 1) * F1_NW + w) * 128 + r];
+        float pend_m = ml[0].x, pend_l = 0.f, pend_w[F1_NW];
+#pragma unroll
+        for (int w = 1; w < F1_NW; ++w) pend_m = fmaxf(pend_m, ml[w].x);
+#pragma unroll
+        for (int w = 0; w < F1_NW; ++w) {
+          pend_w[w] = ex2_mufu(ml[w].x - pend_m);
+          pend_l = fmaf(ml[w].y, pend_w[w], pend_l);
+        }
         const float inv = 1.f / pend_l;
         const uint32_t o_addr = lane_addr + F1_COL_O;
         {
@@ -466,7 +453,6 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
         }
         if (ch == 0 && pend_live) *pend_lse = (pend_m + log2f(pend_l)) * kLn2_1;
       }
-      if (prof) atomicAdd(&g_prof_f1[11], (unsigned long long)(clock64() - f0));
     };
     for (int n = 0; ok; ++n) {
       int qt, bh;
@@ -490,13 +476,7 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
         const uint32_t s_addr = lane_addr + F1_COL_S + bsel * 128 + ch * F1_KW;
         // P of a 32-key chunk: 16 columns, at head_dim 64 the first 16 of this warp's own score columns
         const uint32_t p_addr = s_addr;
-        const long long w0 = clock64();
-        F1_PROF(14, last_w3, w0);
         if (ok) ok = mbar_wait(&s_full[bsel], (g >> 1) & 1, 0x5700 | bsel, abort_flag);
-        const long long w1 = clock64();
-        F1_PROF(1, w0, w1);
-        if (prof) atomicAdd(&g_prof_f1[0], 1ull);
-        const long long xw = xw_total;  // exchange cycles before this step
         tc_fence_after();
         bool done = false;
         if (!diag) {
@@ -546,8 +526,6 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
             for (int c = 0; c < F1_NC; ++c) tmem_st16(p_addr + c * 16, pk_all[c]);
             l_run += part;
             done = true;
-          } else if (prof) {
-            atomicAdd(&g_prof_f1[10], 1ull);
           }
         }
         if (!done) {
@@ -595,7 +573,7 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
           // finite after the exchange: the diagonal tile holds key i of every row.  Split accumulators: only the
           // diagonal step needs the partner (a warp whose share of the diagonal tile is masked has no maximum of
           // its own yet); a redone step further out concerns this warp's accumulator alone.
-          if (t == 0) mx = exchange(mx, ok, false);
+          if (t == 0) mx = exchange_max(mx, n);
           m_run = fmaxf(m_run, mx);
           // every earlier P·V must have retired before O is rescaled or this P buffer rewritten (the
           // tensor core retires them in order, so the latest one covers the rest; at the first step of an
@@ -648,27 +626,25 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
 #pragma unroll
                 for (int e = 0; e < 16; ++e) pk[e] = 0u;
               } else {
-                float e_[32];
+                const float d0 = (float)(i - (kbase + c * 32));
+                auto put = [&](int e, float p0, float p1) {
+                  ls4[(2 * e) & 3] += p0;
+                  ls4[(2 * e + 1) & 3] += p1;
+                  const typename Num<T>::T2 h2 = Num<T>::from_f2(p0, p1);
+                  pk[e] = *reinterpret_cast<const uint32_t*>(&h2);
+                };
                 if (!BIAS && cls[c] == 0) {
 #pragma unroll
-                  for (int e = 0; e < 32; ++e) e_[e] = ex2_mufu(fmaf(__uint_as_float(v[e]), c2, neg_m));
+                  for (int e = 0; e < 16; ++e)
+                    put(e, ex2_mufu(fmaf(__uint_as_float(v[2 * e]), c2, neg_m)), ex2_mufu(fmaf(__uint_as_float(v[2 * e + 1]), c2, neg_m)));
                 } else {
-                  const float d0 = (float)(i - (kbase + c * 32));
 #pragma unroll
-                  for (int e = 0; e < 32; e += 2) {
+                  for (int e = 0; e < 16; ++e) {
                     float x0, x1;
-                    f2_unpack(alibi.sub_pair(f2_pack(fmaf(__uint_as_float(v[e]), c2, neg_m), fmaf(__uint_as_float(v[e + 1]), c2, neg_m)),
-                                             d0 - (float)e, d0 - (float)(e + 1)), x0, x1);
-                    e_[e] = (e >= cnt[c]) ? 0.f : ex2_mufu(x0);
-                    e_[e + 1] = (e + 1 >= cnt[c]) ? 0.f : ex2_mufu(x1);
+                    f2_unpack(alibi.sub_pair(f2_pack(fmaf(__uint_as_float(v[2 * e]), c2, neg_m), fmaf(__uint_as_float(v[2 * e + 1]), c2, neg_m)),
+                                             d0 - (float)(2 * e), d0 - (float)(2 * e + 1)), x0, x1);
+                    put(e, (2 * e >= cnt[c]) ? 0.f : ex2_mufu(x0), (2 * e + 1 >= cnt[c]) ? 0.f : ex2_mufu(x1));
                   }
-                }
-#pragma unroll
-                for (int e = 0; e < 32; ++e) ls4[e & 3] += e_[e];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                  const typename Num<T>::T2 h2 = Num<T>::from_f2(e_[2 * e], e_[2 * e + 1]);
-                  pk[e] = *reinterpret_cast<const uint32_t*>(&h2);
                 }
               }
               tmem_st16(p_addr + c * 16, pk);
@@ -676,41 +652,17 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
           }
           l_run += (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
         }
-        const long long w2 = clock64();
         tc_wait_st();  // P is in tensor memory, the score buffer has been read
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_full[bsel]);
-        F1_PROF(2, w1, w2);
-        const long long w3 = clock64();
-        F1_PROF(4, w2, w3);
-        last_w3 = w3;
-        if (prof) {
-          atomicAdd(&g_prof_f1[3], (unsigned long long)(xw_total - xw));
-          if (t == 0) atomicAdd(&g_prof_f1[8], (unsigned long long)(w3 - w0));
-          if (t == 1) atomicAdd(&g_prof_f1[9], (unsigned long long)(w3 - w0));
-        }
         if (t == 0) finish_pending();  // the previous item's tile
       }
-      // the row sum is the sum of the pair's partial sums; the tile itself is finished one step later
-      {
-        // merge the two streams: common maximum, each stream's weight against it, common row sum
-        float m_w[F1_NW], l_w[F1_NW];
-        const long long g0_ = clock64();
-        gather(m_used, ok, m_w);
-        gather(l_run, ok, l_w);
-        if (prof) atomicAdd(&g_prof_f1[13], (unsigned long long)(clock64() - g0_));
-        float m_all = m_w[0];
-#pragma unroll
-        for (int w = 1; w < F1_NW; ++w) m_all = fmaxf(m_all, m_w[w]);
-        pend_l = 0.f;
-#pragma unroll
-        for (int w = 0; w < F1_NW; ++w) {
-          pend_w[w] = ex2_mufu(m_w[w] - m_all);
-          pend_l = fmaf(l_w[w], pend_w[w], pend_l);
-        }
-        pend_m = m_all;
-      }
+      // this warp's part of the item; the tile itself is merged and finished one step later
+      parts[((n & 1) * F1_NW + ch) * 128 + r] = make_float2(m_used, l_run);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&part_bar[qd]);
+      pend_n = n;
       pend_glast = g0 + jlast;
       pend_row = reinterpret_cast<T*>(p.out) + b * p.so_b + h * p.so_h + (int64_t)i * p.so_t + ch * F1_OW;
       pend_lse = p.lse + (int64_t)bh * p.T + i;
@@ -718,13 +670,8 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
       pend_store = pend_live && ch * F1_OW < p.hd;
       pend = true;
       g0 += jlast + 1;
-      if (prof) atomicAdd(&g_prof_f1[5], 1ull);
     }
     finish_pending();  // the CTA's last tile
-    if (prof) {
-      atomicAdd(&g_prof_f1[6], (unsigned long long)(clock64() - t_entry));
-      atomicAdd(&g_prof_f1[12], (unsigned long long)(global_ns() - ns_entry));
-    }
   }
 
   tc_fence_before();
@@ -741,15 +688,6 @@ __global__ void __launch_bounds__(F1Cfg<HD>::THREADS, 1) attn_fwd1_tc05_kernel(c
 }
 
 // ------------------------------------------------------------------------------- host side
-
-// Copies the 16 cycle counters to the host and clears them.
-int attn_fwd1_tc05_counters(unsigned long long* out) {
-  cudaDeviceSynchronize();
-  if (cudaMemcpyFromSymbol(out, g_prof_f1, sizeof(unsigned long long) * 16) != cudaSuccess) return -1;
-  unsigned long long z[16] = {0};
-  cudaMemcpyToSymbol(g_prof_f1, z, sizeof(z));
-  return 0;
-}
 
 int encode_tmap_sw128(CUtensorMap* out, const void* base, int dtype, int rank, const uint64_t* dims,
                       const uint64_t* strides_bytes, const uint32_t* box);

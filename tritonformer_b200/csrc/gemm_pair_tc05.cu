@@ -21,7 +21,6 @@
 
 namespace tfb {
 
-extern std::atomic<int> g_gemm_debug;
 bool gemm_needs_direct(const void* c, int64_t ldc, const void* bias, const void* addend, int64_t ld_addend, const void* mask,
                        int64_t ld_mask);
 
@@ -58,11 +57,7 @@ struct PairParams {
   int relu;
   int direct;          // C, addend, mask or bias cannot go through TMA boxes: element-wise coalesced stores (store_direct)
   int tiles_m, tiles_n;  // in 256 x BN pair tiles
-  int debug;             // bit 6 (64): per-CTA timeline into g_pair_prof (tfb_debug_set key 4)
 };
-
-// Timeline of each CTA for tuning (cycle stamps and wait sums), read through tfb_debug_counters.
-static __device__ unsigned long long g_pair_prof[148][16];
 
 // ---- cluster / pair primitives ------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -139,10 +134,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
-  const bool prof = (p.debug & 64) && blockIdx.x < 148;
-  unsigned long long* pr = g_pair_prof[blockIdx.x < 148 ? blockIdx.x : 0];
-  const long long t_entry = clock64();
-  if (prof && threadIdx.x == 0) { pr[0] = global_ns(); }
   if (threadIdx.x == 0) {
     for (int i = 0; i < GP_STAGES; ++i) {
       mbar_init(&full[i], 1);
@@ -171,7 +162,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
   // set-up above is local to the pair and may overlap the previous kernel's tail; global memory comes after
   grid_dependency_wait();
   allow_dependents();
-  if (prof && threadIdx.x == 0) pr[1] = (unsigned long long)(clock64() - t_entry);  // set-up
 
   const int num_tiles = p.tiles_m * p.tiles_n;
   const int kblocks = (p.K + GP_K - 1) / GP_K;
@@ -187,9 +177,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
         const int m0 = (tile % p.tiles_m) * (2 * GP_M) + (int)rank * GP_M;  // this CTA's rows
         const int n0 = (tile / p.tiles_m) * BN + (int)rank * Cfg::NH;       // this CTA's half of B
         for (int kb = 0; kb < kblocks; ++kb) {
-          const long long w0 = clock64();
           if (!mbar_wait(&empty[stage], phase ^ 1, 0x700 | stage, abort_flag)) { ok = false; break; }
-          if (prof) pr[2] += (unsigned long long)(clock64() - w0);  // producer waiting for a free slot
           uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + GP_A_BYTES;
           // the leader's barrier counts the bytes of both CTAs
@@ -212,7 +200,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
           if (++stage == GP_STAGES) { stage = 0; phase ^= 1; }
         }
       }
-      if (prof) pr[3] = (unsigned long long)(clock64() - t_entry);  // last load issued
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------------- MMA issuer (leader only)
@@ -222,26 +209,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
       constexpr uint32_t idesc = instr_desc_f16(2 * GP_M, BN, std::is_same<T, __nv_bfloat16>::value ? 1 : 0,
                                                 A_MN ? 1 : 0, B_MN ? 1 : 0);
       const uint32_t tb = __shfl_sync(0xffffffffu, tmem_base, 0), s0 = smem_u32(smem);
-      const bool prof = p.debug & 64 && lane == 0 && blockIdx.x < 148;
       int stage = 0;
       uint32_t phase = 0;
       int buf = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
-        const long long a0 = clock64();
         if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], acc_phase ^ 1, 0x800 | buf, abort_flag))) { ok = false; break; }
-        if (prof) pr[4] += (unsigned long long)(clock64() - a0);  // MMA waiting for a free accumulator
         tc_fence_after();
         const uint32_t d_tmem = tb + buf * 256;
         for (int kb = 0; kb < kblocks; ++kb) {
-          const long long f0 = clock64();
           if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], phase, 0x900 | stage, abort_flag))) { ok = false; break; }
-          if (prof) {
-            const long long f1 = clock64();
-            pr[5] += (unsigned long long)(f1 - f0);  // MMA waiting for operands
-            if (pr[6] == 0) pr[6] = (unsigned long long)(f1 - t_entry);  // first operands landed
-          }
           const uint32_t sa = s0 + stage * Cfg::STAGE_BYTES, sb = sa + GP_A_BYTES;
           const uint64_t ad = A_MN ? smem_desc_sw128(sa, 8192, 1024) : smem_desc_sw128(sa, 16, 1024);
           const uint64_t bd = !B_MN ? smem_desc_sw128(sb, 16, 1024)
@@ -260,7 +238,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
         buf ^= 1;
         if (buf == 0) acc_phase ^= 1;
       }
-      if (prof) pr[7] = (unsigned long long)(clock64() - t_entry);  // last MMA issued
     }
   } else {
     // ---------------------------------------------------------------------- epilogue (both CTAs)
@@ -295,22 +272,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
         mbar_expect_tx(&x_full[ew], 4096);
         tma_load_2d(stage_x, &tmX, n0, row0, &x_full[ew]);
       }
-      const long long e0 = clock64();
       if (!mbar_wait(&acc_full[buf], acc_phase, 0xa00 | buf, abort_flag)) { ok = false; break; }
-      const long long e1 = clock64();
-      if (prof && ew == 0 && lane == 0) pr[8] += (unsigned long long)(e1 - e0);  // epilogue waiting for an accumulator
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256 + first;
       if (!dead) epilogue_tile<T>(epi, steps, taddr, row0, n0, lane, x_phase, abort_flag, 0xb00 | ew, ok);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
-      if (prof && ew == 0 && lane == 0) { pr[9] += (unsigned long long)(clock64() - e1); pr[10] += 1; }  // epilogue busy, tiles
       buf ^= 1;
       if (buf == 0) acc_phase ^= 1;
     }
     if (lane == 0) tma_store_wait_read();  // the boxes have been read; the kernel's end completes the writes
-    if (prof && ew == 0 && lane == 0) pr[11] = (unsigned long long)(clock64() - t_entry);  // epilogue done
   }
 
   // Unwind: every role has left its loop (normally or through a bounded wait).
@@ -329,21 +301,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, GP_TMEM_COLS);
   }
-  if (prof && threadIdx.x == 0) { pr[12] = (unsigned long long)(clock64() - t_entry); pr[13] = global_ns(); }
 }
-
-// Copies the timeline of CTA `cta` (16 words) to the host and clears it.
-int gemm_pair_counters(int cta, unsigned long long* out) {
-  if (cta < 0 || cta >= 148) return -1;
-  cudaDeviceSynchronize();
-  if (cudaMemcpyFromSymbol(out, g_pair_prof, sizeof(unsigned long long) * 16, sizeof(unsigned long long) * 16 * cta) !=
-      cudaSuccess)
-    return -1;
-  unsigned long long z[16] = {0};
-  cudaMemcpyToSymbol(g_pair_prof, z, sizeof(z), sizeof(unsigned long long) * 16 * cta);
-  return 0;
-}
-
 
 template <typename T, int BN, bool A_MN, bool B_MN>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmX,
@@ -371,7 +329,8 @@ int64_t gemm_pair_tiles(int64_t M, int64_t N) { return ceil_div(M, 2 * GP_M) * c
 // from the L2, 32 and 28 KB at 62 bytes a cycle), so the narrow tile, which moves an eighth more operand bytes for the
 // same product, is for outputs whose last wave of wide tiles is mostly empty: as many waves of narrow ones.  M 4096 N 1536, two
 // waves of either: K 4608 (B contiguous along K) 49.2 us wide, 45.4 narrow, K 6144 65.6 and 62.1; B contiguous along N:
-// K 1536 20.8 and 19.8, K 6144 65.2 and 64.6.  M 2112 N 3072 K 1024: 15.9 and 15.6.
+// K 1536 20.8 and 19.8, K 6144 65.2 and 64.6.  M 2112 N 3072 K 1024: 15.9 and 15.6.  (Without the time stamps that the kernel
+// carried then: narrow 44.3, 60.8, 19.1, 63.2 and 14.9.)
 int gemm_pair_width(int64_t M, int64_t N, int sms) {
   const int64_t pairs = sms / 2, tm = ceil_div(M, 2 * GP_M);
   const int64_t wide = ceil_div(tm * ceil_div(N, 256), pairs) * 528, narrow = ceil_div(tm * ceil_div(N, 192), pairs) * 462;
@@ -411,7 +370,7 @@ int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, cons
   PairParams p;
   p.C = c; p.bias = bias; p.addend = addend; p.mask = mask;
   p.M = (int)M; p.N = (int)N; p.K = (int)K; p.ldc = ldc; p.ld_addend = ld_addend; p.ld_mask = ld_mask;
-  p.relu = relu; p.direct = direct; p.debug = g_gemm_debug.load();
+  p.relu = relu; p.direct = direct;
   p.tiles_m = (int)ceil_div(M, 2 * GP_M); p.tiles_n = (int)ceil_div(N, width);
   const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
   // The tiles are handed out whole: cutting the tiles of a partial last wave along K (tried, also with the cut tiles done

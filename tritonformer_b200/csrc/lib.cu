@@ -25,10 +25,6 @@ bool gemm_tc05_eligible(const void* a, const void* b, int64_t M, int64_t N, int6
 int64_t gemm_tc05_workspace_bytes();
 int read_dev_status(int reset);
 int launch_wait_probe(unsigned long long limit_ns, int* waited_ok, cudaStream_t st);
-int attn_bwd_tc05_counters(unsigned long long* out);
-int gemm_pair_counters(int cta, unsigned long long* out);
-int attn_fwd1_tc05_counters(unsigned long long* out);
-std::atomic<int> g_counter_select{-1};
 }  // namespace tfb
 
 using namespace tfb;
@@ -47,12 +43,6 @@ extern "C" int tfb_debug_wait_probe(unsigned long long limit_ns, int* waited_ok,
   return launch_wait_probe(limit_ns, waited_ok, (cudaStream_t)stream);
 }
 
-extern "C" int tfb_debug_counters(unsigned long long* out16) {
-  const int sel = g_counter_select.load();
-  if (sel == -3) return attn_fwd1_tc05_counters(out16);
-  return sel >= 0 ? gemm_pair_counters(sel, out16) : attn_bwd_tc05_counters(out16);
-}
-
 extern "C" void tfb_debug_set(int key, int value) {
   if (key == 0) g_force_generic_gemm.store(value);
   if (key == 1) g_force_fallback_attn.store(value);
@@ -60,7 +50,6 @@ extern "C" void tfb_debug_set(int key, int value) {
   if (key == 3) g_plain_launch.store(value);
   if (key == 4) g_gemm_debug.store(value);
   if (key == 6) g_gemm_free_sms.store(value < 0 ? 0 : value);
-  if (key == 5) g_counter_select.store(value);
 }
 
 extern "C" int tfb_debug_gemm_plan(long long M, long long N, long long K, int b_mn) {
