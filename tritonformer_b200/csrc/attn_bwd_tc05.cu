@@ -20,8 +20,8 @@
 // and an MN-major operand with 128 contraction rows, so each of K, V, Q_i, dO_i, dSᵀ sits in
 // shared memory once and serves two products.
 //
-// Roles: warp 0 TMA producer, warp 1 MMA issuer, warps 2-17 compute (thread = TMEM lane, four
-// warps per lane quarter, each taking a quarter of the columns), warps 18-21 drain dQ_i.
+// Roles: warp 0 TMA producer, warp 1 MMA issuer, warps 4-7 drain dQ_i, warps 8-23 compute (thread = TMEM lane, four
+// warps per lane quarter, each taking a quarter of the columns).
 // Pᵀ goes into the 64 TMEM columns that are left instead of shared memory and is
 // the A operand of the dV product.
 // The scores of tile i+1 are issued as soon as the compute warps hold the scores of tile i in
@@ -46,8 +46,16 @@ extern std::atomic<int> g_attn_debug;
 constexpr float kLog2eB = 1.4426950408889634f;
 constexpr int FB_T = 128;           // tile edge (keys and queries)
 constexpr int FB_CWARPS = 16;        // compute warps: 4 TMEM lane quarters x 4 column quarters
-constexpr int FB_THREADS = 64 + 32 * FB_CWARPS + 128;  // TMA, MMA, compute warps, 4 dQ-drain warps
-constexpr int FB_COMPUTE = 256;     // threads in the compute warps
+// Warpgroups: TMA, MMA and two idle warps; four dQ-drain warps; the compute warps.  The block is launched with 80 registers a
+// thread (six warps per scheduler); the first two groups hand theirs on to the compute warps, which spill at 80: with the two
+// small passes, B4 H16 T2048 fp16 189.6 -> 172.2 us, exact slopes 195.9 -> 183.8, B3 H11 T1472 bf16 67.0 -> 61.3, B3 H16 T704 bf16 with the
+// rounded table 38.0 -> 33.8, B2 H12 T1024 fp16 33.8 -> 30.7.
+constexpr int FB_FIRST_C = 8;       // first compute warp
+constexpr int FB_THREADS = 32 * (FB_FIRST_C + FB_CWARPS);
+constexpr int FB_REGS = 80, FB_REGS_ISSUE = 32, FB_REGS_DRAIN = 64, FB_REGS_COMPUTE = 96;
+static_assert(128 * (FB_REGS_ISSUE + FB_REGS_DRAIN + 4 * FB_REGS_COMPUTE) <= FB_THREADS * FB_REGS, "registers of the block");
+template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
 constexpr int HD = 64;
 constexpr int TILE_BYTES = FB_T * 128;   // 128 rows x 64 x 2 B
@@ -77,7 +85,6 @@ constexpr int COL_PT = 256 + 3 * HD;
 struct FbParams {
   const float* lse;
   const float* delta;
-  float* dq_acc;  // (B,H,T,HD) fp32, zero on entry
   void *dk, *dv;
   int64_t sdk_b, sdk_h, sdk_t, sdv_b, sdv_h, sdv_t;
   int H, T, hd;   // hd: the real head_dim, 32 or 64
@@ -85,16 +92,8 @@ struct FbParams {
   float scale;
   int bias_mode;
   const float* slopes;
-  int debug;  // test switch: bit 0 skips the dQ accumulation (timing experiments only)
+  int debug;  // bit 5: per-slice item order (test switch)
 };
-
-// Cycle counters for the timing switch (debug bit 1): [0] CTA iterations, [1..5] compute warp 2:
-// wait scores, math, wait previous products, smem write, barrier+stats; [6..9] MMA thread: wait P/dS,
-// wait Q/dO, wait dQ drain, total; [10,11] drain warp: wait, drain; [12] / [15] MMA thread: time to issue the
-// score products / the gradient products of a tile.
-static __device__ unsigned long long g_prof[16];
-#define PROF_T(var) long long var = prof ? clock64() : 0
-#define PROF_ADD(idx, t0, t1) do { if (prof) atomicAdd(&g_prof[idx], (unsigned long long)((t1) - (t0))); } while (0)
 
 __device__ __forceinline__ float ex2_approx_b(float x) {
   float y;
@@ -207,6 +206,8 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
   const uint32_t tmem_base = *tmem_holder;
   const bool dead = *abort_flag != 0;
 
+  if (warp < 4) {
+  regs_down<FB_REGS_ISSUE>();
   if (warp == 0) {
     // --------------------------------------------------------------------- TMA producer
     if (lane == 0 && !dead) {
@@ -270,8 +271,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       const uint64_t dv_k = smem_desc_sw128(s0 + OFF_V, 16, 1024);
       const uint64_t dds_k = smem_desc_sw128(s0 + OFF_DS, 16, 1024);
       const uint64_t dds_mn = smem_desc_sw128(s0 + OFF_DS, 16384, 1024);
-      const bool prof = (p.debug & 2) && lane == 0;
-      PROF_T(tm_start);
       // every lane waits; the verdict is made uniform so that the warp stays converged
       auto wait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
         return __all_sync(0xffffffffu, mbar_wait(bar, parity, code, abort_flag)) != 0;
@@ -281,12 +280,8 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       auto issue_scores = [&](int g, int n) -> bool {  // g: tiles of the CTA before this one, n: items
         const uint32_t kv = (n % KVS) * 2 * TILE_BYTES;
         const int st = g % QS;
-        PROF_T(a0);
         if (!wait(&q_full[st], (g / QS) & 1, 0x2300 | st)) return false;
-        PROF_T(a1);
-        PROF_ADD(7, a0, a1);
         tc_fence_after();
-        PROF_T(i0_);
         const uint64_t q_k = smem_desc_sw128(s0 + OFF_Q + st * TILE_BYTES, 16, 1024);
         const uint64_t do_k = smem_desc_sw128(s0 + OFF_DO + st * TILE_BYTES, 16, 1024);
 #pragma unroll
@@ -300,8 +295,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           if (elect_one()) tc_mma_ss(tb + COL_DP, desc_advance(dv_k, kv + off), desc_advance(do_k, off), idesc_s, s ? 1u : 0u);
         }
         if (elect_one()) tc_commit(s_full);
-        PROF_T(i1_);
-        PROF_ADD(12, i0_, i1_);
         return true;
       };
       // dV += Pᵀ dO_i, dK += dSᵀ Q_i, dQ_i = dS K
@@ -311,12 +304,8 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         const uint64_t q_mn = smem_desc_sw128(s0 + OFF_Q + st * TILE_BYTES, 16384, 1024);
         const uint64_t do_mn = smem_desc_sw128(s0 + OFF_DO + st * TILE_BYTES, 16384, 1024);
         // the dQ columns still hold the previous tile's dQ until the drain warps are done with it
-        PROF_T(a0);
         if (g > 0 && !wait(dq_free, (g - 1) & 1, 0x2400)) return false;
-        PROF_T(a1);
-        PROF_ADD(8, a0, a1);
         tc_fence_after();
-        PROF_T(i0_);
         const uint32_t acc = it ? 1u : 0u;
 #pragma unroll
         for (int s = 0; s < FB_T / 16; ++s) {  // contraction over the 128 queries of this tile
@@ -337,8 +326,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           tc_commit(dq_full);
           if (last) tc_commit(&kv_empty[n % KVS]);
         }
-        PROF_T(i1_);
-        PROF_ADD(15, i0_, i1_);
         return true;
       };
       Item w = item_of(blockIdx.x);
@@ -361,10 +348,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
             if (!wait(s_free, g & 1, 0x2550)) { ok = false; break; }
             if (!issue_scores(g + 1, last ? n + 1 : n)) { ok = false; break; }
           }
-          PROF_T(a0);
           if (!wait(pds_full, g & 1, 0x2500)) { ok = false; break; }
-          PROF_T(a1);
-          PROF_ADD(6, a0, a1);
           // the first products of an item overwrite dV and dK of the one before
           if (it == 0 && n > 0 && !wait(acc_free, (n - 1) & 1, 0x2560)) { ok = false; break; }
           ok = issue_grads(g, n, it, last);
@@ -372,14 +356,14 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         if (!more) break;
         w = wn;
       }
-      PROF_T(tm_end);
-      PROF_ADD(9, tm_start, tm_end);
     }
     __syncwarp();
-  } else if (warp < 2 + FB_CWARPS) {
+  }
+  } else if (warp >= FB_FIRST_C) {
     // -------------------------------------------------------------------------- compute
+    regs_up<FB_REGS_COMPUTE>();
     if (!dead) {
-      const int cw = warp - 2;           // 0..15
+      const int cw = warp - FB_FIRST_C;  // 0..15
       const int qd = warp & 3;           // TMEM lane quarter
       const int cq = cw >> 2;            // which quarter (32) of the 128 query columns
       const int r = qd * 32 + lane;      // TMEM lane = key row
@@ -387,7 +371,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       const float c2 = p.scale * kLog2eB;
       uint8_t* sds = smem + OFF_DS;
       bool ok = true;
-      const bool prof = (p.debug & 2) && threadIdx.x == 64;
       // Per-query statistics of the warp's 32 query columns: lane l carries lse and delta of
       // column l, fetched one tile ahead (so the global-memory latency is not part of the tile) and handed to the
       // other lanes through a slice of shared memory that belongs to this warp: no barrier across the warps.
@@ -438,7 +421,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       for (int it = 0; it < nq - w.kt; ++it, ++g) {
         const int i0 = (w.kt + it) * FB_T;
         const bool diag = (it == 0);
-        PROF_T(t0);
         // this tile's statistics, double buffered by iteration parity: a lane that is already here may share
         // the warp with one that still reads the previous tile's slice
         float* s_lse2 = s_stat + ((g & 1) * FB_CWARPS + cw) * 64;
@@ -446,23 +428,10 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         s_lse2[lane] = lse_next * kLog2eB;
         s_delta[lane] = delta_next;
         __syncwarp();
-        PROF_T(t1);
         if (it + 1 < nq - w.kt) load_stat(w, it + 1, lse_next, delta_next);  // after the warp barrier, which would wait for it
         if (ok) ok = mbar_wait(s_full, g & 1, 0x2600, abort_flag);
-        PROF_T(t2);
-        PROF_ADD(5, t0, t1);
-        PROF_ADD(1, t1, t2);
-        if (prof) atomicAdd(&g_prof[0], 1ull);
         uint32_t pk[16], dk_[16];  // this thread's 32 columns of Pᵀ and dSᵀ, packed 16-bit pairs
-        long long t3 = 0, t4 = 0;
-        const bool quiet = (p.debug & 128) != 0;  // timing experiment: the compute warps only keep the barriers going
-        if (quiet) {
-#pragma unroll
-          for (int e = 0; e < 16; ++e) pk[e] = dk_[e] = 0u;
-          if (lane == 0) mbar_arrive(s_free);
-          if (g > 0 && ok) ok = mbar_wait(dq_full, (g - 1) & 1, 0x2650, abort_flag);
-        }
-        if (ok && !quiet) {
+        if (ok) {
           tc_fence_after();
           const bool plain = !BIAS && !diag;  // no bias and not the diagonal tile: scale, subtract, 2^x
           // Four chunks of 8 query columns; the tensor-memory loads of a chunk are issued before the chunk ahead of
@@ -471,7 +440,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           // burst makes the load wait 850 cycles, was tried: the wait for the next scores at that point cost more
           // than it saved, 230 against 210 us.)
           uint32_t sv_[2][8], dv_[2][8];
-          PROF_T(tl0);
           tmem_ld8(lane_addr + COL_S + cq * 32, sv_[0]);
           tmem_ld8(lane_addr + COL_DP + cq * 32, dv_[0]);
 #pragma unroll
@@ -486,10 +454,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
               tc_fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive(s_free);
-            }
-            if (c == 0) {
-              PROF_T(tl1);
-              PROF_ADD(14, tl0, tl1);
             }
 #pragma unroll
             for (int e4 = 0; e4 < 2; ++e4) {
@@ -522,11 +486,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
             }
           }
           // Pᵀ / dSᵀ of the previous tile are still being read by its gradient products
-          if (prof) t3 = clock64();
           if (g > 0) ok = mbar_wait(dq_full, (g - 1) & 1, 0x2650, abort_flag);
-          if (prof) t4 = clock64();
-          PROF_ADD(2, t2, t3);
-          PROF_ADD(3, t3, t4);
         }
         // T is a multiple of 64, so a warp's 32 queries are all real or all past the sequence's end.  The latter get exact
         // zeros: what was worked out from the zero-filled rows is NaN where K or V holds an infinity.
@@ -535,12 +495,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           for (int e = 0; e < 16; ++e) pk[e] = dk_[e] = 0u;
         }
         if (it == 0 && n > 0 && ok) store_item(wp);  // (the wait for dq_full above was for its last tile)
-        if (ok && quiet) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(pds_full);
-        }
-        if (ok && !quiet) {
+        if (ok) {
           tmem_st16(lane_addr + COL_PT + cq * 16, pk);  // this thread's 32 queries of Pᵀ
 #pragma unroll
           for (int v4 = 0; v4 < 4; ++v4) {
@@ -549,14 +504,10 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
             *reinterpret_cast<uint4*>(sds + off) = make_uint4(dk_[v4 * 4], dk_[v4 * 4 + 1], dk_[v4 * 4 + 2], dk_[v4 * 4 + 3]);
           }
           tc_wait_st();
-          PROF_T(t45);
           tc_fence_before();
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
           if (lane == 0) mbar_arrive(pds_full);
-          PROF_T(t5);
-          PROF_ADD(4, t4, t5);
-          PROF_ADD(13, t45, t5);
         }
       }
       Item wn = w;
@@ -571,16 +522,17 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       w = wn;
       }
     }
-  } else if (!dead) {
+  } else {
+    regs_down<FB_REGS_DRAIN>();
+    if (!dead) {
     // ---------------------------------------------------------------------------- dQ drain
-    // the last four warps: lanes are query rows here; each warp adds its 32 rows of dQ_i to the fp32 accumulator.
+    // the second warpgroup: lanes are query rows here; each warp adds its 32 rows of dQ_i to the fp32 accumulator.
     // The rows go through swizzled shared-memory boxes and the TMA unit performs the
     // reduction (cp.reduce.async.bulk.tensor), which keeps the load/store path free for the compute warps.
     const int qd = warp & 3;
     const int r = qd * 32 + lane;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
-    const bool prof = (p.debug & 2) && warp == 2 + FB_CWARPS && lane == 0;
-    uint8_t* stage = smem + OFF_DQ + (warp - 2 - FB_CWARPS) * 4096;
+    uint8_t* stage = smem + OFF_DQ + (warp - 4) * 4096;
     if (lane == 0) tma_prefetch_desc(&tmDQ);
     Item w = item_of(blockIdx.x);
     int g = 0;
@@ -589,24 +541,22 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
     const int bh = w.bh;
     for (int it = 0; it < nq - w.kt; ++it, ++g) {
       const int i0 = (w.kt + it) * FB_T;
-      PROF_T(a0);
       if (!mbar_wait(dq_full, g & 1, 0x2700, abort_flag)) { ok = false; break; }
-      PROF_T(a1);
-      PROF_ADD(10, a0, a1);
       tc_fence_after();
-      if (!(p.debug & 64)) {
-        uint32_t v0[32], v1[32];
-        tmem_ld32(lane_addr + COL_DQ, v0);
-        tmem_ld32(lane_addr + COL_DQ + 32, v1);
-        tc_wait_ld();
-        // TMEM is drained: the tensor core may overwrite dQ while the rows travel on
-        tc_fence_before();
+      const int row0 = (int)((int64_t)bh * p.T) + i0 + qd * 32;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {  // chunks of 32 columns
+        uint32_t v[32];
+        tmem_ld32(lane_addr + COL_DQ + c * 32, v);
+        if (lane == 0) tma_store_wait_read();  // the box has been read by the TMA unit
         __syncwarp();
-        if (lane == 0) mbar_arrive(dq_free);
-        const int row0 = (int)((int64_t)bh * p.T) + i0 + qd * 32;
-        auto add_box = [&](const uint32_t (&v)[32], int col) {
-          if (lane == 0) tma_store_wait_read();  // the box has been read by the TMA unit
+        tc_wait_ld();
+        if (c == 1) {  // tensor memory is drained: the tensor core may overwrite dQ while the rows travel on
+          tc_fence_before();
           __syncwarp();
+          if (lane == 0) mbar_arrive(dq_free);
+        }
+        if (c * 32 < p.hd) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {  // 16-byte chunks (4 floats) of this row
             const uint32_t off = lane * 128 + ((j ^ (lane & 7)) << 4);
@@ -615,39 +565,16 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if (!RAGGED || i0 + qd * 32 < p.T) tma_reduce_add_2d(&tmDQ, stage, col, row0);  // the rows past the end are the next slice's
+            if (!RAGGED || i0 + qd * 32 < p.T) tma_reduce_add_2d(&tmDQ, stage, c * 32, row0);  // the rows past the end are the next slice's
             tma_store_commit();
           }
-        };
-        if (!(p.debug & 1)) {
-          add_box(v0, 0);
-          if (p.hd > 32) add_box(v1, 32);
         }
-      } else {
-        float* dq_row = p.dq_acc + ((int64_t)bh * p.T + i0 + r) * p.hd;
-#pragma unroll 1
-        for (int c = 0; c < p.hd / 32; ++c) {
-          uint32_t v[32];
-          tmem_ld32(lane_addr + COL_DQ + c * 32, v);
-          tc_wait_ld();
-          if (!(p.debug & 1) && i0 + r < p.T)
-#pragma unroll
-            for (int e = 0; e < 32; e += 4)
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dq_row + c * 32 + e),
-                           "f"(__uint_as_float(v[e])), "f"(__uint_as_float(v[e + 1])),
-                           "f"(__uint_as_float(v[e + 2])), "f"(__uint_as_float(v[e + 3]))
-                           : "memory");
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(dq_free);
       }
-      PROF_T(a2);
-      PROF_ADD(11, a1, a2);
     }
     ok = __all_sync(0xffffffffu, ok) != 0 && next_of(n, w, false);
     }
     if (lane == 0) tma_store_wait_all();  // every reduction has reached global memory
+    }
   }
 
   tc_fence_before();
@@ -698,15 +625,6 @@ __global__ void __launch_bounds__(256) attn_dq_convert_kernel(const float* __res
 
 // ------------------------------------------------------------------------------- host side
 
-// Copies the timing counters to `out` (16 values) and clears them.  Synchronises the device.
-int attn_bwd_tc05_counters(unsigned long long* out) {
-  cudaDeviceSynchronize();
-  if (cudaMemcpyFromSymbol(out, g_prof, sizeof(unsigned long long) * 16) != cudaSuccess) return -1;
-  unsigned long long z[16] = {0};
-  cudaMemcpyToSymbol(g_prof, z, sizeof(z));
-  return 0;
-}
-
 static int encode_bhtd(CUtensorMap* m, const void* ptr, const AttnStrides& s, int B, int H, int T, int hd, int dtype) {
   const uint64_t dims[4] = {(uint64_t)hd, (uint64_t)T, (uint64_t)H, (uint64_t)B};
   const uint64_t str[3] = {(uint64_t)s.t * 2, (uint64_t)s.h * 2, (uint64_t)s.b * 2};
@@ -720,6 +638,20 @@ bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd) {  // as in the forward
 }
 
 int attn_bwd128_tc05(const AttnArgs& a, int dtype, cudaStream_t st);
+
+// The registers that the warpgroups share out are those of the launch: a build with another number must not run (a group
+// would wait for registers that there are not).
+template <typename F>
+static int check_registers(F func, std::atomic<int>& seen) {
+  if (seen.load(std::memory_order_relaxed) == FB_REGS) return TFB_OK;
+  cudaFuncAttributes attr;
+  const cudaError_t e = cudaFuncGetAttributes(&attr, func);
+  if (e != cudaSuccess) return fail(TFB_ERR_LAUNCH, "attention_bwd(tcgen05): function attributes: %s", cudaGetErrorString(e));
+  if (attr.numRegs != FB_REGS)
+    return fail(TFB_ERR_LAUNCH, "attention_bwd(tcgen05): built with %d registers a thread instead of %d", attr.numRegs, FB_REGS);
+  seen.store(FB_REGS, std::memory_order_relaxed);
+  return TFB_OK;
+}
 
 template <typename T, bool RAGGED>
 static int bwd64_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
@@ -737,7 +669,7 @@ static int bwd64_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   if ((rc = encode_bhtd(&tv, a.v, a.sv, a.B, a.H, a.T, hd, dtype))) return rc;
   if ((rc = encode_bhtd(&tdo, a.d_o, a.sdo, a.B, a.H, a.T, hd, dtype))) return rc;
   FbParams p;
-  p.lse = a.lse; p.delta = a.delta; p.dq_acc = a.dq_acc; p.dk = a.dk; p.dv = a.dv;
+  p.lse = a.lse; p.delta = a.delta; p.dk = a.dk; p.dv = a.dv;
   p.sdk_b = a.sdk.b; p.sdk_h = a.sdk.h; p.sdk_t = a.sdk.t;
   p.sdv_b = a.sdv.b; p.sdv_h = a.sdv.h; p.sdv_t = a.sdv.t;
   p.H = a.H; p.T = a.T; p.hd = hd; p.scale = a.scale; p.bias_mode = a.bias_mode; p.slopes = a.slopes;
@@ -746,11 +678,13 @@ static int bwd64_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   p.group = attn_slices_per_group(a.B * a.H, a.T, HD);
   dim3 grid((unsigned)ceil_div(a.T, FB_T) * a.B * a.H);
   static std::atomic<uint64_t> done[4] = {{0}, {0}, {0}, {0}};
+  static std::atomic<int> regs[4] = {{0}, {0}, {0}, {0}};
 #define FB_LAUNCH(MODE, SLOT)                                                                                       \
   {                                                                                                                 \
     if ((rc = ensure_dynamic_smem(attn_bwd_tc05_kernel<T, MODE, RAGGED>, SMEM_BYTES, done[SLOT],                   \
                                   "attention_bwd(tcgen05)")))                                                       \
       return rc;                                                                                                    \
+    if ((rc = check_registers(attn_bwd_tc05_kernel<T, MODE, RAGGED>, regs[SLOT]))) return rc;                                    \
     launch_overlapped(attn_bwd_tc05_kernel<T, MODE, RAGGED>, grid, dim3(FB_THREADS), SMEM_BYTES, st, tq, tk, \
                       tv, tdo, tdq, p);                                                                             \
   }
