@@ -26,6 +26,8 @@ FLAGS = [
     # relocatable device code: every translation unit shares ONE device-side status word (status.cu)
     "-rdc=true",
 ]
+# kernels whose warpgroups share out registers: ptxas ignores setmaxnreg in relocatable code
+WHOLE = ("attn_bwd_tc05.cu", "attn_bwd128_tc05.cu")
 
 
 def _sources():
@@ -64,7 +66,8 @@ def _compile(path, force, host_flags):
     newest = max(os.path.getmtime(path), _headers_mtime(os.path.dirname(path)))
     if not force and os.path.exists(obj) and os.path.getmtime(obj) > newest:
         return obj
-    _run(([CXX] + host_flags if is_host else [NVCC] + FLAGS) + ["-c", path, "-o", obj], "compiling " + src)
+    flags = [f for f in FLAGS if f != "-rdc=true" or src not in WHOLE]
+    _run(([CXX] + host_flags if is_host else [NVCC] + flags) + ["-c", path, "-o", obj], "compiling " + src)
     return obj
 
 

@@ -16,13 +16,14 @@
 //
 // TMEM columns of a slot: [0,64) Sᵀ, over it Pᵀ (16-bit, at the head of each warp's own score columns: the A operand of the dV
 // product); [64,128) dPᵀ; over both dQ_i (M = 64: row 16 q + r sits in lane 32 q + r).  [256,384) dV, [384,512) dK.
-// Roles: warp 0 TMA producer, warp 1 MMA issuer, then eight compute warps per slot: two per TMEM lane quarter, 32 query columns
+// Roles: warp 0 TMA producer, warp 1 MMA issuer, from warp 4 on eight compute warps per slot: two per TMEM lane quarter, 32 query columns
 // each; they also hand dQ to the TMA unit.
 // A swizzled panel of 64 16-bit values per row is at the same time a K-major operand and an MN-major one, so each of K, V,
 // Q_i, dO_i, dSᵀ sits in shared memory once and serves two products.
 // Sequences are multiples of 64, so every sub-tile of queries is real; keys past the end are zero rows (TMA fill) that the
 // causal mask keeps from every query.  A warp's 32 x 32 block is, as a whole, untouched by the mask, cut by the diagonal, or
 // masked (nothing is computed).
+#define TFB_STATUS_FROM_LAUNCH
 #include "attn.cuh"
 #include "tc05.cuh"
 #include <type_traits>
@@ -41,7 +42,13 @@ constexpr int FB_CWARPS = 8;    // compute warps per slot
 constexpr int HD = 128;
 constexpr int PANELS = 2;          // 64-element (128-byte) panels along head_dim
 constexpr int SLOTS = 2;
-constexpr int THREADS = 64 + 32 * FB_CWARPS * SLOTS;
+// Warpgroups: TMA, MMA and two idle warps; the compute warps.  The block is launched with 96 registers a thread (five warps per
+// scheduler); the first group hands most of its own on to the compute warps: B1 H12 T4096 fp16 222.7 -> 214.8 us, T4032 217 -> 210,
+// B2 H16 T2048 bf16 with the rounded table 177 -> 170.
+constexpr int FIRST_C = 4;         // first compute warp
+constexpr int THREADS = 32 * (FIRST_C + FB_CWARPS * SLOTS);
+constexpr int REGS = 96, REGS_ISSUE = 32, REGS_COMPUTE = 112;
+static_assert(128 * REGS_ISSUE + 32 * FB_CWARPS * SLOTS * REGS_COMPUTE <= THREADS * REGS, "registers of the block");
 constexpr int KV_BYTES = PANELS * FB_K * 128, Q_BYTES = PANELS * FB_Q * 128;
 constexpr int QS = 2;              // Q / dO ring depth
 constexpr int DS_BYTES = FB_K * FB_Q * 2;
@@ -56,6 +63,7 @@ static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 constexpr int COL_DV = SLOTS * 128, COL_DK = COL_DV + HD;
 
 struct FbParams {
+  int* status;    // the library's status word
   const float* lse;
   const float* delta;
   void *dk, *dv;
@@ -71,16 +79,6 @@ __device__ __forceinline__ float fb_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
-}
-__device__ __forceinline__ uint64_t fb_mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t fb_add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
 }
 template <typename T>
 __device__ __forceinline__ uint32_t fb_pack(uint64_t v) {
@@ -159,13 +157,18 @@ __global__ void __launch_bounds__(THREADS, 1)
   // set-up above is CTA-local and may overlap the previous kernel's tail; global memory comes after
   grid_dependency_wait();
   allow_dependents();
-  if (threadIdx.x == 0) *abort_flag = (*(volatile int*)&g_dev_status != 0) ? 1 : 0;
+  if (threadIdx.x == 0) {
+    *status_slot() = p.status;
+    *abort_flag = (*(volatile int*)p.status != 0) ? 1 : 0;
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   const bool dead = *abort_flag != 0;
 
+  if (warp < FIRST_C) {
+  regs_down<REGS_ISSUE>();
   if (warp == 0) {
     // --------------------------------------------------------------------- TMA producer
     if (lane == 0 && !dead) {
@@ -284,7 +287,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           } else if (__any_sync(0xffffffffu, global_ns() - t_idle > kWaitLimitNs)) {
             if (lane == 0) {
               *abort_flag = 1;
-              atomicCAS(&g_dev_status, 0, 0x2550);
+              atomicCAS(dev_status(), 0, 0x2550);
             }
             ok = false;
           } else {
@@ -294,9 +297,12 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
     }
     __syncwarp();
-  } else if (!dead) {
+  }
+  } else {
+    regs_up<REGS_COMPUTE>();
+    if (!dead) {
     // -------------------------------------------------------------------------- compute
-    const int cw = warp - 2;
+    const int cw = warp - FIRST_C;
     const int slot = cw / FB_CWARPS;
     const int qd = warp & 3;                 // TMEM lane quarter
     const int cq = (cw % FB_CWARPS) >> 2;    // which half (32) of the 64 query columns
@@ -433,8 +439,8 @@ __global__ void __launch_bounds__(THREADS, 1)
           for (int k = 0; k < 4; ++k) {
             const int e = v * 8 + 2 * k;
             const float2 dl = *reinterpret_cast<const float2*>(s_lse + 32 + e);
-            const uint64_t d = fb_add2(f2_pack(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])), f2_pack(dl.x, dl.y));
-            w[k] = fb_pack<T>(fb_mul2(pe[e / 2], d));
+            const uint64_t d = f2_add(f2_pack(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])), f2_pack(dl.x, dl.y));
+            w[k] = fb_pack<T>(f2_mul(pe[e / 2], d));
           }
           *reinterpret_cast<uint4*>(sds + (((cq * 4 + v) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
@@ -471,6 +477,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
     }
     if (lane == 0) tma_store_wait_all();  // every reduction has reached global memory
+    }
   }
 
   tc_fence_before();
@@ -516,14 +523,18 @@ static int bwd128_launch(const AttnArgs& a, int dtype, cudaStream_t st) {
   p.sdv_b = a.sdv.b; p.sdv_h = a.sdv.h; p.sdv_t = a.sdv.t;
   p.H = a.H; p.T = a.T; p.scale = a.scale; p.slopes = a.slopes;
   p.debug = g_attn_debug.load();
+  p.status = dev_status_address();
+  if (!p.status) return fail(TFB_ERR_LAUNCH, "attention_bwd(tcgen05): cannot find the status word");
   p.BH = a.B * a.H;
   p.group = attn_slices_per_group(a.B * a.H, a.T, HD);
   const dim3 grid((unsigned)ceil_div(a.T, FB_K) * a.B * a.H);
   static std::atomic<uint64_t> done[4] = {{0}, {0}, {0}, {0}};
+  static std::atomic<int> regs[4] = {{0}, {0}, {0}, {0}};
 #define FB_LAUNCH(MODE, SLOT)                                                                                               \
   {                                                                                                                         \
     if ((rc = ensure_dynamic_smem(attn_bwd128_tc05_kernel<T, MODE>, SMEM_BYTES, done[SLOT], "attention_bwd(tcgen05)"))) \
       return rc;                                                                                                            \
+    if ((rc = check_launch_registers(attn_bwd128_tc05_kernel<T, MODE>, REGS, regs[SLOT], "attention_bwd(tcgen05)"))) return rc;    \
     launch_overlapped(attn_bwd128_tc05_kernel<T, MODE>, grid, dim3(THREADS), SMEM_BYTES, st, tq, tk, tv, tdo, tdq, p); \
   }
   if (a.bias_mode == 0) FB_LAUNCH(0, 0)

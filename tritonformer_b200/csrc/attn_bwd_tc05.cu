@@ -35,6 +35,7 @@
 // 191 at B4 H16 T2048 fp16, 165 against 89 at B1 H8 T4096.  A sub-tile's chain takes 4.3 k cycles even alone on an SM, nearly as
 // long as a whole tile's 5.5 k, and the two CTAs share what it waits for.)
 // TMEM columns: [0,128) Sᵀ; [128,256) dPᵀ; [256,320) dV; then dK; then dQ_i; then Pᵀ.
+#define TFB_STATUS_FROM_LAUNCH
 #include "attn.cuh"
 #include "tc05.cuh"
 #include <type_traits>
@@ -47,15 +48,15 @@ constexpr float kLog2eB = 1.4426950408889634f;
 constexpr int FB_T = 128;           // tile edge (keys and queries)
 constexpr int FB_CWARPS = 16;        // compute warps: 4 TMEM lane quarters x 4 column quarters
 // Warpgroups: TMA, MMA and two idle warps; four dQ-drain warps; the compute warps.  The block is launched with 80 registers a
-// thread (six warps per scheduler); the first two groups hand theirs on to the compute warps, which spill at 80: with the two
-// small passes, B4 H16 T2048 fp16 189.6 -> 172.2 us, exact slopes 195.9 -> 183.8, B3 H11 T1472 bf16 67.0 -> 61.3, B3 H16 T704 bf16 with the
-// rounded table 38.0 -> 33.8, B2 H12 T1024 fp16 33.8 -> 30.7.
+// thread (six warps per scheduler); the first two groups hand some of theirs on to the compute warps.  (More than 88 for these
+// left the MMA warp spilling: 179 against 172 us.)  Backward with its two small passes, in microseconds: in 22 warps with the drain
+// warps last, with the warpgroups, and with the registers moved as well and the packed arithmetic on blocks that know whether
+// they meet the diagonal: B4 H16 T2048 fp16 189.6, 172.2, 171.9, exact slopes 195.9, 183.8, 171.6; B3 H11 T1472 bf16 67.0, 61.3, 62.6;
+// B3 H16 T704 bf16 with the rounded table 38.0, 33.8, 32.7; B2 H12 T1024 fp16 33.8, 30.7, 31.0.
 constexpr int FB_FIRST_C = 8;       // first compute warp
 constexpr int FB_THREADS = 32 * (FB_FIRST_C + FB_CWARPS);
-constexpr int FB_REGS = 80, FB_REGS_ISSUE = 32, FB_REGS_DRAIN = 64, FB_REGS_COMPUTE = 96;
+constexpr int FB_REGS = 80, FB_REGS_ISSUE = 56, FB_REGS_DRAIN = 72, FB_REGS_COMPUTE = 88;
 static_assert(128 * (FB_REGS_ISSUE + FB_REGS_DRAIN + 4 * FB_REGS_COMPUTE) <= FB_THREADS * FB_REGS, "registers of the block");
-template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
 constexpr int HD = 64;
 constexpr int TILE_BYTES = FB_T * 128;   // 128 rows x 64 x 2 B
@@ -83,6 +84,7 @@ constexpr int COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 256 + HD, COL_DQ =
 constexpr int COL_PT = 256 + 3 * HD;
 
 struct FbParams {
+  int* status;    // the library's status word
   const float* lse;
   const float* delta;
   void *dk, *dv;
@@ -199,7 +201,10 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
   // set-up above is CTA-local and may overlap the previous kernel's tail; global memory comes after
   grid_dependency_wait();
   allow_dependents();
-  if (threadIdx.x == 0) *abort_flag = (*(volatile int*)&g_dev_status != 0) ? 1 : 0;
+  if (threadIdx.x == 0) {
+    *status_slot() = p.status;
+    *abort_flag = (*(volatile int*)p.status != 0) ? 1 : 0;
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -369,6 +374,7 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       const int r = qd * 32 + lane;      // TMEM lane = key row
       const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
       const float c2 = p.scale * kLog2eB;
+      const uint64_t c2p = f2_pack(c2, c2);
       uint8_t* sds = smem + OFF_DS;
       bool ok = true;
       // Per-query statistics of the warp's 32 query columns: lane l carries lse and delta of
@@ -420,69 +426,72 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
       const int j = w.kt * FB_T + r;     // this thread's key
       for (int it = 0; it < nq - w.kt; ++it, ++g) {
         const int i0 = (w.kt + it) * FB_T;
-        const bool diag = (it == 0);
+        // the warp's 32 x 32 block against the diagonal: < 0 masked, 0 cut, > 0 untouched
+        const int rel = it * 4 + cq - qd;
         // this tile's statistics, double buffered by iteration parity: a lane that is already here may share
         // the warp with one that still reads the previous tile's slice
         float* s_lse2 = s_stat + ((g & 1) * FB_CWARPS + cw) * 64;
         float* s_delta = s_lse2 + 32;
-        s_lse2[lane] = lse_next * kLog2eB;
-        s_delta[lane] = delta_next;
+        s_lse2[lane] = -lse_next * kLog2eB;
+        s_delta[lane] = -delta_next;
         __syncwarp();
         if (it + 1 < nq - w.kt) load_stat(w, it + 1, lse_next, delta_next);  // after the warp barrier, which would wait for it
         if (ok) ok = mbar_wait(s_full, g & 1, 0x2600, abort_flag);
         uint32_t pk[16], dk_[16];  // this thread's 32 columns of Pᵀ and dSᵀ, packed 16-bit pairs
         if (ok) {
           tc_fence_after();
-          const bool plain = !BIAS && !diag;  // no bias and not the diagonal tile: scale, subtract, 2^x
-          // Four chunks of 8 query columns; the tensor-memory loads of a chunk are issued before the chunk ahead of
-          // it is worked on (two register sets of 8 + 8 values), so only the first load's latency is exposed.
-          // (Requesting a tile's first chunk at the end of the tile before it, ahead of the gradient products whose
-          // burst makes the load wait 850 cycles, was tried: the wait for the next scores at that point cost more
-          // than it saved, 230 against 210 us.)
-          uint32_t sv_[2][8], dv_[2][8];
-          tmem_ld8(lane_addr + COL_S + cq * 32, sv_[0]);
-          tmem_ld8(lane_addr + COL_DP + cq * 32, dv_[0]);
+          if (rel < 0) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(s_free);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int col0 = cq * 32 + c * 8;
-            const float d0 = (float)(i0 + col0 - j);  // distance of the chunk's first query to this thread's key
-            tc_wait_ld();
-            if (c + 1 < 4) {
-              tmem_ld8(lane_addr + COL_S + col0 + 8, sv_[(c + 1) & 1]);
-              tmem_ld8(lane_addr + COL_DP + col0 + 8, dv_[(c + 1) & 1]);
-            } else {  // this warp's share of Sᵀ and dPᵀ is in registers
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(s_free);
-            }
+            for (int e = 0; e < 16; ++e) pk[e] = dk_[e] = 0u;
+          } else {
+            const int first = rel == 0 ? lane : 0;  // first of the warp's query columns that sees this thread's key
+            // Four chunks of 8 query columns; the tensor-memory loads of a chunk are issued before the chunk ahead of
+            // it is worked on (two register sets of 8 + 8 values), so only the first load's latency is exposed.
+            // (Requesting a tile's first chunk at the end of the tile before it, ahead of the gradient products whose
+            // burst makes the load wait 850 cycles, was tried: the wait for the next scores at that point cost more
+            // than it saved, 230 against 210 us.  All 64 values at once do not fit the registers.)
+            uint32_t sv_[2][8], dv_[2][8];
+            tmem_ld8(lane_addr + COL_S + cq * 32, sv_[0]);
+            tmem_ld8(lane_addr + COL_DP + cq * 32, dv_[0]);
 #pragma unroll
-            for (int e4 = 0; e4 < 2; ++e4) {
-              const float4 l4 = *reinterpret_cast<const float4*>(s_lse2 + c * 8 + e4 * 4);
-              const float4 d4 = *reinterpret_cast<const float4*>(s_delta + c * 8 + e4 * 4);
-              const float lv[4] = {l4.x, l4.y, l4.z, l4.w};
-              const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
-              float pe[4], de[4];
-#pragma unroll
-              for (int k = 0; k < 4; k += 2) {
-                const int e = e4 * 4 + k;
-                float x0 = fmaf(__uint_as_float(sv_[c & 1][e]), c2, -lv[k]), x1 = fmaf(__uint_as_float(sv_[c & 1][e + 1]), c2, -lv[k + 1]);
-                if (plain) {
-                  pe[k] = ex2_approx_b(x0);  // (one exponential in four on the FMA pipe, as in the forward, changed nothing here)
-                  pe[k + 1] = ex2_approx_b(x1);
-                } else {
-                  const int i = i0 + col0 + e;
-                  // a key above the diagonal (negative distance) is masked below
-                  f2_unpack(alibi.sub_pair(f2_pack(x0, x1), d0 + (float)e, d0 + (float)(e + 1)), x0, x1);
-                  pe[k] = (j > i) ? 0.f : ex2_approx_b(x0);
-                  pe[k + 1] = (j > i + 1) ? 0.f : ex2_approx_b(x1);
-                }
-                de[k] = pe[k] * (__uint_as_float(dv_[c & 1][e]) - dl[k]);
-                de[k + 1] = pe[k + 1] * (__uint_as_float(dv_[c & 1][e + 1]) - dl[k + 1]);
+            for (int c = 0; c < 4; ++c) {
+              const int col0 = cq * 32 + c * 8;
+              const float d0 = (float)(i0 + col0 - j);  // distance of the chunk's first query to this thread's key
+              tc_wait_ld();
+              if (c + 1 < 4) {
+                tmem_ld8(lane_addr + COL_S + col0 + 8, sv_[(c + 1) & 1]);
+                tmem_ld8(lane_addr + COL_DP + col0 + 8, dv_[(c + 1) & 1]);
+              } else {  // this warp's share of Sᵀ and dPᵀ is in registers
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_free);
               }
-              pk[c * 4 + e4 * 2] = pack2<T>(pe[0], pe[1]);
-              pk[c * 4 + e4 * 2 + 1] = pack2<T>(pe[2], pe[3]);
-              dk_[c * 4 + e4 * 2] = pack2<T>(de[0], de[1]);
-              dk_[c * 4 + e4 * 2 + 1] = pack2<T>(de[2], de[3]);
+              const uint32_t *sv = sv_[c & 1], *dv = dv_[c & 1];
+#pragma unroll
+              for (int e4 = 0; e4 < 8; e4 += 4) {
+                const float4 l4 = *reinterpret_cast<const float4*>(s_lse2 + c * 8 + e4);
+                const float4 d4 = *reinterpret_cast<const float4*>(s_delta + c * 8 + e4);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                  const int e = e4 + 2 * k;
+                  uint64_t x = f2_fma(f2_pack(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), c2p,
+                                      k ? f2_pack(l4.z, l4.w) : f2_pack(l4.x, l4.y));
+                  if (BIAS) x = alibi.sub_pair(x, d0 + (float)e, d0 + (float)(e + 1));
+                  float x0, x1, s0, s1;
+                  f2_unpack(x, x0, x1);
+                  // (one exponential in four on the FMA pipe, as in the forward, changed nothing here)
+                  x0 = c * 8 + e < first ? 0.f : ex2_approx_b(x0);
+                  x1 = c * 8 + e + 1 < first ? 0.f : ex2_approx_b(x1);
+                  const uint64_t d = f2_add(f2_pack(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])),
+                                            k ? f2_pack(d4.z, d4.w) : f2_pack(d4.x, d4.y));
+                  f2_unpack(f2_mul(f2_pack(x0, x1), d), s0, s1);
+                  pk[c * 4 + e / 2] = pack2<T>(x0, x1);
+                  dk_[c * 4 + e / 2] = pack2<T>(s0, s1);
+                }
+              }
             }
           }
           // Pᵀ / dSᵀ of the previous tile are still being read by its gradient products
@@ -639,20 +648,6 @@ bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd) {  // as in the forward
 
 int attn_bwd128_tc05(const AttnArgs& a, int dtype, cudaStream_t st);
 
-// The registers that the warpgroups share out are those of the launch: a build with another number must not run (a group
-// would wait for registers that there are not).
-template <typename F>
-static int check_registers(F func, std::atomic<int>& seen) {
-  if (seen.load(std::memory_order_relaxed) == FB_REGS) return TFB_OK;
-  cudaFuncAttributes attr;
-  const cudaError_t e = cudaFuncGetAttributes(&attr, func);
-  if (e != cudaSuccess) return fail(TFB_ERR_LAUNCH, "attention_bwd(tcgen05): function attributes: %s", cudaGetErrorString(e));
-  if (attr.numRegs != FB_REGS)
-    return fail(TFB_ERR_LAUNCH, "attention_bwd(tcgen05): built with %d registers a thread instead of %d", attr.numRegs, FB_REGS);
-  seen.store(FB_REGS, std::memory_order_relaxed);
-  return TFB_OK;
-}
-
 template <typename T, bool RAGGED>
 static int bwd64_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   int rc;
@@ -674,6 +669,8 @@ static int bwd64_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   p.sdv_b = a.sdv.b; p.sdv_h = a.sdv.h; p.sdv_t = a.sdv.t;
   p.H = a.H; p.T = a.T; p.hd = hd; p.scale = a.scale; p.bias_mode = a.bias_mode; p.slopes = a.slopes;
   p.debug = g_attn_debug.load();
+  p.status = dev_status_address();
+  if (!p.status) return fail(TFB_ERR_LAUNCH, "attention_bwd(tcgen05): cannot find the status word");
   p.BH = a.B * a.H;
   p.group = attn_slices_per_group(a.B * a.H, a.T, HD);
   dim3 grid((unsigned)ceil_div(a.T, FB_T) * a.B * a.H);
@@ -684,7 +681,7 @@ static int bwd64_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
     if ((rc = ensure_dynamic_smem(attn_bwd_tc05_kernel<T, MODE, RAGGED>, SMEM_BYTES, done[SLOT],                   \
                                   "attention_bwd(tcgen05)")))                                                       \
       return rc;                                                                                                    \
-    if ((rc = check_registers(attn_bwd_tc05_kernel<T, MODE, RAGGED>, regs[SLOT]))) return rc;                                    \
+    if ((rc = check_launch_registers(attn_bwd_tc05_kernel<T, MODE, RAGGED>, FB_REGS, regs[SLOT], "attention_bwd(tcgen05)"))) return rc; \
     launch_overlapped(attn_bwd_tc05_kernel<T, MODE, RAGGED>, grid, dim3(FB_THREADS), SMEM_BYTES, st, tq, tk, \
                       tv, tdo, tdq, p);                                                                             \
   }

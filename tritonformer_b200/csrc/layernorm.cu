@@ -251,16 +251,6 @@ __global__ void __launch_bounds__(MAXT) ln_bwd_kernel(
 // 10.2 -> 7.7, 512 x 256 8.0 -> 4.2, 4096 x 2048 25.9 -> 23.0, 32768 x 1024 58.3 -> 50.6 (5.3 TB/s).
 constexpr int LN_WARPS = 12;  // of a CTA, at most
 constexpr int ln_groups(int g) { return LN_WARPS / g; }
-__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 template <typename T>
 __device__ __forceinline__ void unpack8_pairs(const uint4& raw, uint64_t (&v)[4]) {
   float f[8];

@@ -18,6 +18,20 @@ int read_dev_status(int reset) {
   return v;
 }
 
+int* dev_status_address() {
+  static std::atomic<int*> known[64] = {};
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  int* p = known[dev].load(std::memory_order_acquire);
+  if (!p) {
+    void* at = nullptr;
+    if (cudaGetSymbolAddress(&at, g_dev_status) != cudaSuccess) return nullptr;
+    p = static_cast<int*>(at);
+    known[dev].store(p, std::memory_order_release);
+  }
+  return p;
+}
+
 constexpr int kProbeCode = 0x7e00;
 
 // One CTA, one warp: takes 32 columns of tensor memory like a real kernel would, then waits on an

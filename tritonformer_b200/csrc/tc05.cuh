@@ -11,8 +11,21 @@ namespace tfb {
 // Sticky status word of the library, one per GPU (defined in status.cu): 0 = fine, otherwise the code
 // of the first wait that gave up or of the first bad token id.  Every tcgen05 kernel returns at once
 // while it is non-zero; read_dev_status() fetches (and optionally clears) it for the current device.
+// A kernel that shares its registers out between warpgroups (setmaxnreg) cannot be built as relocatable code, which is what
+// refers to a variable of another file: such a file defines TFB_STATUS_FROM_LAUNCH, its kernels get the word's
+// address as a parameter and put it into *status_slot() before the first wait.
+#ifndef TFB_STATUS_FROM_LAUNCH
 extern __device__ int g_dev_status;
+__device__ __forceinline__ int* dev_status() { return &g_dev_status; }
+#else
+__device__ __forceinline__ int** status_slot() {
+  __shared__ int* slot;
+  return &slot;
+}
+__device__ __forceinline__ int* dev_status() { return *status_slot(); }
+#endif
 int read_dev_status(int reset);
+int* dev_status_address();  // on the current device; null if that fails
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -78,7 +91,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int co
     if (global_ns() - t0 > limit_ns) break;
   }
   *abort_flag = 1;
-  atomicCAS(&g_dev_status, 0, code);
+  atomicCAS(dev_status(), 0, code);
   return false;
 }
 
@@ -292,6 +305,24 @@ __device__ __forceinline__ bool elect_one() {
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(pred));
   return pred != 0;
+}
+
+// ---- registers of a warpgroup (all four warps execute these): what some hand back, others may take.  The sum over the block
+// must not exceed the registers that it was launched with, or a group waits for ever.
+template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// Host side of the same: a build of the kernel with another number of registers than the split was worked out for is not
+// launched.  Asked for once per kernel (`seen`).
+template <typename F>
+inline int check_launch_registers(F func, int regs, std::atomic<int>& seen, const char* what) {
+  if (seen.load(std::memory_order_relaxed) == regs) return TFB_OK;
+  cudaFuncAttributes attr;
+  const cudaError_t e = cudaFuncGetAttributes(&attr, func);
+  if (e != cudaSuccess) return fail(TFB_ERR_LAUNCH, "%s: function attributes: %s", what, cudaGetErrorString(e));
+  if (attr.numRegs != regs) return fail(TFB_ERR_LAUNCH, "%s: built with %d registers a thread instead of %d", what, attr.numRegs, regs);
+  seen.store(regs, std::memory_order_relaxed);
+  return TFB_OK;
 }
 
 // ---- host: tensor maps ------------------------------------------------------------------
