@@ -70,10 +70,6 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -155,8 +151,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
   }
   tc_fence_before();
   __syncthreads();
-  // the peer's barriers and tensor memory are ready before anything is signalled across the pair
-  cluster_sync_all();
+  // The peer's barriers and tensor memory are ready before anything is signalled across the pair.  (The barriers'
+  // initialisation has a fence of its own: the arrival orders nothing else, and costs 1 k cycles less that way.)
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   // set-up above is local to the pair and may overlap the previous kernel's tail; global memory comes after

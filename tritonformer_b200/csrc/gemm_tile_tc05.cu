@@ -13,6 +13,9 @@
 //     distributed shared memory: each sums and finishes its share of the tile's columns, in rank order (the sum does not
 //     depend on timing).  Through a workspace in global memory with arrival counters the same exchange took 4-5 us;
 //   - short rolled code everywhere (see gemm_epi.cuh).
+// Back to back, L2 hot, fp16, with the cluster's first barrier in its release form and the exchange of a split eight columns and one
+// latency at a time, and now: M 2048 N 768 K 768 6.8 and 6.2 us (with addend 7.4, 6.9), M 2048 N 768 K 3072 with addend 17.1 and 14.1, without
+// 13.0 and 12.9, M 2048 N 2304 K 768 9.6 and 9.0, M 768 N 768 K 2048 8.7 and 8.0, M 64 N 768 K 3072 (cold) 6.5 and 6.0.
 // Warps: 0 TMA producer, 1 MMA issuer (of the pair's first CTA), then the epilogue.
 #include "gemm_epi.cuh"
 #include <string.h>
@@ -143,6 +146,69 @@ __device__ __forceinline__ void finish_row8(const TileParams& p, float (&f)[8], 
   }
 }
 
+// What a split's worker finishes of one row at a time: sixteen columns.  The addend and mask vectors are requested a chunk
+// ahead (`Extra`), where the pitches allow vectors and all sixteen columns exist.
+struct Extra {
+  uint4 add[2], mask[2];
+};
+template <typename T>
+__device__ __forceinline__ bool row16_vectors(const TileParams& p, int row, int col) {
+  return !p.direct && row < p.M && col + 16 <= p.N;
+}
+template <typename T>
+__device__ __forceinline__ void request_extra(const TileParams& p, Extra& x, int row, int col) {
+  if (!row16_vectors<T>(p, row, col)) return;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (p.addend) x.add[h] = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.addend) + (int64_t)row * p.ld_addend + col + 8 * h);
+    if (p.mask) x.mask[h] = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.mask) + (int64_t)row * p.ld_mask + col + 8 * h);
+  }
+}
+template <typename T>
+__device__ __forceinline__ void finish_row16(const TileParams& p, float (&f)[16], const Extra& x, int row, int col) {
+  if (!row16_vectors<T>(p, row, col)) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float g[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] = f[8 * h + j];
+      finish_row8<T>(p, g, row, col + 8 * h);
+    }
+    return;
+  }
+  const T* bias = reinterpret_cast<const T*>(p.bias);
+  uint4* c = reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.C) + (int64_t)row * p.ldc + col);
+  uint4 out[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float g[8], t[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) g[j] = f[8 * h + j];
+    if (bias) {
+      unpack8<T>(__ldg(reinterpret_cast<const uint4*>(bias + col) + h), t);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] += t[j];
+    }
+    if (p.relu) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] = fmaxf(g[j], 0.f);
+    }
+    if (p.addend) {
+      unpack8<T>(x.add[h], t);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] += t[j];
+    }
+    if (p.mask) {
+      unpack8<T>(x.mask[h], t);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] = t[j] > 0.f ? g[j] : 0.f;
+    }
+    out[h] = pack8<T>(g);
+  }
+  c[0] = out[0];
+  c[1] = out[1];
+}
+
 template <typename T, int BN, bool PAIR, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
     gemm_tile_tc05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -204,8 +270,12 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
   }
   tc_fence_before();
   __syncthreads();
-  // every CTA of the cluster runs, with its barriers and tensor memory ready, before another one signals or writes to it
-  if (PAIR || p.split > 1) gt_cluster_sync();
+  // Every CTA of the cluster runs, with its barriers and tensor memory ready, before another one signals or writes to it.
+  // (The barriers' initialisation has a fence of its own: the arrival orders nothing else.)
+  if (PAIR || p.split > 1) {
+    gt_cluster_arrive_relaxed();
+    gt_cluster_wait();
+  }
   tc_fence_after();
   const uint32_t tmem_base = tmem_holder;
   // everything above touches only this cluster's shared memory, tensor memory and kernel parameters (and the L2)
@@ -315,21 +385,33 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
       }
       if (lane == 0) tma_store_wait_read();  // the boxes have been read; the kernel's end completes the writes
     } else {
-      bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
-      tc_fence_after();
       // Column slice r of the tile goes to worker r (the CTA of the same side): [source][group of 4 columns][row], so that the
       // 32 lanes of a warp write 512 contiguous bytes.  Sources are numbered without the receiver itself.  The columns of a
       // slice are shared by the HALVES warps of a lane quarter.
+      // What this costs is latencies, so columns move 16 at a time (32 in the exchange) with the next chunk's addend on its way.
       const int slice = BN / p.split, lo = half * (slice / HALVES), hi = lo + slice / HALVES;
-      const int trow = q * 32 + lane;
+      const int trow = q * 32 + lane, row = row0 + lane, first = n0 + part * slice;
+      Extra ex;
+      if (!dead && hi - lo >= 16) request_extra<T>(p, ex, row, first + lo);
+      bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
+      tc_fence_after();
       if (ok) {
 #pragma unroll 1
         for (int i = 1; i < p.split; ++i) {
           const int to = (part + i) % p.split;
           const int slot = part < to ? part : part - 1;
           const uint32_t dst = gt_map(smem_u32(recv + slot * (slice / 4) * GT_M + trow), (uint32_t)(to * WIDTH + side));
+          int c = lo;
 #pragma unroll 1
-          for (int c = lo; c < hi; c += 8) {
+          for (; c + 32 <= hi; c += 32) {
+            uint32_t v[32];
+            tmem_ld32(taddr + to * slice + c, v);
+            tc_wait_ld();
+#pragma unroll
+            for (int e = 0; e < 8; ++e) gt_store_remote(dst + (c / 4 + e) * GT_M * 16, v + 4 * e);
+          }
+#pragma unroll 1
+          for (; c < hi; c += 8) {
             uint32_t v[8];
             tmem_ld8(taddr + to * slice + c, v);
             tc_wait_ld();
@@ -341,8 +423,35 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
       __syncwarp();
       gt_cluster_sync();
       if (ok && !dead && *abort_flag == 0) {
+        int c = lo;
 #pragma unroll 1
-        for (int c = lo; c < hi; c += 8) {
+        for (; c + 16 <= hi; c += 16) {
+          uint32_t own[16];
+          tmem_ld16(taddr + part * slice + c, own);
+          const Extra now = ex;
+          if (c + 32 <= hi) request_extra<T>(p, ex, row, first + c + 16);
+          float f[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) f[j] = 0.f;
+          tc_wait_ld();
+#pragma unroll 1
+          for (int r = 0; r < p.split; ++r) {  // in rank order
+            if (r == part) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) f[j] += __uint_as_float(own[j]);
+            } else {
+              const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + c / 4) * GT_M + trow;
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float4 v = src[e * GT_M];
+                f[4 * e] += v.x; f[4 * e + 1] += v.y; f[4 * e + 2] += v.z; f[4 * e + 3] += v.w;
+              }
+            }
+          }
+          finish_row16<T>(p, f, now, row, first + c);
+        }
+#pragma unroll 1
+        for (; c < hi; c += 8) {
           uint32_t own[8];
           tmem_ld8(taddr + part * slice + c, own);
           tc_wait_ld();
@@ -363,7 +472,7 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
             f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
             f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
           }
-          finish_row8<T>(p, f, row0 + lane, n0 + part * slice + c);
+          finish_row8<T>(p, f, row, first + c);
         }
       }
     }
