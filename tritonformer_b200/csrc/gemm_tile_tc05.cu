@@ -11,7 +11,8 @@
 //     the operand bytes per flop at 256 x 256);
 //   - the contraction is cut over the workers of a cluster (1, 2, 4 or 8), which exchange fp32 partial tiles through
 //     distributed shared memory: each sums and finishes its share of the tile's columns, in rank order (the sum does not
-//     depend on timing).  Through a workspace in global memory with arrival counters the same exchange took 4-5 us;
+//     depend on timing), a row per thread (through staging in the ring, so that a warp's stores are consecutive, was slower:
+//     M 2048 N 768 K 3072 13.7 against 12.9 us).  Through a workspace in global memory with arrival counters the same exchange took 4-5 us;
 //   - short rolled code everywhere (see gemm_epi.cuh).
 // Back to back, L2 hot, fp16, with the cluster's first barrier in its release form and the exchange of a split eight columns and one
 // latency at a time, and now: M 2048 N 768 K 768 6.8 and 6.2 us (with addend 7.4, 6.9), M 2048 N 768 K 3072 with addend 17.1 and 14.1, without
@@ -235,7 +236,9 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
   const int kblocks = (p.K + GT_K - 1) / GT_K;
   const int kb0 = kblocks * part / p.split, kb1 = kblocks * (part + 1) / p.split;
 
-  if (threadIdx.x == 0) {
+  // the three parts of the set-up run on warps of their own (on two of them, one part after the other: M 2048 N 768
+  // K 3072 12.9, now 12.5 us, M 768 N 3072 K 2048 11.9 and 11.7, M 768 N 768 K 2048 8.0 and 7.8)
+  if (warp == 2 && lane == 0) {
     for (int i = 0; i < p.stages; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
@@ -245,7 +248,7 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
     abort_word = 0;
     mbar_fence_init();
   }
-  if (warp == 0 && lane == 0) {
+  if (warp == 3 && lane == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
 #pragma unroll 1
