@@ -78,6 +78,37 @@ def test_grad_rows_at_the_edges_of_a_warps_columns(rows, cols):
         test_grad_rows(rows, cols, torch.float16, offset)
 
 
+@pytest.mark.parametrize("rows,cols", [(9472, 9), (9480, 247), (9472, 248), (9473, 249), (4736, 495), (4749, 496), (4737, 497), (1200, 2049)])
+def test_grad_rows_with_several_rows_a_warp(rows, cols):
+    """From two misaligned rows per warp on: the kernel whose lanes take the misaligned halves from their neighbours."""
+    for offset in range(8):
+        test_grad_rows(rows, cols, torch.float16, offset)
+    test_grad_rows(rows, cols, torch.bfloat16, 3)
+
+
+@pytest.mark.parametrize("rows,cols,pitch,offset,shifted", [
+    (9472, 249, 249, 0, True), (9472, 249, 256, 0, False), (9472, 249, 256, 1, True), (9472, 256, 256, 0, False),
+    (4735, 249, 249, 0, False), (64, 65, 65, 0, False)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_only_misaligned_rows_are_shifted(rows, cols, pitch, offset, shifted, masked):
+    """Aligned rows, and misaligned ones of which a warp has less than two, keep the kernel that loads them as they lie."""
+    from torch.profiler import ProfilerActivity, profile
+    from tritonformer_b200 import _lib as L
+    src = torch.randn(rows * pitch + 8, device="cuda").half()[offset:]
+    dz = torch.empty(rows, -(-cols // 8) * 8, device="cuda", dtype=torch.half)
+    call = (src.data_ptr(), src.data_ptr() if masked else None, dz.data_ptr(), None, None, 0, rows, cols, pitch, pitch, dz.shape[1],
+            L.dtype_code(torch.half), L.stream_ptr(dz.device))
+    L.check(L.lib.tfb_grad_rows(*call))
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        L.check(L.lib.tfb_grad_rows(*call))
+        torch.cuda.synchronize()
+    names = [e.key for e in p.key_averages() if "grad_rows" in e.key]
+    assert len(names) == 1 and ("grad_rows_kernel<__half>" in names[0]) != shifted, names
+    want = src[:rows * pitch].view(rows, pitch)[:, :cols]
+    assert torch.equal(dz[:, :cols], want.clamp_min(0.0) if masked else want)
+
+
 @pytest.mark.parametrize("cols", [1, 7, 9, 2047, 2049, 50257])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_lm_loss_of_an_odd_vocabulary(cols, dtype):

@@ -77,14 +77,75 @@ __global__ void __launch_bounds__(256) colsum_kernel(const T* __restrict__ x, fl
 // dz = act > 0 ? dy : 0 (act may be null: a copy) with the column sums of dz on the way: what the backward of a linear
 // layer needs before its two products, in one pass over dy and act.  dy and act may have any alignment and pitch; dz has
 // 16-byte aligned rows, so that the products can read it through TMA whatever the layer's width (a copy with act and
-// sums null packs an operand the same way).
+// sums null packs an operand the same way).  The work of a CTA is the one of colsum_kernel, four rows of a thread in
+// flight; each lane fetches what its eight elements lie in, one aligned vector or two.  Both kernels add the rows of a column in the same
+// order.
+constexpr int GR_ROWS = 4, GR_COLS = 248;
+template <typename T>
+__global__ void __launch_bounds__(256) grad_rows_kernel(const T* __restrict__ dy, const T* __restrict__ act,
+                                                        T* __restrict__ dz, float* __restrict__ partials, int64_t rows,
+                                                        int cols, int64_t dy_ld, int64_t act_ld, int64_t dz_ld) {
+  grid_dependency_wait();
+  allow_dependents();
+  __shared__ float sm[8][32][9];
+  const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5;
+  const int c0 = (blockIdx.x * 32 + cl) * 8;
+  const int n = min(8, cols - c0);
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+  if (n > 0) {
+    const int64_t step = (int64_t)gridDim.y * 8;
+    for (int64_t r0 = (int64_t)blockIdx.y * 8 + rl; r0 < rows; r0 += step * GR_ROWS) {
+      uint4 g[GR_ROWS], a[GR_ROWS];
+#pragma unroll
+      for (int i = 0; i < GR_ROWS; ++i) {
+        const int64_t r = r0 + i * step;
+        if (r >= rows) continue;
+        g[i] = load8_any(dy + r * dy_ld + c0, n);
+        if (act) a[i] = load8_any(act + r * act_ld + c0, n);
+      }
+#pragma unroll
+      for (int i = 0; i < GR_ROWS; ++i) {
+        const int64_t r = r0 + i * step;
+        if (r >= rows) continue;
+        float f[8];
+        unpack8<T>(g[i], f);
+        if (act) {
+          float m[8];
+          unpack8<T>(a[i], m);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] = m[j] > 0.f ? f[j] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (j >= n) f[j] = 0.f;  // the padding of a row
+          acc[j] += f[j];
+        }
+        *reinterpret_cast<uint4*>(dz + r * dz_ld + c0) = pack8<T>(f);
+      }
+    }
+  }
+  if (!partials) return;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sm[rl][cl][j] = acc[j];
+  __syncthreads();
+  const int cc = threadIdx.x, col = blockIdx.x * 256 + cc;
+  if (col < cols) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += sm[i][cc >> 3][cc & 7];
+    partials[(int64_t)blockIdx.y * cols + col] = s;
+  }
+}
+
+// The same for misaligned rows, several of them per warp.
 // A warp takes 31 output vectors (248 columns) of a row.  All lanes of a row share one misalignment: lane l loads the aligned
 // vector that the l-th output begins in, and the rest of that output is in its neighbour's, so a row is loaded once.  Bound by
 // the loads: a thread requests its vectors of GR_ROWS rows before it uses the first.  (Each lane fetching both of its aligned vectors
 // itself made every row two dependent loads deep per lane.)  Cold L2, fp16: 5015 x 2930 with mask and sums and their fold
 // 39.6 -> 25.6 us (3.4 TB/s of dy, act and dz), a copy of 5015 x 1477 12.0 -> 8.7, of 1477 x 2930 7.4 -> 5.9, of 1024 x 50257
 // 57.5 -> 43.1 (4.8 TB/s).
-constexpr int GR_ROWS = 4, GR_COLS = 248;
 // Loads that vector.  One that holds no wanted byte is not touched; one that does never crosses the end of an allocation.
 template <typename T>
 __device__ __forceinline__ uint4 load_row_vec(const T* row, int c0, int cols) {
@@ -108,9 +169,10 @@ __device__ __forceinline__ uint4 shift_row_vec(const uint4& v, uint32_t off) {
                     __funnelshift_r(w[3], w[4], bits));
 }
 template <typename T, bool ACT>
-__global__ void __launch_bounds__(256, ACT ? 3 : 4) grad_rows_kernel(const T* __restrict__ dy, const T* __restrict__ act,
-                                                           T* __restrict__ dz, float* __restrict__ partials, int64_t rows,
-                                                           int cols, int64_t dy_ld, int64_t act_ld, int64_t dz_ld) {
+__global__ void __launch_bounds__(256, ACT ? 3 : 4) grad_rows_shift_kernel(const T* __restrict__ dy, const T* __restrict__ act,
+                                                                                 T* __restrict__ dz, float* __restrict__ partials,
+                                                                                 int64_t rows, int cols, int64_t dy_ld, int64_t act_ld,
+                                                                                 int64_t dz_ld) {
   grid_dependency_wait();
   allow_dependents();
   __shared__ float sm[8][32][9];
@@ -177,16 +239,28 @@ extern "C" int tfb_grad_rows(const void* dy, const void* act, void* dz, void* su
               "grad_rows: scratch must hold tfb_colsum_partials() rows");
   if (rows == 0 && !sums) return TFB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const dim3 grid((unsigned)ceil_div(cols, GR_COLS), (unsigned)tfb_colsum_partials(rows, cols));
+  // Rows that begin on 16-byte boundaries (the ordinary widths) need no shifting, and 248 columns a CTA would leave a width like 256 a
+  // second block of CTAs with one lane at work; with less than two rows a warp the shifting has nothing to overlap with.  Warm L2, fp16,
+  // plain kernel and shifting one: 8192 x 1024 with mask 6.8 and 11.9 us, 1920 x 256 1.7 and 2.9, 5015 x 2928 13.7 and 19.9;
+  // misaligned, 1 row a warp: 475 x 1346 2.2 and 2.45, 2048 x 498 3.1 and 3.8; 1.5 rows: 7168 x 250 3.6 and 6.0; from 2 rows on they are within
+  // 5 % (10000 x 130 4.4 and 4.5, 2000 x 1111 4.5 and 4.6) or the shifting one is ahead (60000 x 205 22.7 and 17.0), and with a cold L2
+  // it is by 9-78 % (2000 x 1111 7.6 and 6.0, 1000 x 3999 10.9 and 8.4).
+  const int64_t slices = tfb_colsum_partials(rows, cols);
+  const bool whole = aligned16(dy) && dy_ld % 8 == 0 && (!act || (aligned16(act) && act_ld % 8 == 0));
+  const bool shift = !whole && rows >= 16 * slices;  // eight warps share a slice's rows
+  const dim3 grid((unsigned)ceil_div(cols, shift ? GR_COLS : 256), (unsigned)slices);
+#define TFB_GRAD_ROWS(...)                                                                                        \
+  launch_overlapped(__VA_ARGS__, grid, dim3(256), 0, st, (const T*)dy, (const T*)act, (T*)dz, sums ? partials : nullptr, rows, \
+                    (int)cols, dy_ld, act_ld, dz_ld)
   TFB_DISPATCH_16(dtype, T, {
-    if (act) launch_overlapped(grad_rows_kernel<T, true>, grid, dim3(256), 0, st, (const T*)dy, (const T*)act, (T*)dz, sums ? partials : nullptr,
-                               rows, (int)cols, dy_ld, act_ld, dz_ld);
-    else launch_overlapped(grad_rows_kernel<T, false>, grid, dim3(256), 0, st, (const T*)dy, (const T*)act, (T*)dz, sums ? partials : nullptr,
-                           rows, (int)cols, dy_ld, act_ld, dz_ld);
+    if (!shift) TFB_GRAD_ROWS(grad_rows_kernel<T>);
+    else if (act) TFB_GRAD_ROWS((grad_rows_shift_kernel<T, true>));
+    else TFB_GRAD_ROWS((grad_rows_shift_kernel<T, false>));
     const int rc = launched("grad_rows");
     if (rc || !sums) return rc;
     return finalize_partials<T>(partials, n_partials, (int)cols, (int)cols, sums, nullptr, st, 0);
   })
+#undef TFB_GRAD_ROWS
 }
 
 extern "C" int tfb_relu_bwd(const void* dy, const void* act, void* dz, int64_t n, int dtype,
