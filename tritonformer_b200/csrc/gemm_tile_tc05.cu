@@ -391,91 +391,136 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
       // Column slice r of the tile goes to worker r (the CTA of the same side): [source][group of 4 columns][row], so that the
       // 32 lanes of a warp write 512 contiguous bytes.  Sources are numbered without the receiver itself.  The columns of a
       // slice are shared by the HALVES warps of a lane quarter.
-      // What this costs is latencies, so columns move 16 at a time (32 in the exchange) with the next chunk's addend on its way.
       const int slice = BN / p.split, lo = half * (slice / HALVES), hi = lo + slice / HALVES;
       const int trow = q * 32 + lane, row = row0 + lane, first = n0 + part * slice;
-      Extra ex;
-      if (!dead && hi - lo >= 16) request_extra<T>(p, ex, row, first + lo);
-      bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
-      tc_fence_after();
-      if (ok) {
+      if (hi - lo < 16) {
+        // Eight columns a warp (64 columns cut eight ways).  As the rest of the wide form's loops, with the other instructions of
+        // these in between, M 128 N 704 K 832 took 4.95 us and M 448 N 64 K 1024 4.68; so 4.44 and 4.12.
+        bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
+        tc_fence_after();
+        if (ok) {
 #pragma unroll 1
-        for (int i = 1; i < p.split; ++i) {
-          const int to = (part + i) % p.split;
-          const int slot = part < to ? part : part - 1;
-          const uint32_t dst = gt_map(smem_u32(recv + slot * (slice / 4) * GT_M + trow), (uint32_t)(to * WIDTH + side));
-          int c = lo;
-#pragma unroll 1
-          for (; c + 32 <= hi; c += 32) {
-            uint32_t v[32];
-            tmem_ld32(taddr + to * slice + c, v);
-            tc_wait_ld();
-#pragma unroll
-            for (int e = 0; e < 8; ++e) gt_store_remote(dst + (c / 4 + e) * GT_M * 16, v + 4 * e);
-          }
-#pragma unroll 1
-          for (; c < hi; c += 8) {
+          for (int i = 1; i < p.split; ++i) {
+            const int to = (part + i) % p.split;
+            const int slot = part < to ? part : part - 1;
+            const uint32_t dst = gt_map(smem_u32(recv + (slot * (slice / 4) + lo / 4) * GT_M + trow), (uint32_t)(to * WIDTH + side));
             uint32_t v[8];
-            tmem_ld8(taddr + to * slice + c, v);
+            tmem_ld8(taddr + to * slice + lo, v);
             tc_wait_ld();
-            gt_store_remote(dst + (c / 4) * GT_M * 16, v);
-            gt_store_remote(dst + (c / 4 + 1) * GT_M * 16, v + 4);
+            gt_store_remote(dst, v);
+            gt_store_remote(dst + GT_M * 16, v + 4);
           }
         }
-      }
-      __syncwarp();
-      gt_cluster_sync();
-      if (ok && !dead && *abort_flag == 0) {
-        int c = lo;
-#pragma unroll 1
-        for (; c + 16 <= hi; c += 16) {
-          uint32_t own[16];
-          tmem_ld16(taddr + part * slice + c, own);
-          const Extra now = ex;
-          if (c + 32 <= hi) request_extra<T>(p, ex, row, first + c + 16);
-          float f[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) f[j] = 0.f;
-          tc_wait_ld();
-#pragma unroll 1
-          for (int r = 0; r < p.split; ++r) {  // in rank order
-            if (r == part) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) f[j] += __uint_as_float(own[j]);
-            } else {
-              const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + c / 4) * GT_M + trow;
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float4 v = src[e * GT_M];
-                f[4 * e] += v.x; f[4 * e + 1] += v.y; f[4 * e + 2] += v.z; f[4 * e + 3] += v.w;
-              }
-            }
-          }
-          finish_row16<T>(p, f, now, row, first + c);
-        }
-#pragma unroll 1
-        for (; c < hi; c += 8) {
+        __syncwarp();
+        gt_cluster_sync();
+        if (ok && !dead && *abort_flag == 0) {
           uint32_t own[8];
-          tmem_ld8(taddr + part * slice + c, own);
+          tmem_ld8(taddr + part * slice + lo, own);
           tc_wait_ld();
           float f[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) f[j] = 0.f;
 #pragma unroll 1
-          for (int r = 0; r < p.split; ++r) {
+          for (int r = 0; r < p.split; ++r) {  // in rank order
             float4 a, b;
             if (r == part) {
               a = make_float4(__uint_as_float(own[0]), __uint_as_float(own[1]), __uint_as_float(own[2]), __uint_as_float(own[3]));
               b = make_float4(__uint_as_float(own[4]), __uint_as_float(own[5]), __uint_as_float(own[6]), __uint_as_float(own[7]));
             } else {
-              const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + c / 4) * GT_M + trow;
+              const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + lo / 4) * GT_M + trow;
               a = src[0];
               b = src[GT_M];
             }
             f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
             f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
           }
-          finish_row8<T>(p, f, row, first + c);
+          finish_row8<T>(p, f, row, first + lo);
+        }
+      } else {
+        // What this costs is latencies, so columns move 16 at a time (32 in the exchange) with the next chunk's addend on its way.
+        Extra ex;
+        if (!dead) request_extra<T>(p, ex, row, first + lo);
+        bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
+        tc_fence_after();
+        if (ok) {
+#pragma unroll 1
+          for (int i = 1; i < p.split; ++i) {
+            const int to = (part + i) % p.split;
+            const int slot = part < to ? part : part - 1;
+            const uint32_t dst = gt_map(smem_u32(recv + slot * (slice / 4) * GT_M + trow), (uint32_t)(to * WIDTH + side));
+            int c = lo;
+#pragma unroll 1
+            for (; c + 32 <= hi; c += 32) {
+              uint32_t v[32];
+              tmem_ld32(taddr + to * slice + c, v);
+              tc_wait_ld();
+#pragma unroll
+              for (int e = 0; e < 8; ++e) gt_store_remote(dst + (c / 4 + e) * GT_M * 16, v + 4 * e);
+            }
+#pragma unroll 1
+            for (; c < hi; c += 8) {
+              uint32_t v[8];
+              tmem_ld8(taddr + to * slice + c, v);
+              tc_wait_ld();
+              gt_store_remote(dst + (c / 4) * GT_M * 16, v);
+              gt_store_remote(dst + (c / 4 + 1) * GT_M * 16, v + 4);
+            }
+          }
+        }
+        __syncwarp();
+        gt_cluster_sync();
+        if (ok && !dead && *abort_flag == 0) {
+          int c = lo;
+#pragma unroll 1
+          for (; c + 16 <= hi; c += 16) {
+            uint32_t own[16];
+            tmem_ld16(taddr + part * slice + c, own);
+            const Extra now = ex;
+            if (c + 32 <= hi) request_extra<T>(p, ex, row, first + c + 16);
+            float f[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) f[j] = 0.f;
+            tc_wait_ld();
+#pragma unroll 1
+            for (int r = 0; r < p.split; ++r) {  // in rank order
+              if (r == part) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) f[j] += __uint_as_float(own[j]);
+              } else {
+                const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + c / 4) * GT_M + trow;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float4 v = src[e * GT_M];
+                  f[4 * e] += v.x; f[4 * e + 1] += v.y; f[4 * e + 2] += v.z; f[4 * e + 3] += v.w;
+                }
+              }
+            }
+            finish_row16<T>(p, f, now, row, first + c);
+          }
+#pragma unroll 1
+          for (; c < hi; c += 8) {
+            uint32_t own[8];
+            tmem_ld8(taddr + part * slice + c, own);
+            tc_wait_ld();
+            float f[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] = 0.f;
+#pragma unroll 1
+            for (int r = 0; r < p.split; ++r) {
+              float4 a, b;
+              if (r == part) {
+                a = make_float4(__uint_as_float(own[0]), __uint_as_float(own[1]), __uint_as_float(own[2]), __uint_as_float(own[3]));
+                b = make_float4(__uint_as_float(own[4]), __uint_as_float(own[5]), __uint_as_float(own[6]), __uint_as_float(own[7]));
+              } else {
+                const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + c / 4) * GT_M + trow;
+                a = src[0];
+                b = src[GT_M];
+              }
+              f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+              f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+            }
+            finish_row8<T>(p, f, row, first + c);
+          }
         }
       }
     }
