@@ -600,7 +600,8 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
 }
 
 // dq = round(scale * dq_acc), written with the caller's strides.  Bound by memory; one slice per grid row, vectors of eight
-// columns, 1 << vshift of them per row (no 64-bit divisions to find a vector's row; figures at attn_delta_kernel).
+// columns, 1 << vshift of them per row (no 64-bit divisions to find a vector's row).  Backward before and with this and the delta pass
+// of that time: B4 H16 T2048 hd64 fp16 191.5 -> 189.6 us, B3 H11 T1472 hd64 bf16 69.0 -> 67.0, B1 H12 T4096 hd128 226.5 -> 222.7.
 constexpr int DQ_VECS = 2;  // of a thread
 template <typename T>
 __global__ void __launch_bounds__(256) attn_dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq,

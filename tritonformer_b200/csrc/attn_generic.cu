@@ -223,50 +223,37 @@ __global__ void __launch_bounds__(AT_THREADS) attn_fwd_kernel(const AttnArgs a) 
 
 // delta[b,h,i] = sum_d dO[i,d] * O[i,d]; hd/8 lanes per row, one 16-byte load of each operand per lane.
 // `clear` (may be null): contiguous fp32 (B,H,T,HD) buffer; each lane zeroes the eight floats under its chunk.
-// Bound by memory: DELTA_ROWS rows of a thread in flight, one slice per grid row, no 64-bit divisions (four of them per
-// thread before).  Backward with this and the conversion's new form: B4 H16 T2048 hd64 fp16 191.5 -> 189.6 us, B3 H11 T1472 hd64 bf16
-// 69.0 -> 67.0, B1 H12 T4096 hd128 226.5 -> 222.7.
-constexpr int DELTA_ROWS = 2;
+// Bound by memory and by latency; 32-bit divisions, one per block and one for its slice (four 64-bit ones per thread before).  One row
+// of a thread, and blocks that follow each other in different slices: with two rows in flight and a slice's blocks in a row the pass
+// alone was as fast, but not behind a forward that fills the SMs, beside whose blocks the first ones of this pass wait (forward and backward
+// one after the other, with 64-bit divisions, two rows and this form: B3 H14 T320 hd64 29.9, 31.2, 29.2 us, B7 H27 T128 hd32 29.4, 30.2, 28.1,
+// B1 H18 T832 hd64 42.7, 43.2, 41.1; over 110 shapes of T 64 to 4096 the worst is 1.025 times the first, and was 0.96).
 template <typename T, int HD>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const AttnArgs a, float* __restrict__ clear) {
   grid_dependency_wait();
   allow_dependents();
   constexpr int LPR = HD / 8;          // lanes per row
-  constexpr int RPB = 256 / LPR;       // rows of a block at a time
-  const int sub = threadIdx.x % LPR, r0 = blockIdx.x * (RPB * DELTA_ROWS) + threadIdx.x / LPR;
-  const int bh = blockIdx.y, b = bh / a.H, h = bh % a.H;
-  const T* op = (const T*)a.o + b * a.so.b + h * a.so.h + sub * 8;
-  const T* gp = (const T*)a.d_o + b * a.sdo.b + h * a.sdo.h + sub * 8;
-  uint4 x[DELTA_ROWS], y[DELTA_ROWS];
+  constexpr int RPB = 256 / LPR;       // rows of a block
+  const uint32_t slices = a.B * a.H, part = blockIdx.x / slices;
+  const int bh = blockIdx.x - part * slices, b = bh / a.H, h = bh % a.H;
+  const int sub = threadIdx.x % LPR, i = part * RPB + threadIdx.x / LPR;
+  const int64_t row = (int64_t)bh * a.T + i;
+  float s = 0.f;
+  if (i < a.T) {
+    float x[8], y[8];
+    unpack8<T>(ld_stream16((const T*)a.o + b * a.so.b + h * a.so.h + i * a.so.t + sub * 8), x);
+    unpack8<T>(ld_stream16((const T*)a.d_o + b * a.sdo.b + h * a.sdo.h + i * a.sdo.t + sub * 8), y);
 #pragma unroll
-  for (int u = 0; u < DELTA_ROWS; ++u) {
-    const int i = r0 + u * RPB;
-    if (i < a.T) {
-      x[u] = ld_stream16(op + i * a.so.t);
-      y[u] = ld_stream16(gp + i * a.sdo.t);
+    for (int j = 0; j < 8; ++j) s += x[j] * y[j];
+    if (clear) {
+      float4* z = reinterpret_cast<float4*>(clear + row * HD + sub * 8);
+      z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+      z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
 #pragma unroll
-  for (int u = 0; u < DELTA_ROWS; ++u) {
-    const int i = r0 + u * RPB;
-    const int64_t row = (int64_t)bh * a.T + i;
-    float s = 0.f;
-    if (i < a.T) {
-      float p[8], q[8];
-      unpack8<T>(x[u], p);
-      unpack8<T>(y[u], q);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s += p[j] * q[j];
-      if (clear) {
-        float4* z = reinterpret_cast<float4*>(clear + row * HD + sub * 8);
-        z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-        z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-#pragma unroll
-    for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (i < a.T && sub == 0) a.delta[row] = s;
-  }
+  for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (i < a.T && sub == 0) a.delta[row] = s;
 }
 
 // --------------------------------------------------------------------------- backward: dK, dV
@@ -556,7 +543,7 @@ static int bwd_launch(const AttnArgs& a, cudaStream_t st) {
 }
 
 int attn_delta(const AttnArgs& a, int hd, int dtype, cudaStream_t st, float* clear) {
-  const dim3 grid((unsigned)ceil_div(a.T, 256 / (hd / 8) * DELTA_ROWS), (unsigned)(a.B * a.H));
+  const dim3 grid((unsigned)(ceil_div(a.T, 256 / (hd / 8)) * a.B * a.H));
   TFB_DISPATCH_16(dtype, T, {
     if (hd == 32) launch_overlapped(attn_delta_kernel<T, 32>, grid, dim3(256), 0, st, a, clear);
     else if (hd == 64) launch_overlapped(attn_delta_kernel<T, 64>, grid, dim3(256), 0, st, a, clear);
