@@ -20,7 +20,9 @@ extern "C" {
  *          no persistent CTA-pair kernel, bit 7 (128) no one-wave kernel, bits 16-27 the one plan the one-wave kernel
  *          may use (tfb_debug_gemm_plan).
  *   key 6: how many SMs the persistent GEMM grids leave free (for a collective that runs beside
- *          them on another stream); 0 by default.                                */
+ *          them on another stream); 0 by default.
+ *   key 7: the registers a thread that the attention backward's kernels are taken to have been built with; 0: what they
+ *          have.  Where the number does not cover a kernel's split of its registers, the mma.sync kernels take the call.  */
 void tfb_debug_set(int key, int value);
 /* What the one-wave GEMM kernel does with an M x N x K product (b_mn: B is contiguous along N) under the switches in force:
  * 0 if the product goes to the persistent kernels, else 1 + tile width / 64 * 2 + (on CTA pairs ? 1 : 0) + 16 * the number

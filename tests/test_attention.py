@@ -218,3 +218,32 @@ def test_walks_of_every_short_length(t, hd, slopes):
     for got, ref in pairs:
         err = (got.double() - ref).flatten(2).norm(dim=2) / ref.flatten(2).norm(dim=2)
         assert err.max().item() < 4 * 2.0 ** -11
+
+
+@pytest.mark.parametrize("hd,registers,path", [(64, 0, 1), (64, 80, 1), (64, 72, 0), (64, 96, 0), (32, 72, 0), (128, 0, 1),
+                                               (128, 96, 1), (128, 88, 0), (128, 120, 0)])
+@pytest.mark.parametrize("t,dtype", [(320, torch.float16), (256, torch.bfloat16)])
+def test_backward_of_a_build_with_other_registers(hd, registers, path, t, dtype):
+    """A kernel whose registers do not cover the split between its warpgroups is not launched: the mma.sync backward takes the
+    call.  Against 64 bits, per head in the 2-norm: P, dS, the saved output (in delta) and the result are each rounded."""
+    import ctypes
+    from tritonformer_b200 import _lib as L
+    from tritonformer_b200 import attention as A
+    q, k, v, dy = _make((2, 3, t, hd), dtype, True)
+    out, lse, _ = A.attention_forward(q.detach(), k.detach(), v.detach(), A._Bias())
+    grads = [torch.full_like(x, 7.0) for x in (q, k, v)]
+    n = L.lib.tfb_attention_bwd_scratch_bytes(2, 3, t, hd)
+    scratch, ran = torch.empty(n, dtype=torch.uint8, device="cuda"), ctypes.c_int(-1)
+    L.lib.tfb_debug_set(7, registers)
+    try:
+        L.check(L.lib.tfb_attention_bwd(
+            *(x.data_ptr() for x in (q, k, v, out, dy, lse, *grads)), 2, 3, t, hd, *(L.strides3(x) for x in (q, k, v, out, dy, *grads)),
+            None, 0, None, 0, 0, scratch.data_ptr(), n, L.dtype_code(dtype), L.stream_ptr(q.device), ctypes.byref(ran)))
+    finally:
+        L.lib.tfb_debug_set(7, 0)
+    assert ran.value == path
+    qd, kd, vd = (x.detach().double().requires_grad_() for x in (q, k, v))
+    s = (qd @ kd.transpose(-1, -2) / hd ** 0.5).masked_fill(torch.ones(t, t, device="cuda").triu(1) > 0, float("-inf"))
+    for got, ref in zip(grads, torch.autograd.grad(torch.softmax(s, -1) @ vd, (qd, kd, vd), dy.double())):
+        err = (got.double() - ref).flatten(2).norm(dim=2) / ref.flatten(2).norm(dim=2)
+        assert err.max().item() < 4 * (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8)

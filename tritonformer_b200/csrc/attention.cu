@@ -7,6 +7,7 @@ extern std::atomic<int> g_attn_debug;
 bool attn_tc05_fwd_eligible(const AttnArgs& a, int hd);
 int attn_fwd1_tc05(const AttnArgs& a, int hd, int dtype, cudaStream_t st);
 bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd);
+int attn_tc05_bwd_fits(const AttnArgs& a, int hd, int dtype, bool& fit);
 int attn_tc05_bwd(const AttnArgs& a, int hd, int dtype, cudaStream_t st);
 }  // namespace tfb
 
@@ -89,7 +90,8 @@ extern "C" int tfb_attention_bwd(const void* q, const void* k, const void* v, co
   a.bias_mode = slopes ? (alibi_round == 1 ? 2 : alibi_round == 2 ? 4 : 1) : (bias ? 3 : 0);
   a.slopes = slopes; a.bias = bias; a.bias_sh = bias_sh; a.bias_si = bias_si;
   a.dq_acc = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(scratch) + ((B * H * T * 4 + 255) / 256) * 256);
-  const bool fast = !g_force_fallback_attn.load() && attn_tc05_bwd_eligible(a, (int)hd);
+  bool fast = !g_force_fallback_attn.load() && attn_tc05_bwd_eligible(a, (int)hd);
+  if (fast && (rc = attn_tc05_bwd_fits(a, (int)hd, dtype, fast))) return rc;
   if (path) *path = fast ? 1 : 0;
   if (fast) return attn_tc05_bwd(a, (int)hd, dtype, (cudaStream_t)stream);
   return attn_generic_bwd(a, (int)hd, dtype, (cudaStream_t)stream);

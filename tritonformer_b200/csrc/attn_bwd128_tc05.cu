@@ -501,6 +501,24 @@ static int encode_rows(CUtensorMap* m, const void* ptr, const AttnStrides& s, co
   return encode_tmap_sw128(m, ptr, dtype, 4, dims, str, box);
 }
 
+template <typename T>
+struct Bwd128 {
+  using Kernel = decltype(&attn_bwd128_tc05_kernel<T, 0>);
+  static inline std::atomic<uint64_t> smem_done[5] = {};
+  static inline std::atomic<int> registers[5] = {};
+  static Kernel kernel(int mode) {
+    return mode == 0 ? attn_bwd128_tc05_kernel<T, 0> : mode == 1 ? attn_bwd128_tc05_kernel<T, 1>
+         : mode == 2 ? attn_bwd128_tc05_kernel<T, 2> : attn_bwd128_tc05_kernel<T, 4>;
+  }
+};
+
+int attn_bwd128_fits(const AttnArgs& a, int dtype, bool& fit) {
+  TFB_DISPATCH_16(dtype, T, {
+    return registers_fit(Bwd128<T>::kernel(a.bias_mode), REGS, REGS_COMPUTE, Bwd128<T>::registers[a.bias_mode],
+                         "attention_bwd(tcgen05)", fit);
+  })
+}
+
 // The walk over all items; the delta pass before it and the conversion of the dQ accumulator after it are the caller's.
 template <typename T>
 static int bwd128_launch(const AttnArgs& a, int dtype, cudaStream_t st) {
@@ -528,20 +546,9 @@ static int bwd128_launch(const AttnArgs& a, int dtype, cudaStream_t st) {
   p.BH = a.B * a.H;
   p.group = attn_slices_per_group(a.B * a.H, a.T, HD);
   const dim3 grid((unsigned)ceil_div(a.T, FB_K) * a.B * a.H);
-  static std::atomic<uint64_t> done[4] = {{0}, {0}, {0}, {0}};
-  static std::atomic<int> regs[4] = {{0}, {0}, {0}, {0}};
-#define FB_LAUNCH(MODE, SLOT)                                                                                               \
-  {                                                                                                                         \
-    if ((rc = ensure_dynamic_smem(attn_bwd128_tc05_kernel<T, MODE>, SMEM_BYTES, done[SLOT], "attention_bwd(tcgen05)"))) \
-      return rc;                                                                                                            \
-    if ((rc = check_launch_registers(attn_bwd128_tc05_kernel<T, MODE>, REGS, regs[SLOT], "attention_bwd(tcgen05)"))) return rc;    \
-    launch_overlapped(attn_bwd128_tc05_kernel<T, MODE>, grid, dim3(THREADS), SMEM_BYTES, st, tq, tk, tv, tdo, tdq, p); \
-  }
-  if (a.bias_mode == 0) FB_LAUNCH(0, 0)
-  else if (a.bias_mode == 1) FB_LAUNCH(1, 1)
-  else if (a.bias_mode == 2) FB_LAUNCH(2, 2)
-  else FB_LAUNCH(4, 3)
-#undef FB_LAUNCH
+  const auto kernel = Bwd128<T>::kernel(a.bias_mode);
+  if ((rc = ensure_dynamic_smem(kernel, SMEM_BYTES, Bwd128<T>::smem_done[a.bias_mode], "attention_bwd(tcgen05)"))) return rc;
+  launch_overlapped(kernel, grid, dim3(THREADS), SMEM_BYTES, st, tq, tk, tv, tdo, tdq, p);
   return launched("attention_bwd(tcgen05, head_dim 128)");
 }
 

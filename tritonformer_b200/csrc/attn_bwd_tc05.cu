@@ -648,6 +648,27 @@ bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd) {  // as in the forward
 }
 
 int attn_bwd128_tc05(const AttnArgs& a, int dtype, cudaStream_t st);
+int attn_bwd128_fits(const AttnArgs& a, int dtype, bool& fit);
+
+template <typename T, bool RAGGED>
+struct Bwd64 {
+  using Kernel = decltype(&attn_bwd_tc05_kernel<T, 0, RAGGED>);
+  static inline std::atomic<uint64_t> smem_done[5] = {};
+  static inline std::atomic<int> registers[5] = {};
+  static Kernel kernel(int mode) {
+    return mode == 0 ? attn_bwd_tc05_kernel<T, 0, RAGGED> : mode == 1 ? attn_bwd_tc05_kernel<T, 1, RAGGED>
+         : mode == 2 ? attn_bwd_tc05_kernel<T, 2, RAGGED> : attn_bwd_tc05_kernel<T, 4, RAGGED>;
+  }
+  static int fits(const AttnArgs& a, bool& fit) {
+    return registers_fit(kernel(a.bias_mode), FB_REGS, FB_REGS_COMPUTE, registers[a.bias_mode], "attention_bwd(tcgen05)", fit);
+  }
+};
+
+// Whether the kernel that would take the call has the registers that its split counts on.  If not, the mma.sync kernels take it.
+int attn_tc05_bwd_fits(const AttnArgs& a, int hd, int dtype, bool& fit) {
+  if (hd == 128) return attn_bwd128_fits(a, dtype, fit);
+  TFB_DISPATCH_16(dtype, T, { return a.T % FB_T ? Bwd64<T, true>::fits(a, fit) : Bwd64<T, false>::fits(a, fit); })
+}
 
 template <typename T, bool RAGGED>
 static int bwd64_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
@@ -675,22 +696,10 @@ static int bwd64_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   p.BH = a.B * a.H;
   p.group = attn_slices_per_group(a.B * a.H, a.T, HD);
   dim3 grid((unsigned)ceil_div(a.T, FB_T) * a.B * a.H);
-  static std::atomic<uint64_t> done[4] = {{0}, {0}, {0}, {0}};
-  static std::atomic<int> regs[4] = {{0}, {0}, {0}, {0}};
-#define FB_LAUNCH(MODE, SLOT)                                                                                       \
-  {                                                                                                                 \
-    if ((rc = ensure_dynamic_smem(attn_bwd_tc05_kernel<T, MODE, RAGGED>, SMEM_BYTES, done[SLOT],                   \
-                                  "attention_bwd(tcgen05)")))                                                       \
-      return rc;                                                                                                    \
-    if ((rc = check_launch_registers(attn_bwd_tc05_kernel<T, MODE, RAGGED>, FB_REGS, regs[SLOT], "attention_bwd(tcgen05)"))) return rc; \
-    launch_overlapped(attn_bwd_tc05_kernel<T, MODE, RAGGED>, grid, dim3(FB_THREADS), SMEM_BYTES, st, tq, tk, \
-                      tv, tdo, tdq, p);                                                                             \
-  }
-  if (a.bias_mode == 0) FB_LAUNCH(0, 0)
-  else if (a.bias_mode == 1) FB_LAUNCH(1, 1)
-  else if (a.bias_mode == 2) FB_LAUNCH(2, 2)
-  else FB_LAUNCH(4, 3)
-#undef FB_LAUNCH
+  using Form = Bwd64<T, RAGGED>;
+  const auto kernel = Form::kernel(a.bias_mode);
+  if ((rc = ensure_dynamic_smem(kernel, SMEM_BYTES, Form::smem_done[a.bias_mode], "attention_bwd(tcgen05)"))) return rc;
+  launch_overlapped(kernel, grid, dim3(FB_THREADS), SMEM_BYTES, st, tq, tk, tv, tdo, tdq, p);
   return launched("attention_bwd(tcgen05)");
 }
 

@@ -8,6 +8,7 @@ thread_local char g_err[512] = {0};
 std::atomic<int64_t> g_launches{0};
 std::atomic<int> g_force_generic_gemm{0};
 std::atomic<int> g_force_fallback_attn{0};
+std::atomic<int> g_debug_registers{0};
 std::atomic<int> g_attn_debug{0};
 std::atomic<int> g_plain_launch{0};
 std::atomic<int> g_gemm_debug{0};
@@ -49,6 +50,7 @@ extern "C" void tfb_debug_set(int key, int value) {
   if (key == 2) g_attn_debug.store(value);
   if (key == 3) g_plain_launch.store(value);
   if (key == 4) g_gemm_debug.store(value);
+  if (key == 7) g_debug_registers.store(value < 0 ? 0 : value);
   if (key == 6) g_gemm_free_sms.store(value < 0 ? 0 : value);
 }
 

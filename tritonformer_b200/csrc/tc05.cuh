@@ -333,16 +333,22 @@ __device__ __forceinline__ bool elect_one() {
 template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
-// Host side of the same: a build of the kernel with another number of registers than the split was worked out for is not
-// launched.  Asked for once per kernel (`seen`).
+// Host side of the same: `fit` says whether the kernel may be launched with a split that needs `lowest` registers a thread of the
+// whole block and raises no group above `highest`.  The compiler chooses the number (the launch bounds fix it in an ordinary build; a debug
+// build or another toolkit may choose another).  Asked for once per kernel (`known`).
+extern std::atomic<int> g_debug_registers;  // test switch: the number that kernels are taken to have, 0 for their own
 template <typename F>
-inline int check_launch_registers(F func, int regs, std::atomic<int>& seen, const char* what) {
-  if (seen.load(std::memory_order_relaxed) == regs) return TFB_OK;
-  cudaFuncAttributes attr;
-  const cudaError_t e = cudaFuncGetAttributes(&attr, func);
-  if (e != cudaSuccess) return fail(TFB_ERR_LAUNCH, "%s: function attributes: %s", what, cudaGetErrorString(e));
-  if (attr.numRegs != regs) return fail(TFB_ERR_LAUNCH, "%s: built with %d registers a thread instead of %d", what, attr.numRegs, regs);
-  seen.store(regs, std::memory_order_relaxed);
+inline int registers_fit(F func, int lowest, int highest, std::atomic<int>& known, const char* what, bool& fit) {
+  int n = known.load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaFuncAttributes attr;
+    const cudaError_t e = cudaFuncGetAttributes(&attr, func);
+    if (e != cudaSuccess) return fail(TFB_ERR_LAUNCH, "%s: function attributes: %s", what, cudaGetErrorString(e));
+    n = (attr.numRegs + 7) / 8 * 8;  // in the units that a warp gets them in
+    known.store(n, std::memory_order_relaxed);
+  }
+  if (const int pretended = g_debug_registers.load(std::memory_order_relaxed)) n = pretended;
+  fit = n >= lowest && n <= highest;
   return TFB_OK;
 }
 
