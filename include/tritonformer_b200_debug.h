@@ -22,8 +22,12 @@ extern "C" {
  *   key 6: how many SMs the persistent GEMM grids leave free (for a collective that runs beside
  *          them on another stream); 0 by default.
  *   key 7: the registers a thread that the attention backward's kernels are taken to have been built with; 0: what they
- *          have.  Where the number does not cover a kernel's split of its registers, the mma.sync kernels take the call.  */
+ *          have.  Where the number does not cover a kernel's split of its registers, the mma.sync kernels take the call.
+ * Accepted and without effect, for hosts that still set them: key 5, bits 0, 1, 6 and 7 of key 2, bit 6 of key 4 (they belonged to
+ * the cycle counters and to timing experiments of earlier kernels).                                  */
 void tfb_debug_set(int key, int value);
+/* The kernels count no cycles any more.  Sets out16 to zeros and returns the error code of what is not supported.  */
+int tfb_debug_counters(unsigned long long* out16);
 /* What the one-wave GEMM kernel does with an M x N x K product (b_mn: B is contiguous along N) under the switches in force:
  * 0 if the product goes to the persistent kernels, else 1 + tile width / 64 * 2 + (on CTA pairs ? 1 : 0) + 16 * the number
  * of workers that share a tile's contraction.                                              */

@@ -67,3 +67,9 @@ def test_argument_checks_without_device():
     rc = L.lib.tfb_embedding_bwd(None, None, one, None, None, 0, 2, 8, 64, 100, 0, 0, None)
     assert rc == -1 and b"scratch" in L.lib.tfb_last_error()
     assert L.lib.tfb_embedding_bwd(None, None, None, None, None, 0, 2, 8, 64, 100, 0, 0, None) == 0  # both tables frozen
+
+
+def test_the_cycle_counters_answer_that_there_are_none():
+    out = (ctypes.c_uint64 * 16)(*([7] * 16))
+    assert L.lib.tfb_debug_counters(out) == -2 and list(out) == [0] * 16 and b"cycle counters" in L.lib.tfb_last_error()
+    assert L.lib.tfb_debug_counters(None) == -2

@@ -44,6 +44,12 @@ extern "C" int tfb_debug_wait_probe(unsigned long long limit_ns, int* waited_ok,
   return launch_wait_probe(limit_ns, waited_ok, (cudaStream_t)stream);
 }
 
+extern "C" int tfb_debug_counters(unsigned long long* out16) {
+  if (out16)
+    for (int i = 0; i < 16; ++i) out16[i] = 0;
+  return fail(TFB_ERR_UNSUPPORTED, "the kernels have no cycle counters");
+}
+
 extern "C" void tfb_debug_set(int key, int value) {
   if (key == 0) g_force_generic_gemm.store(value);
   if (key == 1) g_force_fallback_attn.store(value);
