@@ -32,6 +32,9 @@ int tfb_debug_counters(unsigned long long* out16);
  * 0 if the product goes to the persistent kernels, else 1 + tile width / 64 * 2 + (on CTA pairs ? 1 : 0) + 16 * the number
  * of workers that share a tile's contraction.                                              */
 int tfb_debug_gemm_plan(long long M, long long N, long long K, int b_mn);
+/* The width of the tiles that the persistent CTA-pair kernel gives such a product, 0 if it does not get it (a_mn: A is contiguous
+ * along M; b_rows_64: the rows of B begin on 64-byte boundaries).                                              */
+int tfb_debug_gemm_pair_width(long long M, long long N, long long K, int a_mn, int b_mn, int b_rows_64);
 /* Launches a one-warp kernel that takes tensor memory, waits `limit_ns` nanoseconds on an mbarrier
  * that nothing arrives at, gives up, records 0x7e00 in the device status word, frees its tensor memory
  * and returns: the expiry path of the library's bounded waits, without a fault, a trap or an unbounded

@@ -144,3 +144,31 @@ def test_narrow_tiles_of_the_pair_kernel(m, n, k, dtype, layout):
     wide, narrow = (-(-(-(-m // 256) * -(-n // bn)) // pairs) for bn in (256, 192))
     assert wide == narrow == 2 and _lib.lib.tfb_debug_gemm_plan(m, n, k, int(layout[1] == "n")) == 0
     _check_all_epilogues(m, n, k, layout, dtype)
+
+
+@pytest.mark.parametrize("layout", ["kn", "kk", "mk"])
+@pytest.mark.parametrize("m,n,k,dtype", [(3328, 1536, 136, torch.float16), (3304, 1440, 1000, torch.bfloat16), (3304, 1376, 200, torch.float16)])
+def test_every_narrow_form_of_the_pair_kernel(m, n, k, dtype, layout):
+    """256 x 192 tiles, whole and with one or two of the last tile's three 64-column steps outside the output."""
+    from tritonformer_b200 import _lib
+    assert _lib.lib.tfb_debug_gemm_pair_width(m, n, k, int(layout[0] == "m"), int(layout[1] == "n"), 1) == 192
+    _check_all_epilogues(m, n, k, layout, dtype)
+
+
+def test_where_the_pair_kernel_takes_narrow_tiles():
+    """Not where both operands are contiguous along the output, nor where rows of B along N begin off 64-byte boundaries."""
+    from tritonformer_b200 import _lib
+    for k in (64, 1000, 8192):
+        for a_mn, b_mn, rows_64, want in ((0, 0, 0, 192), (1, 0, 0, 192), (0, 1, 1, 192), (0, 1, 0, 256), (1, 1, 1, 256), (1, 1, 0, 256)):
+            assert _lib.lib.tfb_debug_gemm_pair_width(3328, 1528, k, a_mn, b_mn, rows_64) == want
+            assert _lib.lib.tfb_debug_gemm_pair_width(4096, 4608, k, a_mn, b_mn, rows_64) == 256  # four waves of wide tiles, six of narrow ones
+    assert _lib.lib.tfb_debug_gemm_pair_width(512, 512, 512, 0, 0, 1) == 0  # the one-wave kernel's
+
+
+@pytest.mark.parametrize("n", [1464, 1528])
+def test_rows_of_b_off_64_byte_boundaries(n):
+    """A little more than a wave of 256 x 256 tiles whose B, contiguous along N, keeps the wide tiles."""
+    from tritonformer_b200 import _lib
+    assert _lib.lib.tfb_debug_gemm_pair_width(3320, n, 200, 0, 1, 0) == 256
+    for layout in ("kn", "mn"):
+        _check_all_epilogues(3320, n, 200, layout)

@@ -28,6 +28,7 @@ _SIGNATURES = {
     "tfb_debug_set": (None, [_i32, _i32]),
     "tfb_debug_counters": (_i32, [_c.POINTER(_c.c_uint64)]),
     "tfb_debug_gemm_plan": (_i32, [_c.c_longlong] * 3 + [_i32]),
+    "tfb_debug_gemm_pair_width": (_i32, [_c.c_longlong] * 3 + [_i32] * 3),
     "tfb_debug_wait_probe": (_i32, [_c.c_uint64, _vp, _vp]),
     "tfb_layernorm_fwd": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _f32, _i32, _vp]),
     "tfb_layernorm_bwd_partials": (_i64, [_i64, _i64]),

@@ -314,7 +314,8 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
 template <typename T, int BN>
 static int dispatch_pair(bool a_mn, bool b_mn, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
                          const CUtensorMap& tmX, const PairParams& p, int grid, cudaStream_t st) {
-  if (a_mn && b_mn) return launch_pair<T, BN, true, true>(tmA, tmB, tmC, tmX, p, grid, st);
+  if constexpr (BN == 256)  // (see gemm_pair_width)
+    if (a_mn && b_mn) return launch_pair<T, BN, true, true>(tmA, tmB, tmC, tmX, p, grid, st);
   if (a_mn) return launch_pair<T, BN, true, false>(tmA, tmB, tmC, tmX, p, grid, st);
   if (b_mn) return launch_pair<T, BN, false, true>(tmA, tmB, tmC, tmX, p, grid, st);
   return launch_pair<T, BN, false, false>(tmA, tmB, tmC, tmX, p, grid, st);
@@ -324,12 +325,16 @@ static int dispatch_pair(bool a_mn, bool b_mn, const CUtensorMap& tmA, const CUt
 int64_t gemm_pair_tiles(int64_t M, int64_t N) { return ceil_div(M, 2 * GP_M) * ceil_div(N, 256); }
 
 // Tile width.  A k-block of a 256 x 256 tile takes 528 cycles of its pair and one of a 256 x 192 tile 462 (what an SM takes in
-// from the L2, 32 and 28 KB at 62 bytes a cycle), so the narrow tile, which moves an eighth more operand bytes for the
+// from the L2, 32 and 28 KB at 62 bytes a cycle), so the narrow tile, which moves a sixth more operand bytes for the
 // same product, is for outputs whose last wave of wide tiles is mostly empty: as many waves of narrow ones.  M 4096 N 1536, two
-// waves of either: K 4608 (B contiguous along K) 49.2 us wide, 45.4 narrow, K 6144 65.6 and 62.1; B contiguous along N:
-// K 1536 20.8 and 19.8, K 6144 65.2 and 64.6.  M 2112 N 3072 K 1024: 15.9 and 15.6.  (Without the time stamps that the kernel
-// carried then: narrow 44.3, 60.8, 19.1, 63.2 and 14.9.)
-int gemm_pair_width(int64_t M, int64_t N, int sms) {
+// waves of either, wide and narrow: B contiguous along K: K 4608 49.0 and 42.7 us, K 6144 64.4 and 59.3; along N: K 1536 21.6 and 19.7,
+// K 6144 66.9 and 61.6; M 2112 N 3072 K 1024 16.4 and 15.3 (35 such products with B along K: 1.02 to 1.17 times as fast).
+// B contiguous along N comes in rows of 64 bytes, and rows that do not begin on multiples of 64 touch a half more of the L2's
+// sectors instead of a quarter: M 3320 N 1464 K 1840 24.6 and 27.5, M 2960 N 2296 K 1808 26.6 and 28.8, M 3328 N 1488 K 1184 16.3 and
+// 15.9.  With A contiguous along M as well the narrow tile wins nothing even on aligned rows: M 1448 N 6624 K 952 21.0 and 21.5, M 968
+// N 6464 K 5576 66.5 and 66.9, M 1552 N 5696 K 2544 41.4 and 41.2.
+int gemm_pair_width(int64_t M, int64_t N, bool a_mn, bool b_mn, bool b_rows_64, int sms) {
+  if (b_mn && (a_mn || !b_rows_64)) return 256;
   const int64_t pairs = sms / 2, tm = ceil_div(M, 2 * GP_M);
   const int64_t wide = ceil_div(tm * ceil_div(N, 256), pairs) * 528, narrow = ceil_div(tm * ceil_div(N, 192), pairs) * 462;
   return narrow * 100 < wide * 95 ? 192 : 256;
@@ -339,7 +344,7 @@ int gemm_pair_tc05(const void* a, const void* b, void* c, const void* bias, cons
                    const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
                    int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, int sms, cudaStream_t st) {
   const bool a_mn = (a_sk != 1), b_mn = (b_sk != 1);
-  const int width = gemm_pair_width(M, N, sms);
+  const int width = gemm_pair_width(M, N, a_mn, b_mn, reinterpret_cast<uintptr_t>(b) % 64 == 0 && b_sk % 32 == 0, sms);
   CUtensorMap tmA, tmB, tmC, tmX;
   int rc;
   const bool direct = gemm_needs_direct(c, ldc, bias, addend, ld_addend, mask, ld_mask);

@@ -23,6 +23,7 @@ struct TilePlan {
 };
 TilePlan gemm_tile_plan(int64_t M, int64_t N, int64_t K, bool b_mn, int sms);
 TilePlan gemm_plan(int64_t M, int64_t N, int64_t K, bool b_mn);  // with the switches in force
+int gemm_pair_plan(int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn, bool b_rows_64);  // the same for the pair kernel's tile width
 
 constexpr int kFlagBytes = 8192;  // head of the workspace: arrival counters, zero between kernels
 

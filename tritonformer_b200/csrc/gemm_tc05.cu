@@ -30,6 +30,7 @@ namespace tfb {
 extern std::atomic<int> g_gemm_debug;
 extern std::atomic<int> g_gemm_free_sms;
 int64_t gemm_pair_tiles(int64_t M, int64_t N);
+int gemm_pair_width(int64_t M, int64_t N, bool a_mn, bool b_mn, bool b_rows_64, int sms);
 bool gemm_needs_direct(const void* c, int64_t ldc, const void* bias, const void* addend, int64_t ld_addend, const void* mask,
                        int64_t ld_mask);
 int gemm_tile_tc05(const TilePlan& plan, const void* a, const void* b, void* c, const void* bias, const void* addend,
@@ -404,6 +405,17 @@ TilePlan gemm_plan(int64_t M, int64_t N, int64_t K, bool b_mn) {
   return gemm_tile_plan(M, N, K, b_mn, gemm_sms());
 }
 
+// Outputs with a 256 x 256 tile for every pair of SMs run on CTA pairs (a third less operand traffic per flop).
+static bool takes_pairs(int64_t M, int64_t N, int sms) {
+  return !(g_gemm_debug.load() & 32) && M >= 256 && N >= 256 && gemm_pair_tiles(M, N) >= sms / 2;
+}
+
+int gemm_pair_plan(int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn, bool b_rows_64) {
+  const int sms = gemm_sms();
+  if (gemm_plan(M, N, K, b_mn).bn || !takes_pairs(M, N, sms)) return 0;
+  return gemm_pair_width(M, N, a_mn, b_mn, b_rows_64, sms);
+}
+
 int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const void* addend, int64_t ld_addend,
               const void* mask, int64_t ld_mask, int64_t M, int64_t N, int64_t K, int64_t a_sm, int64_t a_sk,
               int64_t b_sk, int64_t b_sn, int64_t ldc, int relu, int dtype, void* workspace,
@@ -419,8 +431,7 @@ int gemm_tc05(const void* a, const void* b, void* c, const void* bias, const voi
   if (const TilePlan plan = gemm_plan(M, N, K, b_mn); plan.bn)
     return gemm_tile_tc05(plan, a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk, b_sn, ldc, relu,
                           dtype, st);
-  // Outputs with a 256 x 256 tile for every pair of SMs run on CTA pairs (a third less operand traffic per flop).
-  if (!(dbg & 32) && M >= 256 && N >= 256 && gemm_pair_tiles(M, N) >= sms / 2)
+  if (takes_pairs(M, N, sms))
     return gemm_pair_tc05(a, b, c, bias, addend, ld_addend, mask, ld_mask, M, N, K, a_sm, a_sk, b_sk, b_sn, ldc, relu, dtype,
                           sms, st);
   // Tile width: fewest "waves x tile cost" over the SMs; the wide tile moves fewer operand bytes per

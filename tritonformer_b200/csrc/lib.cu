@@ -64,6 +64,10 @@ extern "C" int tfb_debug_gemm_plan(long long M, long long N, long long K, int b_
   return gemm_plan(M, N, K, b_mn != 0).code();
 }
 
+extern "C" int tfb_debug_gemm_pair_width(long long M, long long N, long long K, int a_mn, int b_mn, int b_rows_64) {
+  return gemm_pair_plan(M, N, K, a_mn != 0, b_mn != 0, b_rows_64 != 0);
+}
+
 extern "C" int64_t tfb_gemm_workspace_bytes(void) { return gemm_tc05_workspace_bytes(); }
 
 extern "C" int tfb_gemm_fused(const void* a, const void* b, void* c, const void* bias, const void* addend,
