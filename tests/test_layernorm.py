@@ -85,3 +85,33 @@ def test_ln_backward_adds_parameter_gradients_into_given_buffers():
     # one fp32 add of the fp32 column sum and the old value, one rounding
     assert_close(buf_a, old_a.float() + da.float(), 2e-2, "dalpha", rtol=2e-3)
     assert_close(buf_b, old_b.float() + db.float(), 2e-2, "dbeta", rtol=2e-3)
+
+
+@pytest.mark.parametrize("d", [8, 248, 256, 264, 520, 776, 1032, 1280, 1288, 1536, 1544, 1792, 1800, 2040, 2048])
+@pytest.mark.parametrize("rows", [1, 17, 4737])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_backward_of_every_group_of_warps(d, rows, dtype):
+    """One to eight warps share a row, the last one whole or partly idle; with and without the residual gradient.  Against 64
+    bits: one rounding of each result, and fp32 sums of d (a row) or `rows` (a column) products, each cut by half a unit."""
+    from tritonformer_b200.layernorm import layernorm_backward, layernorm_forward
+    gen = torch.Generator(device="cuda").manual_seed(d + rows)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    x, dy, res, alpha = (r(rows, d) + 0.5).to(dtype), r(rows, d).to(dtype), r(rows, d).to(dtype), (1.0 + 0.1 * r(d)).to(dtype)
+    _, stats = layernorm_forward(x, alpha, torch.zeros_like(alpha), 1e-5)
+    xd, gd, ad = x.double(), dy.double(), alpha.double()
+    rstd = (xd.var(1, unbiased=False, keepdim=True) + 1e-5).rsqrt()
+    mean = xd.mean(1, keepdim=True)
+    h = (xd - mean) * rstd
+    g = gd * ad
+    plain = rstd * (g - h * (g * h).mean(1, keepdim=True) - g.mean(1, keepdim=True))
+    eps, unit = (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8), 2.0 ** -24
+    small = 2.0 ** -25  # half of fp16's smallest step
+    # what roundings act on: h is x * rstd - mean * rstd; a row's g, h g and their means; a column's products
+    hs = h.abs() + (xd.abs() + mean.abs()) * rstd
+    in_row = (rstd * (g.abs() + hs * (g.abs() * hs).mean(1, keepdim=True) + g.abs().mean(1, keepdim=True))).amax(1, keepdim=True)
+    for dres, want in ((None, plain), (res, plain + res.double())):
+        dx, da, db = layernorm_backward(dy, x, alpha, stats, dres)
+        err = (dx.double() - want).abs()
+        assert (err <= 1.01 * eps * want.abs() + (d ** 0.5 + 16) * unit * (in_row + want.abs()) + small).all()
+        for got, ref, size in ((da, (gd * h).sum(0), (gd.abs() * hs).sum(0)), (db, gd.sum(0), gd.abs().sum(0))):
+            assert ((got.double() - ref).abs() <= 1.01 * eps * ref.abs() + (16 + rows ** 0.5) * unit * size + small).all()
