@@ -13,10 +13,10 @@
 //     distributed shared memory: each sums and finishes its share of the tile's columns, in rank order (the sum does not
 //     depend on timing), a row per thread (through staging in the ring, so that a warp's stores are consecutive, was slower:
 //     M 2048 N 768 K 3072 13.7 against 12.9 us).  Through a workspace in global memory with arrival counters the same exchange took 4-5 us;
-//   - short rolled code everywhere (see gemm_epi.cuh).
-// Back to back, L2 hot, fp16, with the cluster's first barrier in its release form and the exchange of a split eight columns and one
-// latency at a time, and now: M 2048 N 768 K 768 6.8 and 6.2 us (with addend 7.4, 6.9), M 2048 N 768 K 3072 with addend 17.1 and 14.1, without
-// 13.0 and 12.9, M 2048 N 2304 K 768 9.6 and 9.0, M 768 N 768 K 2048 8.7 and 8.0, M 64 N 768 K 3072 (cold) 6.5 and 6.0.
+//   - little code: the roles' loops are rolled, and a tile's last steps run once per CTA (see gemm_epi.cuh).
+// Back to back, L2 hot, fp16, with the cluster's first barrier in its release form, one thread that sets everything up, no early
+// addend and the rolled epilogue, and now: M 2048 N 768 K 768 6.9 and 6.0 us (with addend 7.5, 6.8), M 2048 N 768 K 3072 13.6 and 12.9 (with
+// addend 17.2, 14.0), M 2048 N 2304 K 768 9.6 and 8.2, M 768 N 768 K 2048 8.8 and 8.1, M 64 N 768 K 3072 with addend 6.7 and 5.8.
 // Warps: 0 TMA producer, 1 MMA issuer (of the pair's first CTA), then the epilogue.
 #include "gemm_epi.cuh"
 #include <string.h>
@@ -104,9 +104,19 @@ __device__ __forceinline__ void gt_commit_pair(uint64_t* bar, uint16_t ctas) {
                : "memory");
 }
 
-// Eight columns of one row straight to global memory (vectors where the pitches allow them).
+// Eight columns of one row straight to global memory (vectors where the pitches allow them).  Their addend and mask vectors are
+// requested ahead (`Extra`).
+struct Extra {
+  uint4 add, mask;
+};
 template <typename T>
-__device__ __forceinline__ void finish_row8(const TileParams& p, float (&f)[8], int row, int col) {
+__device__ __forceinline__ void request_extra(const TileParams& p, Extra& x, int row, int col) {
+  if (p.direct || row >= p.M || col + 8 > p.N) return;
+  if (p.addend) x.add = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.addend) + (int64_t)row * p.ld_addend + col);
+  if (p.mask) x.mask = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.mask) + (int64_t)row * p.ld_mask + col);
+}
+template <typename T>
+__device__ __forceinline__ void finish_row8(const TileParams& p, float (&f)[8], const Extra& x, int row, int col) {
   if (row >= p.M || col >= p.N) return;
   const T *bias = reinterpret_cast<const T*>(p.bias), *addend = reinterpret_cast<const T*>(p.addend),
           *mask = reinterpret_cast<const T*>(p.mask);
@@ -123,12 +133,12 @@ __device__ __forceinline__ void finish_row8(const TileParams& p, float (&f)[8], 
       for (int j = 0; j < 8; ++j) f[j] = fmaxf(f[j], 0.f);
     }
     if (addend) {
-      unpack8<T>(*reinterpret_cast<const uint4*>(addend + (int64_t)row * p.ld_addend + col), t);
+      unpack8<T>(x.add, t);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] += t[j];
     }
     if (mask) {
-      unpack8<T>(*reinterpret_cast<const uint4*>(mask + (int64_t)row * p.ld_mask + col), t);
+      unpack8<T>(x.mask, t);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] = t[j] > 0.f ? f[j] : 0.f;
     }
@@ -145,69 +155,6 @@ __device__ __forceinline__ void finish_row8(const TileParams& p, float (&f)[8], 
     if (mask && !(Num<T>::to_f(mask[(int64_t)row * p.ld_mask + col + j]) > 0.f)) v = 0.f;
     c[j] = Num<T>::from_f(v);
   }
-}
-
-// What a split's worker finishes of one row at a time: sixteen columns.  The addend and mask vectors are requested a chunk
-// ahead (`Extra`), where the pitches allow vectors and all sixteen columns exist.
-struct Extra {
-  uint4 add[2], mask[2];
-};
-template <typename T>
-__device__ __forceinline__ bool row16_vectors(const TileParams& p, int row, int col) {
-  return !p.direct && row < p.M && col + 16 <= p.N;
-}
-template <typename T>
-__device__ __forceinline__ void request_extra(const TileParams& p, Extra& x, int row, int col) {
-  if (!row16_vectors<T>(p, row, col)) return;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    if (p.addend) x.add[h] = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.addend) + (int64_t)row * p.ld_addend + col + 8 * h);
-    if (p.mask) x.mask[h] = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.mask) + (int64_t)row * p.ld_mask + col + 8 * h);
-  }
-}
-template <typename T>
-__device__ __forceinline__ void finish_row16(const TileParams& p, float (&f)[16], const Extra& x, int row, int col) {
-  if (!row16_vectors<T>(p, row, col)) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float g[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) g[j] = f[8 * h + j];
-      finish_row8<T>(p, g, row, col + 8 * h);
-    }
-    return;
-  }
-  const T* bias = reinterpret_cast<const T*>(p.bias);
-  uint4* c = reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.C) + (int64_t)row * p.ldc + col);
-  uint4 out[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    float g[8], t[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) g[j] = f[8 * h + j];
-    if (bias) {
-      unpack8<T>(__ldg(reinterpret_cast<const uint4*>(bias + col) + h), t);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) g[j] += t[j];
-    }
-    if (p.relu) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) g[j] = fmaxf(g[j], 0.f);
-    }
-    if (p.addend) {
-      unpack8<T>(x.add[h], t);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) g[j] += t[j];
-    }
-    if (p.mask) {
-      unpack8<T>(x.mask[h], t);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) g[j] = t[j] > 0.f ? g[j] : 0.f;
-    }
-    out[h] = pack8<T>(g);
-  }
-  c[0] = out[0];
-  c[1] = out[1];
 }
 
 template <typename T, int BN, bool PAIR, bool A_MN, bool B_MN>
@@ -391,35 +338,44 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
       // Column slice r of the tile goes to worker r (the CTA of the same side): [source][group of 4 columns][row], so that the
       // 32 lanes of a warp write 512 contiguous bytes.  Sources are numbered without the receiver itself.  The columns of a
       // slice are shared by the HALVES warps of a lane quarter.
+      // Eight columns at a time, with the next ones' addend on its way: what this costs is latencies and the fetching of its
+      // instructions.  (32 columns at a time in the exchange and 16 behind it, in code of three times the size, was as fast or up to 5 % faster
+      // in a loop over one product, but not where products follow each other: a linear layer's three of 1344 x 320 x 960 20.0 us
+      // against 19.7, of 2048 x 1792 x 320 26.2 against 25.4, with a cold L2 27.0 against 25.2 and 33.5 against 31.0; the layer of
+      // 8512 x 256 x 2624 85.5 against 77.6.)
       const int slice = BN / p.split, lo = half * (slice / HALVES), hi = lo + slice / HALVES;
       const int trow = q * 32 + lane, row = row0 + lane, first = n0 + part * slice;
-      if (hi - lo < 16) {
-        // Eight columns a warp (64 columns cut eight ways).  As the rest of the wide form's loops, with the other instructions of
-        // these in between, M 128 N 704 K 832 took 4.95 us and M 448 N 64 K 1024 4.68; so 4.44 and 4.12.
-        bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
-        tc_fence_after();
-        if (ok) {
+      Extra ex;
+      if (!dead) request_extra<T>(p, ex, row, first + lo);
+      bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
+      tc_fence_after();
+      if (ok) {
 #pragma unroll 1
-          for (int i = 1; i < p.split; ++i) {
-            const int to = (part + i) % p.split;
-            const int slot = part < to ? part : part - 1;
-            const uint32_t dst = gt_map(smem_u32(recv + (slot * (slice / 4) + lo / 4) * GT_M + trow), (uint32_t)(to * WIDTH + side));
+        for (int i = 1; i < p.split; ++i) {
+          const int to = (part + i) % p.split;
+          const int slot = part < to ? part : part - 1;
+          const uint32_t dst = gt_map(smem_u32(recv + slot * (slice / 4) * GT_M + trow), (uint32_t)(to * WIDTH + side));
+#pragma unroll 1
+          for (int c = lo; c < hi; c += 8) {
             uint32_t v[8];
-            tmem_ld8(taddr + to * slice + lo, v);
+            tmem_ld8(taddr + to * slice + c, v);
             tc_wait_ld();
-            gt_store_remote(dst, v);
-            gt_store_remote(dst + GT_M * 16, v + 4);
+            gt_store_remote(dst + (c / 4) * GT_M * 16, v);
+            gt_store_remote(dst + (c / 4 + 1) * GT_M * 16, v + 4);
           }
         }
-        __syncwarp();
-        gt_cluster_sync();
-        if (ok && !dead && *abort_flag == 0) {
+      }
+      __syncwarp();
+      gt_cluster_sync();
+      if (ok && !dead && *abort_flag == 0) {
+#pragma unroll 1
+        for (int c = lo; c < hi; c += 8) {
           uint32_t own[8];
-          tmem_ld8(taddr + part * slice + lo, own);
-          tc_wait_ld();
+          tmem_ld8(taddr + part * slice + c, own);
           float f[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) f[j] = 0.f;
+          tc_wait_ld();
 #pragma unroll 1
           for (int r = 0; r < p.split; ++r) {  // in rank order
             float4 a, b;
@@ -427,100 +383,15 @@ __global__ void __launch_bounds__(TileCfg<BN, PAIR, B_MN>::THREADS, 1)
               a = make_float4(__uint_as_float(own[0]), __uint_as_float(own[1]), __uint_as_float(own[2]), __uint_as_float(own[3]));
               b = make_float4(__uint_as_float(own[4]), __uint_as_float(own[5]), __uint_as_float(own[6]), __uint_as_float(own[7]));
             } else {
-              const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + lo / 4) * GT_M + trow;
+              const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + c / 4) * GT_M + trow;
               a = src[0];
               b = src[GT_M];
             }
             f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
             f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
           }
-          finish_row8<T>(p, f, row, first + lo);
-        }
-      } else {
-        // What this costs is latencies, so columns move 16 at a time (32 in the exchange) with the next chunk's addend on its way.
-        Extra ex;
-        if (!dead) request_extra<T>(p, ex, row, first + lo);
-        bool ok = mbar_wait(acc_full, 0, 0x400, abort_flag);
-        tc_fence_after();
-        if (ok) {
-#pragma unroll 1
-          for (int i = 1; i < p.split; ++i) {
-            const int to = (part + i) % p.split;
-            const int slot = part < to ? part : part - 1;
-            const uint32_t dst = gt_map(smem_u32(recv + slot * (slice / 4) * GT_M + trow), (uint32_t)(to * WIDTH + side));
-            int c = lo;
-#pragma unroll 1
-            for (; c + 32 <= hi; c += 32) {
-              uint32_t v[32];
-              tmem_ld32(taddr + to * slice + c, v);
-              tc_wait_ld();
-#pragma unroll
-              for (int e = 0; e < 8; ++e) gt_store_remote(dst + (c / 4 + e) * GT_M * 16, v + 4 * e);
-            }
-#pragma unroll 1
-            for (; c < hi; c += 8) {
-              uint32_t v[8];
-              tmem_ld8(taddr + to * slice + c, v);
-              tc_wait_ld();
-              gt_store_remote(dst + (c / 4) * GT_M * 16, v);
-              gt_store_remote(dst + (c / 4 + 1) * GT_M * 16, v + 4);
-            }
-          }
-        }
-        __syncwarp();
-        gt_cluster_sync();
-        if (ok && !dead && *abort_flag == 0) {
-          int c = lo;
-#pragma unroll 1
-          for (; c + 16 <= hi; c += 16) {
-            uint32_t own[16];
-            tmem_ld16(taddr + part * slice + c, own);
-            const Extra now = ex;
-            if (c + 32 <= hi) request_extra<T>(p, ex, row, first + c + 16);
-            float f[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) f[j] = 0.f;
-            tc_wait_ld();
-#pragma unroll 1
-            for (int r = 0; r < p.split; ++r) {  // in rank order
-              if (r == part) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) f[j] += __uint_as_float(own[j]);
-              } else {
-                const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + c / 4) * GT_M + trow;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float4 v = src[e * GT_M];
-                  f[4 * e] += v.x; f[4 * e + 1] += v.y; f[4 * e + 2] += v.z; f[4 * e + 3] += v.w;
-                }
-              }
-            }
-            finish_row16<T>(p, f, now, row, first + c);
-          }
-#pragma unroll 1
-          for (; c < hi; c += 8) {
-            uint32_t own[8];
-            tmem_ld8(taddr + part * slice + c, own);
-            tc_wait_ld();
-            float f[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = 0.f;
-#pragma unroll 1
-            for (int r = 0; r < p.split; ++r) {
-              float4 a, b;
-              if (r == part) {
-                a = make_float4(__uint_as_float(own[0]), __uint_as_float(own[1]), __uint_as_float(own[2]), __uint_as_float(own[3]));
-                b = make_float4(__uint_as_float(own[4]), __uint_as_float(own[5]), __uint_as_float(own[6]), __uint_as_float(own[7]));
-              } else {
-                const float4* src = recv + ((r < part ? r : r - 1) * (slice / 4) + c / 4) * GT_M + trow;
-                a = src[0];
-                b = src[GT_M];
-              }
-              f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
-              f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
-            }
-            finish_row8<T>(p, f, row, first + c);
-          }
+          finish_row8<T>(p, f, ex, row, first + c);
+          if (c + 8 < hi) request_extra<T>(p, ex, row, first + c + 8);
         }
       }
     }
