@@ -247,3 +247,32 @@ def test_backward_of_a_build_with_other_registers(hd, registers, path, t, dtype)
     for got, ref in zip(grads, torch.autograd.grad(torch.softmax(s, -1) @ vd, (qd, kd, vd), dy.double())):
         err = (got.double() - ref).flatten(2).norm(dim=2) / ref.flatten(2).norm(dim=2)
         assert err.max().item() < 4 * (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_backward_of_two_copies_of_the_library_in_one_process(hd, tmp_path):
+    """What is done once per kernel (shared-memory limits, register counts) is done by each copy for its own kernels."""
+    import ctypes
+    import shutil
+    from tritonformer_b200 import _lib as L
+    from tritonformer_b200 import attention as A
+    q, k, v, dy = (x.detach() for x in _make((1, 2, 192, hd), torch.float16, True))
+    out, lse, _ = A.attention_forward(q, k, v, A._Bias())
+    n = L.lib.tfb_attention_bwd_scratch_bytes(1, 2, 192, hd)
+    scratch = torch.empty(n, dtype=torch.uint8, device="cuda")
+
+    def grads_of(lib):
+        grads = [torch.full_like(x, 7.0) for x in (q, k, v)]
+        rc = lib.tfb_attention_bwd(
+            *(x.data_ptr() for x in (q, k, v, out, dy, lse, *grads)), 1, 2, 192, hd, *(L.strides3(x) for x in (q, k, v, out, dy, *grads)),
+            None, 0, None, 0, 0, scratch.data_ptr(), n, L.dtype_code(q.dtype), L.stream_ptr(q.device), None)
+        torch.cuda.synchronize()
+        return rc, grads
+
+    rc, want = grads_of(L.lib)
+    assert rc == 0
+    path = shutil.copy(L.LIB_PATH, tmp_path / "copy.so")
+    copy = ctypes.CDLL(str(path))
+    copy.tfb_attention_bwd.argtypes, copy.tfb_attention_bwd.restype = L.lib.tfb_attention_bwd.argtypes, ctypes.c_int
+    rc, got = grads_of(copy)
+    assert rc == 0 and all(torch.equal(a, b) for a, b in zip(got, want))

@@ -501,6 +501,7 @@ static int encode_rows(CUtensorMap* m, const void* ptr, const AttnStrides& s, co
   return encode_tmap_sw128(m, ptr, dtype, 4, dims, str, box);
 }
 
+namespace {  // (not shared with another copy of the library in the process)
 template <typename T>
 struct Bwd128 {
   using Kernel = decltype(&attn_bwd128_tc05_kernel<T, 0>);
@@ -511,6 +512,7 @@ struct Bwd128 {
          : mode == 2 ? attn_bwd128_tc05_kernel<T, 2> : attn_bwd128_tc05_kernel<T, 4>;
   }
 };
+}  // namespace
 
 int attn_bwd128_fits(const AttnArgs& a, int dtype, bool& fit) {
   TFB_DISPATCH_16(dtype, T, {

@@ -650,6 +650,7 @@ bool attn_tc05_bwd_eligible(const AttnArgs& a, int hd) {  // as in the forward
 int attn_bwd128_tc05(const AttnArgs& a, int dtype, cudaStream_t st);
 int attn_bwd128_fits(const AttnArgs& a, int dtype, bool& fit);
 
+namespace {  // (not shared with another copy of the library in the process)
 template <typename T, bool RAGGED>
 struct Bwd64 {
   using Kernel = decltype(&attn_bwd_tc05_kernel<T, 0, RAGGED>);
@@ -663,6 +664,7 @@ struct Bwd64 {
     return registers_fit(kernel(a.bias_mode), FB_REGS, FB_REGS_COMPUTE, registers[a.bias_mode], "attention_bwd(tcgen05)", fit);
   }
 };
+}  // namespace
 
 // Whether the kernel that would take the call has the registers that its split counts on.  If not, the mma.sync kernels take it.
 int attn_tc05_bwd_fits(const AttnArgs& a, int hd, int dtype, bool& fit) {
