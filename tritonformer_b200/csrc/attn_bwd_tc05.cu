@@ -92,7 +92,6 @@ struct FbParams {
   int H, T, hd;   // hd: the real head_dim, 32 or 64
   int BH, group;  // batch*heads; how many of them are walked together (their tiles share the L2)
   float scale;
-  int bias_mode;
   const float* slopes;
   int debug;  // bit 5: per-slice item order (test switch)
 };
@@ -291,12 +290,12 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
         const uint64_t do_k = smem_desc_sw128(s0 + OFF_DO + st * TILE_BYTES, 16, 1024);
 #pragma unroll
         for (int s = 0; s < HD / 16; ++s) {
-          const uint32_t off = (s / 4) * 16384 + (s % 4) * 32;
+          const uint32_t off = s * 32;
           if (elect_one()) tc_mma_ss(tb + COL_S, desc_advance(dk_k, kv + off), desc_advance(q_k, off), idesc_s, s ? 1u : 0u);
         }
 #pragma unroll
         for (int s = 0; s < HD / 16; ++s) {
-          const uint32_t off = (s / 4) * 16384 + (s % 4) * 32;
+          const uint32_t off = s * 32;
           if (elect_one()) tc_mma_ss(tb + COL_DP, desc_advance(dv_k, kv + off), desc_advance(do_k, off), idesc_s, s ? 1u : 0u);
         }
         if (elect_one()) tc_commit(s_full);
@@ -539,7 +538,6 @@ __global__ void __launch_bounds__(FB_THREADS, 1) attn_bwd_tc05_kernel(const __gr
     // The rows go through swizzled shared-memory boxes and the TMA unit performs the
     // reduction (cp.reduce.async.bulk.tensor), which keeps the load/store path free for the compute warps.
     const int qd = warp & 3;
-    const int r = qd * 32 + lane;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(qd * 32) << 16);
     uint8_t* stage = smem + OFF_DQ + (warp - 4) * 4096;
     if (lane == 0) tma_prefetch_desc(&tmDQ);
@@ -691,7 +689,7 @@ static int bwd64_launch(const AttnArgs& a, int hd, int dtype, cudaStream_t st) {
   p.lse = a.lse; p.delta = a.delta; p.dk = a.dk; p.dv = a.dv;
   p.sdk_b = a.sdk.b; p.sdk_h = a.sdk.h; p.sdk_t = a.sdk.t;
   p.sdv_b = a.sdv.b; p.sdv_h = a.sdv.h; p.sdv_t = a.sdv.t;
-  p.H = a.H; p.T = a.T; p.hd = hd; p.scale = a.scale; p.bias_mode = a.bias_mode; p.slopes = a.slopes;
+  p.H = a.H; p.T = a.T; p.hd = hd; p.scale = a.scale; p.slopes = a.slopes;
   p.debug = g_attn_debug.load();
   p.status = dev_status_address();
   if (!p.status) return fail(TFB_ERR_LAUNCH, "attention_bwd(tcgen05): cannot find the status word");
