@@ -49,10 +49,11 @@ constexpr int FB_T = 128;           // tile edge (keys and queries)
 constexpr int FB_CWARPS = 16;        // compute warps: 4 TMEM lane quarters x 4 column quarters
 // Warpgroups: TMA, MMA and two idle warps; four dQ-drain warps; the compute warps.  The block is launched with 80 registers a
 // thread (six warps per scheduler); the first two groups hand some of theirs on to the compute warps.  (More than 88 for these
-// left the MMA warp spilling: 179 against 172 us.)  Backward with its two small passes, in microseconds: in 22 warps with the drain
-// warps last, with the warpgroups, and with the registers moved as well and the packed arithmetic on blocks that know whether
-// they meet the diagonal: B4 H16 T2048 fp16 189.6, 172.2, 171.9, exact slopes 195.9, 183.8, 171.6; B3 H11 T1472 bf16 67.0, 61.3, 62.6;
-// B3 H16 T704 bf16 with the rounded table 38.0, 33.8, 32.7; B2 H12 T1024 fp16 33.8, 30.7, 31.0.
+// left the MMA warp spilling: 179 against 172 us.  At 88 they still spill, 16 to 32 bytes a thread; how much depends on as little as the
+// layout of the parameters.)  Backward with its two small passes, in microseconds: in 22 warps with the drain
+// warps last, with the warpgroups, and now, with the registers moved as well and the packed arithmetic on blocks that know whether
+// they meet the diagonal: B4 H16 T2048 fp16 189.6, 172.2, 172.3, exact slopes 195.9, 183.8, 175.2; B3 H11 T1472 bf16 67.0, 61.3, 61.7;
+// B3 H16 T704 bf16 with the rounded table 38.0, 33.8, 32.0; B2 H12 T1024 fp16 33.8, 30.7, 30.8.
 constexpr int FB_FIRST_C = 8;       // first compute warp
 constexpr int FB_THREADS = 32 * (FB_FIRST_C + FB_CWARPS);
 constexpr int FB_REGS = 80, FB_REGS_ISSUE = 56, FB_REGS_DRAIN = 72, FB_REGS_COMPUTE = 88;

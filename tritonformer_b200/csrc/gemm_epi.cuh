@@ -1,13 +1,14 @@
 // Epilogue shared by the tcgen05 GEMM kernels: a warp turns its 32 rows x (64 STEPS) columns of the accumulator in tensor
 // memory into 16-bit output, 64 columns (one swizzled 32 x 64 box in shared memory, one TMA store) at a time.
 //
-// A tile's epilogue runs a few times per CTA, so what it costs is latencies and the fetching of its instructions: unrolled over 64 columns with every option inside the innermost loop it took 2.4-3.4 k cycles per 64 columns
-// whatever the options were (per-CTA time stamps, warm or cold); in rolled steps of 16 columns with each option behind one
-// uniform branch 1.7 k, four latencies of tensor memory among them; with all 64 columns read at once and each option a pass
-// over them behind its branch, less.  (Where different kernels follow each other with a cold L2, the longer code costs some of
-// that again: a linear layer's three products of 1280 x 128 x 896 19.5 us with the rolled form, 22.2 so, with a warm L2 16.6 and 16.7.)
-// Products of M 2048, fp16, L2 hot, rolled and now: N 3072 K 768 with mask 14.2 and 12.4 us, without
-// 12.4 and 11.8, N 2304 K 768 8.8 and 8.1, N 768 K 768 6.2 and 5.8; M 768 N 3072 K 2048 11.7 and 11.1; M 8192 N 1024 K 4096 55.8 and 54.
+// A tile's epilogue runs a few times per CTA, so what it costs is latencies and the fetching of its instructions: unrolled over 64
+// columns with every option inside the innermost loop it took 2.4-3.4 k cycles per 64 columns whatever the options were (per-CTA time
+// stamps, warm or cold); in rolled steps of 16 columns with each option behind one uniform branch 1.7 k, four latencies of tensor memory
+// among them; with all 64 columns read at once and each option a pass over them behind its branch, less.  (Where different
+// kernels follow each other with a cold L2, the longer code costs some of that again: a linear layer's three products of
+// 1280 x 128 x 896 19.5 us with the rolled form, 22.2 so, with a warm L2 16.6 and 16.7.)  Products of M 2048, fp16, L2 hot, rolled and now:
+// N 3072 K 768 with mask 14.2 and 12.4 us, without 12.4 and 11.8, N 2304 K 768 8.8 and 8.1, N 768 K 768 6.2 and 5.8; M 768 N 3072 K 2048
+// 11.7 and 11.1; M 8192 N 1024 K 4096 55.8 and 54.
 #pragma once
 #include "gemm_sched.cuh"
 

@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(MAXT) ln_bwd_kernel(
 // registers.  The two row sums are reduced by warp shuffles and exchanged between the G warps through shared memory behind
 // a named barrier (double-buffered).
 // What bounds it: the instructions a warp issues per row, one in 7 cycles at four warps per scheduler.  So the arithmetic is
-// packed (two columns an instruction), nothing is copied through shared memory, and six warps fit a scheduler.  With a
+// packed (two columns an instruction), nothing is copied through shared memory, and two CTAs, all that the grid has for an SM, give a
+// scheduler six warps (widths up to 1024 and of 1281-1536; five at 1025-1280, three and a half at 1537-1792, four above).  With a
 // cp.async ring per lane, G a power of two and four warps per scheduler: 31 instructions per element.  With the residual
 // gradient and the fold of the partials, cold L2, fp16: 8192 x 1024 22.8 -> 18.0 us, 4096 x 1536 24.1 -> 15.5, 2048 x 768
 // 10.2 -> 7.7, 512 x 256 8.0 -> 4.2, 4096 x 2048 25.9 -> 23.0, 32768 x 1024 58.3 -> 50.6 (5.3 TB/s).
