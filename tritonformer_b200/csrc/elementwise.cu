@@ -283,7 +283,8 @@ extern "C" int tfb_relu_bwd(const void* dy, const void* act, void* dz, int64_t n
 }
 
 extern "C" int64_t tfb_colsum_partials(int64_t rows, int64_t cols) {
-  // enough row slices to fill the machine given ceil(cols/256) column CTAs
+  // enough row slices to fill the machine given ceil(cols/256) column CTAs, four of them per SM (what grad_rows_shift_kernel makes of it is
+  // its 248 columns, and three per SM with a mask: its grid then runs a few CTAs, or a third of them, past a wave)
   const int64_t col_ctas = ceil_div(cols, 256);
   int64_t n = ceil_div(148 * 4, col_ctas);
   const int64_t max_n = ceil_div(rows, 8);

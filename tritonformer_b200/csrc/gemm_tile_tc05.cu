@@ -468,6 +468,7 @@ static int dispatch_tile(bool a_mn, bool b_mn, const CUtensorMap& tmA, const CUt
 // Cycles of the one-wave kernel for a plan: a fixed chain of latencies, the k-blocks of a CTA, the exchange of a split.  What
 // a k-block costs is mostly what an SM can take in from the L2, about 62 bytes a cycle (measured over tiles, splits and
 // contraction lengths: 24 KB 400-430 cycles, 32 KB 480-540, whatever the tensor core would need).
+// (The fixed part, the per-column part and the exchange were fitted to an epilogue and a set-up that were slower than the present ones.)
 static int64_t tile_cycles(int bn, bool pair, int split, bool b_mn, int64_t kblocks) {
   const int64_t bytes = 16384 + (pair ? (b_mn ? (bn / 2 + 63) / 64 * 8192 : bn / 2 * 128) : bn * 128);
   const int64_t mma = pair ? bn * 2 : bn * 2 + 60;
