@@ -424,10 +424,10 @@ def run_b200_arm(args):
         achieved = gflop / in_step_s / 1e12
         mhz = lambda c: c.get("sm_mhz") if c else None
         # one launch of the dominant kernel under ncu (profiles/ncu_gemm_tc05.md): the forward product of the first
-        # MLP linear, M8192 N4096 K1024 fp16.  DRAM read 25.29 MB = X (16.8 MB) + W (8.4 MB) once; 18.76 MB of the
+        # MLP linear, M8192 N4096 K1024 fp16.  DRAM read 25.28 MB = X (16.8 MB) + W (8.4 MB) once; 17.08 MB of the
         # 67.1 MB output had been written back when the kernel ended (the rest was still in the L2).
         traffic = {"launch": "gemm_pair_tc05_kernel, forward fc1 M8192 N4096 K1024 fp16 (profiles/ncu_gemm_tc05.md)",
-                   "dram_bytes_read": 25.29e6, "dram_bytes_written": 18.76e6,
+                   "dram_bytes_read": 25.28e6, "dram_bytes_written": 17.08e6,
                    "algorithmic_bytes_read": 2.0 * (8192 * 1024 + 1024 * 4096),
                    "algorithmic_bytes_written": 2.0 * 8192 * 4096}
         roof = {"bound": "tensor",
@@ -456,7 +456,7 @@ def run_b200_arm(args):
                      # DRAM bytes of one forward + one backward launch, from the ncu captures of the B2 H16 T2048
                      # hd64 case scaled by batch*heads (the traffic is q, k, v, dO read once: proportional);
                      # only for the configuration the captures cover
-                     "traffic": (2 * (25.23e6 + 50.92e6 + 1.83e6) * (B * cfg.num_attention_heads) / 64.0
+                     "traffic": (2 * (25.23e6 + 50.95e6 + 1.51e6) * (B * cfg.num_attention_heads) / 64.0
                                  if (cfg.head_dim == 64 and T == 2048) else None),
                      "traffic_detail": "profiles/ncu_attention_fwd.md, profiles/ncu_attention_bwd.md",
                      "calls": n_attn, "fwd_ms_per_step": fwd_t * 1e3, "bwd_ms_per_step": bwd_t * 1e3,
